@@ -18,8 +18,10 @@
 // w_in [E][2 * ff][width] (an expert's gate rows, then its up rows), w_out [E][width][ff]. An
 // expert without a gate (`single`: y = relu(W_up h)^2) has w_in [E][ff][width].
 //
-// The tile products run on the CUDA cores with fp32 FMA for float32 and on the warp-level
-// tensor cores (mma.sync m16n8k16, fp32 accumulators) for bfloat16.
+// The tile products run on the CUDA cores with fp32 FMA for float32. In bfloat16 they run on the
+// 5th-generation tensor cores in tiles of 128 pairs once an expert gets that many (moe_tc.cuh),
+// and on the warp-level ones (mma.sync m16n8k16, fp32 accumulators) in tiles of 32 below, and
+// where an operand breaks TMA's alignment rule.
 #include <limits.h>
 
 #include "common.cuh"
@@ -27,7 +29,7 @@
 namespace ayk {
 
 constexpr int MOE_TM = 32;   // pairs per tile: few rows, and float32
-constexpr int MOE_TM_WIDE = 128;  // pairs per tile of the tensor-core products of many rows
+constexpr int MOE_TM_WIDE = 128;  // pairs per tile of the tcgen05 products of many rows
 constexpr int MOE_TN = 64;   // output columns per tile
 constexpr int MOE_TK = 32;   // k per turn on the CUDA cores (the tensor-core tiles take 64)
 constexpr int MOE_MAX_EXPERTS = 1024;
@@ -197,10 +199,11 @@ __global__ void moe_route_scored_kernel(const float* __restrict__ logits, int ld
 }
 
 // One CTA. sorted: [max_tiles * tile_rows] pair indices or -1; tile_expert: [max_tiles], -1 for a
-// tile past the last.
+// tile past the last; tile_first (unless null): [max_tiles], the pairs before the tile's first.
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ chosen, int pairs, int E, int max_tiles, int tile_rows,
-                 int* __restrict__ sorted, int* __restrict__ tile_expert) {
+                 int* __restrict__ sorted, int* __restrict__ tile_expert,
+                 int* __restrict__ tile_first) {
   __shared__ int counts[MOE_MAX_EXPERTS];
   __shared__ int starts[MOE_MAX_EXPERTS];
   pdl_launch_dependents();
@@ -215,11 +218,15 @@ moe_align_kernel(const int* __restrict__ chosen, int pairs, int E, int max_tiles
   for (int i = tid; i < max_tiles * tile_rows; i += blockDim.x) sorted[i] = -1;
   __syncthreads();
   if (tid == 0) {
-    int tile = 0;
+    int tile = 0, before = 0;
     for (int e = 0; e < E; ++e) {
       starts[e] = tile * tile_rows;
       const int tiles = (counts[e] + tile_rows - 1) / tile_rows;
-      for (int t = 0; t < tiles && tile < max_tiles; ++t) tile_expert[tile++] = e;
+      for (int t = 0; t < tiles && tile < max_tiles; ++t) {
+        if (tile_first != nullptr) tile_first[tile] = before + t * tile_rows;
+        tile_expert[tile++] = e;
+      }
+      before += counts[e];
       counts[e] = 0;  // now the cursor of the expert's stretch
     }
     for (; tile < max_tiles; ++tile) tile_expert[tile] = -1;
@@ -247,10 +254,16 @@ __device__ __forceinline__ float expert_unit(float g, float u, float limit, floa
   return g / (1.f + expf(-alpha * g)) * (u + shift);
 }
 
-template <typename T, int PHASE, int TM> struct TileAcc;
+}  // namespace ayk
+
+#include "moe_tc.cuh"
+
+namespace ayk {
+
+template <typename T, int PHASE> struct TileAcc;
 
 // fp32: thread (ty, tx) of 16 x 16 owns rows 2 ty .. +1 and columns 4 tx .. +3
-template <int PHASE> struct TileAcc<float, PHASE, MOE_TM> {
+template <int PHASE> struct TileAcc<float, PHASE> {
   static constexpr int TK = MOE_TK;
   static constexpr int LDS = MOE_TK + 1;
   float acc[PHASE == 0 ? 2 : 1][2][4];
@@ -298,29 +311,22 @@ template <int PHASE> struct TileAcc<float, PHASE, MOE_TM> {
   }
 };
 
-// bfloat16: eight warps as (TM / 16 MT) x the rest; a warp holds MT x NT m16n8 accumulators
-// per matrix (tiles of 32 pairs: 2 x 4 warps of 16 x 16; of 128 pairs: 4 x 2 warps of
-// 32 x 32, four times the products per turn and a quarter of the weights' re-reads). Shared
-// rows are padded by 8 entries so that the eight rows of an ldmatrix tile fall into
-// different banks.
-template <int PHASE, int TM> struct TileAcc<__nv_bfloat16, PHASE, TM> {
+// bfloat16: eight warps as 2 x 4, each 16 x 16: NT m16n8 accumulators per matrix. Shared rows
+// are padded by 8 entries so that the eight rows of an ldmatrix tile fall into different banks.
+template <int PHASE> struct TileAcc<__nv_bfloat16, PHASE> {
   static constexpr int TK = 64;
   static constexpr int LDS = TK + 8;
-  static constexpr int MT = TM >= 128 ? 2 : 1;    // m16 tiles of a warp
-  static constexpr int WARPS_M = TM / (16 * MT);  // warps down the rows
-  static constexpr int WARPS_N = 8 / WARPS_M;
-  static constexpr int NT = MOE_TN / (8 * WARPS_N);  // n8 tiles of a warp (2 or 4)
+  static constexpr int WARPS_N = 8 / (MOE_TM / 16);
+  static constexpr int NT = MOE_TN / (8 * WARPS_N);  // n8 tiles of a warp
   static constexpr int W = PHASE == 0 ? 2 : 1;
-  float acc[W][MT][NT][4];
+  float acc[W][NT][4];
   __device__ __forceinline__ void zero() {
 #pragma unroll
     for (int w = 0; w < W; ++w)
 #pragma unroll
-      for (int m = 0; m < MT; ++m)
+      for (int n = 0; n < NT; ++n)
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[w][m][n][i] = 0.f;
+        for (int i = 0; i < 4; ++i) acc[w][n][i] = 0.f;
   }
   static __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4],
                                              uint32_t b0, uint32_t b1) {
@@ -340,7 +346,7 @@ template <int PHASE, int TM> struct TileAcc<__nv_bfloat16, PHASE, TM> {
   __device__ __forceinline__ void step(const __nv_bfloat16* As, const __nv_bfloat16* Bs,
                                        const __nv_bfloat16* Bs2, bool both) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = (warp / WARPS_N) * 16 * MT, n0 = (warp % WARPS_N) * 8 * NT;
+    const int m0 = (warp / WARPS_N) * 16, n0 = (warp % WARPS_N) * 8 * NT;
     // A: lanes 0-15 give rows 0-15 at k, lanes 16-31 the same rows at k + 8 (a0..a3);
     // B (kept [n][k]): lanes 0-7 rows n.. at k, 8-15 the same at k + 8 (b0, b1 of eight
     // columns), 16-31 likewise for the next eight
@@ -348,24 +354,17 @@ template <int PHASE, int TM> struct TileAcc<__nv_bfloat16, PHASE, TM> {
     const int b_offset = (n0 + (lane >> 4) * 8 + (lane & 7)) * LDS + ((lane >> 3) & 1) * 8;
 #pragma unroll
     for (int k0 = 0; k0 < TK; k0 += 16) {
-      uint32_t a[MT][4], b[4];
-#pragma unroll
-      for (int m = 0; m < MT; ++m) load_tiles(a[m], a_at + m * 16 * LDS + k0);
+      uint32_t a[4], b[4];
+      load_tiles(a, a_at + k0);
 #pragma unroll
       for (int n = 0; n < NT; n += 2) {
         load_tiles(b, Bs + b_offset + n * 8 * LDS + k0);
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          mma(acc[0][m][n], a[m], b[0], b[1]);
-          mma(acc[0][m][n + 1], a[m], b[2], b[3]);
-        }
+        mma(acc[0][n], a, b[0], b[1]);
+        mma(acc[0][n + 1], a, b[2], b[3]);
         if (PHASE == 0 && both) {
           load_tiles(b, Bs2 + b_offset + n * 8 * LDS + k0);
-#pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            mma(acc[W - 1][m][n], a[m], b[0], b[1]);
-            mma(acc[W - 1][m][n + 1], a[m], b[2], b[3]);
-          }
+          mma(acc[W - 1][n], a, b[0], b[1]);
+          mma(acc[W - 1][n + 1], a, b[2], b[3]);
         }
       }
     }
@@ -373,26 +372,25 @@ template <int PHASE, int TM> struct TileAcc<__nv_bfloat16, PHASE, TM> {
   template <typename F> __device__ __forceinline__ void each(F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int m0 = (warp / WARPS_N) * 16 * MT, n0 = (warp % WARPS_N) * 8 * NT;
+    const int m0 = (warp / WARPS_N) * 16, n0 = (warp % WARPS_N) * 8 * NT;
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          f(m0 + 16 * m + g + (i >> 1) * 8, n0 + 8 * n + 2 * t + (i & 1), acc[0][m][n][i],
-            acc[W - 1][m][n][i]);
-        }
+      for (int i = 0; i < 4; ++i) {
+        f(m0 + g + (i >> 1) * 8, n0 + 8 * n + 2 * t + (i & 1), acc[0][n][i], acc[W - 1][n][i]);
+      }
   }
 };
 
-template <typename T, int PHASE, int TM>
+// A list made for tiles of `tile_rows` (32 or 128) pairs is walked 32 pairs at a time.
+template <typename T, int PHASE>
 __global__ void __launch_bounds__(256, 2)  // two CTAs an SM: one's copies under the other's products
 moe_tile_kernel(const T* __restrict__ a, int lda, const T* __restrict__ weight,
                 const int* __restrict__ sorted, const int* __restrict__ tile_expert, int top,
                 int K, int N, float limit, float alpha, float shift, T* __restrict__ y, int ld_y,
-                float* __restrict__ out, int ld_out, int wide, int single) {
-  using Acc = TileAcc<T, PHASE, TM>;
+                float* __restrict__ out, int ld_out, int tile_rows, int wide, int single) {
+  using Acc = TileAcc<T, PHASE>;
+  constexpr int TM = MOE_TM;
   constexpr int LDS = Acc::LDS, TK = Acc::TK;
   constexpr bool BF16 = sizeof(T) == 2;
   __shared__ __align__(16) T As[TM * LDS];
@@ -402,7 +400,7 @@ moe_tile_kernel(const T* __restrict__ a, int lda, const T* __restrict__ weight,
   pdl_launch_dependents();
   const int tile = blockIdx.x, n0 = blockIdx.y * MOE_TN, tid = threadIdx.x;
   pdl_wait_for(a, sorted, tile_expert);
-  const int e = tile_expert[tile];
+  const int e = tile_expert[tile / (tile_rows / TM)];
   if (e < 0) return;
   if (tid < TM) pair_s[tid] = sorted[tile * TM + tid];
   __syncthreads();
@@ -584,10 +582,10 @@ __global__ void moe_join_kernel(const float* __restrict__ pair_out, int ld, cons
   }
 }
 
-template <typename T, int TM>
+template <typename T>
 int moe_experts(const void* hidden, int ld_hidden, const void* w_in, const void* w_out,
-                const int* sorted, const int* tile_expert, int max_tiles, int top, int width,
-                int ff, float limit, float alpha, float shift, int single, void* y, int ld_y,
+                const int* sorted, const int* tile_expert, int max_tiles, int tile_rows, int top,
+                int width, int ff, float limit, float alpha, float shift, int single, void* y, int ld_y,
                 float* pair_out, int ld_out, cudaStream_t stream) {
   // 16-byte pieces when every row of every operand starts on a 16-byte boundary
   const auto aligned = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
@@ -597,23 +595,25 @@ int moe_experts(const void* hidden, int ld_hidden, const void* w_in, const void*
                        aligned(w_out);
   // (room in shared memory for two CTAs an SM: the default split may leave less)
   static const bool carved = [] {
-    cudaFuncSetAttribute(moe_tile_kernel<T, 0, TM>,
+    cudaFuncSetAttribute(moe_tile_kernel<T, 0>,
                          cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(moe_tile_kernel<T, 1, TM>,
+    cudaFuncSetAttribute(moe_tile_kernel<T, 1>,
                          cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return true;
   }();
   (void)carved;
-  const dim3 grid_in(max_tiles, (ff + MOE_TN - 1) / MOE_TN);
-  int status = launch_kernel(moe_tile_kernel<T, 0, TM>, grid_in, dim3(256), 0, stream, 1,
+  const int row_tiles = max_tiles * (tile_rows / MOE_TM);
+  const dim3 grid_in(row_tiles, (ff + MOE_TN - 1) / MOE_TN);
+  int status = launch_kernel(moe_tile_kernel<T, 0>, grid_in, dim3(256), 0, stream, 1,
                              (const T*)hidden, ld_hidden, (const T*)w_in, sorted, tile_expert,
                              top, width, ff, limit, alpha, shift, (T*)y, ld_y, (float*)nullptr, 0,
-                             wide_in, single);
+                             tile_rows, wide_in, single);
   if (status != AYK_OK) return status;
-  const dim3 grid_out(max_tiles, (width + MOE_TN - 1) / MOE_TN);
-  return launch_kernel(moe_tile_kernel<T, 1, TM>, grid_out, dim3(256), 0, stream, 1, (const T*)y,
+  const dim3 grid_out(row_tiles, (width + MOE_TN - 1) / MOE_TN);
+  return launch_kernel(moe_tile_kernel<T, 1>, grid_out, dim3(256), 0, stream, 1, (const T*)y,
                        ld_y, (const T*)w_out, sorted, tile_expert, top, ff, width, limit, alpha, shift,
-                       (T*)nullptr, 0, pair_out, ld_out, wide_out, 0);
+                       (T*)nullptr, 0, pair_out, ld_out, tile_rows,
+                       wide_out, 0);
 }
 
 }  // namespace ayk
@@ -661,14 +661,16 @@ AYK_API int ayk_moe_route_scored(const float* logits, int ld, int rows, int expe
 }
 
 // Three launches: align, the two grouped products. `sorted` holds max_tiles * tile_rows ints,
-// `tile_expert` max_tiles, `y` max_tiles * tile_rows rows of ff, `pair_out` rows * top rows
+// `tile_expert` max_tiles (twice that for tiles of 128), `y` max_tiles * tile_rows rows of ff, `pair_out` rows * top rows
 // of width. type: 0 = float32, 1 = bfloat16. tile_rows: 32, or 128 (bfloat16 only).
+// A tcgen05 product whose bounded wait ran out says so in `device_status`.
 AYK_API int ayk_moe_experts(const void* hidden, int ld_hidden, const void* w_in,
                             const void* w_out, const int* chosen, int rows, int experts, int top,
                             int width, int ff, float limit, float alpha, float shift, int single,
                             int* sorted,
                             int* tile_expert, int max_tiles, int tile_rows, void* y, int ld_y,
-                            float* pair_out, int ld_out, int type, void* stream) {
+                            float* pair_out, int ld_out, int type, int* device_status,
+                            void* stream) {
   using namespace ayk;
   if (rows == 0) return AYK_OK;
   const long long pairs = (long long)rows * top;
@@ -677,29 +679,32 @@ AYK_API int ayk_moe_experts(const void* hidden, int ld_hidden, const void* w_in,
       tile_expert == nullptr || y == nullptr || pair_out == nullptr || ld_hidden < width ||
       ld_y < ff || ld_out < width || !(limit > 0.f) ||
       (tile_rows != MOE_TM && !(tile_rows == MOE_TM_WIDE && type == 1)) ||
-      (long long)max_tiles * tile_rows <
+      device_status == nullptr || (long long)max_tiles * tile_rows <
           pairs + (long long)min(experts, (int)pairs) * (tile_rows - 1)) {
     return AYK_BAD_ARGUMENT;
   }
   if (experts > MOE_MAX_EXPERTS || max_tiles > 2000000) return AYK_TOO_LARGE;
   cudaStream_t s = (cudaStream_t)stream;
+  const bool wide = tile_rows == MOE_TM_WIDE &&
+                    moe_tc_takes(hidden, ld_hidden, w_in, w_out, width, ff, y, ld_y, pair_out, ld_out);
+  int* tile_first = wide ? tile_expert + max_tiles : nullptr;
   int status = launch_kernel(moe_align_kernel, dim3(1), dim3(1024), 0, s, 1, chosen, (int)pairs,
-                             experts, max_tiles, tile_rows, sorted, tile_expert);
+                             experts, max_tiles, tile_rows, sorted, tile_expert, tile_first);
   if (status != AYK_OK) return status;
-  if (type == 0) {
-    return moe_experts<float, MOE_TM>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert, max_tiles,
-                              top, width, ff, limit, alpha, shift, single, y, ld_y, pair_out,
-                              ld_out, s);
+  if (wide) {
+    return moe_experts_tc(hidden, ld_hidden, w_in, w_out, sorted, tile_expert, tile_first,
+                          max_tiles, rows, experts, top, width, ff, MoeUnit{limit, alpha, shift, single}, y, ld_y,
+                          pair_out, ld_out, device_status, s);
   }
-  if (type == 1 && tile_rows == MOE_TM_WIDE) {
-    return moe_experts<__nv_bfloat16, MOE_TM_WIDE>(hidden, ld_hidden, w_in, w_out, sorted,
-                                                   tile_expert, max_tiles, top, width, ff, limit,
-                                                   alpha, shift, single, y, ld_y, pair_out, ld_out, s);
+  if (type == 0) {
+    return moe_experts<float>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert, max_tiles,
+                              tile_rows, top, width, ff, limit, alpha, shift, single, y, ld_y,
+                              pair_out, ld_out, s);
   }
   if (type == 1) {
-    return moe_experts<__nv_bfloat16, MOE_TM>(hidden, ld_hidden, w_in, w_out, sorted,
-                                              tile_expert, max_tiles, top, width, ff, limit,
-                                              alpha, shift, single, y, ld_y, pair_out, ld_out, s);
+    return moe_experts<__nv_bfloat16>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert,
+                                      max_tiles, tile_rows, top, width, ff, limit, alpha, shift,
+                                      single, y, ld_y, pair_out, ld_out, s);
   }
   return AYK_BAD_ARGUMENT;
 }

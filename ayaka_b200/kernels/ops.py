@@ -1456,9 +1456,12 @@ def moe_max_tiles(rows: int, experts: int, top: int, tile_rows: int = MOE_TILE_R
 
 
 def moe_tile_rows(rows: int, experts: int, top: int, dtype: torch.dtype) -> int:
-    """Rows of a tile :func:`moe_experts` uses: the wide tile in bfloat16 once an expert gets
-    two narrow tiles' worth of pairs on average, else the narrow one."""
-    wide = dtype == torch.bfloat16 and rows * top >= 2 * MOE_TILE_ROWS * experts
+    """Rows of a tile :func:`moe_experts` uses: the wide tile (tcgen05 products) in bfloat16
+    once an expert gets a narrow tile's worth of pairs on average, else the narrow one (both
+    products of 16 experts, narrow against wide: 16 pairs an expert, 2,048 x 2,048, 155 against
+    126 us, but 8 pairs at 1,024 x 1,024 56 against 73; 32 pairs 208 against 126 and 75 against
+    48; 512 pairs 1,631 against 235)."""
+    wide = dtype == torch.bfloat16 and rows * top >= MOE_TILE_ROWS * experts
     return MOE_TILE_ROWS_WIDE if wide else MOE_TILE_ROWS
 
 
@@ -1467,7 +1470,8 @@ def moe_scratch(rows: int, experts: int, top: int) -> tuple[int, int]:
     of ``tile_expert`` any tile size needs for up to ``rows`` rows."""
     sizes = (MOE_TILE_ROWS, MOE_TILE_ROWS_WIDE)
     return (max(moe_max_tiles(rows, experts, top, t) * t for t in sizes),
-            max(moe_max_tiles(rows, experts, top, t) for t in sizes))
+            max(moe_max_tiles(rows, experts, top, MOE_TILE_ROWS),
+                2 * moe_max_tiles(rows, experts, top, MOE_TILE_ROWS_WIDE)))
 
 
 def moe_route(logits: torch.Tensor, chosen: torch.Tensor, share: torch.Tensor, *, top: int,
@@ -1501,7 +1505,7 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
     ``g = min(W_gate h, limit)``, ``u = clamp(W_up h, -limit, limit)``,
     ``y = g * sigmoid(alpha * g) * (u + shift)`` and ``pair_out[p] = W_down y`` (float32
     ``[N * top, width]``, unweighted); ``limit=inf, alpha=1, shift=0`` is ``silu(g) * u``. Scratch: ``sorted_pairs`` (int32, ``tiles * tile
-    rows``), ``tile_expert`` (int32, ``tiles``) and ``inner`` (``[tiles * tile rows, ff]``,
+    rows``), ``tile_expert`` (int32, two per wide tile) and ``inner`` (``[tiles * tile rows, ff]``,
     compute dtype) sized by :func:`moe_scratch`. With ``single`` an expert has no gate:
     ``w_in`` is ``[experts * ff, width]`` and ``y = relu(W_up h)^2``."""
     op = "moe_experts"
@@ -1518,16 +1522,17 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
     width, ff = hidden.shape[1], w_out.shape[1]
     tile_rows = moe_tile_rows(rows, experts, top, hidden.dtype)
     tiles = moe_max_tiles(rows, experts, top, tile_rows)
+    kept_tiles = tiles * (2 if tile_rows > MOE_TILE_ROWS else 1)  # and each one's first row
     if hidden.dtype not in _TYPE or not w_in.is_contiguous() or not w_out.is_contiguous() or \
             tuple(w_in.shape) != (experts * (1 if single else 2) * ff, width) or \
             tuple(w_out.shape) != (experts * width, ff) or inner.shape[1] != ff or \
             pair_out.shape[1] != width or rows > hidden.shape[0] or \
             chosen.shape[0] < rows * top or pair_out.shape[0] < rows * top or \
-            sorted_pairs.shape[0] < tiles * tile_rows or tile_expert.shape[0] < tiles or \
+            sorted_pairs.shape[0] < tiles * tile_rows or tile_expert.shape[0] < kept_tiles or \
             inner.shape[0] < tiles * tile_rows:
         raise BackendError(f"{op}: shapes do not fit")
     global _launches
-    _launches += 2  # align and two products
+    _launches += 2 + (tile_rows > MOE_TILE_ROWS)  # align, (the rows grouped,) two products
     status = library("moe").ayk_moe_experts(
         _ptr(hidden), c_int(hidden.stride(0)), _ptr(w_in), _ptr(w_out), _ptr(chosen),
         c_int(rows), c_int(experts), c_int(top), c_int(width), c_int(ff), c_float(limit),
@@ -1536,7 +1541,7 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
         c_int(tile_rows),
         _ptr(inner),
         c_int(inner.stride(0)), _ptr(pair_out), c_int(pair_out.stride(0)),
-        c_int(_TYPE[hidden.dtype]), _stream())
+        c_int(_TYPE[hidden.dtype]), _ptr(_status_word(hidden.device)), _stream())
     check(status, op)
 
 
