@@ -1,84 +1,186 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias, activation, residual) on the CUDA cores with fp32 FMA.
 //
 // This is the true 32-bit matrix product of the float32 path (tensor cores have no fp32 x fp32
-// mode) and the plain on-device reference of the tensor-core kernel in bfloat16. Every output
-// element is accumulated over k = 0..K-1 in that order in one fp32 register, whatever M, N or
-// the tile it falls in, so a row's result does not depend on what else is in the batch.
-// Any M, N, K and leading dimensions; no alignment rule.
-#include "common.cuh"
+// mode) and the plain on-device reference of the tensor-core kernel in bfloat16. K is cut into
+// `simt_splits(N, K)` equal stretches; every output element is, per stretch, two fp32 sums over
+// the even and over the odd k upward, and these are added up in the stretches' order, whatever M
+// or the tile it falls in, so a row's result does not depend on what else is in the batch. Any M,
+// N, K and leading dimensions; no alignment rule.
+//
+// Bound by FMA issue and by what shared memory can feed, so a thread owns 8 x 8 elements (a
+// quarter of a shared float per FMA, all that the 128 bytes a clock allow) and the products are
+// packed pairs (fma.rn.f32x2, two exact fp32 FMAs an instruction): a pair is two neighbouring k of
+// one element, which lie side by side in shared memory as the operands do in global memory; pairs
+// along m or n would need moves. Tiles travel by cp.async through a ring of four stages of 16 k;
+// rows of 20 floats let the eight rows that a quarter of a warp reads 16 bytes of fall into
+// different banks. The stretches of K run in the CTAs of a cluster, each of which adds up its share
+// of the tile's rows through distributed shared memory: a few hundred rows of a model's products
+// are too few tiles for the device.
+// Measured on a B200 at 513 rows (2304 x 768, 768 x 768, 3072 x 768, 768 x 3072), against
+// tiles of 64 x 64 with 4 x 4 elements a thread:  123, 76, 123, 287 -> 92, 37, 94, 111
+// microseconds (cold caches); at 64 rows 83, 82, 84, 318 -> 23, 16, 27, 25.
+#include "tc_common.cuh"
 
 namespace ayk {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int BK = 16, LDK = BK + 4, SIMT_STAGES = 4;
+constexpr int SIMT_THREADS = 64;  // 8 x 8
+
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
+                                                   unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ void simt_copy16(float* dst, const float* src, bool in) {
+  // (with a source size of 0 nothing is read and the 16 bytes are zeros)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 16 : 0)
+               : "memory");
+}
+
+// 16 k from k0 of rows r0 .. r0 + ROWS of a matrix with `rows` rows, zeros outside it; `vec`: fp32,
+// rows of whole aligned 16-byte pieces.
+template <int ROWS, typename T>
+__device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src, int ld, int r0,
+                                           int rows, int k0, int K, bool vec) {
+  if (sizeof(T) == 4 && vec) {
+#pragma unroll
+    for (int idx = threadIdx.x; idx < ROWS * (BK / 4); idx += SIMT_THREADS) {
+      const int r = idx / (BK / 4), k = idx % (BK / 4) * 4;
+      const bool in = r0 + r < rows && k0 + k < K;  // (K is a multiple of 4)
+      simt_copy16(dst + r * LDK + k,
+                  reinterpret_cast<const float*>(src) + (in ? (size_t)(r0 + r) * ld + k0 + k : 0), in);
+    }
+  } else {
+    for (int idx = threadIdx.x; idx < ROWS * BK; idx += SIMT_THREADS) {
+      const int r = idx / BK, k = idx % BK;
+      dst[r * LDK + k] =
+          r0 + r < rows && k0 + k < K ? ldf(src + (size_t)(r0 + r) * ld + k0 + k) : 0.f;
+    }
+  }
+}
 
 // MODE 0: out[m,n] = act(acc + bias[n]) stored as TOut.   MODE 1: out(fp32)[m,n] += acc + bias[n].
-template <typename TA, typename TW, typename TOut, int MODE>
-__global__ void __launch_bounds__(256)
+template <typename TOut, int MODE>
+__device__ __forceinline__ void simt_store(TOut* __restrict__ out, int ldo, int m, int n, float v,
+                                           const float* __restrict__ bias, int act) {
+  if (bias != nullptr) v += bias[n];
+  TOut* dst = out + (size_t)m * ldo + n;
+  if (MODE == 1) {
+    stf(dst, ldf(dst) + v);
+  } else {
+    stf(dst, activate(v, act));
+  }
+}
+
+// 8 x 8 threads; a thread owns T x T elements, rows and columns 8 apart. A cluster of `splits` CTAs
+// along grid.x works on a tile of 8 T x 8 T; CTA r's stretch of K starts at r * k_split.
+template <typename TA, typename TW, typename TOut, int MODE, int T>
+__global__ void __launch_bounds__(SIMT_THREADS)
 gemm_simt_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, int ldw,
                  const float* __restrict__ bias, TOut* __restrict__ out, int ldo, int M, int N,
-                 int K, int act) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Ws[BK][BN + 4];
+                 int K, int act, int vec, int splits, int k_split) {
+  constexpr int B = 8 * T, TILE = B * LDK;
+  __shared__ __align__(16) float ring[SIMT_STAGES * 2 * TILE];  // and the tile's sums at the end
+  static_assert(SIMT_STAGES * 2 * TILE >= B * B, "the sums fit the ring");
   pdl_launch_dependents();
-  pdl_wait_for(a);
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int ty = tid >> 4, tx = tid & 15;
-  const int lrow = tid >> 2, lk = (tid & 3) * 4;
-  float acc[4][4];
+  const int ty = threadIdx.x >> 3, tx = threadIdx.x & 7;
+  const int rank = splits > 1 ? (int)(blockIdx.x % splits) : 0;
+  const int m0 = blockIdx.y * B, n0 = (int)(blockIdx.x / splits) * B;
+  const int k_first = rank * k_split, k_last = min(K, k_first + k_split);
+  const int num_kb = (k_last - k_first + BK - 1) / BK;
+  unsigned long long acc[T][T];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < T; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < T; ++j) acc[i][j] = 0ull;  // (two zeros)
+  pdl_wait_for(a, out);
+  auto stage = [&](int kb) {
+    if (kb < num_kb) {
+      float* at = ring + kb % SIMT_STAGES * 2 * TILE;
+      stage_rows<B>(at, a, lda, m0, M, k_first + kb * BK, k_last, vec);
+      stage_rows<B>(at + TILE, w, ldw, n0, N, k_first + kb * BK, k_last, vec);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int kb = 0; kb < SIMT_STAGES - 1; ++kb) stage(kb);
+  for (int kb = 0; kb < num_kb; ++kb) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(SIMT_STAGES - 2) : "memory");
+    __syncthreads();  // block kb has landed, and everyone is done with block kb - 1
+    stage(kb + SIMT_STAGES - 1);
+    const float* a_s = ring + kb % SIMT_STAGES * 2 * TILE + ty * LDK;
+    const float* w_s = ring + kb % SIMT_STAGES * 2 * TILE + TILE + tx * LDK;
+#pragma unroll
+    for (int k = 0; k < BK; k += 4) {
+      ulonglong2 av[T], wv[T];
+#pragma unroll
+      for (int i = 0; i < T; ++i) {
+        av[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * 8 * LDK + k);
+        wv[i] = *reinterpret_cast<const ulonglong2*>(w_s + i * 8 * LDK + k);
+      }
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) acc[i][j] = fma2(av[i].x, wv[j].x, acc[i][j]);
+#pragma unroll
+      for (int i = 0; i < T; ++i)
+#pragma unroll
+        for (int j = 0; j < T; ++j) acc[i][j] = fma2(av[i].y, wv[j].y, acc[i][j]);
+    }
+  }
+  auto sum = [&](int i, int j) {
+    return __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
+  };
+  if (splits == 1) {
+#pragma unroll
+    for (int i = 0; i < T; ++i) {
+      const int m = m0 + ty + 8 * i;
+#pragma unroll
+      for (int j = 0; j < T; ++j) {
+        const int n = n0 + tx + 8 * j;
+        if (m < M && n < N) simt_store<TOut, MODE>(out, ldo, m, n, sum(i, j), bias, act);
+      }
+    }
+    return;
+  }
+  __syncthreads();  // (every copy has landed: the last blocks' waits covered them)
+#pragma unroll
+  for (int i = 0; i < T; ++i)
+#pragma unroll
+    for (int j = 0; j < T; ++j) ring[(ty + 8 * i) * B + tx + 8 * j] = sum(i, j);
+  cluster_sync_all();
+  const int share = B / splits;  // this CTA's rows of the tile
+  for (int idx = threadIdx.x; idx < share * B; idx += SIMT_THREADS) {
+    const int at = rank * share * B + idx, m = m0 + at / B, n = n0 + at % B;
+    float v = 0.f;
+    for (int r = 0; r < splits; ++r) v += ld_peer_f32(ring + at, r);
+    if (m < M && n < N) simt_store<TOut, MODE>(out, ldo, m, n, v, bias, act);
+  }
+  cluster_sync_all();  // nobody leaves while a peer may still read its sums
+}
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    {
-      const int m = m0 + lrow;
-      const TA* src = a + (size_t)m * lda + k0 + lk;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        As[lk + i][lrow] = (m < M && k0 + lk + i < K) ? ldf(src + i) : 0.f;
-      }
-      const int n = n0 + lrow;
-      const TW* wsrc = w + (size_t)n * ldw + k0 + lk;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        Ws[lk + i][lrow] = (n < N && k0 + lk + i < K) ? ldf(wsrc + i) : 0.f;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float av[4], wv[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) av[i] = As[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) wv[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      if (bias != nullptr) v += bias[n];
-      TOut* dst = out + (size_t)m * ldo + n;
-      if (MODE == 1) {
-        stf(dst, ldf(dst) + v);
-      } else {
-        stf(dst, activate(v, act));
-      }
-    }
-  }
+// Stretches of K, by N and K alone: 1, 2, 4 or 8, so that a row of 64-wide tiles comes to about
+// 128 CTAs as long as a stretch has at least 192 k.
+inline int simt_splits(int N, int K) {
+  const int tiles = (N + 63) / 64;
+  int splits = 1;
+  while (splits < 8 && 2 * splits * tiles <= 128 && K >= 2 * splits * 192) splits *= 2;
+  return splits;
+}
+
+template <typename TA, typename TW, typename TOut, int MODE, int T>
+int launch_simt(const TA* a, int lda, const TW* w, int ldw, const float* bias, TOut* out, int ldo,
+                int M, int N, int K, int act, int vec, int splits, cudaStream_t stream) {
+  const long long gy = (M + 8 * T - 1) / (8 * T);
+  if (gy > 65535) return AYK_TOO_LARGE;
+  const int k_split = ((K + splits - 1) / splits + BK - 1) / BK * BK;
+  return launch_kernel_x(gemm_simt_kernel<TA, TW, TOut, MODE, T>,
+                         dim3((N + 8 * T - 1) / (8 * T) * splits, (unsigned)gy),
+                         dim3(SIMT_THREADS), 0, stream, splits, a, lda, w, ldw, bias, out, ldo, M,
+                         N, K, act, vec, splits, k_split);
 }
 
 template <typename TA, typename TW, typename TOut, int MODE>
@@ -87,11 +189,18 @@ int gemm_simt(const void* a, int lda, const void* w, int ldw, const float* bias,
   if (M == 0 || N == 0) return AYK_OK;
   if (M < 0 || N < 0 || K < 1 || lda < K || ldw < K || ldo < N) return AYK_BAD_ARGUMENT;
   if (act < ACT_NONE || act > ACT_RELU_SQUARED) return AYK_BAD_ARGUMENT;
-  const long long gy = (M + BM - 1) / BM;
-  if (gy > 65535) return AYK_TOO_LARGE;
-  dim3 grid((N + BN - 1) / BN, (unsigned)gy);
-  return launch_kernel(gemm_simt_kernel<TA, TW, TOut, MODE>, grid, dim3(256), 0, stream, 1,
-                       (const TA*)a, lda, (const TW*)w, ldw, bias, (TOut*)out, ldo, M, N, K, act);
+  const int vec = sizeof(TA) == 4 && sizeof(TW) == 4 && K % 4 == 0 && lda % 4 == 0 &&
+                  ldw % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0;
+  const int splits = simt_splits(N, K);
+  const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64) * splits;
+  // 32 x 32 tiles while those of 64 x 64 leave SMs without one (an M that the small tile's grid
+  // cannot count takes the large one)
+  if (tiles < sm_count() && M <= 65535 * 32) {
+    return launch_simt<TA, TW, TOut, MODE, 4>((const TA*)a, lda, (const TW*)w, ldw, bias,
+                                              (TOut*)out, ldo, M, N, K, act, vec, splits, stream);
+  }
+  return launch_simt<TA, TW, TOut, MODE, 8>((const TA*)a, lda, (const TW*)w, ldw, bias, (TOut*)out,
+                                            ldo, M, N, K, act, vec, splits, stream);
 }
 
 }  // namespace ayk
