@@ -35,6 +35,18 @@ template <> struct Elem<__nv_bfloat16> {
 template <typename T> __device__ __forceinline__ float ldf(const T* p) { return Elem<T>::load(p); }
 template <typename T> __device__ __forceinline__ void stf(T* p, float v) { Elem<T>::store(p, v); }
 
+// Two fp32 numbers side by side (the lower address in the low half), each rounded on its own: half
+// the instructions of the same arithmetic one by one.
+typedef unsigned long long float_pair;
+__device__ __forceinline__ float_pair fma2(float_pair a, float_pair b, float_pair c) {
+  float_pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ float sum2(float_pair a) {
+  return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32));
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -26,12 +26,6 @@ namespace ayk {
 constexpr int BK = 16, LDK = BK + 4, SIMT_STAGES = 4;
 constexpr int SIMT_THREADS = 64;  // 8 x 8
 
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b,
-                                                   unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 __device__ __forceinline__ void simt_copy16(float* dst, const float* src, bool in) {
   // (with a source size of 0 nothing is read and the 16 bytes are zeros)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
@@ -91,7 +85,7 @@ gemm_simt_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, in
   const int m0 = blockIdx.y * B, n0 = (int)(blockIdx.x / splits) * B;
   const int k_first = rank * k_split, k_last = min(K, k_first + k_split);
   const int num_kb = (k_last - k_first + BK - 1) / BK;
-  unsigned long long acc[T][T];
+  float_pair acc[T][T];
 #pragma unroll
   for (int i = 0; i < T; ++i)
 #pragma unroll
@@ -131,9 +125,7 @@ gemm_simt_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, in
         for (int j = 0; j < T; ++j) acc[i][j] = fma2(av[i].y, wv[j].y, acc[i][j]);
     }
   }
-  auto sum = [&](int i, int j) {
-    return __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
-  };
+  auto sum = [&](int i, int j) { return sum2(acc[i][j]); };
   if (splits == 1) {
 #pragma unroll
     for (int i = 0; i < T; ++i) {

@@ -26,6 +26,8 @@
 // with Kt = G k, Qt = G q, R = B T, Kh = T^T (D_(C-1) k) is all the scan computes. Decays only
 // ever appear as products of factors in [0, 1] (never as quotients), so nothing overflows and a
 // channel that forgets at once is exact. A chunk's missing rows have k = q = 0, beta = 0, g = 1.
+#include <type_traits>
+
 #include "common.cuh"
 #include "rope.cuh"
 
@@ -38,7 +40,8 @@ constexpr int LA_MAX_TAPS = 16;
 constexpr int LA_CONV_ROWS = 8;    // rows per CTA of the portions' convolution
 constexpr int LA_THREADS = 256;
 
-enum DecayMode : int { DECAY_FIXED = 0, DECAY_HEAD = 1, DECAY_CHANNEL = 2 };
+// (DECAY_SIGMOID: per key channel, sigmoid(raw)^(1/tau); portions only)
+enum DecayMode : int { DECAY_FIXED = 0, DECAY_HEAD = 1, DECAY_CHANNEL = 2, DECAY_SIGMOID = 3 };
 enum HeadGate : int { HEAD_GATE_NONE = 0, HEAD_GATE_SIGMOID = 1, HEAD_GATE_SILU = 2 };
 
 // What both paths need to know of a layer and a step (packed once per call by the host).
@@ -71,6 +74,9 @@ struct LinearArgs {
   int rot_dims, rot_layout;
   int requests, chunks;
   float q_scale, k_scale, eps, unit_eps;
+  // portions only
+  float inv_tau;   // DECAY_SIGMOID
+  int transposed;  // the state's slots hold S as [head][P][N]
 };
 
 __device__ __forceinline__ float la_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
@@ -81,6 +87,10 @@ __device__ __forceinline__ float la_softplus(float z) {  // log(1 + e^z), for an
 // a decay; rate = -exp(A_log)
 __device__ __forceinline__ float la_decay(float rate, float raw) {
   return expf(rate * la_softplus(raw));
+}
+// sigmoid(raw)^inv_tau
+__device__ __forceinline__ float la_sigmoid_decay(float raw, float inv_tau) {
+  return expf((fminf(raw, 0.f) - log1pf(expf(-fabsf(raw)))) * inv_tau);
 }
 __device__ __forceinline__ void la_sincos(int position, double f, float& s, float& c) {
   // the angle and its reduction to [-pi, pi] in double precision (see rope.cuh)
@@ -174,11 +184,11 @@ la_conv_kernel(const float* __restrict__ in, int ld_in, const float* __restrict_
 }
 
 // ---------------------------------------------------------------------------------------------
-// A chunk's matrices in the scratch, per (chunk, head): M [N][2 C] (Kt of the C rows, then Qt),
-// Kh [N][C], G [N] (padded to a multiple of 4), R [C][C].
+// A chunk's matrices in the scratch, per (chunk, head): M [N][2 C] (Kt of the C rows, then Qt; Qt
+// alone, [N][C], without the delta rule), Kh [N][C], G [N] (padded to a multiple of 4), R [C][C].
 __host__ __device__ __forceinline__ int la_pad4(int n) { return (n + 3) & ~3; }
-__host__ __device__ __forceinline__ int la_chunk_floats(int N) {
-  return 3 * LA_C * N + la_pad4(N) + LA_C * LA_C;
+__host__ __device__ __forceinline__ int la_chunk_floats(int N, bool delta) {
+  return (delta ? 3 : 2) * LA_C * N + la_pad4(N) + LA_C * LA_C;
 }
 
 // The request that owns chunk `index` of the step and the chunk's first row in it.
@@ -222,7 +232,8 @@ la_prepare_kernel(const LinearArgs a) {
   pdl_wait_for(in, raw, decay_raw, scratch);
   if (!found) return;
   const int r0 = a.row_start[b] + t0;
-  const float rate = a.decay_mode == DECAY_FIXED ? 0.f : -expf(a.a_log[h]);
+  const float rate =
+      a.decay_mode == DECAY_HEAD || a.decay_mode == DECAY_CHANNEL ? -expf(a.a_log[h]) : 0.f;
   if (tid < LA_C * LA_C) {
     A[tid / LA_C][tid % LA_C] = 0.f;
     B[tid / LA_C][tid % LA_C] = 0.f;
@@ -247,9 +258,12 @@ la_prepare_kernel(const LinearArgs a) {
       q[m] = live ? src[a.q_at + kv * N + n] : 0.f;
       g[m] = shared_g;
       if (CHANNEL) {
-        g[m] = live ? la_decay(rate, decay_raw[(size_t)(r0 + i) * a.ld_decay + h * N + n] +
-                                         a.dt_bias[h * N + n])
-                    : 1.f;
+        g[m] = 1.f;
+        if (live) {
+          const float z = decay_raw[(size_t)(r0 + i) * a.ld_decay + h * N + n];
+          g[m] = a.decay_mode == DECAY_SIGMOID ? la_sigmoid_decay(z, a.inv_tau)
+                                               : la_decay(rate, z + a.dt_bias[h * N + n]);
+        }
       }
     }
     if (lane == 0) {
@@ -311,9 +325,9 @@ la_prepare_kernel(const LinearArgs a) {
     }
   }
   __syncthreads();
-  float* chunk = scratch + ((size_t)blockIdx.x * a.heads + h) * la_chunk_floats(N);
+  float* chunk = scratch + ((size_t)blockIdx.x * a.heads + h) * la_chunk_floats(N, a.delta);
   float* m_out = chunk;
-  float* kh_out = m_out + 2 * LA_C * N;
+  float* kh_out = m_out + (a.delta ? 2 : 1) * LA_C * N;
   float* g_out = kh_out + LA_C * N;
   float* r_out = g_out + la_pad4(N);
   {
@@ -385,9 +399,10 @@ la_prepare_kernel(const LinearArgs a) {
       }
     }
   } else {  // meanwhile Kt and Qt (four rows of a channel a thread) and G
-    for (int idx = tid - 32; idx < N * 8; idx += LA_THREADS - 32) {
-      const int n = idx >> 3, part = idx & 7, first = (part & 3) * 4;
-      const float* x = part < 4 ? k_s : q_s;
+    const int parts = a.delta ? 8 : 4;
+    for (int idx = tid - 32; idx < N * parts; idx += LA_THREADS - 32) {
+      const int n = idx / parts, part = idx % parts, first = (part & 3) * 4;
+      const float* x = part < parts - 4 ? k_s : q_s;
       float g = 1.f;
       for (int i = 0; i < first; ++i) g *= g_s[i * NS + n];
       float v[4];
@@ -396,7 +411,7 @@ la_prepare_kernel(const LinearArgs a) {
         g *= g_s[(first + i) * NS + n];
         v[i] = g * x[(first + i) * NS + n];
       }
-      *reinterpret_cast<float4*>(m_out + (size_t)n * 2 * LA_C + part * 4) =
+      *reinterpret_cast<float4*>(m_out + (size_t)n * parts * 4 + part * 4) =
           make_float4(v[0], v[1], v[2], v[3]);
       if (part == 3) g_out[n] = g;
     }
@@ -440,8 +455,8 @@ template <int N> __device__ __forceinline__ void la_wait() {
 }
 
 // floats of one stage (a chunk's matrices and its values) and of the rest of shared memory
-__host__ __device__ __forceinline__ int la_stage_floats(int N) {
-  return la_chunk_floats(N) + LA_C * LA_COLS;
+__host__ __device__ __forceinline__ int la_stage_floats(int N, bool delta) {
+  return la_chunk_floats(N, delta) + LA_C * LA_COLS;
 }
 __host__ __device__ __forceinline__ int la_fixed_floats(int N) {
   return N * LA_COLS + 8 * 2 * LA_C * LA_COLS + LA_C * LA_COLS;
@@ -449,15 +464,16 @@ __host__ __device__ __forceinline__ int la_fixed_floats(int N) {
 
 // grid (heads, requests, tiles of LA_COLS columns). Per chunk: [Kt; Qt] S_0 with the channels
 // shared out over the eight warps (a warp's lanes hold 4 x 4 pieces of the 32 x 16 result), the
-// warps' shares added up, W; then O and the new state from W.
-template <int STAGES>
+// warps' shares added up, W; then O and the new state from W. Without the delta rule there is no
+// Kt and W is V: half a warp holds the 16 x 16 result, the halves share out the channels too.
+template <int STAGES, bool DELTA>
 __global__ void __launch_bounds__(LA_THREADS)
 la_scan_kernel(const LinearArgs a, int vec) {
   extern __shared__ __align__(16) float la_smem[];
   pdl_launch_dependents();
   const int N = a.N, P = a.P, h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * LA_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int stage_floats = la_stage_floats(N), chunk_floats = la_chunk_floats(N);
+  const int stage_floats = la_stage_floats(N, DELTA), chunk_floats = la_chunk_floats(N, DELTA);
   float* s_s = la_smem + (size_t)STAGES * stage_floats;  // [N][LA_COLS]
   float* red = s_s + N * LA_COLS;                        // [8 warps][4][32 lanes][4]
   float* w_s = red + 8 * 2 * LA_C * LA_COLS;             // [C][LA_COLS]
@@ -505,14 +521,19 @@ la_scan_kernel(const LinearArgs a, int vec) {
     }
   }
   for (int idx = tid; idx < N * LA_COLS; idx += LA_THREADS) {
-    const int n = idx / LA_COLS, c = idx % LA_COLS;
-    s_s[idx] = p0 + c < P ? mine[(size_t)n * P + p0 + c] : 0.f;
+    if (a.transposed) {
+      const int c = idx / N, n = idx % N;
+      s_s[n * LA_COLS + c] = p0 + c < P ? mine[(size_t)(p0 + c) * N + n] : 0.f;
+    } else {
+      const int n = idx / LA_COLS, c = idx % LA_COLS;
+      s_s[idx] = p0 + c < P ? mine[(size_t)n * P + p0 + c] : 0.f;
+    }
   }
-  const int rg = lane >> 2, cg = lane & 3;
+  const int rg = DELTA ? lane >> 2 : (lane >> 2) & 3, cg = lane & 3;
   // the result's element this thread finishes: its two rows of a warp lie in different quads of
   // rows at the same place, so that a warp reads 32 neighbouring floats of a share
   const int pr = tid >> 4, col = tid & 15;
-  const int row = (pr & 1) * 4 + ((pr >> 1) & 3) + (pr >> 3) * 8;
+  const int row = DELTA ? (pr & 1) * 4 + ((pr >> 1) & 3) + (pr >> 3) * 8 : pr;
   const int red_at = ((row & 3) * 32 + (row >> 2) * 4) * 4 + col;
   for (int c = 0; c < chunks; ++c) {
     if (STAGES == 1) {
@@ -528,18 +549,20 @@ la_scan_kernel(const LinearArgs a, int vec) {
       la_commit();
     }
     const float* m_s = la_smem + (size_t)(STAGES == 1 ? 0 : c % STAGES) * stage_floats;
-    const float* kh_s = m_s + 2 * LA_C * N;
+    const float* kh_s = m_s + (DELTA ? 2 : 1) * LA_C * N;
     const float* g_s = kh_s + LA_C * N;
     const float* r_s = g_s + la_pad4(N);
     const float* v_s = m_s + chunk_floats;
+    const float* used_s = DELTA ? w_s : v_s;  // W
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 #pragma unroll 4
-    for (int n = warp; n < N; n += 8) {
-      const float4 m = *reinterpret_cast<const float4*>(m_s + (size_t)n * 2 * LA_C + rg * 4);
+    for (int n = DELTA ? warp : 2 * warp + (lane >> 4); n < N; n += DELTA ? 8 : 16) {
+      const float4 m =
+          *reinterpret_cast<const float4*>(m_s + (size_t)n * (DELTA ? 2 : 1) * LA_C + rg * 4);
       const float4 s = *reinterpret_cast<const float4*>(s_s + n * LA_COLS + cg * 4);
       const float mv[4] = {m.x, m.y, m.z, m.w}, sv[4] = {s.x, s.y, s.z, s.w};
 #pragma unroll
@@ -547,24 +570,39 @@ la_scan_kernel(const LinearArgs a, int vec) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(mv[i], sv[j], acc[i][j]);
     }
+    float o = 0.f;
+    if (DELTA) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      *reinterpret_cast<float4*>(red + ((warp * 4 + i) * 32 + lane) * 4) =
-          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    }
-    __syncthreads();
-    float seen = 0.f, o = 0.f;
+      for (int i = 0; i < 4; ++i) {
+        *reinterpret_cast<float4*>(red + ((warp * 4 + i) * 32 + lane) * 4) =
+            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      }
+      __syncthreads();
+      float seen = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      seen += red[w * 512 + red_at];
-      o += red[w * 512 + red_at + 64];  // the same place of the rows of Qt (16 rows on)
+      for (int w = 0; w < 8; ++w) {
+        seen += red[w * 512 + red_at];
+        o += red[w * 512 + red_at + 64];  // the same place of the rows of Qt (16 rows on)
+      }
+      w_s[row * LA_COLS + col] = v_s[row * LA_COLS + col] - seen;
+      __syncthreads();
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += __shfl_xor_sync(0xffffffffu, acc[i][j], 16);
+        if (lane < 16) {
+          *reinterpret_cast<float4*>(red + (warp * LA_C + rg * 4 + i) * LA_COLS + cg * 4) =
+              make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < 8; ++w) o += red[w * LA_C * LA_COLS + tid];
     }
-    const float v = v_s[row * LA_COLS + col];
-    w_s[row * LA_COLS + col] = a.delta ? v - seen : v;
-    __syncthreads();
     float wc[LA_C];
 #pragma unroll
-    for (int j = 0; j < LA_C; ++j) wc[j] = w_s[j * LA_COLS + col];
+    for (int j = 0; j < LA_C; ++j) wc[j] = used_s[j * LA_COLS + col];
 #pragma unroll
     for (int j = 0; j < LA_C; j += 4) {
       const float4 r = *reinterpret_cast<const float4*>(r_s + row * LA_C + j);
@@ -575,34 +613,67 @@ la_scan_kernel(const LinearArgs a, int vec) {
     }
     const int t = c * LA_C + row;
     if (t < rows && p0 + col < P) a.out[(size_t)(r0 + t) * a.ld_out + h * P + p0 + col] = o;
-    for (int item = tid; item < N * 4; item += LA_THREADS) {
-      const int n = item >> 2, cq = (item & 3) * 4;
-      float4 s = *reinterpret_cast<float4*>(s_s + n * LA_COLS + cq);
-      const float g = g_s[n];
-      s.x *= g;
-      s.y *= g;
-      s.z *= g;
-      s.w *= g;
+    // four columns of a channel a thread; of more than LA_THREADS / 4 channels two a thread, which
+    // share what they fetch of W
+    auto update = [&](auto channels, int first) {
+      constexpr int CH = decltype(channels)::value;
+      const int cq = (first & 3) * 4;
+      float4 s[CH];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int n = (first >> 2) + i * (LA_THREADS / 4);
+        s[i] = *reinterpret_cast<float4*>(s_s + n * LA_COLS + cq);
+        const float g = g_s[n];
+        s[i].x *= g;
+        s[i].y *= g;
+        s[i].z *= g;
+        s[i].w *= g;
+      }
 #pragma unroll
       for (int j = 0; j < LA_C; j += 4) {
-        const float4 k = *reinterpret_cast<const float4*>(kh_s + n * LA_C + j);
-        const float kv[4] = {k.x, k.y, k.z, k.w};
+        float kv[CH][4];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+          const int n = (first >> 2) + i * (LA_THREADS / 4);
+          const float4 k = *reinterpret_cast<const float4*>(kh_s + n * LA_C + j);
+          kv[i][0] = k.x;
+          kv[i][1] = k.y;
+          kv[i][2] = k.z;
+          kv[i][3] = k.w;
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float4 w = *reinterpret_cast<const float4*>(w_s + (j + e) * LA_COLS + cq);
-          s.x = fmaf(kv[e], w.x, s.x);
-          s.y = fmaf(kv[e], w.y, s.y);
-          s.z = fmaf(kv[e], w.z, s.z);
-          s.w = fmaf(kv[e], w.w, s.w);
+          const float4 w = *reinterpret_cast<const float4*>(used_s + (j + e) * LA_COLS + cq);
+#pragma unroll
+          for (int i = 0; i < CH; ++i) {
+            s[i].x = fmaf(kv[i][e], w.x, s[i].x);
+            s[i].y = fmaf(kv[i][e], w.y, s[i].y);
+            s[i].z = fmaf(kv[i][e], w.z, s[i].z);
+            s[i].w = fmaf(kv[i][e], w.w, s[i].w);
+          }
         }
       }
-      *reinterpret_cast<float4*>(s_s + n * LA_COLS + cq) = s;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int n = (first >> 2) + i * (LA_THREADS / 4);
+        *reinterpret_cast<float4*>(s_s + n * LA_COLS + cq) = s[i];
+      }
+    };
+    int item = tid;
+    for (; item + LA_THREADS < N * 4; item += 2 * LA_THREADS) {
+      update(std::integral_constant<int, 2>{}, item);
     }
+    if (item < N * 4) update(std::integral_constant<int, 1>{}, item);
   }
   __syncthreads();
   for (int idx = tid; idx < N * LA_COLS; idx += LA_THREADS) {
-    const int n = idx / LA_COLS, c = idx % LA_COLS;
-    if (p0 + c < P) mine[(size_t)n * P + p0 + c] = s_s[idx];
+    if (a.transposed) {
+      const int c = idx / N, n = idx % N;
+      if (p0 + c < P) mine[(size_t)(p0 + c) * N + n] = s_s[n * LA_COLS + c];
+    } else {
+      const int n = idx / LA_COLS, c = idx % LA_COLS;
+      if (p0 + c < P) mine[(size_t)n * P + p0 + c] = s_s[idx];
+    }
   }
 }
 
@@ -892,6 +963,64 @@ static bool la_common_ok(const LinearArgs& a) {
          a.state_stride >= (long long)a.heads * a.N * a.P;
 }
 
+// Prepare and scan; everything but the scratch's alignment and the sizes has been checked.
+static int la_chunks(const LinearArgs& a, cudaStream_t s) {
+  if (((uintptr_t)a.scratch % 16) != 0) return AYK_BAD_ALIGNMENT;
+  const int tiles = (a.P + LA_COLS - 1) / LA_COLS;
+  if (a.N > LA_MAX_N || a.heads > 65535 || a.requests > 65535 || tiles > 65535) {
+    return AYK_TOO_LARGE;
+  }
+  const size_t smem = (size_t)4 * LA_C * la_pad4(a.N) * sizeof(float);
+  int status;
+#define AYK_LA_PREPARE_AS(NREG, CHANNEL)                                                         \
+  {                                                                                              \
+    static const bool allowed =                                                                  \
+        (cudaFuncSetAttribute(la_prepare_kernel<NREG, CHANNEL>,                                  \
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,                       \
+                              4 * LA_C * 32 * NREG * (int)sizeof(float)), true);                 \
+    (void)allowed;                                                                               \
+    status = launch_kernel(la_prepare_kernel<NREG, CHANNEL>, dim3(a.chunks, a.heads),            \
+                           dim3(LA_THREADS), smem, s, 1, a);                                     \
+  }
+#define AYK_LA_PREPARE(NREG)                                                                     \
+  {                                                                                              \
+    if (a.decay_mode >= DECAY_CHANNEL) AYK_LA_PREPARE_AS(NREG, true)                             \
+    else AYK_LA_PREPARE_AS(NREG, false)                                                          \
+  }
+  if (a.N <= 32) AYK_LA_PREPARE(1)
+  else if (a.N <= 64) AYK_LA_PREPARE(2)
+  else if (a.N <= 128) AYK_LA_PREPARE(4)
+  else if (a.N <= 256) AYK_LA_PREPARE(8)
+  else AYK_LA_PREPARE(16)
+#undef AYK_LA_PREPARE
+#undef AYK_LA_PREPARE_AS
+  if (status != AYK_OK) return status;
+  const int vec = ((uintptr_t)a.in % 16) == 0 && a.ld_in % 4 == 0 && a.v_at % 4 == 0 &&
+                  a.P % 4 == 0;
+  const dim3 grid(a.heads, a.requests, tiles);
+#define AYK_LA_SCAN_AS(STAGES, DELTA)                                                            \
+  {                                                                                              \
+    static const bool allowed =                                                                  \
+        (cudaFuncSetAttribute(la_scan_kernel<STAGES, DELTA>,                                     \
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), true);   \
+    (void)allowed;                                                                               \
+    return launch_kernel(la_scan_kernel<STAGES, DELTA>, grid, dim3(LA_THREADS),                  \
+                         ((size_t)STAGES * la_stage_floats(a.N, DELTA) + la_fixed_floats(a.N)) * \
+                             sizeof(float),                                                      \
+                         s, 1, a, vec);                                                          \
+  }
+#define AYK_LA_SCAN(STAGES)                                                                      \
+  {                                                                                              \
+    if (a.delta) AYK_LA_SCAN_AS(STAGES, true)                                                    \
+    AYK_LA_SCAN_AS(STAGES, false)                                                                \
+  }
+  if (a.N <= 128) AYK_LA_SCAN(3)
+  if (a.N <= 320) AYK_LA_SCAN(2)
+  AYK_LA_SCAN(1)
+#undef AYK_LA_SCAN
+#undef AYK_LA_SCAN_AS
+}
+
 }  // namespace ayk
 
 AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
@@ -899,7 +1028,7 @@ AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
 AYK_API int ayk_linear_chunk_rows() { return ayk::LA_C; }
 AYK_API int ayk_linear_args_bytes() { return (int)sizeof(ayk::LinearArgs); }
 // floats of the scratch per (chunk, head)
-AYK_API int ayk_linear_chunk_floats(int n) { return ayk::la_chunk_floats(n); }
+AYK_API int ayk_linear_chunk_floats(int n, int delta) { return ayk::la_chunk_floats(n, delta != 0); }
 
 // `ring`: the first float of slot 0's ring; slots are state_stride floats apart.
 AYK_API int ayk_conv_ring(const float* in, int ld_in, const float* w, float* ring,
@@ -944,55 +1073,52 @@ AYK_API int ayk_linear_chunks(const ayk::LinearArgs* args, void* stream) {
       (a.decay_mode == DECAY_HEAD && a.ld_raw < a.decay_at + a.heads)) {
     return AYK_BAD_ARGUMENT;
   }
-  if (((uintptr_t)a.scratch % 16) != 0) return AYK_BAD_ALIGNMENT;
-  const int tiles = (a.P + LA_COLS - 1) / LA_COLS;
-  if (a.N > LA_MAX_N || a.heads > 65535 || a.requests > 65535 || tiles > 65535) {
-    return AYK_TOO_LARGE;
+  return la_chunks(a, (cudaStream_t)stream);
+}
+
+// The gated linear attention of csrc/recurrent.cu (a decay sigmoid(z)^(1/tau) per key channel, S as
+// [head][P][N]) in chunks; its rows, `z` and the state as there, the scratch as above (no delta
+// rule). AYK_NOT_TAKEN: the scratch does not start on 16 bytes; nothing ran.
+AYK_API int ayk_gla_chunks(const float* proj, int ld_proj, int k_offset, int v_offset, const float* z,
+                           int ld_z, float tau, float q_scale, float* state,
+                           long long state_stride, const int* row_start, const int* state_slot,
+                           float* out, int ld_out, int requests, int chunks, int heads, int N,
+                           int P, float* scratch, void* stream) {
+  using namespace ayk;
+  if (requests == 0 || chunks == 0) return AYK_OK;
+  if (requests < 0 || chunks < 0 || heads < 1 || N < 1 || P < 1 || proj == nullptr || z == nullptr ||
+      state == nullptr || row_start == nullptr || state_slot == nullptr || out == nullptr ||
+      scratch == nullptr || !(tau > 0.f) || ld_out < heads * P || ld_z < heads * N ||
+      ld_proj < max(k_offset + heads * N, v_offset + heads * P) ||
+      state_stride < (long long)heads * N * P) {
+    return AYK_BAD_ARGUMENT;
   }
-  cudaStream_t s = (cudaStream_t)stream;
-  const size_t smem = (size_t)4 * LA_C * la_pad4(a.N) * sizeof(float);
-  int status;
-#define AYK_LA_PREPARE_AS(NREG, CHANNEL)                                                         \
-  {                                                                                              \
-    static const bool allowed =                                                                  \
-        (cudaFuncSetAttribute(la_prepare_kernel<NREG, CHANNEL>,                                  \
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,                       \
-                              4 * LA_C * 32 * NREG * (int)sizeof(float)), true);                 \
-    (void)allowed;                                                                               \
-    status = launch_kernel(la_prepare_kernel<NREG, CHANNEL>, dim3(a.chunks, a.heads),            \
-                           dim3(LA_THREADS), smem, s, 1, a);                                     \
-  }
-#define AYK_LA_PREPARE(NREG)                                                                     \
-  {                                                                                              \
-    if (a.decay_mode == DECAY_CHANNEL) AYK_LA_PREPARE_AS(NREG, true)                             \
-    else AYK_LA_PREPARE_AS(NREG, false)                                                          \
-  }
-  if (a.N <= 32) AYK_LA_PREPARE(1)
-  else if (a.N <= 64) AYK_LA_PREPARE(2)
-  else if (a.N <= 128) AYK_LA_PREPARE(4)
-  else if (a.N <= 256) AYK_LA_PREPARE(8)
-  else AYK_LA_PREPARE(16)
-#undef AYK_LA_PREPARE
-#undef AYK_LA_PREPARE_AS
-  if (status != AYK_OK) return status;
-  const int vec = ((uintptr_t)a.in % 16) == 0 && a.ld_in % 4 == 0 && a.v_at % 4 == 0 &&
-                  a.P % 4 == 0;
-  const dim3 grid(a.heads, a.requests, tiles);
-#define AYK_LA_SCAN(STAGES)                                                                      \
-  {                                                                                              \
-    static const bool allowed =                                                                  \
-        (cudaFuncSetAttribute(la_scan_kernel<STAGES>,                                            \
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), true);   \
-    (void)allowed;                                                                               \
-    return launch_kernel(la_scan_kernel<STAGES>, grid, dim3(LA_THREADS),                         \
-                         ((size_t)STAGES * la_stage_floats(a.N) + la_fixed_floats(a.N)) *        \
-                             sizeof(float),                                                      \
-                         s, 1, a, vec);                                                          \
-  }
-  if (a.N <= 128) AYK_LA_SCAN(3)
-  if (a.N <= 320) AYK_LA_SCAN(2)
-  AYK_LA_SCAN(1)
-#undef AYK_LA_SCAN
+  if (((uintptr_t)scratch % 16) != 0) return AYK_NOT_TAKEN;
+  LinearArgs a = {};
+  a.in = proj;
+  a.decay_raw = z;
+  a.row_start = row_start;
+  a.state_slot = state_slot;
+  a.state = state;
+  a.scratch = scratch;
+  a.out = out;
+  a.state_stride = state_stride;
+  a.ld_in = ld_proj;
+  a.ld_decay = ld_z;
+  a.ld_out = ld_out;
+  a.k_at = k_offset;
+  a.v_at = v_offset;
+  a.heads = a.kv_heads = heads;
+  a.N = N;
+  a.P = P;
+  a.decay_mode = DECAY_SIGMOID;
+  a.requests = requests;
+  a.chunks = chunks;
+  a.q_scale = q_scale;
+  a.k_scale = 1.f;
+  a.inv_tau = 1.f / tau;
+  a.transposed = 1;
+  return la_chunks(a, (cudaStream_t)stream);
 }
 
 // A step of single rows, row r of request r: one launch. type: 0 = float32, 1 = bfloat16, of

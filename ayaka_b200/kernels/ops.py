@@ -1157,15 +1157,77 @@ def causal_conv_silu(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor |
     check(status, op)
 
 
+#: rows of a chunk of the recurrences over prompt portions (``MC_ROWS`` in ``csrc/memory_chunks.cuh``)
+MEMORY_CHUNK = 64
+#: what a step may have more chunks than whole ones (requests of few rows), and the most scratch
+MEMORY_EXTRA_CHUNKS, MEMORY_MAX_FLOATS = 64, 1 << 28
+
+
+def memory_chunks(host_rows: list[int]) -> int:
+    """Chunks that a step of these row counts has."""
+    return sum(-(-rows // MEMORY_CHUNK) for rows in host_rows)
+
+
+def memory_buffers(host_rows: list[int], max_rows: int, heads: int, inner: int,
+                   columns: int) -> tuple[int, int] | None:
+    """``(chunks, floats per chunk)`` of the scratch for the largest step if a step of these row
+    counts is taken in chunks by :func:`mamba2_scan` / :func:`mlstm_scan`, else ``None``: a request
+    brings at least a chunk of rows, and the step is not mostly single rows. (The scan row by row
+    takes about 0.9 microseconds a row of the longest request, whatever else runs beside it; in
+    chunks a step takes about 20 and then 2 a chunk of 2^18 state entries, a single row's chunk
+    as much as a whole one.)"""
+    longest, chunks = max(host_rows, default=0), memory_chunks(host_rows)
+    most, floats = max_rows // MEMORY_CHUNK + MEMORY_EXTRA_CHUNKS, heads * inner * (columns + 1)
+    if longest < MEMORY_CHUNK or 2 * chunks > longest or chunks > most or \
+            most * floats > MEMORY_MAX_FLOATS:
+        return None
+    return most, floats
+
+
+def gla_buffers(host_rows: list[int], max_rows: int, heads: int,
+                dim: int) -> tuple[int, int] | None:
+    """The same for :func:`gla_scan`, whose chunks have ``LINEAR_CHUNK`` rows. (Row by row 0.72
+    microseconds a row of the longest request; in chunks about 20 and then 0.1 a row.)"""
+    longest, chunks = max(host_rows, default=0), linear_chunks(host_rows)
+    most = max_rows // LINEAR_CHUNK + MEMORY_EXTRA_CHUNKS
+    floats = heads * (2 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK)
+    if longest < MEMORY_CHUNK or chunks > longest or chunks > most or \
+            most * floats > MEMORY_MAX_FLOATS:
+        return None
+    return most, floats
+
+
+def _memory_scratch(op: str, host_rows: list[int] | None,
+                    scratch: tuple[torch.Tensor, torch.Tensor] | None, requests: int, heads: int,
+                    inner: int, columns: int, planes: int) -> tuple[int, int] | None:
+    """The step's rows and chunks when it is to run in chunks."""
+    if host_rows is None or scratch is None:
+        return None
+    rows, chunks = sum(host_rows), memory_chunks(host_rows)
+    extra = inner if planes == 3 else 0
+    for tensor, least in zip(scratch, (chunks * heads * (inner * columns + extra),
+                                       planes * rows * heads)):
+        _need(op, "scratch", tensor, torch.float32)
+        if not tensor.is_contiguous() or tensor.numel() < least:
+            raise BackendError(f"{op}: the scratch is too small")
+    if len(host_rows) != requests:
+        raise BackendError(f"{op}: row counts and requests do not match")
+    return rows, chunks
+
+
 def mamba2_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
                 a_log: torch.Tensor, skip: torch.Tensor | None, state: torch.Tensor,
                 y: torch.Tensor, *, row_start: torch.Tensor, state_slot: torch.Tensor,
-                requests: int, heads: int, groups: int, state_size: int, columns: int) -> None:
+                requests: int, heads: int, groups: int, state_size: int, columns: int,
+                host_rows: list[int] | None = None,
+                scratch: tuple[torch.Tensor, torch.Tensor] | None = None) -> None:
     """The state-space recurrence over each request's rows. ``xbc`` float32
     ``[N, heads * columns + 2 * groups * state_size]`` (x, then B, then C, after convolution
     and activation), ``dt_raw`` ``[N, heads]``; per head ``S <- exp(-exp(a_log) dt) S + dt B
     x^T``, ``y = S^T C + skip * x`` with ``dt = softplus(dt_raw + dt_bias)``. ``state``
-    ``[slots, heads * state_size * columns]`` (a view of the matrices' part of the state)."""
+    ``[slots, heads * state_size * columns]`` (a view of the matrices' part of the state). With the
+    step's ``host_rows`` and ``scratch`` (float32: the chunks' states, :func:`memory_buffers`; 2 *
+    heads floats a row) the rows are taken in chunks where the operands allow it."""
     op = "mamba2_scan"
     if _left_out and op in _left_out:
         return
@@ -1178,6 +1240,22 @@ def mamba2_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
     if xbc.shape[1] != heads * columns + 2 * groups * state_size or dt_raw.shape[1] != heads or \
             y.shape[1] != heads * columns or state.shape[1] < heads * state_size * columns:
         raise BackendError(f"{op}: shapes do not fit")
+    in_chunks = _memory_scratch(op, host_rows, scratch, requests, heads, state_size, columns, 2)
+    if in_chunks is not None:
+        rows, chunks = in_chunks
+        if rows > min(xbc.shape[0], dt_raw.shape[0], y.shape[0]):
+            raise BackendError(f"{op}: shapes do not fit")
+        status = library("recurrent").ayk_mamba2_chunks(
+            _ptr(xbc), c_int(xbc.stride(0)), _ptr(dt_raw), c_int(dt_raw.stride(0)),
+            _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state), c_longlong(state.stride(0)),
+            _ptr(row_start), _ptr(state_slot), _ptr(y), c_int(y.stride(0)), c_int(requests),
+            c_int(rows), c_int(chunks), c_int(heads), c_int(groups), c_int(state_size),
+            c_int(columns), _ptr(scratch[0]), _ptr(scratch[1]), _stream())  # type: ignore[index]
+        if status != -6:  # AYK_NOT_TAKEN
+            global _launches
+            _launches += 2  # the gates, the states, the outputs
+            check(status, op)
+            return
     status = library("recurrent").ayk_mamba2_scan(
         _ptr(xbc), c_int(xbc.stride(0)), _ptr(dt_raw), c_int(dt_raw.stride(0)), _ptr(dt_bias),
         _ptr(a_log), _ptr(skip), _ptr(state), c_longlong(state.stride(0)), _ptr(row_start),
@@ -1189,13 +1267,15 @@ def mamba2_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
 def mlstm_scan(proj: torch.Tensor, gate_bias: torch.Tensor | None, state: torch.Tensor,
                out: torch.Tensor, *, row_start: torch.Tensor, state_slot: torch.Tensor,
                requests: int, heads: int, dim: int, columns: int, k_offset: int, v_offset: int,
-               i_offset: int, f_offset: int, cap: float) -> None:
+               i_offset: int, f_offset: int, cap: float, host_rows: list[int] | None = None,
+               scratch: tuple[torch.Tensor, torch.Tensor] | None = None) -> None:
     """The matrix-memory recurrence over each request's rows. ``proj`` float32 rows hold the
     queries at 0, keys at ``k_offset`` (``heads * dim`` each), values at ``v_offset``
     (``heads * columns``) and the raw input and forget gates at ``i_offset`` / ``f_offset``
     (``heads`` each); ``gate_bias`` ``[2 * heads]`` (input, then forget). ``out``
     ``[N, heads * columns]`` is the memory's answer before norm and output gate. ``state``
-    ``[slots, scan_state_floats("mlstm", ...)]``."""
+    ``[slots, scan_state_floats("mlstm", ...)]``. ``host_rows`` and ``scratch`` as for
+    :func:`mamba2_scan` (3 * heads floats a row)."""
     op = "mlstm_scan"
     if _left_out and op in _left_out:
         return
@@ -1209,6 +1289,23 @@ def mlstm_scan(proj: torch.Tensor, gate_bias: torch.Tensor | None, state: torch.
                                 i_offset + heads, f_offset + heads) or \
             (gate_bias is not None and gate_bias.shape[0] != 2 * heads):
         raise BackendError(f"{op}: shapes do not fit")
+    in_chunks = _memory_scratch(op, host_rows, scratch, requests, heads, dim, columns, 3)
+    if in_chunks is not None:
+        rows, chunks = in_chunks
+        if rows > min(proj.shape[0], out.shape[0]):
+            raise BackendError(f"{op}: shapes do not fit")
+        status = library("recurrent").ayk_mlstm_chunks(
+            _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset),
+            c_int(i_offset), c_int(f_offset), _ptr(gate_bias), c_float(cap), _ptr(state),
+            c_longlong(state.stride(0)), _ptr(row_start), _ptr(state_slot), _ptr(out),
+            c_int(out.stride(0)), c_int(requests), c_int(rows), c_int(chunks), c_int(heads),
+            c_int(dim), c_int(columns), _ptr(scratch[0]),  # type: ignore[index]
+            _ptr(scratch[1]), _stream())  # type: ignore[index]
+        if status != -6:  # AYK_NOT_TAKEN
+            global _launches
+            _launches += 2  # the gates, the states, the outputs
+            check(status, op)
+            return
     status = library("recurrent").ayk_mlstm_scan(
         _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset), c_int(i_offset),
         c_int(f_offset), _ptr(gate_bias), c_float(cap), _ptr(state),
@@ -1221,13 +1318,15 @@ def mlstm_scan(proj: torch.Tensor, gate_bias: torch.Tensor | None, state: torch.
 def gla_scan(proj: torch.Tensor, decay_raw: torch.Tensor, state: torch.Tensor,
              out: torch.Tensor, *, row_start: torch.Tensor, state_slot: torch.Tensor,
              requests: int, heads: int, dim: int, columns: int, k_offset: int, v_offset: int,
-             tau: float, q_scale: float) -> None:
+             tau: float, q_scale: float, host_rows: list[int] | None = None,
+             scratch: torch.Tensor | None = None) -> None:
     """Gated linear attention with a decay per key channel over each request's rows. ``proj``
     float32 rows hold the queries at 0, keys at ``k_offset`` (``heads * dim`` each) and values
     at ``v_offset`` (``heads * columns``); ``decay_raw`` ``[N, heads * dim]`` the raw decays
     ``z``. Per head ``S <- diag(sigmoid(z)^(1/tau)) S + k v^T`` (the decay of key channel ``n``
     on row ``n`` of ``S``) and ``out = q_scale * S^T q``. ``state`` ``[slots, heads * dim *
-    columns]`` float32, a slot's ``S`` kept as ``[heads][columns][dim]``."""
+    columns]`` float32, a slot's ``S`` kept as ``[heads][columns][dim]``. With the step's
+    ``host_rows`` and ``scratch`` (float32, :func:`gla_buffers`) the rows are taken in chunks."""
     op = "gla_scan"
     if _left_out and op in _left_out:
         return
@@ -1238,6 +1337,25 @@ def gla_scan(proj: torch.Tensor, decay_raw: torch.Tensor, state: torch.Tensor,
             decay_raw.shape[1] != heads * dim or \
             proj.shape[1] < max(k_offset + heads * dim, v_offset + heads * columns):
         raise BackendError(f"{op}: shapes do not fit")
+    if host_rows is not None and scratch is not None:
+        _need(op, "scratch", scratch, torch.float32)
+        chunks = linear_chunks(host_rows)
+        floats = heads * (2 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK)
+        if not scratch.is_contiguous() or scratch.numel() < chunks * floats or \
+                len(host_rows) != requests or \
+                sum(host_rows) > min(proj.shape[0], decay_raw.shape[0], out.shape[0]):
+            raise BackendError(f"{op}: shapes do not fit")
+        status = library("linear_attention").ayk_gla_chunks(
+            _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset),
+            _ptr(decay_raw), c_int(decay_raw.stride(0)), c_float(tau), c_float(q_scale),
+            _ptr(state), c_longlong(state.stride(0)), _ptr(row_start), _ptr(state_slot),
+            _ptr(out), c_int(out.stride(0)), c_int(requests), c_int(chunks), c_int(heads),
+            c_int(dim), c_int(columns), _ptr(scratch), _stream())
+        if status != -6:  # AYK_NOT_TAKEN
+            global _launches
+            _launches += 1  # the chunks' matrices, then the scan
+            check(status, op)
+            return
     status = library("recurrent").ayk_gla_scan(
         _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset), _ptr(decay_raw),
         c_int(decay_raw.stride(0)), c_float(tau), c_float(q_scale), _ptr(state),
@@ -2188,7 +2306,7 @@ class _LinearArgs(Structure):
             "decay_at", "beta_at", "gate_at", "heads", "kv_heads", "N", "P", "taps", "channels",
             "ring_at", "decay_mode", "delta", "unit", "gate_mode", "decay_rank", "gate_rank",
             "rot_dims", "rot_layout", "requests", "chunks")] + [(name, c_float) for name in (
-                "q_scale", "k_scale", "eps", "unit_eps")]
+                "q_scale", "k_scale", "eps", "unit_eps", "inv_tau")] + [("transposed", c_int)]
 
 
 @dataclass(frozen=True, slots=True)
@@ -2351,7 +2469,8 @@ def linear_chunks(host_rows: list[int]) -> int:
 def linear_chunk_floats(shape: LinearShape) -> int:
     """Scratch floats per chunk (all heads) of :func:`linear_attention_chunks`."""
     pad = -(-shape.dim // 4) * 4
-    return shape.heads * (3 * LINEAR_CHUNK * shape.dim + pad + LINEAR_CHUNK * LINEAR_CHUNK)
+    return shape.heads * ((3 if shape.delta else 2) * LINEAR_CHUNK * shape.dim + pad
+                          + LINEAR_CHUNK * LINEAR_CHUNK)
 
 
 def linear_attention_chunks(qkv: torch.Tensor, proj: torch.Tensor, shape: LinearShape,

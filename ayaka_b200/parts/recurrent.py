@@ -17,6 +17,19 @@ from ayaka_b200.parts.spec import PartSpec
 __all__ = ["MLSTM", "DeltaRule", "GatedLinearAttention", "Mamba2"]
 
 
+def _chunks(step: StepContext, heads: int, inner: int, columns: int,
+            planes: int) -> dict[str, object]:
+    """The scan's further arguments for a step that is taken in chunks of rows (the scratch is
+    sized for the largest step)."""
+    work = step.workspace
+    sizes = ops.memory_buffers(step.host_rows, work.max_rows, heads, inner, columns)
+    if sizes is None:
+        return {}
+    return {"host_rows": step.host_rows,
+            "scratch": (work.buffer("memory.states", sizes[1], torch.float32, rows=sizes[0]),
+                        work.buffer("memory.gates", planes * heads, torch.float32))}
+
+
 @register_part("mixer", "mamba2")
 class Mamba2(Mixer):
     """Selective state-space layer (state-space duality form, scalar decay per head).
@@ -90,7 +103,8 @@ class Mamba2(Mixer):
                         self.skip, state[:, self.kept:], y, row_start=step.row_start,
                         state_slot=step.state_slot, requests=step.num_requests,
                         heads=self.num_heads, groups=self.groups, state_size=self.state,
-                        columns=self.columns)
+                        columns=self.columns,
+                        **_chunks(step, self.num_heads, self.state, self.columns, 2))
         ops.rms_norm(y, self.norm_weight, self.eps, gated, groups=self.norm_groups, count=n,
                      gate=proj[:, :inner], gate_mode="silu_before")
         ops.linear(gated, self.out_weight, None, residual, residual=True, rows=n)
@@ -150,7 +164,8 @@ class MLSTM(Mixer):
                        state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                        dim=self.dim, columns=self.columns, k_offset=self.qk,
                        v_offset=2 * self.qk, i_offset=gate_at + self.inner,
-                       f_offset=gate_at + self.inner + heads, cap=self.gate_cap)
+                       f_offset=gate_at + self.inner + heads, cap=self.gate_cap,
+                       **_chunks(step, heads, self.dim, self.columns, 3))
         # a head is a group of the norm: each divided by its own root mean square
         ops.rms_norm(answer, self.norm_weight, self.eps, gated, groups=heads, count=n,
                      gate=proj[:, gate_at:gate_at + self.inner], gate_mode="sigmoid_after")
@@ -225,10 +240,14 @@ class GatedLinearAttention(Mixer):
         ops.linear(hidden, self.proj_weight, None, proj, rows=n)
         ops.linear(hidden, self.decay_down, None, low, rows=n)
         ops.linear(low, self.decay_up, self.decay_bias, decay, rows=n)
+        sizes = ops.gla_buffers(step.host_rows, work.max_rows, heads, self.dim)
+        chunks: dict[str, object] = {} if sizes is None else {
+            "host_rows": step.host_rows,
+            "scratch": work.buffer("gla.chunks", sizes[1], torch.float32, rows=sizes[0])}
         ops.gla_scan(proj, decay, state, answer, row_start=step.row_start,
                      state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                      dim=self.dim, columns=self.columns, k_offset=self.qk, v_offset=2 * self.qk,
-                     tau=self.tau, q_scale=self.dim ** -0.5)
+                     tau=self.tau, q_scale=self.dim ** -0.5, **chunks)
         # a head is a group of the norm; the weight's `columns` entries repeat for every head
         ops.rms_norm(answer, self.norm_weight, self.eps, gated, groups=heads, count=n,
                      gate=proj[:, 2 * self.qk + self.inner:], gate_mode="silu_after")
