@@ -19,6 +19,7 @@
 // front of the next sublayer may leave the same launch.
 // Everything in fp32, rounded once to the output type. Any width.
 #include "common.cuh"
+#include "row_pieces.cuh"
 
 namespace ayk {
 
@@ -103,6 +104,71 @@ __global__ void rms_norm_kernel(const float* __restrict__ x, int ld_x,
       v *= z * sigmoid_f(z);
     }
     stf(dst + c, v);
+  }
+}
+
+// The same for groups of whole pieces that a CTA's registers hold, without a weight's period.
+// Measured on a B200, 4,024 rows of 2,048 with a gate in front: 67 -> 18 microseconds.
+template <typename TOut>
+__global__ void __launch_bounds__(512)
+rms_norm_pieces_kernel(const float* __restrict__ x, int ld_x, const int* __restrict__ rows,
+                       const float* __restrict__ weight, float weight_offset, float eps,
+                       int group_width, const float* __restrict__ gate, int ld_gate, int gate_mode,
+                       TOut* __restrict__ out, int ld_out) {
+  __shared__ float scratch[33];
+  pdl_launch_dependents();
+  const int r = blockIdx.x, pieces = group_width / 4;
+  const size_t first = (size_t)blockIdx.y * group_width;
+  const int row = rows != nullptr ? rows[r] : r;
+  float4 ws[ROW_PIECES], xs[ROW_PIECES], zs[ROW_PIECES];
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    ws[i] = weight != nullptr ? offset_piece(weight + first, weight_offset,
+                                             threadIdx.x + i * blockDim.x, pieces)
+                              : make_float4(1.f, 1.f, 1.f, 1.f);
+  }
+  pdl_wait_for(x, gate);
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    xs[i] = row_piece(x + (size_t)row * ld_x + first, c, pieces);
+    if (gate_mode != GATE_NONE) {
+      zs[i] = row_piece(gate + (size_t)row * ld_gate + first, c, pieces);
+    }
+  }
+  if (gate_mode != GATE_NONE) {  // the gate's factor
+    const bool silu = gate_mode != GATE_SIGMOID_AFTER;
+#pragma unroll
+    for (int i = 0; i < ROW_PIECES; ++i) {
+      zs[i].x = (silu ? zs[i].x : 1.f) * sigmoid_f(zs[i].x);
+      zs[i].y = (silu ? zs[i].y : 1.f) * sigmoid_f(zs[i].y);
+      zs[i].z = (silu ? zs[i].z : 1.f) * sigmoid_f(zs[i].z);
+      zs[i].w = (silu ? zs[i].w : 1.f) * sigmoid_f(zs[i].w);
+    }
+  }
+  auto times_gate = [&](int i) {
+    xs[i].x *= zs[i].x;
+    xs[i].y *= zs[i].y;
+    xs[i].z *= zs[i].z;
+    xs[i].w *= zs[i].w;
+  };
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    if (gate_mode == GATE_SILU_BEFORE) times_gate(i);
+    s += square_sum(xs[i]);
+  }
+  const float inv = 1.f / sqrtf(block_sum(s, scratch) / (float)group_width + eps);
+  TOut* dst = out + (size_t)r * ld_out + first;
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    xs[i].x = xs[i].x * inv * ws[i].x;
+    xs[i].y = xs[i].y * inv * ws[i].y;
+    xs[i].z = xs[i].z * inv * ws[i].z;
+    xs[i].w = xs[i].w * inv * ws[i].w;
+    if (gate_mode > GATE_SILU_BEFORE) times_gate(i);
+    if (c < pieces) put_piece(dst, c, xs[i]);
   }
 }
 
@@ -194,6 +260,14 @@ int rms_norm(const float* x, int ld_x, const int* rows, const float* weight, flo
     if (group_width <= 128) AYK_NORM_GROUPS(4);
     AYK_NORM_GROUPS(8);
 #undef AYK_NORM_GROUPS
+  }
+  const int by_piece = row_threads(group_width);
+  if (by_piece && weight_period == 0 && row_takes(x, ld_x, group_width, 4) &&
+      row_takes(weight, 0, group_width, 4) && row_takes(gate, ld_gate, group_width, 4) &&
+      row_takes(out, ld_out, group_width, sizeof(TOut))) {
+    return launch_kernel(rms_norm_pieces_kernel<TOut>, dim3(n, groups), dim3(by_piece), 0, stream, 1,
+                         x, ld_x, rows, weight, weight_offset, eps, group_width, gate, ld_gate,
+                         gate_mode, (TOut*)out, ld_out);
   }
   const int threads = group_width >= 2048 ? 512 : (group_width >= 512 ? 256 : 128);
   return launch_kernel(rms_norm_kernel<TOut>, dim3(n, groups), dim3(threads), 0, stream, 1, x,
@@ -326,6 +400,56 @@ __global__ void norm_sum_kernel(Branches in, int count, float eps, float factor,
   }
 }
 
+// norm_sum_kernel for two sides and rows of whole pieces. Measured on a B200, 4,096 rows of 2,048 with
+// the next norm: 113 -> 27 microseconds (168 MB are 26).
+template <typename TOut>
+__global__ void __launch_bounds__(512)
+norm_sum_pieces_kernel(Branches in, float eps, float factor, const float* __restrict__ scale,
+                       float* __restrict__ dst, int ld_dst, int width, int accumulate,
+                       const float* __restrict__ next_weight, float next_offset, float next_eps,
+                       TOut* __restrict__ next_out, int ld_next) {
+  __shared__ float scratch[33], other[33];
+  pdl_launch_dependents();
+  const int r = blockIdx.x, pieces = width / 4;
+  pdl_wait_for(dst, in.x[0], in.x[1]);
+  float4 xs[2][ROW_PIECES], ds[ROW_PIECES];
+  float* to = dst + (size_t)r * ld_dst;
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    xs[0][i] = row_piece(in.x[0] + (size_t)r * in.ld[0], c, pieces);
+    xs[1][i] = row_piece(in.x[1] + (size_t)r * in.ld[1], c, pieces);
+    ds[i] = accumulate ? row_piece(to, c, pieces) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    s0 += square_sum(xs[0][i]);
+    s1 += square_sum(xs[1][i]);
+  }
+  const float inv0 = factor / sqrtf(block_sum(s0, scratch) / (float)width + eps);
+  const float inv1 = factor / sqrtf(block_sum(s1, other) / (float)width + eps);
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < pieces) {
+      const float4 a = row_piece(in.weight[0], c, pieces), b = row_piece(in.weight[1], c, pieces);
+      const float4 f = scale != nullptr ? row_piece(scale, c, pieces)
+                                        : make_float4(1.f, 1.f, 1.f, 1.f);
+      ds[i].x += f.x * (xs[0][i].x * inv0 * a.x + xs[1][i].x * inv1 * b.x);
+      ds[i].y += f.y * (xs[0][i].y * inv0 * a.y + xs[1][i].y * inv1 * b.y);
+      ds[i].z += f.z * (xs[0][i].z * inv0 * a.z + xs[1][i].z * inv1 * b.z);
+      ds[i].w += f.w * (xs[0][i].w * inv0 * a.w + xs[1][i].w * inv1 * b.w);
+      put_piece(to, c, ds[i]);
+      s2 += square_sum(ds[i]);
+    }
+  }
+  if (next_out != nullptr) {
+    next_norm(ds, s2, scratch, width, next_weight, next_offset, next_eps,
+              next_out + (size_t)r * ld_next);
+  }
+}
+
 // dst[r][c] += factor * x[r][c] * rsqrt(mean_c(x[r]^2) + eps) * (offset + w[c]), and, when
 // `copy` is given, copy[r][c] = the new dst[r][c] in the compute type: a sublayer's normed
 // result joins the fp32 residual stream and the next sublayer's input leaves the same pass.
@@ -427,6 +551,65 @@ __global__ void norm_add_kernel(const float* __restrict__ x, int ld_x, float x_f
   }
 }
 
+// norm_add_kernel for rows of whole pieces. Measured on a B200, 4,096 rows of 2,048 with a bfloat16
+// copy: 38 -> 16 microseconds (117 MB are 18).
+template <typename TOut>
+__global__ void __launch_bounds__(512)
+norm_add_pieces_kernel(const float* __restrict__ x, int ld_x, float x_factor,
+                       const float* __restrict__ other, int ld_other, float other_factor,
+                       const float* __restrict__ weight, float offset, float eps, float factor,
+                       float* __restrict__ dst, int ld_dst, TOut* __restrict__ copy, int ld_copy,
+                       int width, const float* __restrict__ next_weight, float next_offset,
+                       float next_eps, TOut* __restrict__ next_out, int ld_next) {
+  __shared__ float scratch[33];
+  pdl_launch_dependents();
+  const int r = blockIdx.x, pieces = width / 4;
+  float4 ws[ROW_PIECES], xs[ROW_PIECES], ds[ROW_PIECES];
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    ws[i] = offset_piece(weight, offset, threadIdx.x + i * blockDim.x, pieces);
+  }
+  pdl_wait_for(x, dst, other);
+  float* to = dst + (size_t)r * ld_dst;
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    xs[i] = row_piece(x + (size_t)r * ld_x, c, pieces);
+    ds[i] = row_piece(to, c, pieces);
+  }
+  if (other != nullptr) {
+#pragma unroll
+    for (int i = 0; i < ROW_PIECES; ++i) {
+      const float4 o = row_piece(other + (size_t)r * ld_other, threadIdx.x + i * blockDim.x, pieces);
+      xs[i].x = xs[i].x * x_factor + o.x * other_factor;
+      xs[i].y = xs[i].y * x_factor + o.y * other_factor;
+      xs[i].z = xs[i].z * x_factor + o.z * other_factor;
+      xs[i].w = xs[i].w * x_factor + o.w * other_factor;
+    }
+  }
+  float s = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) s += square_sum(xs[i]);
+  const float inv = factor / sqrtf(block_sum(s, scratch) / (float)width + eps);
+#pragma unroll
+  for (int i = 0; i < ROW_PIECES; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c < pieces) {
+      ds[i].x += xs[i].x * inv * ws[i].x;
+      ds[i].y += xs[i].y * inv * ws[i].y;
+      ds[i].z += xs[i].z * inv * ws[i].z;
+      ds[i].w += xs[i].w * inv * ws[i].w;
+      put_piece(to, c, ds[i]);
+      if (copy != nullptr) put_piece(copy + (size_t)r * ld_copy, c, ds[i]);
+      s2 += square_sum(ds[i]);
+    }
+  }
+  if (next_out != nullptr) {
+    next_norm(ds, s2, scratch, width, next_weight, next_offset, next_eps,
+              next_out + (size_t)r * ld_next);
+  }
+}
+
 }  // namespace ayk
 
 AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
@@ -473,6 +656,22 @@ AYK_API int ayk_norm_sum(const float* const* x, const int* ld, const float* cons
     in.weight[b] = weight[b];
     in.ld[b] = ld[b];
   }
+  const int by_piece = row_threads(width);
+  if (count == 2 && by_piece && row_takes(x[0], ld[0], width, 4) && row_takes(x[1], ld[1], width, 4) &&
+      row_takes(weight[0], 0, width, 4) && row_takes(weight[1], 0, width, 4) &&
+      row_takes(scale, 0, width, 4) && row_takes(dst, ld_dst, width, 4) &&
+      row_takes(next_weight, 0, width, 4) &&
+      row_takes(next_out, ld_next, width, next_type == 1 ? 2 : 4)) {
+    if (next_out != nullptr && next_type == 1) {
+      return launch_kernel(norm_sum_pieces_kernel<__nv_bfloat16>, dim3(n), dim3(by_piece), 0,
+                           (cudaStream_t)stream, 1, in, eps, factor, scale, dst, ld_dst, width,
+                           accumulate, next_weight, next_offset, next_eps,
+                           (__nv_bfloat16*)next_out, ld_next);
+    }
+    return launch_kernel(norm_sum_pieces_kernel<float>, dim3(n), dim3(by_piece), 0,
+                         (cudaStream_t)stream, 1, in, eps, factor, scale, dst, ld_dst, width,
+                         accumulate, next_weight, next_offset, next_eps, (float*)next_out, ld_next);
+  }
   const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
   if (next_out != nullptr && next_type == 1) {
     return launch_kernel(norm_sum_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0,
@@ -515,8 +714,25 @@ AYK_API int ayk_norm_add_next(const float* x, int ld_x, float x_factor, const fl
                                !(next_eps > 0.f)))) {
     return AYK_BAD_ARGUMENT;
   }
-  const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
   const bool typed = copy != nullptr || next_out != nullptr;
+  const int by_piece = row_threads(width), size = typed && copy_type == 1 ? 2 : 4;
+  if (by_piece && (!typed || copy_type == 0 || copy_type == 1) && row_takes(x, ld_x, width, 4) &&
+      row_takes(other, ld_other, width, 4) && row_takes(weight, 0, width, 4) &&
+      row_takes(dst, ld_dst, width, 4) && row_takes(copy, ld_copy, width, size) &&
+      row_takes(next_weight, 0, width, 4) && row_takes(next_out, ld_next, width, size)) {
+    if (size == 2) {
+      return launch_kernel(norm_add_pieces_kernel<__nv_bfloat16>, dim3(n), dim3(by_piece), 0,
+                           (cudaStream_t)stream, 1, x, ld_x, x_factor, other, ld_other,
+                           other_factor, weight, offset, eps, factor, dst, ld_dst,
+                           (__nv_bfloat16*)copy, ld_copy, width, next_weight, next_offset, next_eps,
+                           (__nv_bfloat16*)next_out, ld_next);
+    }
+    return launch_kernel(norm_add_pieces_kernel<float>, dim3(n), dim3(by_piece), 0,
+                         (cudaStream_t)stream, 1, x, ld_x, x_factor, other, ld_other, other_factor,
+                         weight, offset, eps, factor, dst, ld_dst, (float*)copy, ld_copy, width,
+                         next_weight, next_offset, next_eps, (float*)next_out, ld_next);
+  }
+  const int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
   if (typed && copy_type == 1) {
     return launch_kernel(norm_add_kernel<__nv_bfloat16>, dim3(n), dim3(threads), 0,
                          (cudaStream_t)stream, 1, x, ld_x, x_factor, other, ld_other,
