@@ -177,11 +177,19 @@ class CacheStorage:
         return out
 
     def zero_state_rows(self, rows: list[int]) -> None:
-        if not rows:
-            return
+        # Runs of neighbouring rows, each one fill. (Indexing with the list would send it to the
+        # device from pageable memory, which waits for everything queued so far: the host then
+        # prepares and launches a step while the device has nothing to do.)
+        runs: list[list[int]] = []
+        for row in sorted(rows):
+            if runs and row <= runs[-1][1]:
+                runs[-1][1] = max(runs[-1][1], row + 1)
+            else:
+                runs.append([row, row + 1])
         for state in self.states:
             if state is not None:
-                state[rows] = 0
+                for first, end in runs:
+                    state[first:end].zero_()
 
     def nbytes(self) -> int:
         pooled = [t for pair in self.pooled if pair is not None for t in pair]
