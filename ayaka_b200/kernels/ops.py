@@ -483,8 +483,10 @@ def attention_prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
 
     Request ``b`` owns rows ``row_start[b] .. row_start[b + 1]`` of ``q`` and ``out``, which
     are the last rows of its ``kv_len[b]`` cached tokens; ``host_rows`` is the host copy of
-    the row counts (the grid is sized from it). Head size 64 runs on tcgen05; the other head
-    sizes on a warp-level kernel compiled for the head size (``kernel`` forces one of them).
+    the row counts (the grid is sized from it). Head size 64 runs on tcgen05; so do, with
+    ``keep_first``, ``gate`` and ``sink`` or without, head size 128 and latent rows of 256 entries
+    (``v_pages`` is ``k_pages``); the rest on a warp-level kernel compiled for the head size
+    (``kernel``: ``"tcgen05"``, ``"wide"`` or ``"mma"`` forces one of them where it serves the case).
     The warp-level kernel also takes value rows of another size than key rows (``v_pages``'
     last dimension), ``keep_first`` (with a window: keys before that position stay visible)
     and ``gate`` (float32 ``[N, num_heads * value size]``: the result times its sigmoid);
@@ -538,10 +540,35 @@ def attention_prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         raise BackendError(f"{op}: slopes do not go with pooled rows, a sigmoid not with a sink")
     plain = value_dim == head_dim and gate is None and not (keep_first and window) and \
         not pooled and sink is None and not mode
-    # the tcgen05 kernel works on tiles of 256 rows: a step of short portions only is better
-    # served by the warp-level kernel's tiles of 64
-    which = kernel or (PREFILL_ATTENTION if head_dim == 64 and scale > 0 and plain
-                       and max(host_rows, default=0) >= 256 else "mma")
+    # the tcgen05 kernels work on tiles of 256 and 128 rows: a step of short portions only is better
+    # served by the warp-level kernel's tiles of 64 (mma against wide, 16 heads: 128 rows of head
+    # size 128 16.4 against 14.3 us, 64 rows 14.3 against 12.3; latent rows 22.5 against 16.4, and
+    # twelve requests of 60 20.5 against 25.4; head size 64 with a gate, 128 rows 16.4 against
+    # 18.4, 300 rows 23.3 against 20.5)
+    longest = max(host_rows, default=0)
+    if kernel is not None:
+        which = kernel
+    elif PREFILL_ATTENTION != "tcgen05" or scale <= 0:
+        which = "mma"
+    elif head_dim == 64 and plain:
+        which = "tcgen05" if longest >= 256 else "mma"
+    else:
+        which = "wide" if longest >= (256 if head_dim == 64 else 128) else "mma"
+    if which == "wide" and not pooled and not mode and value_dim == head_dim:
+        lib = library("attention_prefill_wide")
+        tile_rows = lib.ayk_attention_prefill_wide_rows()
+        tiles = sum(-(-rows // tile_rows) for rows in host_rows)
+        status = lib.ayk_attention_prefill_wide(
+            _ptr(q), c_int(q.stride(0)), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+            c_int(block_table.stride(0)), _ptr(row_start), _ptr(kv_len), _ptr(out),
+            c_int(out.stride(0)), c_int(count), c_int(q.shape[0]), c_int(tiles), c_int(num_heads),
+            c_int(kv_heads), c_int(head_dim), c_int(page_size), c_int(k_pages.shape[0]),
+            c_float(scale), c_int(window), c_int(keep_first), _ptr(gate),
+            c_int(0 if gate is None else gate.stride(0)), _ptr(sink),
+            _ptr(_status_word(q.device)), _stream())
+        if status != -6:  # AYK_NOT_TAKEN
+            check(status, op)
+            return
     if which == "tcgen05":
         if head_dim != 64 or not plain:
             raise BackendError(f"{op}: the tcgen05 kernel serves a softmax of head size 64 without "
