@@ -1,0 +1,45 @@
+"""The float32 attention of 32 rows a block against the rows one by one."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dim", [8, 40, 64, 128])
+@pytest.mark.parametrize("rows,lengths,window", [
+    ([333, 180], [333, 180], 0),                     # a block of two requests
+    ([200], [500], 77),
+    ([1, 70, 3, 40, 1, 90], [9, 70, 64, 400, 1, 91], 33),
+    ([1] * 150 + [64], [5 + i for i in range(150)] + [200], 0),  # blocks of single rows
+])
+def test_float32_attention_in_blocks(rows, lengths, window, dim):
+    """Bit for bit what the same rows give a few at a time."""
+    from ayaka_b200.kernels import ops
+
+    heads, kv_heads, page = 4, 2, 16
+    g = torch.Generator("cuda").manual_seed(dim + len(rows))
+    pages = [-(-length // page) for length in lengths]
+    shape = (sum(pages) + 1, kv_heads, page, dim)
+    k, v = (torch.randn(shape, generator=g, device="cuda") for _ in range(2))
+    table = torch.zeros(len(rows), max(pages), dtype=torch.int32, device="cuda")
+    at = 1
+    for b, count in enumerate(pages):
+        table[b, :count] = torch.arange(at, at + count)
+        at += count
+    req = torch.cat([torch.full((n,), b) for b, n in enumerate(rows)]).int().cuda()
+    pos = torch.cat([torch.arange(length - n, length)
+                     for n, length in zip(rows, lengths)]).int().cuda()
+    req[sum(rows) // 2] = -1  # a padding row
+    total = sum(rows)
+    assert total > 192
+    q = torch.randn(total, heads * dim, generator=g, device="cuda")
+    whole, parts = torch.full_like(q, 3.0), torch.full_like(q, 5.0)
+    ops.attention(q, k, v, table, req, pos, whole, num_heads=heads, scale=dim ** -0.5, window=window)
+    for lo in range(0, total, 50):
+        part = slice(lo, min(total, lo + 50))
+        ops.attention(q[part], k, v, table, req[part], pos[part], parts[part], num_heads=heads,
+                      scale=dim ** -0.5, window=window)
+    assert torch.equal(whole, parts)
