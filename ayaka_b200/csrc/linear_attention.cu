@@ -26,6 +26,15 @@
 // with Kt = G k, Qt = G q, R = B T, Kh = T^T (D_(C-1) k) is all the scan computes. Decays only
 // ever appear as products of factors in [0, 1] (never as quotients), so nothing overflows and a
 // channel that forgets at once is exact. A chunk's missing rows have k = q = 0, beta = 0, g = 1.
+//
+// The generalised delta rule of csrc/recurrent.cu, S_t = (diag(w) - (a u) u^T) S_(t-1) + k v^T with the
+// unit key u, takes the same scan: what row i removes along is x_i = u_i . S_(i-1), so with
+// D_ij = w_(j+1) ... w_i and D'_ij = w_(j+1) ... w_(i-1)
+//   X = T (Ut S_0 + Lk V),   T = (I + La)^-1,  Lk_ij = u_i . (D'_ij k_j),  La_ij = u_i . (D'_ij a_j u_j)
+//   O = Rt S_0 + Mk V - Ma X,                  Mk_ij = r_i . (D_ij k_j),   Ma_ij = r_i . (D_ij a_j u_j)
+//   S_C = G S_0 + Kh^T V - Ah^T X,
+// and with X = U' S_0 + T' V folded in (U' = T Ut, T' = T Lk) the scan computes W = -U' S_0,
+//   O = (Rt - Ma U') S_0 + (Mk - Ma T') V,   S_C = G S_0 + (Kh - T'^T Ah)^T V + Ah^T W.
 #include <type_traits>
 
 #include "common.cuh"
@@ -185,10 +194,12 @@ la_conv_kernel(const float* __restrict__ in, int ld_in, const float* __restrict_
 
 // ---------------------------------------------------------------------------------------------
 // A chunk's matrices in the scratch, per (chunk, head): M [N][2 C] (Kt of the C rows, then Qt; Qt
-// alone, [N][C], without the delta rule), Kh [N][C], G [N] (padded to a multiple of 4), R [C][C].
+// alone, [N][C], without the delta rule), Kh [N][C], (MODE_GENERAL: Ah [N][C],) G [N] (padded to a
+// multiple of 4), R [C][C].
+enum ScanMode : int { MODE_PLAIN = 0, MODE_DELTA = 1, MODE_GENERAL = 2 };
 __host__ __device__ __forceinline__ int la_pad4(int n) { return (n + 3) & ~3; }
-__host__ __device__ __forceinline__ int la_chunk_floats(int N, bool delta) {
-  return (delta ? 3 : 2) * LA_C * N + la_pad4(N) + LA_C * LA_C;
+__host__ __device__ __forceinline__ int la_chunk_floats(int N, int mode) {
+  return (2 + mode) * LA_C * N + la_pad4(N) + LA_C * LA_C;
 }
 
 // The request that owns chunk `index` of the step and the chunk's first row in it.
@@ -325,7 +336,7 @@ la_prepare_kernel(const LinearArgs a) {
     }
   }
   __syncthreads();
-  float* chunk = scratch + ((size_t)blockIdx.x * a.heads + h) * la_chunk_floats(N, a.delta);
+  float* chunk = scratch + ((size_t)blockIdx.x * a.heads + h) * la_chunk_floats(N, a.delta ? MODE_DELTA : MODE_PLAIN);
   float* m_out = chunk;
   float* kh_out = m_out + (a.delta ? 2 : 1) * LA_C * N;
   float* g_out = kh_out + LA_C * N;
@@ -440,6 +451,215 @@ la_prepare_kernel(const LinearArgs a) {
   }
 }
 
+// The chunk matrices of the generalised delta rule (see the head of this file), laid out for the scan.
+// grid (chunks, heads). Shared memory: u (then Ut), r (then Rt), k (then Kh), a u (then Ah) and w
+// (then U') as [C][NS].
+struct GeneralArgs {
+  const float* proj;    // r at 0, k at k_at, raw rates at a_at (heads x N each)
+  const float* z;       // raw decays, heads x N a row
+  const float* a_bias;  // heads x N
+  const int* row_start;
+  float* scratch;
+  int ld_proj, ld_z, k_at, a_at, requests, heads, N;
+  float decay_rate;
+};
+
+template <int M>  // ceil(N / 64)
+__global__ void __launch_bounds__(LA_THREADS)
+general_prepare_kernel(const GeneralArgs a) {
+  extern __shared__ __align__(16) float la_smem[];
+  __shared__ __align__(16) float Lk[LA_C][LA_C], La[LA_C][LA_C], Mk[LA_C][LA_C], Ma[LA_C][LA_C];
+  __shared__ __align__(16) float T[LA_C][LA_C], Tk[LA_C][LA_C];
+  const int N = a.N, NS = la_pad4(N), h = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* u_s = la_smem;
+  float* r_s = u_s + LA_C * NS;
+  float* k_s = r_s + LA_C * NS;
+  float* au_s = k_s + LA_C * NS;
+  float* g_s = au_s + LA_C * NS;
+  int b, t0, count;
+  const bool found = la_find_chunk(a.row_start, a.requests, blockIdx.x, b, t0, count);
+  const float* proj = a.proj;
+  const float* z = a.z;
+  float* scratch = a.scratch;
+  pdl_wait_for(proj, z, scratch);
+  if (!found) return;
+  const int r0 = a.row_start[b] + t0;
+  if (tid < LA_C * LA_C) {
+    Lk[tid / LA_C][tid % LA_C] = La[tid / LA_C][tid % LA_C] = 0.f;
+    Mk[tid / LA_C][tid % LA_C] = Ma[tid / LA_C][tid % LA_C] = 0.f;
+  }
+  for (int i = warp; i < LA_C; i += LA_THREADS / 32) {  // a warp per row
+    const bool row = i < count;
+    const float* src = proj + (size_t)(r0 + i) * a.ld_proj + (size_t)h * N;
+    float kk = 0.f;
+    for (int n = lane; n < NS; n += 32) {
+      const float k = row && n < N ? src[a.k_at + n] : 0.f;
+      k_s[i * NS + n] = k;
+      kk = fmaf(k, k, kk);
+    }
+    const float inv = 1.f / sqrtf(warp_sum(kk) + 1e-6f);
+    for (int n = lane; n < NS; n += 32) {
+      const bool live = row && n < N;
+      const float u = k_s[i * NS + n] * inv;
+      u_s[i * NS + n] = u;
+      r_s[i * NS + n] = live ? src[n] : 0.f;
+      au_s[i * NS + n] = live ? u * la_sigmoid(src[a.a_at + n] + a.a_bias[h * N + n]) : 0.f;
+      g_s[i * NS + n] =
+          live ? expf(-a.decay_rate * la_sigmoid(z[(size_t)(r0 + i) * a.ld_z + h * N + n])) : 1.f;
+    }
+  }
+  __syncthreads();
+  {  // the four matrices: warp w takes columns w and C - 1 - w, half a warp each, four neighbouring
+     // channels a lane at a time; what a column's row carries (k_j and a_j u_j, faded) ends as Kh, Ah
+    const int half = lane >> 4, l = lane & 15, j = half ? LA_C - 1 - warp : warp;
+    float4 dk[M], da[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int n = 4 * (l + 16 * m);
+      dk[m] = n < NS ? *reinterpret_cast<const float4*>(k_s + j * NS + n)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
+      da[m] = n < NS ? *reinterpret_cast<const float4*>(au_s + j * NS + n)
+                     : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int i = warp; i < LA_C; ++i) {  // (warp: the smaller of the two columns)
+      float lk = 0.f, la = 0.f, mk = 0.f, ma = 0.f;
+      if (i >= j) {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          const int n = 4 * (l + 16 * m);
+          if (n < NS) {
+            if (i > j) {
+              const float4 u = *reinterpret_cast<const float4*>(u_s + i * NS + n);
+              const float4 g = *reinterpret_cast<const float4*>(g_s + i * NS + n);
+              lk = fmaf(u.x, dk[m].x, fmaf(u.y, dk[m].y, fmaf(u.z, dk[m].z, fmaf(u.w, dk[m].w, lk))));
+              la = fmaf(u.x, da[m].x, fmaf(u.y, da[m].y, fmaf(u.z, da[m].z, fmaf(u.w, da[m].w, la))));
+              dk[m] = make_float4(dk[m].x * g.x, dk[m].y * g.y, dk[m].z * g.z, dk[m].w * g.w);
+              da[m] = make_float4(da[m].x * g.x, da[m].y * g.y, da[m].z * g.z, da[m].w * g.w);
+            }
+            const float4 r = *reinterpret_cast<const float4*>(r_s + i * NS + n);
+            mk = fmaf(r.x, dk[m].x, fmaf(r.y, dk[m].y, fmaf(r.z, dk[m].z, fmaf(r.w, dk[m].w, mk))));
+            ma = fmaf(r.x, da[m].x, fmaf(r.y, da[m].y, fmaf(r.z, da[m].z, fmaf(r.w, da[m].w, ma))));
+          }
+        }
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        lk += __shfl_xor_sync(0xffffffffu, lk, o);
+        la += __shfl_xor_sync(0xffffffffu, la, o);
+        mk += __shfl_xor_sync(0xffffffffu, mk, o);
+        ma += __shfl_xor_sync(0xffffffffu, ma, o);
+      }
+      if (l == 0 && i >= j) {
+        Lk[i][j] = lk;
+        La[i][j] = la;
+        Mk[i][j] = mk;
+        Ma[i][j] = ma;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {  // (nobody else reads these rows)
+      const int n = 4 * (l + 16 * m);
+      if (n < NS) {
+        *reinterpret_cast<float4*>(k_s + j * NS + n) = dk[m];
+        *reinterpret_cast<float4*>(au_s + j * NS + n) = da[m];
+      }
+    }
+  }
+  __syncthreads();
+  float* m_out = scratch + ((size_t)blockIdx.x * a.heads + h) * la_chunk_floats(N, MODE_GENERAL);
+  float* kh_out = m_out + 2 * LA_C * N;
+  float* ah_out = kh_out + LA_C * N;
+  float* g_out = ah_out + LA_C * N;
+  float* r_out = g_out + la_pad4(N);
+  if (warp == 0) {
+    if (lane < LA_C) {  // column `lane` of T, from the top
+      float x[LA_C];
+#pragma unroll
+      for (int i = 0; i < LA_C; ++i) {
+        float s = i == lane ? 1.f : 0.f;
+#pragma unroll
+        for (int m = 0; m < i; ++m) s = fmaf(-La[i][m], x[m], s);
+        x[i] = s;
+        T[i][lane] = s;
+      }
+    }
+  } else {  // meanwhile Ut, Rt and G, a channel a thread
+    for (int n = tid - 32; n < N; n += LA_THREADS - 32) {
+      float g = 1.f;
+      for (int i = 0; i < LA_C; ++i) {
+        u_s[i * NS + n] *= g;
+        g *= g_s[i * NS + n];
+        r_s[i * NS + n] *= g;
+      }
+      g_out[n] = g;
+    }
+  }
+  __syncthreads();
+  if (tid < LA_C * LA_C) {
+    const int i = tid / LA_C, j = tid % LA_C;
+    float s = 0.f;
+#pragma unroll
+    for (int m = 0; m < LA_C; ++m) s = fmaf(T[i][m], Lk[m][j], s);
+    Tk[i][j] = s;
+  }
+  // U' = T Ut into the space of the decays (no longer needed). A thread takes eight rows of a channel,
+  // a warp 32 channels of the same rows: no bank conflicts, and the small matrices are broadcast.
+  for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
+    const int n = idx % N, first = idx / N * 8;
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = 0.f;
+#pragma unroll 4
+    for (int m = 0; m < LA_C; ++m) {  // (T is zero above the diagonal)
+      const float u = u_s[m * NS + n];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] = fmaf(T[first + e][m], u, s[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) g_s[(first + e) * NS + n] = s[e];
+  }
+  __syncthreads();
+  if (tid < LA_C * LA_C) {
+    const int i = tid / LA_C, j = tid % LA_C;
+    float s = Mk[i][j];
+#pragma unroll
+    for (int m = 0; m < LA_C; ++m) s = fmaf(-Ma[i][m], Tk[m][j], s);
+    r_out[tid] = s;
+  }
+  for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
+    const int n = idx % N, first = idx / N * 8;
+    float q[8], kh[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      q[e] = r_s[(first + e) * NS + n];
+      kh[e] = k_s[(first + e) * NS + n];
+    }
+#pragma unroll 4
+    for (int m = 0; m < LA_C; ++m) {
+      const float u = g_s[m * NS + n], d = au_s[m * NS + n];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        q[e] = fmaf(-Ma[first + e][m], u, q[e]);
+        kh[e] = fmaf(-Tk[m][first + e], d, kh[e]);
+      }
+    }
+    float* m_row = m_out + (size_t)n * 2 * LA_C + first;
+#pragma unroll
+    for (int e = 0; e < 8; e += 4) {  // (32 bytes at a time: whole sectors)
+      *reinterpret_cast<float4*>(m_row + e) =
+          make_float4(g_s[(first + e) * NS + n], g_s[(first + e + 1) * NS + n],
+                      g_s[(first + e + 2) * NS + n], g_s[(first + e + 3) * NS + n]);
+      *reinterpret_cast<float4*>(m_row + LA_C + e) = make_float4(q[e], q[e + 1], q[e + 2], q[e + 3]);
+      *reinterpret_cast<float4*>(kh_out + (size_t)n * LA_C + first + e) =
+          make_float4(kh[e], kh[e + 1], kh[e + 2], kh[e + 3]);
+      *reinterpret_cast<float4*>(ah_out + (size_t)n * LA_C + first + e) =
+          make_float4(au_s[(first + e) * NS + n], au_s[(first + e + 1) * NS + n],
+                      au_s[(first + e + 2) * NS + n], au_s[(first + e + 3) * NS + n]);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void la_copy16(float* dst, const float* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -455,8 +675,8 @@ template <int N> __device__ __forceinline__ void la_wait() {
 }
 
 // floats of one stage (a chunk's matrices and its values) and of the rest of shared memory
-__host__ __device__ __forceinline__ int la_stage_floats(int N, bool delta) {
-  return la_chunk_floats(N, delta) + LA_C * LA_COLS;
+__host__ __device__ __forceinline__ int la_stage_floats(int N, int mode) {
+  return la_chunk_floats(N, mode) + LA_C * LA_COLS;
 }
 __host__ __device__ __forceinline__ int la_fixed_floats(int N) {
   return N * LA_COLS + 8 * 2 * LA_C * LA_COLS + LA_C * LA_COLS;
@@ -466,14 +686,15 @@ __host__ __device__ __forceinline__ int la_fixed_floats(int N) {
 // shared out over the eight warps (a warp's lanes hold 4 x 4 pieces of the 32 x 16 result), the
 // warps' shares added up, W; then O and the new state from W. Without the delta rule there is no
 // Kt and W is V: half a warp holds the 16 x 16 result, the halves share out the channels too.
-template <int STAGES, bool DELTA>
+template <int STAGES, int MODE>
 __global__ void __launch_bounds__(LA_THREADS)
 la_scan_kernel(const LinearArgs a, int vec) {
   extern __shared__ __align__(16) float la_smem[];
   pdl_launch_dependents();
   const int N = a.N, P = a.P, h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * LA_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int stage_floats = la_stage_floats(N, DELTA), chunk_floats = la_chunk_floats(N, DELTA);
+  constexpr bool DELTA = MODE != MODE_PLAIN;
+  const int stage_floats = la_stage_floats(N, MODE), chunk_floats = la_chunk_floats(N, MODE);
   float* s_s = la_smem + (size_t)STAGES * stage_floats;  // [N][LA_COLS]
   float* red = s_s + N * LA_COLS;                        // [8 warps][4][32 lanes][4]
   float* w_s = red + 8 * 2 * LA_C * LA_COLS;             // [C][LA_COLS]
@@ -550,10 +771,11 @@ la_scan_kernel(const LinearArgs a, int vec) {
     }
     const float* m_s = la_smem + (size_t)(STAGES == 1 ? 0 : c % STAGES) * stage_floats;
     const float* kh_s = m_s + (DELTA ? 2 : 1) * LA_C * N;
-    const float* g_s = kh_s + LA_C * N;
+    const float* ah_s = kh_s + LA_C * N;
+    const float* g_s = ah_s + (MODE == MODE_GENERAL ? LA_C * N : 0);
     const float* r_s = g_s + la_pad4(N);
     const float* v_s = m_s + chunk_floats;
-    const float* used_s = DELTA ? w_s : v_s;  // W
+    const float* used_s = MODE == MODE_DELTA ? w_s : v_s;
     float acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -584,7 +806,8 @@ la_scan_kernel(const LinearArgs a, int vec) {
         seen += red[w * 512 + red_at];
         o += red[w * 512 + red_at + 64];  // the same place of the rows of Qt (16 rows on)
       }
-      w_s[row * LA_COLS + col] = v_s[row * LA_COLS + col] - seen;
+      w_s[row * LA_COLS + col] =
+          MODE == MODE_DELTA ? v_s[row * LA_COLS + col] - seen : -seen;
       __syncthreads();
     } else {
 #pragma unroll
@@ -650,6 +873,29 @@ la_scan_kernel(const LinearArgs a, int vec) {
             s[i].y = fmaf(kv[i][e], w.y, s[i].y);
             s[i].z = fmaf(kv[i][e], w.z, s[i].z);
             s[i].w = fmaf(kv[i][e], w.w, s[i].w);
+          }
+        }
+        if (MODE == MODE_GENERAL) {
+          float av[CH][4];
+#pragma unroll
+          for (int i = 0; i < CH; ++i) {
+            const int n = (first >> 2) + i * (LA_THREADS / 4);
+            const float4 a4 = *reinterpret_cast<const float4*>(ah_s + n * LA_C + j);
+            av[i][0] = a4.x;
+            av[i][1] = a4.y;
+            av[i][2] = a4.z;
+            av[i][3] = a4.w;
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float4 w = *reinterpret_cast<const float4*>(w_s + (j + e) * LA_COLS + cq);
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+              s[i].x = fmaf(av[i][e], w.x, s[i].x);
+              s[i].y = fmaf(av[i][e], w.y, s[i].y);
+              s[i].z = fmaf(av[i][e], w.z, s[i].z);
+              s[i].w = fmaf(av[i][e], w.w, s[i].w);
+            }
           }
         }
       }
@@ -963,6 +1209,8 @@ static bool la_common_ok(const LinearArgs& a) {
          a.state_stride >= (long long)a.heads * a.N * a.P;
 }
 
+static int la_scan(const LinearArgs& a, int mode, cudaStream_t s);
+
 // Prepare and scan; everything but the scratch's alignment and the sizes has been checked.
 static int la_chunks(const LinearArgs& a, cudaStream_t s) {
   if (((uintptr_t)a.scratch % 16) != 0) return AYK_BAD_ALIGNMENT;
@@ -995,24 +1243,31 @@ static int la_chunks(const LinearArgs& a, cudaStream_t s) {
 #undef AYK_LA_PREPARE
 #undef AYK_LA_PREPARE_AS
   if (status != AYK_OK) return status;
+  return la_scan(a, a.delta ? MODE_DELTA : MODE_PLAIN, s);
+}
+
+// The scan over the chunks' matrices.
+static int la_scan(const LinearArgs& a, int mode, cudaStream_t s) {
+  const int tiles = (a.P + LA_COLS - 1) / LA_COLS;
   const int vec = ((uintptr_t)a.in % 16) == 0 && a.ld_in % 4 == 0 && a.v_at % 4 == 0 &&
                   a.P % 4 == 0;
   const dim3 grid(a.heads, a.requests, tiles);
-#define AYK_LA_SCAN_AS(STAGES, DELTA)                                                            \
+#define AYK_LA_SCAN_AS(STAGES, MODE)                                                             \
   {                                                                                              \
     static const bool allowed =                                                                  \
-        (cudaFuncSetAttribute(la_scan_kernel<STAGES, DELTA>,                                     \
+        (cudaFuncSetAttribute(la_scan_kernel<STAGES, MODE>,                                      \
                               cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024), true);   \
     (void)allowed;                                                                               \
-    return launch_kernel(la_scan_kernel<STAGES, DELTA>, grid, dim3(LA_THREADS),                  \
-                         ((size_t)STAGES * la_stage_floats(a.N, DELTA) + la_fixed_floats(a.N)) * \
+    return launch_kernel(la_scan_kernel<STAGES, MODE>, grid, dim3(LA_THREADS),                   \
+                         ((size_t)STAGES * la_stage_floats(a.N, MODE) + la_fixed_floats(a.N)) *  \
                              sizeof(float),                                                      \
                          s, 1, a, vec);                                                          \
   }
 #define AYK_LA_SCAN(STAGES)                                                                      \
   {                                                                                              \
-    if (a.delta) AYK_LA_SCAN_AS(STAGES, true)                                                    \
-    AYK_LA_SCAN_AS(STAGES, false)                                                                \
+    if (mode == MODE_GENERAL) AYK_LA_SCAN_AS(STAGES, MODE_GENERAL)                               \
+    if (mode == MODE_DELTA) AYK_LA_SCAN_AS(STAGES, MODE_DELTA)                                   \
+    AYK_LA_SCAN_AS(STAGES, MODE_PLAIN)                                                           \
   }
   if (a.N <= 128) AYK_LA_SCAN(3)
   if (a.N <= 320) AYK_LA_SCAN(2)
@@ -1028,7 +1283,9 @@ AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
 AYK_API int ayk_linear_chunk_rows() { return ayk::LA_C; }
 AYK_API int ayk_linear_args_bytes() { return (int)sizeof(ayk::LinearArgs); }
 // floats of the scratch per (chunk, head)
-AYK_API int ayk_linear_chunk_floats(int n, int delta) { return ayk::la_chunk_floats(n, delta != 0); }
+AYK_API int ayk_linear_chunk_floats(int n, int delta) {
+  return ayk::la_chunk_floats(n, delta ? ayk::MODE_DELTA : ayk::MODE_PLAIN);
+}
 
 // `ring`: the first float of slot 0's ring; slots are state_stride floats apart.
 AYK_API int ayk_conv_ring(const float* in, int ld_in, const float* w, float* ring,
@@ -1119,6 +1376,61 @@ AYK_API int ayk_gla_chunks(const float* proj, int ld_proj, int k_offset, int v_o
   a.inv_tau = 1.f / tau;
   a.transposed = 1;
   return la_chunks(a, (cudaStream_t)stream);
+}
+
+// The generalised delta rule of csrc/recurrent.cu in chunks; its operands as there, S as [head][P][N];
+// the scratch holds chunks * heads * ayk_delta_chunk_floats(N) floats. AYK_NOT_TAKEN: more than
+// LA_GENERAL_N key channels or a scratch that does not start on 16 bytes; nothing ran.
+constexpr int LA_GENERAL_N = 256;
+AYK_API int ayk_delta_chunk_floats(int n) { return ayk::la_chunk_floats(n, ayk::MODE_GENERAL); }
+AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v_offset,
+                             int a_offset, const float* a_bias, const float* z, int ld_z,
+                             float decay_rate, float* state, long long state_stride,
+                             const int* row_start, const int* state_slot, float* out, int ld_out,
+                             int requests, int chunks, int heads, int N, int P, float* scratch,
+                             void* stream) {
+  using namespace ayk;
+  if (requests == 0 || chunks == 0) return AYK_OK;
+  if (requests < 0 || chunks < 0 || heads < 1 || N < 1 || P < 1 || proj == nullptr || z == nullptr ||
+      a_bias == nullptr || state == nullptr || row_start == nullptr || state_slot == nullptr ||
+      out == nullptr || scratch == nullptr || !(decay_rate >= 0.f) || ld_out < heads * P ||
+      ld_z < heads * N || k_offset < 0 || v_offset < 0 || a_offset < 0 ||
+      ld_proj < max(max(k_offset, a_offset) + heads * N, v_offset + heads * P) ||
+      state_stride < (long long)heads * N * P) {
+    return AYK_BAD_ARGUMENT;
+  }
+  if (heads > 65535 || requests > 65535 || (P + LA_COLS - 1) / LA_COLS > 65535) return AYK_TOO_LARGE;
+  if (N > LA_GENERAL_N || ((uintptr_t)scratch % 16) != 0) return AYK_NOT_TAKEN;
+  const GeneralArgs g = {proj,    z,    a_bias,   row_start, scratch, ld_proj,
+                         ld_z,    k_offset, a_offset, requests,  heads,   N,
+                         decay_rate};
+  const size_t smem = (size_t)5 * LA_C * la_pad4(N) * sizeof(float);
+  cudaStream_t s = (cudaStream_t)stream;
+  int status;
+#define AYK_GENERAL(M)                                                                             {                                                                                                  static const cudaError_t allowed =                                                                   cudaFuncSetAttribute(general_prepare_kernel<M>,                                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,                                                     5 * LA_C * 64 * M * (int)sizeof(float));                                if (allowed != cudaSuccess) return (int)allowed;                                                 status = launch_kernel(general_prepare_kernel<M>, dim3(chunks, heads), dim3(LA_THREADS),                                smem, s, 1, g);                                                         }
+  if (N <= 64) AYK_GENERAL(1)
+  else if (N <= 128) AYK_GENERAL(2)
+  else AYK_GENERAL(4)
+#undef AYK_GENERAL
+  if (status != AYK_OK) return status;
+  LinearArgs a = {};
+  a.in = proj;
+  a.row_start = row_start;
+  a.state_slot = state_slot;
+  a.state = state;
+  a.scratch = scratch;
+  a.out = out;
+  a.state_stride = state_stride;
+  a.ld_in = ld_proj;
+  a.ld_out = ld_out;
+  a.v_at = v_offset;
+  a.heads = a.kv_heads = heads;
+  a.N = N;
+  a.P = P;
+  a.requests = requests;
+  a.chunks = chunks;
+  a.transposed = 1;
+  return la_scan(a, MODE_GENERAL, s);
 }
 
 // A step of single rows, row r of request r: one launch. type: 0 = float32, 1 = bfloat16, of

@@ -327,10 +327,15 @@ class DeltaRule(Mixer):
         ops.linear(hidden, self.proj_weight, None, proj, rows=n)
         ops.unary_rows(proj[:, self.low_at:], low, activation="tanh", rows=n)
         ops.linear(low, self.decay_up, self.decay_bias, decay, rows=n)
+        sizes = ops.delta_buffers(step.host_rows, work.max_rows, heads, self.dim)
+        chunks: dict[str, object] = {} if sizes is None else {
+            "host_rows": step.host_rows,
+            "scratch": work.buffer("delta.chunks", sizes[1], torch.float32, rows=sizes[0])}
         ops.delta_scan(proj, decay, self.rate_bias, state, answer, row_start=step.row_start,
                        state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                        dim=self.dim, columns=self.columns, k_offset=self.k_at,
-                       v_offset=self.v_at, a_offset=self.a_at, decay_rate=self.decay_rate)
+                       v_offset=self.v_at, a_offset=self.a_at, decay_rate=self.decay_rate,
+                       **chunks)
         # a head is a group of the norm: each divided by its own root mean square
         ops.rms_norm(answer, self.norm_weight, self.eps, gated, groups=heads, count=n,
                      gate=proj[:, self.g_at:self.g_at + self.inner], gate_mode="sigmoid_after")

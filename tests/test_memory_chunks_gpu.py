@@ -1,4 +1,4 @@
-"""Mamba-2, mLSTM and gated linear attention taken in chunks of rows against the recurrences in float64: several requests
+"""Mamba-2, mLSTM, gated linear attention and the generalised delta rule taken in chunks of rows against the recurrences in float64: several requests
 of any length in one step, states that go on from one, sizes with remainders of every tile."""
 
 from __future__ import annotations
@@ -47,7 +47,8 @@ def _close(got, want, tolerance=TOLERANCE):
 
 @pytest.mark.parametrize("rows", ROWS)
 @pytest.mark.parametrize("heads,groups,inner,columns", [(4, 2, 16, 16), (2, 1, 132, 68),
-                                                        (3, 3, 64, 64), (2, 2, 40, 128)])
+                                                        (3, 3, 64, 64), (2, 2, 40, 128),
+                                                        (150, 50, 20, 12)])
 def test_mamba2_in_chunks(heads, groups, inner, columns, rows):
     from ayaka_b200.kernels import ops
 
@@ -77,7 +78,8 @@ def test_mamba2_in_chunks(heads, groups, inner, columns, rows):
 
 
 @pytest.mark.parametrize("rows", ROWS)
-@pytest.mark.parametrize("heads,inner,columns", [(3, 16, 20), (2, 132, 68), (1, 256, 128)])
+@pytest.mark.parametrize("heads,inner,columns", [(3, 16, 20), (2, 132, 68), (1, 256, 128),
+                                                 (150, 20, 12)])
 def test_mlstm_in_chunks(heads, inner, columns, rows):
     from ayaka_b200.kernels import ops
 
@@ -173,6 +175,47 @@ def test_gated_linear_attention_in_chunks(heads, inner, columns, rows):
     before = ops.launch_count()
     ops.gla_scan(proj, z, state, out, heads=heads, dim=inner, columns=columns, k_offset=qk,
                  v_offset=2 * qk, tau=4.0, q_scale=inner ** -0.5, scratch=scratch, **_step(rows))
+    assert ops.launch_count() - before == 2  # not row by row
+    _close(out, want.flatten(1))
+    _close(state, wide.flatten(1))
+
+
+@pytest.mark.parametrize("rows", ROWS)
+@pytest.mark.parametrize("heads,inner,columns", [(3, 16, 20), (2, 130, 33), (2, 64, 64),
+                                                 (2, 65, 7), (1, 256, 40)])
+def test_generalised_delta_rule_in_chunks(heads, inner, columns, rows):
+    from ayaka_b200.kernels import ops
+
+    g = torch.Generator("cuda").manual_seed(inner + sum(rows))
+    total, qk, width = sum(rows), heads * inner, heads * columns
+    proj = torch.randn(total, 3 * qk + width + 3, generator=g, device="cuda")
+    proj[5] = 0.0  # a key of length nothing
+    z = 3.0 * torch.randn(total, qk, generator=g, device="cuda")
+    bias = torch.randn(qk, generator=g, device="cuda")
+    state = torch.randn(len(rows) + 1, heads * inner * columns, generator=g, device="cuda")
+    wide = state.double().view(-1, heads, columns, inner)
+    r, k, y = (proj[:, i * qk:(i + 1) * qk].double().reshape(total, heads, inner) for i in range(3))
+    v = proj[:, 3 * qk:3 * qk + width].double().reshape(total, heads, columns)
+    w = torch.exp(-0.6065 * torch.sigmoid(z.double())).view(total, heads, inner)
+    u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    au = torch.sigmoid(y + bias.double().view(heads, inner)) * u
+    want, first = torch.zeros_like(v), 0
+    for b, count in enumerate(rows):
+        S = wide[len(rows) - b]
+        for t in range(first, first + count):
+            seen = (S @ u[t, :, :, None])[..., 0]
+            S = w[t, :, None, :] * S - seen[:, :, None] * au[t, :, None, :] + \
+                v[t, :, :, None] * k[t, :, None, :]
+            want[t] = (S @ r[t, :, :, None])[..., 0]
+        wide[len(rows) - b] = S
+        first += count
+    floats = heads * (64 * inner + -(-inner // 4) * 4 + 256)
+    scratch = torch.full((ops.linear_chunks(rows), floats), float("nan"), device="cuda")
+    out = torch.zeros(total, width, device="cuda")
+    before = ops.launch_count()
+    ops.delta_scan(proj, z, bias, state, out, heads=heads, dim=inner, columns=columns, k_offset=qk,
+                   a_offset=2 * qk, v_offset=3 * qk, decay_rate=0.6065, scratch=scratch,
+                   **_step(rows))
     assert ops.launch_count() - before == 2  # not row by row
     _close(out, want.flatten(1))
     _close(state, wide.flatten(1))
