@@ -1911,6 +1911,25 @@ def delta_scan(proj: torch.Tensor, decay: torch.Tensor, rate_bias: torch.Tensor,
             out.shape[1] < heads * columns or state.shape[1] < heads * dim * columns or \
             row_start.shape[0] < requests + 1 or state_slot.shape[0] < requests:
         raise BackendError(f"{op}: shapes do not fit")
+    if host_rows is not None and scratch is not None:
+        _need(op, "scratch", scratch, torch.float32)
+        chunks = linear_chunks(host_rows)
+        if not scratch.is_contiguous() or len(host_rows) != requests or \
+                scratch.numel() < chunks * heads * _delta_floats(dim) or \
+                sum(host_rows) > min(proj.shape[0], decay.shape[0], out.shape[0]):
+            raise BackendError(f"{op}: shapes do not fit")
+        status = library("linear_attention").ayk_delta_chunks(
+            _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset),
+            c_int(a_offset), _ptr(rate_bias), _ptr(decay), c_int(decay.stride(0)),
+            c_float(decay_rate), _ptr(state), c_longlong(state.stride(0)), _ptr(row_start),
+            _ptr(state_slot), _ptr(out), c_int(out.stride(0)), c_int(requests), c_int(chunks),
+            c_int(heads), c_int(dim), c_int(columns), _ptr(scratch), _stream())
+        if status != -6:  # AYK_NOT_TAKEN
+            global _launches
+            _launches += 1  # the chunks' matrices, then the scan
+            check(status, op)
+            return
+        _nothing_ran()
     status = library("recurrent").ayk_delta_scan(
         _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset), c_int(a_offset),
         _ptr(rate_bias), _ptr(decay), c_int(decay.stride(0)), c_float(decay_rate), _ptr(state),
@@ -1938,25 +1957,6 @@ def pooled_prepare(proj: torch.Tensor, *, k_offset: int, q_weight: torch.Tensor 
         return
     _need(op, "proj", proj, torch.float32, 2)
     _need(op, "q", q, ndim=2)
-    if host_rows is not None and scratch is not None:
-        _need(op, "scratch", scratch, torch.float32)
-        chunks = linear_chunks(host_rows)
-        if not scratch.is_contiguous() or len(host_rows) != requests or \
-                scratch.numel() < chunks * heads * _delta_floats(dim) or \
-                sum(host_rows) > min(proj.shape[0], decay.shape[0], out.shape[0]):
-            raise BackendError(f"{op}: shapes do not fit")
-        status = library("linear_attention").ayk_delta_chunks(
-            _ptr(proj), c_int(proj.stride(0)), c_int(k_offset), c_int(v_offset),
-            c_int(a_offset), _ptr(rate_bias), _ptr(decay), c_int(decay.stride(0)),
-            c_float(decay_rate), _ptr(state), c_longlong(state.stride(0)), _ptr(row_start),
-            _ptr(state_slot), _ptr(out), c_int(out.stride(0)), c_int(requests), c_int(chunks),
-            c_int(heads), c_int(dim), c_int(columns), _ptr(scratch), _stream())
-        if status != -6:  # AYK_NOT_TAKEN
-            global _launches
-            _launches += 1  # the chunks' matrices, then the scan
-            check(status, op)
-            return
-        _nothing_ran()
     _need(op, "positions", positions, torch.int32, 1)
     if q.dtype not in _TYPE or rows > proj.shape[0] or rows > q.shape[0] or \
             rows > positions.shape[0] or q.shape[1] != heads * dim or \
