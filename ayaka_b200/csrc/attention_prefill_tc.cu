@@ -307,6 +307,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k,
         }
       } while (j <= jhi && !active(g, j));
     };
+    // Only a stage that the producer fills again is handed back: nobody waits for the last ones, and
+    // an arrival of theirs could come when the CTA has left and the next one owns the memory.
+    auto hand_back = [&](uint64_t* empty, int jj) {
+      if (jj + FA_STAGES < num_blocks) umma_commit(&empty[jj % FA_STAGES]);
+    };
 
     if (warp >= FA_FIRST_PRODUCER) {
       // ---- producers: all of them bring Q; then the first FA_PRODUCERS warps bring the K
@@ -458,7 +463,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k,
                      umma_desc_k128(k_tile, k * 32), idesc_s, k != 0);
           }
           umma_commit(&s_full[slot]);
-          if (sg == 1 || !active(1, sj)) umma_commit(&k_empty[stage]);  // the block's last reader
+          if (sg == 1 || !active(1, sj)) hand_back(k_empty, jj);  // the block's last reader
           ++si;
           advance(sg, sj);
         }
@@ -489,7 +494,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k,
                      umma_desc_mn128(v_tile + k * 16 * 128), idesc_o, (npv[pg] | k) != 0);
           }
           umma_commit(&pv_done[slot]);
-          if (pg == 1 || !active(1, pj)) umma_commit(&v_empty[stage]);
+          if (pg == 1 || !active(1, pj)) hand_back(v_empty, jj);
           ++npv[pg];
           ++pi;
           advance(pg, pj);

@@ -264,6 +264,12 @@ attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q,
         constexpr uint32_t idesc_o = umma_idesc_bf16(FW_BM, 64) | (1u << 16);  // B: MN-major
         const uint8_t* q_s = smem + L::Q;
         const uint8_t* p_s = smem + L::P;
+        const int places = SAME ? turns : 2 * turns;
+        // Only a place that the producer fills again is handed back: nobody waits for the last ones,
+        // and an arrival of theirs could come when the CTA has left and the next one owns the memory.
+        auto hand_back = [&](int n) {
+          if (n + E < places) umma_commit(&empty[n % E]);
+        };
         bool ok = mbar_wait(q_full, 0);
         auto scores = [&](int i) {
           const int n = k_place(i), s = n % E;
@@ -280,7 +286,7 @@ attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q,
             }
           }
           umma_commit(&s_full[i & 1]);
-          if (!SAME) umma_commit(&empty[s]);
+          if (!SAME) hand_back(n);
           return true;
         };
         if (ok) ok = scores(0);
@@ -303,7 +309,7 @@ attention_prefill_wide_kernel(const __grid_constant__ CUtensorMap map_q,
             }
           }
           umma_commit(pv_done);
-          umma_commit(&empty[s]);
+          hand_back(n);
         }
         if (!ok) *failed = 1;
       }

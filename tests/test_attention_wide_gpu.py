@@ -120,3 +120,41 @@ def test_far_references():
             torch.ones(n, n, device="cuda").triu(1).bool(), -math.inf)
         want = torch.softmax(s, 1) @ v.double()
         assert (out.double() - want).norm() <= 2.0 ** -7 * want.norm()
+
+
+@pytest.mark.parametrize("kernel,dim", [("wide", 64), ("wide", 128), ("wide", 256),
+                                        ("tcgen05", 64)])
+def test_short_walks_one_after_another(kernel, dim):
+    """Walks of one block up to two rings of blocks, in many more CTAs than fit at one time, so that a
+    CTA's shared memory is the next one's as soon as it has left: the bits of a launch alone."""
+    from ayaka_b200.kernels import gemm_tc, ops
+
+    page, heads = 64, 16
+    latent = dim == 256
+    kv_heads = 1 if latent else heads
+    rows = [2 + 67 * b for b in range(8)] * 6
+    g = torch.Generator("cuda").manual_seed(dim)
+    randn = lambda *shape: torch.randn(*shape, generator=g, device="cuda").bfloat16()  # noqa: E731
+    counts = [-(-n // page) for n in rows]
+    table = torch.zeros(len(rows), max(counts), dtype=torch.int32, device="cuda")
+    at = 1
+    for b, count in enumerate(counts):
+        table[b, :count] = torch.arange(at, at + count)
+        at += count
+    k_pages = randn(at, kv_heads, page, dim)
+    v_pages = k_pages if latent else randn(at, kv_heads, page, dim)
+    q = randn(sum(rows), heads * dim)
+
+    def run(first, last):
+        own = slice(sum(rows[:first]), sum(rows[:last]))
+        out = torch.zeros_like(q[own])
+        lengths = torch.tensor(rows[first:last]).int().cuda()
+        starts = torch.tensor([0, *rows[first:last]]).cumsum(0).int().cuda()
+        ops.attention_prefill(q[own], k_pages, v_pages, table[first:last], starts, lengths, out,
+                              num_heads=heads, scale=dim ** -0.5, host_rows=rows[first:last],
+                              kernel=kernel)
+        gemm_tc.check_status(out.device)
+        return out
+
+    whole = run(0, len(rows))
+    assert torch.equal(whole, torch.cat([run(b, b + 1) for b in range(len(rows))]))
