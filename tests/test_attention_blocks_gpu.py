@@ -43,3 +43,39 @@ def test_float32_attention_in_blocks(rows, lengths, window, dim):
         ops.attention(q[part], k, v, table, req[part], pos[part], parts[part], num_heads=heads,
                       scale=dim ** -0.5, window=window)
     assert torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("order", ["descending", "every second", "twice", "any", "stretches"])
+@pytest.mark.parametrize("window", [0, 50])
+def test_rows_at_any_positions(order, window, dtype):
+    """A request's rows need not be neighbours in the order of their positions: every row against
+    float64, and bit for bit what it gives alone."""
+    from ayaka_b200.kernels import ops
+
+    heads, kv_heads, page, dim, length, n = 2, 1, 16, 40, 256, 250
+    g = torch.Generator("cuda").manual_seed(5)
+    k, v = (torch.randn(length // page + 1, kv_heads, page, dim, generator=g, device="cuda").to(dtype)
+            for _ in range(2))
+    table = torch.arange(1, length // page + 1, dtype=torch.int32, device="cuda").view(1, -1)
+    at = torch.arange(n, device="cuda")
+    pos = {"descending": n - 1 - at, "every second": 2 * at % length, "twice": at // 2,
+           "any": torch.randint(0, length, (n,), generator=g, device="cuda"),
+           "stretches": at % 11 + 16 * (at // 11 % 15)}[order].int()
+    req = torch.zeros(n, dtype=torch.int32, device="cuda")
+    q = torch.randn(n, heads * dim, generator=g, device="cuda").to(dtype)
+    whole, alone = torch.full_like(q, 3.0), torch.full_like(q, 5.0)
+    ops.attention(q, k, v, table, req, pos, whole, num_heads=heads, scale=dim ** -0.5, window=window)
+    for i in range(n):
+        one = slice(i, i + 1)
+        ops.attention(q[one], k, v, table, req[one], pos[one], alone[one], num_heads=heads,
+                      scale=dim ** -0.5, window=window)
+    assert torch.equal(whole, alone)
+    keys, values = (x[1:].reshape(length, dim).double() for x in (k, v))
+    key, last = torch.arange(length, device="cuda"), pos[:, None]
+    seen = (key <= last) & ((key > last - window) | (window == 0))
+    s = q.double().view(n, heads, dim) @ keys.T * dim ** -0.5
+    want = torch.softmax(s.masked_fill(~seen[:, None], -torch.inf), -1) @ values
+    # fp32 sums of up to 256 terms, or one rounding to bfloat16
+    tolerance = 2e-6 if dtype == torch.float32 else 2.0 ** -8
+    assert (whole.double().view_as(want) - want).norm() <= tolerance * want.norm()
