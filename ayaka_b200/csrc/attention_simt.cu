@@ -19,9 +19,14 @@ namespace ayk {
 
 constexpr int ATT_WARPS = 4;
 constexpr int ATT_MAX_HD = 256;
-// A step of more rows than this brings prompt portions as a rule; of fewer, the rows one by one are
-// more warps at work (a decode step of so many requests would be four rows a warp).
+// Blocks of 32 rows serve steps of more than ATT_ROWS_FROM rows (of fewer, the rows one by one are more
+// warps at work) that bring at least ATT_ROWS_A_REQUEST rows a request: of fewer, 32 rows are more
+// stretches than a block shares and are taken one by one, for which the kernel of rows has room for
+// more warps. 256 single rows behind 300 keys, 12 heads of 64 and 16 of 128: blocks 117 and 388
+// microseconds, rows 137 and 285; a portion of 200 rows behind 32 single ones 84 and 197 against 123
+// and 254.
 constexpr int ATT_ROWS_FROM = 192;
+constexpr int ATT_ROWS_A_REQUEST = 6;
 
 template <typename T> struct Vec8;
 template <> struct Vec8<float> {
@@ -153,7 +158,11 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
 // attend_row: the results are the same bits. Rows that are not a few stretches of neighbouring
 // positions (of several requests, or asked for in any other order) are taken one by one.
 // Measured on a B200, GPT-2 small's 12 heads of 64, prompts of 333 and 180: 111 -> 61 microseconds.
+// ATT_TILE_PARTS CTAs a block: where its rows are taken one by one each has a warp for every row of its
+// part (one CTA for all 32 walked four rows a warp: 32 single rows and a portion of 200, 12 heads of 64,
+// 240 microseconds where this takes 84), else the first one works for all.
 constexpr int ATT_TILE_WARPS = 8, ATT_TILE_ROWS = 32;
+constexpr int ATT_TILE_PARTS = ATT_TILE_ROWS / ATT_TILE_WARPS;
 constexpr int ATT_TILE_STRETCHES = 4;  // of more stretches the 32 rows are taken one by one
 template <typename T, int NI>  // ceil(head_dim / 32)
 __global__ void __launch_bounds__(ATT_TILE_WARPS * 32)
@@ -173,7 +182,8 @@ attention_simt_tile_kernel(const T* __restrict__ q, int ld_q, const T* __restric
   pdl_wait_for(q, k_pages, v_pages);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = blockIdx.y;
   // the last rows first: they see the most keys
-  const int tile0 = (int)(gridDim.x - 1 - blockIdx.x) * ATT_TILE_ROWS;
+  const int tile0 = (int)(gridDim.x / ATT_TILE_PARTS - 1 - blockIdx.x / ATT_TILE_PARTS) * ATT_TILE_ROWS;
+  const int part = blockIdx.x % ATT_TILE_PARTS;
   const int all = min(ATT_TILE_ROWS, num_rows - tile0);
   // where a row does not follow the row before it at the next position of the same request (bit r:
   // row r)
@@ -185,15 +195,16 @@ attention_simt_tile_kernel(const T* __restrict__ q, int ld_q, const T* __restric
       0xffffffffu,
       lane < all && (lane == 0 || own != ahead || own < 0 || place != place_ahead + 1));
   if (__popc(starts) > ATT_TILE_STRETCHES) {
-    for (int r = warp; r < all; r += ATT_TILE_WARPS) {
+    const int r = part * ATT_TILE_WARPS + warp;
+    if (r < all) {
       attend_row(q, ld_q, k_pages, v_pages, block_table, table_stride, request_of_row, positions,
                  out, ld_out, tile0 + r, head, num_kv_heads, group, head_dim, page_size, scale,
                  window, q_s + warp * head_dim, &p_s[warp][0][0],
                  reinterpret_cast<long long*>(&p_s[warp][8][0]));
-      __syncwarp();
     }
     return;
   }
+  if (part != 0) return;
   for (int begin = 0; begin < all;) {  // one stretch at a time
     const uint32_t later = begin < 31 ? starts >> (begin + 1) : 0u;
     const int end = later ? begin + __ffs(later) : all;
@@ -388,7 +399,7 @@ int attention_simt(const void* q, int ld_q, const void* k_pages, const void* v_p
                    const int* block_table, int table_stride, const int* request_of_row,
                    const int* positions, void* out, int ld_out, int num_rows, int num_heads,
                    int num_kv_heads, int head_dim, int page_size, float scale, int window,
-                   cudaStream_t stream) {
+                   int requests, cudaStream_t stream) {
   if (num_rows == 0) return AYK_OK;
   if (num_rows < 0 || num_heads < 1 || num_kv_heads < 1 || num_heads % num_kv_heads ||
       page_size < 1 || table_stride < 1 || window < 0) {
@@ -398,7 +409,8 @@ int attention_simt(const void* q, int ld_q, const void* k_pages, const void* v_p
   if (head_dim > ATT_MAX_HD || num_heads > 65535) return AYK_TOO_LARGE;
   const size_t vec = 8 * sizeof(T);
   if (((uintptr_t)k_pages % vec) || ((uintptr_t)v_pages % vec)) return AYK_BAD_ALIGNMENT;
-  if (num_rows > ATT_ROWS_FROM && head_dim <= 128) {
+  const bool portions = num_rows / ATT_ROWS_A_REQUEST >= requests;
+  if (num_rows > ATT_ROWS_FROM && portions && head_dim <= 128) {
     const int ni = (head_dim + 31) / 32;
     const auto kernel = ni == 1   ? attention_simt_tile_kernel<T, 1>
                         : ni == 2 ? attention_simt_tile_kernel<T, 2>
@@ -408,7 +420,8 @@ int attention_simt(const void* q, int ld_q, const void* k_pages, const void* v_p
     const cudaError_t e =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return launch_kernel(kernel, dim3((num_rows + ATT_TILE_ROWS - 1) / ATT_TILE_ROWS, num_heads),
+    const int tiles = (num_rows + ATT_TILE_ROWS - 1) / ATT_TILE_ROWS;
+    return launch_kernel(kernel, dim3(tiles * ATT_TILE_PARTS, num_heads),
                          dim3(ATT_TILE_WARPS * 32), smem, stream, 1, (const T*)q, ld_q,
                          (const T*)k_pages, (const T*)v_pages, block_table, table_stride,
                          request_of_row, positions, (T*)out, ld_out, num_rows, num_kv_heads,
@@ -451,23 +464,24 @@ using bf16 = __nv_bfloat16;
 
 AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
 
-// type: 0 = float32, 1 = bfloat16 (queries, pages and output share it).
+// type: 0 = float32, 1 = bfloat16 (queries, pages and output share it). `requests`: rows of the block
+// table (which kernel serves the step hangs on it, no result).
 AYK_API int ayk_attention_simt(const void* q, int ld_q, const void* k_pages, const void* v_pages,
                                const int* block_table, int table_stride,
                                const int* request_of_row, const int* positions, void* out,
                                int ld_out, int num_rows, int num_heads, int num_kv_heads,
-                               int head_dim, int page_size, float scale, int window, int type,
-                               void* stream) {
+                               int head_dim, int page_size, float scale, int window,
+                               int requests, int type, void* stream) {
   if (type == 0) {
     return ayk::attention_simt<float>(q, ld_q, k_pages, v_pages, block_table, table_stride,
                                       request_of_row, positions, out, ld_out, num_rows, num_heads,
-                                      num_kv_heads, head_dim, page_size, scale, window,
+                                      num_kv_heads, head_dim, page_size, scale, window, requests,
                                       (cudaStream_t)stream);
   }
   if (type == 1) {
     return ayk::attention_simt<bf16>(q, ld_q, k_pages, v_pages, block_table, table_stride,
                                      request_of_row, positions, out, ld_out, num_rows, num_heads,
-                                     num_kv_heads, head_dim, page_size, scale, window,
+                                     num_kv_heads, head_dim, page_size, scale, window, requests,
                                      (cudaStream_t)stream);
   }
   return AYK_BAD_ARGUMENT;

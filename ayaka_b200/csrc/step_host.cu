@@ -37,7 +37,7 @@ typedef int (*AttnDecodeFn)(const void*, int, const void*, const void*, const in
                             int, void*, int);
 typedef int (*AttnSimtFn)(const void*, int, const void*, const void*, const int*, int,
                           const int*, const int*, void*, int, int, int, int, int, int, float, int,
-                          int, void*);
+                          int, int, void*);
 typedef int (*AttnPrefillFn)(const void*, int, const void*, const void*, const int*, int,
                              const int*, const int*, void*, int, int, int, int, int, int, int,
                              float, int, int, int, const float*, int, void*);
@@ -319,8 +319,8 @@ int attention_half(const AykAttentionPart* p, AykStep* step, float* residual, vo
     r = ((AttnSimtFn)k.attention_simt)(q, ld_qkv, k_pages, v_pages, g.block_table,
                                        g.table_stride, step->request_of_row, step->positions,
                                        p->attended, q_width, n, p->num_heads, p->num_kv_heads,
-                                       p->head_dim, g.page_size, p->scale, p->window, p->type,
-                                       step->stream);
+                                       p->head_dim, g.page_size, p->scale, p->window,
+                                       step->num_requests, p->type, step->stream);
   }
   if (r != AYK_OK) return r;
   return linear(k, step, p->type, p->attended, q_width, p->out_weight, q_width, p->out_bias,

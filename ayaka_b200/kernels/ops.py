@@ -466,7 +466,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                 c_int(block_table.stride(0)), _ptr(request_of_row), _ptr(positions), _ptr(out),
                 c_int(out.stride(0)), c_int(n), c_int(num_heads), c_int(kv_heads),
                 c_int(head_dim), c_int(page_size), c_float(scale), c_int(window),
-                c_int(_TYPE[q.dtype]), _stream())
+                c_int(block_table.shape[0]), c_int(_TYPE[q.dtype]), _stream())
     check(status, op)
 
 

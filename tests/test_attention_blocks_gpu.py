@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
     ([333, 180], [333, 180], 0),                     # a block of two requests
     ([200], [500], 77),
     ([1, 70, 3, 40, 1, 90], [9, 70, 64, 400, 1, 91], 33),
-    ([1] * 150 + [64], [5 + i for i in range(150)] + [200], 0),  # blocks of single rows
+    ([1] * 150 + [64], [5 + i for i in range(150)] + [200], 0),  # single rows: not in blocks
+    ([1] * 40 + [2] * 9 + [301], [5 + i for i in range(49)] + [400], 20),  # blocks of single rows
 ])
 def test_float32_attention_in_blocks(rows, lengths, window, dim):
     """Bit for bit what the same rows give a few at a time."""
