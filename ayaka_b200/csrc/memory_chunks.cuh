@@ -422,7 +422,10 @@ memory_outputs_kernel(const MemoryArgs a) {
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) m_s[(ty + 8 * i) * MC_LDA + tx + 16 * j] *= own[i][j];
+    for (int j = 0; j < 4; ++j) {
+      // (a later row's entry stays the zero it is: its product may be no number)
+      if (tx + 16 * j <= ty + 8 * i) m_s[(ty + 8 * i) * MC_LDA + tx + 16 * j] *= own[i][j];
+    }
   if (NORM) dot_s[tid] = dot;
   __syncthreads();
 #pragma unroll
@@ -443,10 +446,22 @@ memory_outputs_kernel(const MemoryArgs a) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float ae[4] = {av[i].x, av[i].y, av[i].z, av[i].w};
-      o[i][0] += dot4(ae, vv[0].x, vv[1].x, vv[2].x, vv[3].x);
-      o[i][1] += dot4(ae, vv[0].y, vv[1].y, vv[2].y, vv[3].y);
-      o[i][2] += dot4(ae, vv[0].z, vv[1].z, vv[2].z, vv[3].z);
-      o[i][3] += dot4(ae, vv[0].w, vv[1].w, vv[2].w, vv[3].w);
+      // rows j + 1 + seen .. of the chunk are later than this one: zero times what they hold would
+      // not be zero for an infinity
+      const int seen = ty + 8 * i - j;
+      if (seen >= 3) {
+        o[i][0] += dot4(ae, vv[0].x, vv[1].x, vv[2].x, vv[3].x);
+        o[i][1] += dot4(ae, vv[0].y, vv[1].y, vv[2].y, vv[3].y);
+        o[i][2] += dot4(ae, vv[0].z, vv[1].z, vv[2].z, vv[3].z);
+        o[i][3] += dot4(ae, vv[0].w, vv[1].w, vv[2].w, vv[3].w);
+      } else if (seen >= 0) {
+        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v1 = seen >= 1 ? vv[1] : none, v2 = seen >= 2 ? vv[2] : none;
+        o[i][0] += dot4(ae, vv[0].x, v1.x, v2.x, 0.f);
+        o[i][1] += dot4(ae, vv[0].y, v1.y, v2.y, 0.f);
+        o[i][2] += dot4(ae, vv[0].z, v1.z, v2.z, 0.f);
+        o[i][3] += dot4(ae, vv[0].w, v1.w, v2.w, 0.f);
+      }
     }
   }
   if (NORM) {  // the denominators: two threads a row

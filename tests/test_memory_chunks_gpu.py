@@ -219,3 +219,53 @@ def test_generalised_delta_rule_in_chunks(heads, inner, columns, rows):
     assert ops.launch_count() - before == 2  # not row by row
     _close(out, want.flatten(1))
     _close(state, wide.flatten(1))
+
+
+def _rows_before(run, operands, row, rows):
+    """``run(**operands)``: outputs of a step whose request 1 has an infinity, then a NaN, in every
+    entry of its row ``row`` of one operand after the other: the request's rows before it and the other
+    requests are what they were."""
+    first = rows[0] + row
+    clean = run(**operands)
+    for name, operand in operands.items():
+        for value in (float("inf"), -float("inf"), float("nan")):
+            bad = operand.clone()
+            bad[first] = value
+            got = run(**{**operands, name: bad})
+            assert torch.equal(got[:first], clean[:first]), (name, value)
+            assert torch.equal(got[sum(rows[:2]):], clean[sum(rows[:2]):]), (name, value)
+
+
+@pytest.mark.parametrize("row", [0, 1, 37, 63, 90])
+def test_mamba2_and_mlstm_take_no_later_row_into_an_earlier_one(row):
+    from ayaka_b200.kernels import ops
+
+    rows, heads, inner, columns = [70, 130, 66], 2, 36, 68
+    g = torch.Generator("cuda").manual_seed(row)
+    randn = lambda *shape: torch.randn(*shape, generator=g, device="cuda")  # noqa: E731
+    total, qk, width = sum(rows), heads * inner, heads * columns
+    dt_bias, a_log, skip = randn(heads), randn(heads), randn(heads)
+
+    def mamba2(x, B, C, dt):
+        y = torch.zeros(total, width, device="cuda")
+        ops.mamba2_scan(torch.cat([x, B, C], 1), dt, dt_bias, a_log, skip,
+                        torch.zeros(4, heads * inner * columns, device="cuda"), y, heads=heads,
+                        groups=heads, state_size=inner, columns=columns,
+                        scratch=_scratch(rows, heads, inner, columns, 2), **_step(rows))
+        return y
+
+    _rows_before(mamba2, dict(x=randn(total, width), B=randn(total, qk), C=randn(total, qk),
+                              dt=randn(total, heads)), row, rows)
+    floats = ops.scan_state_floats("mlstm", heads=heads, inner=inner, columns=columns)
+
+    def mlstm(q, k, v, i, f):
+        out = torch.zeros(total, width, device="cuda")
+        ops.mlstm_scan(torch.cat([q, k, v, i, f], 1), None,
+                       torch.zeros(4, floats, device="cuda"), out, heads=heads, dim=inner,
+                       columns=columns, k_offset=qk, v_offset=2 * qk, i_offset=2 * qk + width,
+                       f_offset=2 * qk + width + heads, cap=15.0,
+                       scratch=_scratch(rows, heads, inner, columns, 3), **_step(rows))
+        return out
+
+    _rows_before(mlstm, dict(q=randn(total, qk), k=randn(total, qk), v=randn(total, width),
+                             i=randn(total, heads), f=randn(total, heads)), row, rows)
