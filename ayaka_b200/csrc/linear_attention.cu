@@ -600,21 +600,31 @@ general_prepare_kernel(const GeneralArgs a) {
     const int i = tid / LA_C, j = tid % LA_C;
     float s = 0.f;
 #pragma unroll
-    for (int m = 0; m < LA_C; ++m) s = fmaf(T[i][m], Lk[m][j], s);
+    for (int m = 0; m < LA_C; ++m) {
+      if (m <= i) s = fmaf(T[i][m], Lk[m][j], s);
+    }
     Tk[i][j] = s;
   }
   // U' = T Ut into the space of the decays (no longer needed). A thread takes eight rows of a channel,
   // a warp 32 channels of the same rows: no bank conflicts, and the small matrices are broadcast.
+  // What lies above a matrix's diagonal is never multiplied: an entry of a later row may be infinite,
+  // and zero times that is not zero.
   for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
     const int n = idx % N, first = idx / N * 8;
     float s[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) s[e] = 0.f;
 #pragma unroll 4
-    for (int m = 0; m < LA_C; ++m) {  // (T is zero above the diagonal)
+    for (int m = 0; m < first; ++m) {
       const float u = u_s[m * NS + n];
 #pragma unroll
       for (int e = 0; e < 8; ++e) s[e] = fmaf(T[first + e][m], u, s[e]);
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const float u = u_s[(first + m) * NS + n];
+#pragma unroll
+      for (int e = m; e < 8; ++e) s[e] = fmaf(T[first + e][first + m], u, s[e]);
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) g_s[(first + e) * NS + n] = s[e];
@@ -624,7 +634,9 @@ general_prepare_kernel(const GeneralArgs a) {
     const int i = tid / LA_C, j = tid % LA_C;
     float s = Mk[i][j];
 #pragma unroll
-    for (int m = 0; m < LA_C; ++m) s = fmaf(-Ma[i][m], Tk[m][j], s);
+    for (int m = 0; m < LA_C; ++m) {
+      if (m <= i) s = fmaf(-Ma[i][m], Tk[m][j], s);
+    }
     r_out[tid] = s;
   }
   for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
@@ -635,14 +647,30 @@ general_prepare_kernel(const GeneralArgs a) {
       q[e] = r_s[(first + e) * NS + n];
       kh[e] = k_s[(first + e) * NS + n];
     }
+    // (Ma is zero above the diagonal, Tk on it too)
 #pragma unroll 4
-    for (int m = 0; m < LA_C; ++m) {
-      const float u = g_s[m * NS + n], d = au_s[m * NS + n];
+    for (int m = 0; m < first; ++m) {
+      const float u = g_s[m * NS + n];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[e] = fmaf(-Ma[first + e][m], u, q[e]);
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const float u = g_s[(first + m) * NS + n], d = au_s[(first + m) * NS + n];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        q[e] = fmaf(-Ma[first + e][m], u, q[e]);
-        kh[e] = fmaf(-Tk[m][first + e], d, kh[e]);
+        if (e >= m) {
+          q[e] = fmaf(-Ma[first + e][first + m], u, q[e]);
+        } else {
+          kh[e] = fmaf(-Tk[first + m][first + e], d, kh[e]);
+        }
       }
+    }
+#pragma unroll 4
+    for (int m = first + 8; m < LA_C; ++m) {
+      const float d = au_s[m * NS + n];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) kh[e] = fmaf(-Tk[m][first + e], d, kh[e]);
     }
     float* m_row = m_out + (size_t)n * 2 * LA_C + first;
 #pragma unroll
@@ -828,11 +856,12 @@ la_scan_kernel(const LinearArgs a, int vec) {
     for (int j = 0; j < LA_C; ++j) wc[j] = used_s[j * LA_COLS + col];
 #pragma unroll
     for (int j = 0; j < LA_C; j += 4) {
+      // (R is zero above the diagonal, but a later row's W may be no number)
       const float4 r = *reinterpret_cast<const float4*>(r_s + row * LA_C + j);
-      o = fmaf(r.x, wc[j], o);
-      o = fmaf(r.y, wc[j + 1], o);
-      o = fmaf(r.z, wc[j + 2], o);
-      o = fmaf(r.w, wc[j + 3], o);
+      if (j <= row) o = fmaf(r.x, wc[j], o);
+      if (j + 1 <= row) o = fmaf(r.y, wc[j + 1], o);
+      if (j + 2 <= row) o = fmaf(r.z, wc[j + 2], o);
+      if (j + 3 <= row) o = fmaf(r.w, wc[j + 3], o);
     }
     const int t = c * LA_C + row;
     if (t < rows && p0 + col < P) a.out[(size_t)(r0 + t) * a.ld_out + h * P + p0 + col] = o;

@@ -269,3 +269,37 @@ def test_mamba2_and_mlstm_take_no_later_row_into_an_earlier_one(row):
 
     _rows_before(mlstm, dict(q=randn(total, qk), k=randn(total, qk), v=randn(total, width),
                              i=randn(total, heads), f=randn(total, heads)), row, rows)
+
+
+@pytest.mark.parametrize("row", [1, 10, 15, 37, 63, 90])
+def test_gated_and_delta_scans_take_no_later_row_into_an_earlier_one(row):
+    from ayaka_b200.kernels import ops
+
+    rows, heads, inner, columns = [70, 130, 66], 2, 40, 36
+    g = torch.Generator("cuda").manual_seed(row)
+    randn = lambda *shape: torch.randn(*shape, generator=g, device="cuda")  # noqa: E731
+    total, qk, width = sum(rows), heads * inner, heads * columns
+    bias = randn(qk)
+
+    def scratch(floats):
+        return torch.full((ops.linear_chunks(rows), heads * (floats * inner + inner + 256)),
+                          float("nan"), device="cuda")
+
+    def gated(q, k, v, z):
+        out = torch.zeros(total, width, device="cuda")
+        ops.gla_scan(torch.cat([q, k, v], 1), z, torch.zeros(4, qk * columns, device="cuda"), out,
+                     heads=heads, dim=inner, columns=columns, k_offset=qk, v_offset=2 * qk, tau=4.0,
+                     q_scale=0.2, scratch=scratch(32), **_step(rows))
+        return out
+
+    def delta(r, k, y, v, z):
+        out = torch.zeros(total, width, device="cuda")
+        ops.delta_scan(torch.cat([r, k, y, v], 1), z, bias,
+                       torch.zeros(4, qk * columns, device="cuda"), out, heads=heads, dim=inner,
+                       columns=columns, k_offset=qk, a_offset=2 * qk, v_offset=3 * qk,
+                       decay_rate=0.6065, scratch=scratch(64), **_step(rows))
+        return out
+
+    operands = dict(k=randn(total, qk), v=randn(total, width), z=randn(total, qk))
+    _rows_before(gated, dict(q=randn(total, qk), **operands), row, rows)
+    _rows_before(delta, dict(r=randn(total, qk), y=randn(total, qk), **operands), row, rows)
