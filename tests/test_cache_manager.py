@@ -6,9 +6,10 @@ from __future__ import annotations
 import random
 
 import pytest
+import torch
 
 from ayaka_b200.cache.manager import CacheManager, PagePool
-from ayaka_b200.cache.storage import plan_cache
+from ayaka_b200.cache.storage import CacheStorage, plan_cache
 from ayaka_b200.errors import CapacityError, ConfigError, EngineError
 from ayaka_b200.parts.base import CacheNeed, StateNeed
 from ayaka_b200.parts.spec import Run
@@ -174,3 +175,43 @@ def test_plan_groups_runs_by_need_and_shares_read_caches():
     assert plan.bytes_per_page(0, 2, 16) == 2 * 2 * 4 * 16 * 16 * 2
     with pytest.raises(ConfigError):
         plan_cache((Run(0), Run(1, reads_cache_of=0)), [(FULL, None), (WINDOW, None)])
+
+
+class _Writes(torch.utils._python_dispatch.TorchDispatchMode):
+    """Counts the operations that write a state tensor."""
+
+    count = 0
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.count += func._schema.name in ("aten::zero_", "aten::fill_", "aten::index_fill_",
+                                            "aten::index_put_", "aten::_index_put_impl_")
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("rows", [[], [5], [3, 4, 5, 6], [6, 3, 5, 4, 4], [1, 9], [-1, 0, 7],
+                                  list(range(1, 12, 2)), list(range(12))])
+def test_fresh_state_rows_are_zeroed_and_no_others(rows, device):
+    plan = plan_cache([Run(i) for i in range(3)],
+                      [(None, StateNeed((7,))), (None, None), (None, StateNeed((2, 3)))])
+    storage = CacheStorage(plan, [], 16, 12, torch.float32, torch.device(device))
+    states = [state for state in storage.states if state is not None]
+    assert len(states) == 2
+    for state in states:
+        state.fill_(5.0)
+    if device == "cuda":  # a wait for the device would leave it without work
+        torch.cuda.set_sync_debug_mode("error")
+    try:
+        with _Writes() as writes:
+            storage.zero_state_rows(rows)
+    finally:
+        if device == "cuda":
+            torch.cuda.set_sync_debug_mode("default")
+    assert writes.count <= len(states)  # however many stretches of rows there are
+    for state in states:
+        for row in range(12):
+            assert torch.all(state[row] == (0.0 if row in rows or row - 12 in rows else 5.0))
+    for bad in (12, -13):
+        with pytest.raises(IndexError):
+            storage.zero_state_rows([0, bad])
+    assert torch.all(states[0][0] == (0.0 if 0 in rows else 5.0))
