@@ -45,18 +45,55 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 // u[t - l] is a row of this step if the request has it in this step, else one of the last
 // taps - 1 inputs kept in the request's state (conv[k] = the input taps - 1 - k rows before the
 // step's first), zeros before the sequence's start.
-// Bound by memory (every input read and every output written once): a thread takes CONV_ROWS rows of
-// a channel, so that with up to four taps an input of rows inside one request is fetched once.
-// Measured on a B200, 4,024 rows of 2,304 channels, four taps: a row a thread 99 microseconds,
-// this 25.
+// Steps of few rows or of few rows a request: a row a thread. Bound by a chain of dependent loads (which
+// request, its slot, its inputs), which a thread of several rows has as many times: conv_rows below.
+template <int TAPS>
+__global__ void causal_conv_silu_kernel(const float* __restrict__ in, int ld_in,
+                                        const float* __restrict__ w,
+                                        const float* __restrict__ bias,
+                                        const float* __restrict__ state, long long state_stride,
+                                        const int* __restrict__ request_of_row,
+                                        const int* __restrict__ row_start,
+                                        const int* __restrict__ state_slot,
+                                        float* __restrict__ out, int ld_out, int rows, int channels,
+                                        int taps) {
+  pdl_launch_dependents();
+  const int c = blockIdx.y * blockDim.x + threadIdx.x, r = blockIdx.x;
+  const int b = request_of_row[r];
+  if (c >= channels || b < 0) return;
+  const int j = r - row_start[b];
+  const float* kept = state + (size_t)state_slot[b] * state_stride;
+  float wv[TAPS];
+#pragma unroll
+  for (int l = 0; l < TAPS; ++l) wv[l] = l < taps ? w[(size_t)c * taps + taps - 1 - l] : 0.f;
+  float acc = bias != nullptr ? bias[c] : 0.f;
+  pdl_wait_for(in, kept);
+#pragma unroll
+  for (int l = 0; l < TAPS; ++l) {
+    if (l < taps) {
+      const float u = j - l >= 0 ? in[(size_t)(r - l) * ld_in + c]
+                                 : kept[(size_t)(taps - 1 + j - l) * channels + c];
+      acc = fmaf(wv[l], u, acc);
+    }
+  }
+  out[(size_t)r * ld_out + c] = silu_f(acc);
+}
+
+// Portions: bound by memory (every input read and every output written once), so a thread takes
+// CONV_ROWS rows of a channel: with up to four taps an input of rows inside one request is fetched once,
+// and a channel's weights are.
+// Measured on a B200, microseconds a step with the update of the kept inputs, by a row and by eight rows
+// a thread. 2,304 channels, four taps: 8 requests of a row 4.0 and 11.5, one of 64 rows 4.3 and 8.0,
+// of 200 rows 7.7 and 8.3, 2,324 rows of two 51 and 16; 4,352 channels, 200 rows 11.4 and 9.7; eight taps,
+// 2,324 rows 176 and 111.
 constexpr int CONV_ROWS = 8;
 template <int TAPS>
 __global__ void __launch_bounds__(128)
-causal_conv_silu_kernel(const float* __restrict__ in, int ld_in, const float* __restrict__ w,
-                        const float* __restrict__ bias, const float* __restrict__ state,
-                        long long state_stride, const int* __restrict__ request_of_row,
-                        const int* __restrict__ row_start, const int* __restrict__ state_slot,
-                        float* __restrict__ out, int ld_out, int rows, int channels, int taps) {
+causal_conv_silu_rows_kernel(const float* __restrict__ in, int ld_in, const float* __restrict__ w,
+                             const float* __restrict__ bias, const float* __restrict__ state,
+                             long long state_stride, const int* __restrict__ request_of_row,
+                             const int* __restrict__ row_start, const int* __restrict__ state_slot,
+                             float* __restrict__ out, int ld_out, int rows, int channels, int taps) {
   pdl_launch_dependents();
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= channels) return;
@@ -64,28 +101,32 @@ causal_conv_silu_kernel(const float* __restrict__ in, int ld_in, const float* __
 #pragma unroll
   for (int l = 0; l < TAPS; ++l) wv[l] = l < taps ? w[(size_t)c * taps + taps - 1 - l] : 0.f;
   const float start = bias != nullptr ? bias[c] : 0.f;
-  pdl_wait_for(in, state);
   const int first = blockIdx.x * CONV_ROWS, last = min(rows, first + CONV_ROWS);
-  if (TAPS <= 4 && last - first == CONV_ROWS) {
+  bool whole = TAPS <= 4 && last - first == CONV_ROWS;
+  if (whole) {  // rows of one request and of inputs of this step (a row of padding may lie anywhere)
     const int b = request_of_row[first];
-    if (b >= 0 && b == request_of_row[last - 1] && first - row_start[b] >= taps - 1) {
-      float u[CONV_ROWS + TAPS - 1];
+    whole = b >= 0 && first - row_start[b] >= taps - 1;
 #pragma unroll
-      for (int i = 0; i < CONV_ROWS + TAPS - 1; ++i) {
-        const int r = first + i - (TAPS - 1);
-        u[i] = r >= first - (taps - 1) ? in[(size_t)r * ld_in + c] : 0.f;
-      }
+    for (int i = 1; i < CONV_ROWS; ++i) whole &= request_of_row[first + i] == b;
+  }
+  pdl_wait_for(in, state);
+  if (whole) {
+    float u[CONV_ROWS + TAPS - 1];
 #pragma unroll
-      for (int i = 0; i < CONV_ROWS; ++i) {
-        float acc = start;
-#pragma unroll
-        for (int l = 0; l < TAPS; ++l) {
-          if (l < taps) acc = fmaf(wv[l], u[i + TAPS - 1 - l], acc);
-        }
-        out[(size_t)(first + i) * ld_out + c] = silu_f(acc);
-      }
-      return;
+    for (int i = 0; i < CONV_ROWS + TAPS - 1; ++i) {
+      const int r = first + i - (TAPS - 1);
+      u[i] = r >= first - (taps - 1) ? in[(size_t)r * ld_in + c] : 0.f;
     }
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i) {
+      float acc = start;
+#pragma unroll
+      for (int l = 0; l < TAPS; ++l) {
+        if (l < taps) acc = fmaf(wv[l], u[i + TAPS - 1 - l], acc);
+      }
+      out[(size_t)(first + i) * ld_out + c] = silu_f(acc);
+    }
+    return;
   }
   for (int r = first; r < last; ++r) {
     const int b = request_of_row[r];
@@ -103,6 +144,11 @@ causal_conv_silu_kernel(const float* __restrict__ in, int ld_in, const float* __
     }
     out[(size_t)r * ld_out + c] = silu_f(acc);
   }
+}
+// Rows a thread of the convolution takes: CONV_ROWS where most of such stretches lie inside a request and
+// the threads still fill the device (half a million entries are 3.5 warps a scheduler).
+inline int conv_rows(int rows, int requests, int channels) {
+  return rows / 16 >= requests && (long long)rows * channels >= (1 << 19) ? CONV_ROWS : 1;
 }
 
 // After the convolution has read it, the kept inputs move on: conv[k] <- the input
@@ -669,6 +715,10 @@ inline int scan_vec(const float* base, long long ld, int n, int P,
 
 AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
 
+// Rows a thread of the convolution takes in a step of these sizes.
+AYK_API int ayk_causal_conv_rows(int rows, int requests, int channels) {
+  return ayk::conv_rows(rows, requests, channels);
+}
 AYK_API int ayk_scan_columns() { return ayk::SCAN_COLS; }
 
 // `in`: the step's rows, column 0 = channel 0 (a column range of the projection output);
@@ -690,11 +740,14 @@ AYK_API int ayk_causal_conv_silu(const float* in, int ld_in, const float* w, con
   const int threads = 128, tiles = (channels + threads - 1) / threads;
   if (taps > CONV_MAX_TAPS || tiles > 65535) return AYK_TOO_LARGE;
   cudaStream_t s = (cudaStream_t)stream;
-  const int status = launch_kernel(
-      taps <= 4 ? causal_conv_silu_kernel<4> : causal_conv_silu_kernel<CONV_MAX_TAPS>,
-      dim3((rows + CONV_ROWS - 1) / CONV_ROWS, tiles), dim3(threads), 0, s, 1, in, ld_in, w, bias,
-      (const float*)state, state_stride, request_of_row, row_start, state_slot, out, ld_out, rows,
-      channels, taps);
+  const int each = conv_rows(rows, requests, channels);
+  const auto kernel =
+      each > 1 ? (taps <= 4 ? causal_conv_silu_rows_kernel<4> : causal_conv_silu_rows_kernel<CONV_MAX_TAPS>)
+               : (taps <= 4 ? causal_conv_silu_kernel<4> : causal_conv_silu_kernel<CONV_MAX_TAPS>);
+  const int status = launch_kernel(kernel, dim3((rows + each - 1) / each, tiles), dim3(threads), 0, s,
+                                   1, in, ld_in, w, bias, (const float*)state, state_stride,
+                                   request_of_row, row_start, state_slot, out, ld_out, rows, channels,
+                                   taps);
   if (status != AYK_OK || taps == 1) return status;
   return launch_kernel(conv_state_update_kernel, dim3(tiles, requests), dim3(threads), 0, s, 1,
                        in, ld_in, state, state_stride, row_start, state_slot, channels, taps);
