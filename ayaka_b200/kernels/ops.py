@@ -1193,8 +1193,8 @@ def causal_conv_silu(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor |
 
 #: rows of a chunk of the recurrences over prompt portions (``MC_ROWS`` in ``csrc/memory_chunks.cuh``)
 MEMORY_CHUNK = 64
-#: what a step may have more chunks than whole ones (requests of few rows), and the most scratch
-MEMORY_EXTRA_CHUNKS, MEMORY_MAX_FLOATS = 64, 1 << 28
+#: the most scratch floats of a step that is taken in chunks (1 GiB)
+MEMORY_MAX_FLOATS = 1 << 28
 
 
 def memory_chunks(host_rows: list[int]) -> int:
@@ -1202,49 +1202,52 @@ def memory_chunks(host_rows: list[int]) -> int:
     return sum(-(-rows // MEMORY_CHUNK) for rows in host_rows)
 
 
-def memory_buffers(host_rows: list[int], max_rows: int, heads: int, inner: int,
+def _chunk_buffers(chunks: int, floats: int) -> tuple[int, int] | None:
+    """The scratch of a step of so many chunks, by the step alone (what the engine allows in one
+    says nothing of this one): a power of two of them, so that growing steps settle soon."""
+    if chunks * floats > MEMORY_MAX_FLOATS:
+        return None
+    return min(1 << (chunks - 1).bit_length(), MEMORY_MAX_FLOATS // floats), floats
+
+
+def memory_buffers(host_rows: list[int], heads: int, inner: int,
                    columns: int) -> tuple[int, int] | None:
-    """``(chunks, floats per chunk)`` of the scratch for the largest step if a step of these row
+    """``(chunks, floats per chunk)`` of the scratch if a step of these row
     counts is taken in chunks by :func:`mamba2_scan` / :func:`mlstm_scan`, else ``None``: a request
     brings at least a chunk of rows, and the step is not mostly single rows. (The scan row by row
     takes about 0.9 microseconds a row of the longest request, whatever else runs beside it; in
     chunks a step takes about 20 and then 2 a chunk of 2^18 state entries, a single row's chunk
     as much as a whole one.)"""
     longest, chunks = max(host_rows, default=0), memory_chunks(host_rows)
-    most, floats = max_rows // MEMORY_CHUNK + MEMORY_EXTRA_CHUNKS, heads * inner * (columns + 1)
-    if longest < MEMORY_CHUNK or 2 * chunks > longest or chunks > most or \
-            most * floats > MEMORY_MAX_FLOATS:
+    if longest < MEMORY_CHUNK or 2 * chunks > longest:
         return None
-    return most, floats
+    return _chunk_buffers(chunks, heads * inner * (columns + 1))
 
 
-def delta_buffers(host_rows: list[int], max_rows: int, heads: int,
-                  dim: int) -> tuple[int, int] | None:
+def delta_buffers(host_rows: list[int], heads: int, dim: int) -> tuple[int, int] | None:
     """The same for :func:`delta_scan`. (Row by row 0.48 microseconds a row of the longest request;
     in chunks about 20 and then 0.13 a row.)"""
     longest, chunks = max(host_rows, default=0), linear_chunks(host_rows)
-    most, floats = max_rows // LINEAR_CHUNK + MEMORY_EXTRA_CHUNKS, heads * _delta_floats(dim)
-    if longest < MEMORY_CHUNK or chunks > longest or chunks > most or dim > 256 or \
-            most * floats > MEMORY_MAX_FLOATS:
+    if longest < MEMORY_CHUNK or chunks > longest or dim > 256:
         return None
-    return most, floats
+    return _chunk_buffers(chunks, heads * _delta_floats(dim))
 
 
 def _delta_floats(dim: int) -> int:
     return 4 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK
 
 
-def gla_buffers(host_rows: list[int], max_rows: int, heads: int,
-                dim: int) -> tuple[int, int] | None:
+def gla_buffers(host_rows: list[int], heads: int, dim: int) -> tuple[int, int] | None:
     """The same for :func:`gla_scan`, whose chunks have ``LINEAR_CHUNK`` rows. (Row by row 0.72
     microseconds a row of the longest request; in chunks about 20 and then 0.1 a row.)"""
     longest, chunks = max(host_rows, default=0), linear_chunks(host_rows)
-    most = max_rows // LINEAR_CHUNK + MEMORY_EXTRA_CHUNKS
-    floats = heads * (2 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK)
-    if longest < MEMORY_CHUNK or chunks > longest or chunks > most or \
-            most * floats > MEMORY_MAX_FLOATS:
+    if longest < MEMORY_CHUNK or chunks > longest:
         return None
-    return most, floats
+    return _chunk_buffers(chunks, heads * _gla_floats(dim))
+
+
+def _gla_floats(dim: int) -> int:
+    return 2 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK
 
 
 def _memory_scratch(op: str, host_rows: list[int] | None,
@@ -1392,8 +1395,8 @@ def gla_scan(proj: torch.Tensor, decay_raw: torch.Tensor, state: torch.Tensor,
     if host_rows is not None and scratch is not None:
         _need(op, "scratch", scratch, torch.float32)
         chunks = linear_chunks(host_rows)
-        floats = heads * (2 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK)
-        if not scratch.is_contiguous() or scratch.numel() < chunks * floats or \
+        if not scratch.is_contiguous() or \
+                scratch.numel() < chunks * heads * _gla_floats(dim) or \
                 len(host_rows) != requests or \
                 sum(host_rows) > min(proj.shape[0], decay_raw.shape[0], out.shape[0]):
             raise BackendError(f"{op}: shapes do not fit")

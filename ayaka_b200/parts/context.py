@@ -26,6 +26,8 @@ class Workspace:
         self._buffers: dict[tuple[str, int, torch.dtype], torch.Tensor] = {}
         # a buffer that had to grow is kept: a captured graph may still hold its address
         self._retired: list[torch.Tensor] = []
+        # rows of a spare buffer that the device had no room for
+        self._refused: dict[tuple[str, int, torch.dtype], int] = {}
 
     def buffer(self, name: str, width: int, dtype: torch.dtype,
                rows: int | None = None) -> torch.Tensor:
@@ -39,6 +41,25 @@ class Workspace:
             found = torch.zeros((want, width), dtype=dtype, device=self.device)
             self._buffers[key] = found
         return found
+
+    def spare(self, name: str, width: int, dtype: torch.dtype,
+              rows: int) -> torch.Tensor | None:
+        """A buffer of at least ``rows`` rows that a part can do without and no captured graph
+        uses: ``None`` where the device has no room for it (nor is it asked for so many again); one
+        that has to grow gives its memory back first."""
+        key = (name, width, dtype)
+        found = self._buffers.get(key)
+        if found is not None and found.shape[0] >= rows:
+            return found
+        if rows >= self._refused.get(key, rows + 1):
+            return None
+        del found
+        self._buffers.pop(key, None)
+        try:
+            return self.buffer(name, width, dtype, rows=rows)
+        except torch.OutOfMemoryError:
+            self._refused[key] = rows
+            return None
 
     def nbytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in self._buffers.values())

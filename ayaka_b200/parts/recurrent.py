@@ -17,17 +17,23 @@ from ayaka_b200.parts.spec import PartSpec
 __all__ = ["MLSTM", "DeltaRule", "GatedLinearAttention", "Mamba2"]
 
 
+def _scratch(step: StepContext, name: str,
+             sizes: tuple[int, int] | None) -> torch.Tensor | None:
+    """Room for the chunks of a step that is taken in chunks of rows; ``None`` (the scan goes row by
+    row) for other steps and where the device has none left."""
+    return None if sizes is None else \
+        step.workspace.spare(name, sizes[1], torch.float32, rows=sizes[0])
+
+
 def _chunks(step: StepContext, heads: int, inner: int, columns: int,
             planes: int) -> dict[str, object]:
-    """The scan's further arguments for a step that is taken in chunks of rows (the scratch is
-    sized for the largest step)."""
-    work = step.workspace
-    sizes = ops.memory_buffers(step.host_rows, work.max_rows, heads, inner, columns)
-    if sizes is None:
+    """The scan's further arguments for a step that is taken in chunks of rows."""
+    states = _scratch(step, "memory.states",
+                      ops.memory_buffers(step.host_rows, heads, inner, columns))
+    if states is None:
         return {}
-    return {"host_rows": step.host_rows,
-            "scratch": (work.buffer("memory.states", sizes[1], torch.float32, rows=sizes[0]),
-                        work.buffer("memory.gates", planes * heads, torch.float32))}
+    gates = step.workspace.buffer("memory.gates", planes * heads, torch.float32)
+    return {"host_rows": step.host_rows, "scratch": (states, gates)}
 
 
 @register_part("mixer", "mamba2")
@@ -240,14 +246,12 @@ class GatedLinearAttention(Mixer):
         ops.linear(hidden, self.proj_weight, None, proj, rows=n)
         ops.linear(hidden, self.decay_down, None, low, rows=n)
         ops.linear(low, self.decay_up, self.decay_bias, decay, rows=n)
-        sizes = ops.gla_buffers(step.host_rows, work.max_rows, heads, self.dim)
-        chunks: dict[str, object] = {} if sizes is None else {
-            "host_rows": step.host_rows,
-            "scratch": work.buffer("gla.chunks", sizes[1], torch.float32, rows=sizes[0])}
+        scratch = _scratch(step, "gla.chunks", ops.gla_buffers(step.host_rows, heads, self.dim))
         ops.gla_scan(proj, decay, state, answer, row_start=step.row_start,
                      state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                      dim=self.dim, columns=self.columns, k_offset=self.qk, v_offset=2 * self.qk,
-                     tau=self.tau, q_scale=self.dim ** -0.5, **chunks)
+                     tau=self.tau, q_scale=self.dim ** -0.5,
+                     host_rows=step.host_rows, scratch=scratch)
         # a head is a group of the norm; the weight's `columns` entries repeat for every head
         ops.rms_norm(answer, self.norm_weight, self.eps, gated, groups=heads, count=n,
                      gate=proj[:, 2 * self.qk + self.inner:], gate_mode="silu_after")
@@ -327,15 +331,13 @@ class DeltaRule(Mixer):
         ops.linear(hidden, self.proj_weight, None, proj, rows=n)
         ops.unary_rows(proj[:, self.low_at:], low, activation="tanh", rows=n)
         ops.linear(low, self.decay_up, self.decay_bias, decay, rows=n)
-        sizes = ops.delta_buffers(step.host_rows, work.max_rows, heads, self.dim)
-        chunks: dict[str, object] = {} if sizes is None else {
-            "host_rows": step.host_rows,
-            "scratch": work.buffer("delta.chunks", sizes[1], torch.float32, rows=sizes[0])}
+        scratch = _scratch(step, "delta.chunks",
+                           ops.delta_buffers(step.host_rows, heads, self.dim))
         ops.delta_scan(proj, decay, self.rate_bias, state, answer, row_start=step.row_start,
                        state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                        dim=self.dim, columns=self.columns, k_offset=self.k_at,
                        v_offset=self.v_at, a_offset=self.a_at, decay_rate=self.decay_rate,
-                       **chunks)
+                       host_rows=step.host_rows, scratch=scratch)
         # a head is a group of the norm: each divided by its own root mean square
         ops.rms_norm(answer, self.norm_weight, self.eps, gated, groups=heads, count=n,
                      gate=proj[:, self.g_at:self.g_at + self.inner], gate_mode="sigmoid_after")
