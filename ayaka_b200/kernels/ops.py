@@ -492,7 +492,8 @@ def attention_prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
     the row counts (the grid is sized from it). Head size 64 runs on tcgen05; so do, with
     ``keep_first``, ``gate`` and ``sink`` or without, head size 128 and latent rows of 256 entries
     (``v_pages`` is ``k_pages``); the rest on a warp-level kernel compiled for the head size
-    (``kernel``: ``"tcgen05"``, ``"wide"`` or ``"mma"`` forces one of them where it serves the case).
+    (``kernel``: ``"tcgen05"``, ``"wide"`` or ``"mma"`` forces one of them, an error where it does not
+    serve the case).
     The warp-level kernel also takes value rows of another size than key rows (``v_pages``'
     last dimension), ``keep_first`` (with a window: keys before that position stay visible)
     and ``gate`` (float32 ``[N, num_heads * value size]``: the result times its sigmoid);
@@ -576,6 +577,9 @@ def attention_prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
             check(status, op)
             return
         _nothing_ran()
+    if kernel == "wide":
+        raise BackendError(f"{op}: the wide kernel does not serve this case (head size {head_dim}, "
+                           f"pages of {page_size})")
     if which == "tcgen05":
         if head_dim != 64 or not plain:
             raise BackendError(f"{op}: the tcgen05 kernel serves a softmax of head size 64 without "

@@ -158,3 +158,35 @@ def test_short_walks_one_after_another(kernel, dim):
 
     whole = run(0, len(rows))
     assert torch.equal(whole, torch.cat([run(b, b + 1) for b in range(len(rows))]))
+
+
+@pytest.mark.parametrize("dim,page,more", [
+    (96, 16, {}), (256, 16, {}), (128, 4, {}), (128, 24, {}), (128, 16, {"scale": 0.0}),
+    (64, 16, {"scores": "sigmoid"}), (128, 16, {"gate": "aside"})])
+def test_a_kernel_that_is_asked_for_runs_or_says_so(dim, page, more):
+    """What the wide kernel does not serve: an error for who asks for it, another kernel (with no
+    launch counted for the first) for who does not."""
+    from ayaka_b200.errors import BackendError
+    from ayaka_b200.kernels import gemm_tc, ops
+
+    n, heads = 192, 2
+    pages = -(-n // page)
+    q = torch.randn(n, heads * dim, device="cuda").bfloat16()
+    k_pages, v_pages = (torch.randn(pages + 1, 1, page, dim, device="cuda").bfloat16()
+                        for _ in range(2))
+    table = torch.arange(1, pages + 1, dtype=torch.int32, device="cuda").view(1, -1)
+    if more.get("gate"):  # rows of raw gates that do not start on 16 bytes
+        more = {"gate": torch.randn(n, heads * dim + 1, device="cuda")[:, 1:]}
+    args = dict(num_heads=heads, host_rows=[n], **{"scale": dim ** -0.5, **more})
+    tensors = (q, k_pages, v_pages, table, torch.tensor([0, n]).int().cuda(),
+               torch.tensor([n]).int().cuda())
+    out, plain = (torch.full_like(q, 3.0) for _ in range(2))
+    before = ops.launch_count()
+    with pytest.raises(BackendError):
+        ops.attention_prefill(*tensors, out, kernel="wide", **args)
+    assert torch.all(out == 3.0) and ops.launch_count() == before
+    ops.attention_prefill(*tensors, out, **args)
+    assert ops.launch_count() == before + 1
+    ops.attention_prefill(*tensors, plain, kernel="mma", **args)
+    gemm_tc.check_status(out.device)
+    assert torch.equal(out, plain)
