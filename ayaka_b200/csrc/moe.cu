@@ -729,15 +729,18 @@ AYK_API int ayk_moe_route_scored(const float* logits, int ld, int rows, int expe
 // Three launches: align, the two grouped products. `sorted` holds max_tiles * tile_rows ints,
 // `tile_expert` max_tiles (twice that for tiles of 128), `y` max_tiles * tile_rows rows of ff, `pair_out` rows * top rows
 // of width. type: 0 = float32, 1 = bfloat16. tile_rows: 32, or 128 (bfloat16 only).
-// A tcgen05 product whose bounded wait ran out says so in `device_status`.
+// A tcgen05 product whose bounded wait ran out says so in `device_status`. `launches` (on the host): the
+// kernels that were launched.
 AYK_API int ayk_moe_experts(const void* hidden, int ld_hidden, const void* w_in,
                             const void* w_out, const int* chosen, int rows, int experts, int top,
                             int width, int ff, float limit, float alpha, float shift, int single,
                             int* sorted,
                             int* tile_expert, int max_tiles, int tile_rows, void* y, int ld_y,
                             float* pair_out, int ld_out, int type, int* device_status,
-                            void* stream) {
+                            int* launches, void* stream) {
   using namespace ayk;
+  if (launches == nullptr) return AYK_BAD_ARGUMENT;
+  *launches = 0;
   if (rows == 0) return AYK_OK;
   const long long pairs = (long long)rows * top;
   if (rows < 0 || experts < 1 || top < 1 || width < 1 || ff < 1 || hidden == nullptr ||
@@ -754,6 +757,7 @@ AYK_API int ayk_moe_experts(const void* hidden, int ld_hidden, const void* w_in,
   const bool wide = tile_rows == MOE_TM_WIDE &&
                     moe_tc_takes(hidden, ld_hidden, w_in, w_out, width, ff, y, ld_y, pair_out, ld_out);
   int* tile_first = wide ? tile_expert + max_tiles : nullptr;
+  *launches = wide ? 4 : 3;  // align, (the rows grouped,) two products
   int status = launch_kernel(moe_align_kernel, dim3(1), dim3(1024), 0, s, 1, chosen, (int)pairs,
                              experts, max_tiles, tile_rows, sorted, tile_expert, tile_first);
   if (status != AYK_OK) return status;

@@ -1709,8 +1709,7 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
             sorted_pairs.shape[0] < tiles * tile_rows or tile_expert.shape[0] < kept_tiles or \
             inner.shape[0] < tiles * tile_rows:
         raise BackendError(f"{op}: shapes do not fit")
-    global _launches
-    _launches += 2 + (tile_rows > MOE_TILE_ROWS)  # align, (the rows grouped,) two products
+    launches = c_int(0)
     status = library("moe").ayk_moe_experts(
         _ptr(hidden), c_int(hidden.stride(0)), _ptr(w_in), _ptr(w_out), _ptr(chosen),
         c_int(rows), c_int(experts), c_int(top), c_int(width), c_int(ff), c_float(limit),
@@ -1719,7 +1718,9 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
         c_int(tile_rows),
         _ptr(inner),
         c_int(inner.stride(0)), _ptr(pair_out), c_int(pair_out.stride(0)),
-        c_int(_TYPE[hidden.dtype]), _ptr(_status_word(hidden.device)), _stream())
+        c_int(_TYPE[hidden.dtype]), _ptr(_status_word(hidden.device)), byref(launches), _stream())
+    global _launches
+    _launches += launches.value - 1  # (_stream counted one)
     check(status, op)
 
 

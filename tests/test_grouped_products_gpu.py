@@ -38,11 +38,14 @@ def test_grouped_products(rows, experts, top, width, ff, gated):
     assert ops.moe_tile_rows(rows, experts, top, torch.bfloat16) == 128
     places, tiles = ops.moe_scratch(rows, experts, top)
     pair_out = torch.full((rows * top, width), float("nan"), device="cuda")
+    before = ops.launch_count()
     ops.moe_experts(hidden, w_in, w_out, chosen, pair_out, experts=experts, top=top,
                     limit=7.0, alpha=1.702, shift=1.0, rows=rows, single=not gated,
                     sorted_pairs=torch.empty(places, dtype=torch.int32, device="cuda"),
                     tile_expert=torch.empty(tiles, dtype=torch.int32, device="cuda"),
                     inner=torch.full((places, ff), float("nan"), **dev))
+    # (the tensor-core products run over a copy of the rows: a launch more)
+    assert ops.launch_count() - before == (4 if width % 8 == 0 and ff % 8 == 0 else 3)
     w_in, w_out = w_in.double().view(experts, parts * ff, width), w_out.double()
     for e in range(experts):
         pairs = (chosen == e).nonzero()[:, 0]
