@@ -1624,6 +1624,9 @@ def scale_add(x: torch.Tensor, scale: torch.Tensor, dst: torch.Tensor, *, rows: 
 #: and per tile of the bfloat16 products of steps with many rows (``MOE_TM_WIDE``)
 MOE_TILE_ROWS = 32
 MOE_TILE_ROWS_WIDE = 128
+#: CTAs of the narrow tiles that are resident at one time: two on each of 148 SMs, and a few more
+#: since some are a nearly empty tile's (316 still took one round, 336 two)
+MOE_NARROW_SLOTS = 318
 
 
 def moe_max_tiles(rows: int, experts: int, top: int, tile_rows: int = MOE_TILE_ROWS) -> int:
@@ -1633,14 +1636,25 @@ def moe_max_tiles(rows: int, experts: int, top: int, tile_rows: int = MOE_TILE_R
     return -(-(pairs + min(experts, pairs) * (tile_rows - 1)) // tile_rows)
 
 
-def moe_tile_rows(rows: int, experts: int, top: int, dtype: torch.dtype) -> int:
-    """Rows of a tile :func:`moe_experts` uses: the wide tile (tcgen05 products) in bfloat16
-    once an expert gets a narrow tile's worth of pairs on average, else the narrow one (both
-    products of 16 experts, narrow against wide: 16 pairs an expert, 2,048 x 2,048, 155 against
-    126 us, but 8 pairs at 1,024 x 1,024 56 against 73; 32 pairs 208 against 126 and 75 against
-    48; 512 pairs 1,631 against 235)."""
-    wide = dtype == torch.bfloat16 and rows * top >= MOE_TILE_ROWS * experts
-    return MOE_TILE_ROWS_WIDE if wide else MOE_TILE_ROWS
+def moe_tile_rows(rows: int, experts: int, top: int, dtype: torch.dtype, width: int = 0,
+                  ff: int = 0) -> int:
+    """Rows of a tile :func:`moe_experts` uses: in bfloat16 the wide tile (tcgen05 products) once an
+    expert gets a narrow tile's worth of pairs on average, unless the experts are so few and
+    small that the narrow tiles are done first (``width`` and ``ff`` 0: large ones). A narrow
+    product takes rounds of two tiles of 64 columns an SM, each as long as its sum; the wide ones
+    have more to do ahead of their first sum and are faster at it. Both products, cold matrices,
+    narrow against wide tiles, microseconds. 32 pairs an expert: 8 experts of 1,024 x 1,024 48
+    against 64, 16 of them 85 against 73, 64 of them 218 against 142, 256 of 1,024 x 256 261
+    against 192, 16 of 2,048 x 2,048 208 against 128 (skewed choices 208 against 128); 64 pairs, 4 of
+    512 x 512 28 against 50, 16 of 2,048 x 2,048 314 against 128."""
+    pairs = rows * top
+    if dtype != torch.bfloat16 or pairs < MOE_TILE_ROWS * experts:
+        return MOE_TILE_ROWS
+    tiles = pairs / MOE_TILE_ROWS + experts / 2  # (half of every expert's last tile is empty)
+    narrow = sum(math.ceil(tiles * -(-columns // 64) / MOE_NARROW_SLOTS) * depth
+                 for columns, depth in ((ff, width), (width, ff)))
+    few = width and narrow < 1800 + 0.62 * (width + ff)
+    return MOE_TILE_ROWS if few else MOE_TILE_ROWS_WIDE
 
 
 def moe_scratch(rows: int, experts: int, top: int) -> tuple[int, int]:
@@ -1676,16 +1690,17 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
                 chosen: torch.Tensor, pair_out: torch.Tensor, *, experts: int, top: int,
                 limit: float, alpha: float, sorted_pairs: torch.Tensor,
                 tile_expert: torch.Tensor, inner: torch.Tensor, rows: int,
-                shift: float = 1.0, single: bool = False) -> None:
+                shift: float = 1.0, single: bool = False, tile_rows: int | None = None) -> None:
     """The chosen experts of every row, as two products grouped by expert. ``w_in``
     ``[experts * 2 * ff, width]`` holds each expert's gate rows, then its up rows; ``w_out``
     ``[experts * width, ff]`` its down matrix. Pair ``p = row * top + choice`` computes
     ``g = min(W_gate h, limit)``, ``u = clamp(W_up h, -limit, limit)``,
     ``y = g * sigmoid(alpha * g) * (u + shift)`` and ``pair_out[p] = W_down y`` (float32
-    ``[N * top, width]``, unweighted); ``limit=inf, alpha=1, shift=0`` is ``silu(g) * u``. Scratch: ``sorted_pairs`` (int32, ``tiles * tile
-    rows``), ``tile_expert`` (int32, two per wide tile) and ``inner`` (``[tiles * tile rows, ff]``,
-    compute dtype) sized by :func:`moe_scratch`. With ``single`` an expert has no gate:
-    ``w_in`` is ``[experts * ff, width]`` and ``y = relu(W_up h)^2``."""
+    ``[N * top, width]``, unweighted); ``limit=inf, alpha=1, shift=0`` is ``silu(g) * u``.
+    Scratch: ``sorted_pairs`` (int32, ``tiles * tile rows``), ``tile_expert`` (int32, two per wide
+    tile) and ``inner`` (``[tiles * tile rows, ff]``, compute dtype) sized by :func:`moe_scratch`.
+    With ``single`` an expert has no gate: ``w_in`` is ``[experts * ff, width]`` and
+    ``y = relu(W_up h)^2``. ``tile_rows`` forces the narrow or the wide tiles."""
     op = "moe_experts"
     if _left_out and op in _left_out:
         return
@@ -1698,7 +1713,8 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
     _need(op, "sorted_pairs", sorted_pairs, torch.int32, 1)
     _need(op, "tile_expert", tile_expert, torch.int32, 1)
     width, ff = hidden.shape[1], w_out.shape[1]
-    tile_rows = moe_tile_rows(rows, experts, top, hidden.dtype)
+    if tile_rows is None:
+        tile_rows = moe_tile_rows(rows, experts, top, hidden.dtype, width, ff)
     tiles = moe_max_tiles(rows, experts, top, tile_rows)
     kept_tiles = tiles * (2 if tile_rows > MOE_TILE_ROWS else 1)  # and each one's first row
     if hidden.dtype not in _TYPE or not w_in.is_contiguous() or not w_out.is_contiguous() or \

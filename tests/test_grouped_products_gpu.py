@@ -35,12 +35,12 @@ def test_grouped_products(rows, experts, top, width, ff, gated):
     chosen[rows // 2, 0] = experts - 1
     chosen[3, top - 1] = experts
     chosen = chosen.to(torch.int32).view(-1).cuda()
-    assert ops.moe_tile_rows(rows, experts, top, torch.bfloat16) == 128
+    assert ops.moe_tile_rows(rows, experts, top, torch.bfloat16) == 128  # were they large ones
     places, tiles = ops.moe_scratch(rows, experts, top)
     pair_out = torch.full((rows * top, width), float("nan"), device="cuda")
     before = ops.launch_count()
     ops.moe_experts(hidden, w_in, w_out, chosen, pair_out, experts=experts, top=top,
-                    limit=7.0, alpha=1.702, shift=1.0, rows=rows, single=not gated,
+                    limit=7.0, alpha=1.702, shift=1.0, rows=rows, single=not gated, tile_rows=128,
                     sorted_pairs=torch.empty(places, dtype=torch.int32, device="cuda"),
                     tile_expert=torch.empty(tiles, dtype=torch.int32, device="cuda"),
                     inner=torch.full((places, ff), float("nan"), **dev))
