@@ -19,9 +19,10 @@
 // expert without a gate (`single`: y = relu(W_up h)^2) has w_in [E][ff][width].
 //
 // The tile products run on the CUDA cores with fp32 FMA for float32. In bfloat16 they run on the
-// 5th-generation tensor cores in tiles of 128 pairs once an expert gets that many (moe_tc.cuh),
-// and on the warp-level ones (mma.sync m16n8k16, fp32 accumulators) in tiles of 32 below, and
-// where an operand breaks TMA's alignment rule.
+// 5th-generation tensor cores in tiles of 128 pairs (moe_tc.cuh) where an expert gets 32 pairs or
+// more on average and is not so small that the tiles of 32 are done first; else, and where an operand
+// breaks TMA's alignment rule, on the warp-level tensor cores (mma.sync m16n8k16, fp32 accumulators)
+// in tiles of 32 pairs, or of 128 without that alignment (the caller chooses).
 #include <limits.h>
 
 #include "common.cuh"
@@ -30,7 +31,7 @@
 namespace ayk {
 
 constexpr int MOE_TM = 32;   // pairs per tile: few rows, and float32
-constexpr int MOE_TM_WIDE = 128;  // pairs per tile of the tcgen05 products of many rows
+constexpr int MOE_TM_WIDE = 128;  // pairs per tile of the products of many rows
 constexpr int MOE_TN = 64;   // output columns per tile
 constexpr int MOE_TK = 32;   // k per turn on the CUDA cores (the tensor-core tiles take 64)
 constexpr int MOE_MAX_EXPERTS = 1024;
@@ -261,10 +262,10 @@ __device__ __forceinline__ float expert_unit(float g, float u, float limit, floa
 
 namespace ayk {
 
-template <typename T, int PHASE> struct TileAcc;
+template <typename T, int PHASE, int TM> struct TileAcc;
 
 // fp32: thread (ty, tx) of 16 x 16 owns rows 2 ty .. +1 and columns 4 tx .. +3
-template <int PHASE> struct TileAcc<float, PHASE> {
+template <int PHASE> struct TileAcc<float, PHASE, MOE_TM> {
   static constexpr int TK = MOE_TK;
   static constexpr int LDS = MOE_TK + 1;
   float acc[PHASE == 0 ? 2 : 1][2][4];
@@ -312,22 +313,30 @@ template <int PHASE> struct TileAcc<float, PHASE> {
   }
 };
 
-// bfloat16: eight warps as 2 x 4, each 16 x 16: NT m16n8 accumulators per matrix. Shared rows
-// are padded by 8 entries so that the eight rows of an ldmatrix tile fall into different banks.
-template <int PHASE> struct TileAcc<__nv_bfloat16, PHASE> {
+// bfloat16: eight warps as (TM / 16 MT) x the rest; a warp holds MT x NT m16n8 accumulators
+// per matrix (tiles of 32 pairs: 2 x 4 warps of 16 x 16; of 128 pairs: 4 x 2 warps of
+// 32 x 32, four times the products per turn and a quarter of the weights' re-reads, for many rows that
+// TMA does not take: 64 experts of 2,044 x 1,020 with 64 pairs each 2,317 microseconds where tiles of 32
+// take 2,638). Shared rows are padded by 8 entries so that the eight rows of an ldmatrix tile fall
+// into different banks.
+template <int PHASE, int TM> struct TileAcc<__nv_bfloat16, PHASE, TM> {
   static constexpr int TK = 64;
   static constexpr int LDS = TK + 8;
-  static constexpr int WARPS_N = 8 / (MOE_TM / 16);
-  static constexpr int NT = MOE_TN / (8 * WARPS_N);  // n8 tiles of a warp
+  static constexpr int MT = TM >= 128 ? 2 : 1;    // m16 tiles of a warp
+  static constexpr int WARPS_M = TM / (16 * MT);  // warps down the rows
+  static constexpr int WARPS_N = 8 / WARPS_M;
+  static constexpr int NT = MOE_TN / (8 * WARPS_N);  // n8 tiles of a warp (2 or 4)
   static constexpr int W = PHASE == 0 ? 2 : 1;
-  float acc[W][NT][4];
+  float acc[W][MT][NT][4];
   __device__ __forceinline__ void zero() {
 #pragma unroll
     for (int w = 0; w < W; ++w)
 #pragma unroll
-      for (int n = 0; n < NT; ++n)
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[w][n][i] = 0.f;
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[w][m][n][i] = 0.f;
   }
   static __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4],
                                              uint32_t b0, uint32_t b1) {
@@ -347,7 +356,7 @@ template <int PHASE> struct TileAcc<__nv_bfloat16, PHASE> {
   __device__ __forceinline__ void step(const __nv_bfloat16* As, const __nv_bfloat16* Bs,
                                        const __nv_bfloat16* Bs2, bool both) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = (warp / WARPS_N) * 16, n0 = (warp % WARPS_N) * 8 * NT;
+    const int m0 = (warp / WARPS_N) * 16 * MT, n0 = (warp % WARPS_N) * 8 * NT;
     // A: lanes 0-15 give rows 0-15 at k, lanes 16-31 the same rows at k + 8 (a0..a3);
     // B (kept [n][k]): lanes 0-7 rows n.. at k, 8-15 the same at k + 8 (b0, b1 of eight
     // columns), 16-31 likewise for the next eight
@@ -355,17 +364,24 @@ template <int PHASE> struct TileAcc<__nv_bfloat16, PHASE> {
     const int b_offset = (n0 + (lane >> 4) * 8 + (lane & 7)) * LDS + ((lane >> 3) & 1) * 8;
 #pragma unroll
     for (int k0 = 0; k0 < TK; k0 += 16) {
-      uint32_t a[4], b[4];
-      load_tiles(a, a_at + k0);
+      uint32_t a[MT][4], b[4];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) load_tiles(a[m], a_at + m * 16 * LDS + k0);
 #pragma unroll
       for (int n = 0; n < NT; n += 2) {
         load_tiles(b, Bs + b_offset + n * 8 * LDS + k0);
-        mma(acc[0][n], a, b[0], b[1]);
-        mma(acc[0][n + 1], a, b[2], b[3]);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          mma(acc[0][m][n], a[m], b[0], b[1]);
+          mma(acc[0][m][n + 1], a[m], b[2], b[3]);
+        }
         if (PHASE == 0 && both) {
           load_tiles(b, Bs2 + b_offset + n * 8 * LDS + k0);
-          mma(acc[W - 1][n], a, b[0], b[1]);
-          mma(acc[W - 1][n + 1], a, b[2], b[3]);
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            mma(acc[W - 1][m][n], a[m], b[0], b[1]);
+            mma(acc[W - 1][m][n + 1], a[m], b[2], b[3]);
+          }
         }
       }
     }
@@ -373,25 +389,26 @@ template <int PHASE> struct TileAcc<__nv_bfloat16, PHASE> {
   template <typename F> __device__ __forceinline__ void each(F f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int m0 = (warp / WARPS_N) * 16, n0 = (warp % WARPS_N) * 8 * NT;
+    const int m0 = (warp / WARPS_N) * 16 * MT, n0 = (warp % WARPS_N) * 8 * NT;
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        f(m0 + g + (i >> 1) * 8, n0 + 8 * n + 2 * t + (i & 1), acc[0][n][i], acc[W - 1][n][i]);
-      }
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          f(m0 + 16 * m + g + (i >> 1) * 8, n0 + 8 * n + 2 * t + (i & 1), acc[0][m][n][i],
+            acc[W - 1][m][n][i]);
+        }
   }
 };
 
-// A list made for tiles of `tile_rows` (32 or 128) pairs is walked 32 pairs at a time.
-template <typename T, int PHASE>
+template <typename T, int PHASE, int TM>
 __global__ void __launch_bounds__(256, 2)  // two CTAs an SM: one's copies under the other's products
 moe_tile_kernel(const T* __restrict__ a, int lda, const T* __restrict__ weight,
                 const int* __restrict__ sorted, const int* __restrict__ tile_expert, int top,
                 int K, int N, float limit, float alpha, float shift, T* __restrict__ y, int ld_y,
-                float* __restrict__ out, int ld_out, int tile_rows, int wide, int single) {
-  using Acc = TileAcc<T, PHASE>;
-  constexpr int TM = MOE_TM;
+                float* __restrict__ out, int ld_out, int wide, int single) {
+  using Acc = TileAcc<T, PHASE, TM>;
   constexpr int LDS = Acc::LDS, TK = Acc::TK;
   constexpr bool BF16 = sizeof(T) == 2;
   __shared__ __align__(16) T As[TM * LDS];
@@ -401,7 +418,7 @@ moe_tile_kernel(const T* __restrict__ a, int lda, const T* __restrict__ weight,
   pdl_launch_dependents();
   const int tile = blockIdx.x, n0 = blockIdx.y * MOE_TN, tid = threadIdx.x;
   pdl_wait_for(a, sorted, tile_expert);
-  const int e = tile_expert[tile / (tile_rows / TM)];
+  const int e = tile_expert[tile];
   if (e < 0) return;
   if (tid < TM) pair_s[tid] = sorted[tile * TM + tid];
   __syncthreads();
@@ -648,10 +665,10 @@ moe_join_pieces_kernel(const float* __restrict__ pair_out, int ld, const float* 
   }
 }
 
-template <typename T>
+template <typename T, int TM>
 int moe_experts(const void* hidden, int ld_hidden, const void* w_in, const void* w_out,
-                const int* sorted, const int* tile_expert, int max_tiles, int tile_rows, int top,
-                int width, int ff, float limit, float alpha, float shift, int single, void* y, int ld_y,
+                const int* sorted, const int* tile_expert, int max_tiles, int top, int width,
+                int ff, float limit, float alpha, float shift, int single, void* y, int ld_y,
                 float* pair_out, int ld_out, cudaStream_t stream) {
   // 16-byte pieces when every row of every operand starts on a 16-byte boundary
   const auto aligned = [](const void* p) { return ((uintptr_t)p % 16) == 0; };
@@ -661,25 +678,23 @@ int moe_experts(const void* hidden, int ld_hidden, const void* w_in, const void*
                        aligned(w_out);
   // (room in shared memory for two CTAs an SM: the default split may leave less)
   static const bool carved = [] {
-    cudaFuncSetAttribute(moe_tile_kernel<T, 0>,
+    cudaFuncSetAttribute(moe_tile_kernel<T, 0, TM>,
                          cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(moe_tile_kernel<T, 1>,
+    cudaFuncSetAttribute(moe_tile_kernel<T, 1, TM>,
                          cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return true;
   }();
   (void)carved;
-  const int row_tiles = max_tiles * (tile_rows / MOE_TM);
-  const dim3 grid_in(row_tiles, (ff + MOE_TN - 1) / MOE_TN);
-  int status = launch_kernel(moe_tile_kernel<T, 0>, grid_in, dim3(256), 0, stream, 1,
+  const dim3 grid_in(max_tiles, (ff + MOE_TN - 1) / MOE_TN);
+  int status = launch_kernel(moe_tile_kernel<T, 0, TM>, grid_in, dim3(256), 0, stream, 1,
                              (const T*)hidden, ld_hidden, (const T*)w_in, sorted, tile_expert,
                              top, width, ff, limit, alpha, shift, (T*)y, ld_y, (float*)nullptr, 0,
-                             tile_rows, wide_in, single);
+                             wide_in, single);
   if (status != AYK_OK) return status;
-  const dim3 grid_out(row_tiles, (width + MOE_TN - 1) / MOE_TN);
-  return launch_kernel(moe_tile_kernel<T, 1>, grid_out, dim3(256), 0, stream, 1, (const T*)y,
+  const dim3 grid_out(max_tiles, (width + MOE_TN - 1) / MOE_TN);
+  return launch_kernel(moe_tile_kernel<T, 1, TM>, grid_out, dim3(256), 0, stream, 1, (const T*)y,
                        ld_y, (const T*)w_out, sorted, tile_expert, top, ff, width, limit, alpha, shift,
-                       (T*)nullptr, 0, pair_out, ld_out, tile_rows,
-                       wide_out, 0);
+                       (T*)nullptr, 0, pair_out, ld_out, wide_out, 0);
 }
 
 }  // namespace ayk
@@ -727,8 +742,8 @@ AYK_API int ayk_moe_route_scored(const float* logits, int ld, int rows, int expe
 }
 
 // Three launches: align, the two grouped products. `sorted` holds max_tiles * tile_rows ints,
-// `tile_expert` max_tiles (twice that for tiles of 128), `y` max_tiles * tile_rows rows of ff, `pair_out` rows * top rows
-// of width. type: 0 = float32, 1 = bfloat16. tile_rows: 32, or 128 (bfloat16 only).
+// `tile_expert` max_tiles (twice that for tiles of 128), `y` max_tiles * tile_rows rows of ff,
+// `pair_out` rows * top rows of width. type: 0 = float32, 1 = bfloat16. tile_rows: 32, or 128 (bfloat16 only).
 // A tcgen05 product whose bounded wait ran out says so in `device_status`. `launches` (on the host): the
 // kernels that were launched.
 AYK_API int ayk_moe_experts(const void* hidden, int ld_hidden, const void* w_in,
@@ -767,14 +782,19 @@ AYK_API int ayk_moe_experts(const void* hidden, int ld_hidden, const void* w_in,
                           pair_out, ld_out, device_status, s);
   }
   if (type == 0) {
-    return moe_experts<float>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert, max_tiles,
-                              tile_rows, top, width, ff, limit, alpha, shift, single, y, ld_y,
-                              pair_out, ld_out, s);
+    return moe_experts<float, MOE_TM>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert, max_tiles,
+                                      top, width, ff, limit, alpha, shift, single, y, ld_y, pair_out,
+                                      ld_out, s);
+  }
+  if (type == 1 && tile_rows == MOE_TM_WIDE) {
+    return moe_experts<__nv_bfloat16, MOE_TM_WIDE>(hidden, ld_hidden, w_in, w_out, sorted,
+                                                   tile_expert, max_tiles, top, width, ff, limit,
+                                                   alpha, shift, single, y, ld_y, pair_out, ld_out, s);
   }
   if (type == 1) {
-    return moe_experts<__nv_bfloat16>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert,
-                                      max_tiles, tile_rows, top, width, ff, limit, alpha, shift,
-                                      single, y, ld_y, pair_out, ld_out, s);
+    return moe_experts<__nv_bfloat16, MOE_TM>(hidden, ld_hidden, w_in, w_out, sorted, tile_expert,
+                                              max_tiles, top, width, ff, limit, alpha, shift, single, y,
+                                              ld_y, pair_out, ld_out, s);
   }
   return AYK_BAD_ARGUMENT;
 }

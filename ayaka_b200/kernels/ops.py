@@ -1637,7 +1637,7 @@ def moe_max_tiles(rows: int, experts: int, top: int, tile_rows: int = MOE_TILE_R
 
 
 def moe_tile_rows(rows: int, experts: int, top: int, dtype: torch.dtype, width: int = 0,
-                  ff: int = 0) -> int:
+                  ff: int = 0, tma: bool = True) -> int:
     """Rows of a tile :func:`moe_experts` uses: in bfloat16 the wide tile (tcgen05 products) once an
     expert gets a narrow tile's worth of pairs on average, unless the experts are so few and
     small that the narrow tiles are done first (``width`` and ``ff`` 0: large ones). A narrow
@@ -1646,10 +1646,13 @@ def moe_tile_rows(rows: int, experts: int, top: int, dtype: torch.dtype, width: 
     narrow against wide tiles, microseconds. 32 pairs an expert: 8 experts of 1,024 x 1,024 48
     against 64, 16 of them 85 against 73, 64 of them 218 against 142, 256 of 1,024 x 256 261
     against 192, 16 of 2,048 x 2,048 208 against 128 (skewed choices 208 against 128); 64 pairs, 4 of
-    512 x 512 28 against 50, 16 of 2,048 x 2,048 314 against 128."""
+    512 x 512 28 against 50, 16 of 2,048 x 2,048 314 against 128. Operands that TMA does not take
+    have wide tiles on the warp-level tensor cores, from two narrow tiles' worth of pairs on."""
     pairs = rows * top
-    if dtype != torch.bfloat16 or pairs < MOE_TILE_ROWS * experts:
+    if dtype != torch.bfloat16 or pairs < (1 if tma else 2) * MOE_TILE_ROWS * experts:
         return MOE_TILE_ROWS
+    if not tma:
+        return MOE_TILE_ROWS_WIDE
     tiles = pairs / MOE_TILE_ROWS + experts / 2  # (half of every expert's last tile is empty)
     narrow = sum(math.ceil(tiles * -(-columns // 64) / MOE_NARROW_SLOTS) * depth
                  for columns, depth in ((ff, width), (width, ff)))
@@ -1714,7 +1717,11 @@ def moe_experts(hidden: torch.Tensor, w_in: torch.Tensor, w_out: torch.Tensor,
     _need(op, "tile_expert", tile_expert, torch.int32, 1)
     width, ff = hidden.shape[1], w_out.shape[1]
     if tile_rows is None:
-        tile_rows = moe_tile_rows(rows, experts, top, hidden.dtype, width, ff)
+        # (what moe_tc_takes in csrc/moe_tc.cuh asks for)
+        tma = not ((width | ff | hidden.stride(0) | inner.stride(0)) % 8 or
+                   pair_out.stride(0) % 4 or
+                   any(t.data_ptr() % 16 for t in (hidden, w_in, w_out, inner, pair_out)))
+        tile_rows = moe_tile_rows(rows, experts, top, hidden.dtype, width, ff, tma)
     tiles = moe_max_tiles(rows, experts, top, tile_rows)
     kept_tiles = tiles * (2 if tile_rows > MOE_TILE_ROWS else 1)  # and each one's first row
     if hidden.dtype not in _TYPE or not w_in.is_contiguous() or not w_out.is_contiguous() or \

@@ -28,6 +28,13 @@ def test_wide_tiles_where_they_are_faster(experts, width, ff, wide_from):
 
 
 @pytest.mark.parametrize("experts", [2, 16, 64])
+def test_operands_that_tma_does_not_take(experts):
+    for pairs, tile in ((32, 32), (63, 32), (64, 128), (1000, 128)):
+        assert ops.moe_tile_rows(pairs * experts, experts, 1, torch.bfloat16, 2044, 1020,
+                                 tma=False) == tile
+
+
+@pytest.mark.parametrize("experts", [2, 16, 64])
 def test_the_scratch_serves_both_tiles(experts):
     for rows in (1, 33, 700):
         places, tiles = ops.moe_scratch(rows, experts, 2)

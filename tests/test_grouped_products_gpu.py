@@ -1,5 +1,5 @@
-"""The experts' grouped products in tiles of 128 pairs (tcgen05, and the narrow tiles that take a
-list made for 128) against float64."""
+"""The experts' grouped products in tiles of 128 pairs (tcgen05, and mma.sync for rows that TMA does
+not take) against float64."""
 
 from __future__ import annotations
 
@@ -15,7 +15,9 @@ CASES = [
     (301, 4, 1, 328, 264, False),  # K and N tails of an expert without a gate
     (513, 2, 2, 256, 128, True),   # whole tiles and a single pair behind them
     (700, 5, 2, 1032, 520, True),  # more tiles than a ring, columns of three tiles
-    (150, 4, 2, 36, 20, True),     # rows TMA does not take: narrow tiles over the same list
+    (150, 4, 2, 36, 20, True),     # rows TMA does not take: less than a tile
+    (301, 3, 2, 140, 196, True),   # and tiles in every direction with remainders
+    (280, 3, 1, 132, 76, False),   # and an expert without a gate
 ]
 
 
