@@ -11,14 +11,15 @@
 // quarter of a shared float per FMA, all that the 128 bytes a clock allow) and the products are
 // packed pairs (fma.rn.f32x2, two exact fp32 FMAs an instruction): a pair is two neighbouring k of
 // one element, which lie side by side in shared memory as the operands do in global memory; pairs
-// along m or n would need moves. Tiles travel by cp.async through a ring of four stages of 16 k;
-// rows of 20 floats let the eight rows that a quarter of a warp reads 16 bytes of fall into
+// along m or n would need moves. Tiles travel through a ring of four stages of 16 k (by cp.async, 16-bit
+// operands through registers: RowStage); rows of 20 floats let the eight rows that a quarter of a warp reads 16 bytes of fall into
 // different banks. The stretches of K run in the CTAs of a cluster, each of which adds up its share
 // of the tile's rows through distributed shared memory: a few hundred rows of a model's products
 // are too few tiles for the device.
 // Measured on a B200 at 513 rows (2304 x 768, 768 x 768, 3072 x 768, 768 x 3072), against
 // tiles of 64 x 64 with 4 x 4 elements a thread:  123, 76, 123, 287 -> 92, 37, 94, 111
-// microseconds (cold caches); at 64 rows 83, 82, 84, 318 -> 23, 16, 27, 25.
+// microseconds (cold caches); at 64 rows 83, 82, 84, 318 -> 19, 13, 27, 22. Rows of 769 entries, which
+// are no whole pieces, 3072 x 769: 513 rows 131 -> 101, 8 rows 97 -> 24; in bfloat16 128 -> 98, 85 -> 29.
 #include "tc_common.cuh"
 
 namespace ayk {
@@ -26,35 +27,72 @@ namespace ayk {
 constexpr int BK = 16, LDK = BK + 4, SIMT_STAGES = 4;
 constexpr int SIMT_THREADS = 64;  // 8 x 8
 
-__device__ __forceinline__ void simt_copy16(float* dst, const float* src, bool in) {
-  // (with a source size of 0 nothing is read and the 16 bytes are zeros)
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(in ? 16 : 0)
-               : "memory");
-}
+// How a block of 16 k of a matrix's rows gets to shared memory (zeros outside the matrix). COPY 16 and 4:
+// fp32 by cp.async in pieces of so many bytes (16: rows of whole aligned pieces). COPY 0: the 16-bit
+// types, which cp.async cannot widen, through a thread's registers; they are fetched a block ahead, so
+// that the trip to memory is under the products.
+template <int COPY, int ROWS, typename T> struct RowStage {
+  static constexpr int APART = SIMT_THREADS / BK;  // rows between two entries of a thread
+  static constexpr int EACH = ROWS / APART;
+  T held[COPY == 0 ? EACH : 1];
 
-// 16 k from k0 of rows r0 .. r0 + ROWS of a matrix with `rows` rows, zeros outside it; `vec`: fp32,
-// rows of whole aligned 16-byte pieces.
-template <int ROWS, typename T>
-__device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src, int ld, int r0,
-                                           int rows, int k0, int K, bool vec) {
-  if (sizeof(T) == 4 && vec) {
-#pragma unroll
-    for (int idx = threadIdx.x; idx < ROWS * (BK / 4); idx += SIMT_THREADS) {
-      const int r = idx / (BK / 4), k = idx % (BK / 4) * 4;
-      const bool in = r0 + r < rows && k0 + k < K;  // (K is a multiple of 4)
-      simt_copy16(dst + r * LDK + k,
-                  reinterpret_cast<const float*>(src) + (in ? (size_t)(r0 + r) * ld + k0 + k : 0), in);
-    }
-  } else {
-    for (int idx = threadIdx.x; idx < ROWS * BK; idx += SIMT_THREADS) {
-      const int r = idx / BK, k = idx % BK;
-      dst[r * LDK + k] =
-          r0 + r < rows && k0 + k < K ? ldf(src + (size_t)(r0 + r) * ld + k0 + k) : 0.f;
+  static __device__ __forceinline__ void copy(float* dst, const T* src, bool in) {
+    // (with a source size of 0 nothing is read and the bytes are zeros)
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    if (COPY == 16) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src),
+                   "r"(in ? 16 : 0)
+                   : "memory");
+    } else {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to), "l"(src),
+                   "r"(in ? 4 : 0)
+                   : "memory");
     }
   }
-}
+  // COPY > 0: 16 k from k0 of rows r0 .. r0 + ROWS are on their way to `dst`
+  static __device__ __forceinline__ void bring(float* dst, const T* __restrict__ src, int ld, int r0,
+                                               int rows, int k0, int K) {
+    if (COPY == 16) {
+#pragma unroll
+      for (int idx = threadIdx.x; idx < ROWS * (BK / 4); idx += SIMT_THREADS) {
+        const int r = idx / (BK / 4), k = idx % (BK / 4) * 4;
+        const bool in = r0 + r < rows && k0 + k < K;  // (K is a multiple of 4)
+        copy(dst + r * LDK + k, src + (in ? (size_t)(r0 + r) * ld + k0 + k : 0), in);
+      }
+    } else {
+      const int r = threadIdx.x / BK, k = threadIdx.x % BK;
+      const T* from = src + (size_t)(r0 + r) * ld + k0 + k;
+#pragma unroll
+      for (int i = 0; i < EACH; ++i) {
+        const bool in = r0 + r + APART * i < rows && k0 + k < K;
+        copy(dst + (r + APART * i) * LDK + k, in ? from + (size_t)(APART * i) * ld : src, in);
+      }
+    }
+  }
+  // COPY 0: the same into registers, and from there
+  __device__ __forceinline__ void fetch(const T* __restrict__ src, int ld, int r0, int rows, int k0,
+                                        int K) {
+    const int r = threadIdx.x / BK, k = threadIdx.x % BK;
+    const T* from = src + (size_t)(r0 + r) * ld + k0 + k;
+    if (r0 + ROWS <= rows && k0 + BK <= K) {  // nothing is outside
+#pragma unroll
+      for (int i = 0; i < EACH; ++i, from += (size_t)APART * ld) held[COPY == 0 ? i : 0] = *from;
+    } else {
+#pragma unroll
+      for (int i = 0; i < EACH; ++i, from += (size_t)APART * ld) {
+        const bool in = r0 + r + APART * i < rows && k0 + k < K;
+        held[COPY == 0 ? i : 0] = in ? *from : T(0.f);
+      }
+    }
+  }
+  __device__ __forceinline__ void put(float* dst) const {
+    const int r = threadIdx.x / BK, k = threadIdx.x % BK;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+      dst[(r + APART * i) * LDK + k] = ldf(&held[COPY == 0 ? i : 0]);
+    }
+  }
+};
 
 // MODE 0: out[m,n] = act(acc + bias[n]) stored as TOut.   MODE 1: out(fp32)[m,n] += acc + bias[n].
 template <typename TOut, int MODE>
@@ -71,11 +109,11 @@ __device__ __forceinline__ void simt_store(TOut* __restrict__ out, int ldo, int 
 
 // 8 x 8 threads; a thread owns T x T elements, rows and columns 8 apart. A cluster of `splits` CTAs
 // along grid.x works on a tile of 8 T x 8 T; CTA r's stretch of K starts at r * k_split.
-template <typename TA, typename TW, typename TOut, int MODE, int T>
+template <typename TA, typename TW, typename TOut, int MODE, int T, int COPY>
 __global__ void __launch_bounds__(SIMT_THREADS)
 gemm_simt_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, int ldw,
                  const float* __restrict__ bias, TOut* __restrict__ out, int ldo, int M, int N,
-                 int K, int act, int vec, int splits, int k_split) {
+                 int K, int act, int splits, int k_split) {
   constexpr int B = 8 * T, TILE = B * LDK;
   __shared__ __align__(16) float ring[SIMT_STAGES * 2 * TILE];  // and the tile's sums at the end
   static_assert(SIMT_STAGES * 2 * TILE >= B * B, "the sums fit the ring");
@@ -91,20 +129,38 @@ gemm_simt_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, in
 #pragma unroll
     for (int j = 0; j < T; ++j) acc[i][j] = 0ull;  // (two zeros)
   pdl_wait_for(a, out);
-  auto stage = [&](int kb) {
+  RowStage<COPY, B, TA> a_rows;
+  RowStage<COPY, B, TW> w_rows;
+  auto stage = [&](int kb) {  // block kb comes to its place in the ring (COPY 0: from the registers)
+    float* at = ring + kb % SIMT_STAGES * 2 * TILE;
     if (kb < num_kb) {
-      float* at = ring + kb % SIMT_STAGES * 2 * TILE;
-      stage_rows<B>(at, a, lda, m0, M, k_first + kb * BK, k_last, vec);
-      stage_rows<B>(at + TILE, w, ldw, n0, N, k_first + kb * BK, k_last, vec);
+      if (COPY > 0) {
+        a_rows.bring(at, a, lda, m0, M, k_first + kb * BK, k_last);
+        w_rows.bring(at + TILE, w, ldw, n0, N, k_first + kb * BK, k_last);
+      } else {
+        a_rows.put(at);
+        w_rows.put(at + TILE);
+      }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (COPY > 0) asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto fetch = [&](int kb) {
+    if (COPY == 0 && kb < num_kb) {
+      a_rows.fetch(a, lda, m0, M, k_first + kb * BK, k_last);
+      w_rows.fetch(w, ldw, n0, N, k_first + kb * BK, k_last);
+    }
   };
 #pragma unroll
-  for (int kb = 0; kb < SIMT_STAGES - 1; ++kb) stage(kb);
+  for (int kb = 0; kb < SIMT_STAGES - 1; ++kb) {
+    fetch(kb);
+    stage(kb);
+  }
+  fetch(SIMT_STAGES - 1);
   for (int kb = 0; kb < num_kb; ++kb) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(SIMT_STAGES - 2) : "memory");
+    if (COPY > 0) asm volatile("cp.async.wait_group %0;" ::"n"(SIMT_STAGES - 2) : "memory");
     __syncthreads();  // block kb has landed, and everyone is done with block kb - 1
     stage(kb + SIMT_STAGES - 1);
+    fetch(kb + SIMT_STAGES);
     const float* a_s = ring + kb % SIMT_STAGES * 2 * TILE + ty * LDK;
     const float* w_s = ring + kb % SIMT_STAGES * 2 * TILE + TILE + tx * LDK;
 #pragma unroll
@@ -163,16 +219,16 @@ inline int simt_splits(int N, int K) {
   return splits;
 }
 
-template <typename TA, typename TW, typename TOut, int MODE, int T>
+template <typename TA, typename TW, typename TOut, int MODE, int T, int COPY>
 int launch_simt(const TA* a, int lda, const TW* w, int ldw, const float* bias, TOut* out, int ldo,
-                int M, int N, int K, int act, int vec, int splits, cudaStream_t stream) {
+                int M, int N, int K, int act, int splits, cudaStream_t stream) {
   const long long gy = (M + 8 * T - 1) / (8 * T);
   if (gy > 65535) return AYK_TOO_LARGE;
   const int k_split = ((K + splits - 1) / splits + BK - 1) / BK * BK;
-  return launch_kernel_x(gemm_simt_kernel<TA, TW, TOut, MODE, T>,
+  return launch_kernel_x(gemm_simt_kernel<TA, TW, TOut, MODE, T, COPY>,
                          dim3((N + 8 * T - 1) / (8 * T) * splits, (unsigned)gy),
                          dim3(SIMT_THREADS), 0, stream, splits, a, lda, w, ldw, bias, out, ldo, M,
-                         N, K, act, vec, splits, k_split);
+                         N, K, act, splits, k_split);
 }
 
 template <typename TA, typename TW, typename TOut, int MODE>
@@ -181,18 +237,28 @@ int gemm_simt(const void* a, int lda, const void* w, int ldw, const float* bias,
   if (M == 0 || N == 0) return AYK_OK;
   if (M < 0 || N < 0 || K < 1 || lda < K || ldw < K || ldo < N) return AYK_BAD_ARGUMENT;
   if (act < ACT_NONE || act > ACT_RELU_SQUARED) return AYK_BAD_ARGUMENT;
-  const int vec = sizeof(TA) == 4 && sizeof(TW) == 4 && K % 4 == 0 && lda % 4 == 0 &&
-                  ldw % 4 == 0 && (uintptr_t)a % 16 == 0 && (uintptr_t)w % 16 == 0;
   const int splits = simt_splits(N, K);
   const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64) * splits;
   // 32 x 32 tiles while those of 64 x 64 leave SMs without one (an M that the small tile's grid
   // cannot count takes the large one)
-  if (tiles < sm_count() && M <= 65535 * 32) {
-    return launch_simt<TA, TW, TOut, MODE, 4>((const TA*)a, lda, (const TW*)w, ldw, bias,
-                                              (TOut*)out, ldo, M, N, K, act, vec, splits, stream);
+  const bool small = tiles < sm_count() && M <= 65535 * 32;
+#define AYK_SIMT(COPY)                                                                              \
+  return small ? launch_simt<TA, TW, TOut, MODE, 4, COPY>((const TA*)a, lda, (const TW*)w, ldw, bias, \
+                                                          (TOut*)out, ldo, M, N, K, act, splits,    \
+                                                          stream)                                   \
+               : launch_simt<TA, TW, TOut, MODE, 8, COPY>((const TA*)a, lda, (const TW*)w, ldw, bias, \
+                                                          (TOut*)out, ldo, M, N, K, act, splits,    \
+                                                          stream)
+  if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
+    if (K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (uintptr_t)a % 16 == 0 &&
+        (uintptr_t)w % 16 == 0) {
+      AYK_SIMT(16);
+    }
+    AYK_SIMT(4);
+  } else {
+    AYK_SIMT(0);
   }
-  return launch_simt<TA, TW, TOut, MODE, 8>((const TA*)a, lda, (const TW*)w, ldw, bias, (TOut*)out,
-                                            ldo, M, N, K, act, vec, splits, stream);
+#undef AYK_SIMT
 }
 
 }  // namespace ayk
