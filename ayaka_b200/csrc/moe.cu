@@ -562,7 +562,7 @@ __global__ void moe_join_kernel(const float* __restrict__ pair_out, int ld, cons
     for (int i = 0; i < KEEP; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
       if (c < width) {
-        ds[i] += scale != nullptr ? sum[i] * scale[c] : sum[i];
+        ds[i] = __fadd_rn(ds[i], scale != nullptr ? __fmul_rn(sum[i], scale[c]) : sum[i]);
         dst[(size_t)row * ld_dst + c] = ds[i];
         s2 += ds[i] * ds[i];
       }
@@ -585,9 +585,9 @@ __global__ void moe_join_kernel(const float* __restrict__ pair_out, int ld, cons
       sum = fmaf(share[pair],
                  identity ? ldf(hidden + (size_t)row * ld_hidden + c) : pair_out[pair * ld + c], sum);
     }
-    if (scale != nullptr) sum *= scale[c];
+    if (scale != nullptr) sum = __fmul_rn(sum, scale[c]);
     float* to = dst + (size_t)row * ld_dst + c;
-    const float v = accumulate ? *to + sum : sum;
+    const float v = accumulate ? __fadd_rn(*to, sum) : sum;
     *to = v;
     s2 += v * v;
   }
@@ -600,10 +600,11 @@ __global__ void moe_join_kernel(const float* __restrict__ pair_out, int ld, cons
   }
 }
 
+constexpr int JOIN_PIECES_ROWS = 128;
 // moe_join_kernel for rows of whole pieces of four entries (csrc/row_pieces.cuh). Bound by reading the
-// pairs' rows. Measured on a B200, 4,096 rows of 2,048, two choices, without a next norm: 74 -> 23
-// microseconds (101 MB are 16).
-template <typename T>
+// pairs' rows. Measured on a B200 with cold operands, 4,096 rows of 2,048, two choices: 102 -> 39
+// microseconds (134 MB are 21), with the next norm 102 -> 43, and 8 rows 4.3 -> 2.8.
+template <typename T, int P>
 __global__ void __launch_bounds__(512)
 moe_join_pieces_kernel(const float* __restrict__ pair_out, int ld, const float* __restrict__ share,
                        const int* __restrict__ chosen, const T* hidden, int ld_hidden, int experts,
@@ -613,11 +614,12 @@ moe_join_pieces_kernel(const float* __restrict__ pair_out, int ld, const float* 
   __shared__ float scratch[33];
   pdl_launch_dependents();
   const int row = blockIdx.x, pieces = width / 4;
+  const RowWeights<P> scales(scale, pieces, 1.f), next(next_weight, pieces, 0.f);
   pdl_wait_for(pair_out, share, chosen, hidden, dst);
   float* to = dst + (size_t)row * ld_dst;
-  float4 sum[ROW_PIECES], ds[ROW_PIECES];
+  float4 sum[P], ds[P];
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     sum[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     ds[i] = accumulate ? row_piece(to, threadIdx.x + i * blockDim.x, pieces) : sum[i];
   }
@@ -627,7 +629,7 @@ moe_join_pieces_kernel(const float* __restrict__ pair_out, int ld, const float* 
     const bool identity = hidden != nullptr && chosen[pair] >= experts;
     const float weight = share[pair];
 #pragma unroll
-    for (int i = 0; i < ROW_PIECES; ++i) {
+    for (int i = 0; i < P; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
       if (c < pieces) {
         const float4 v = identity ? load_piece(hidden + (size_t)row * ld_hidden, c)
@@ -641,26 +643,22 @@ moe_join_pieces_kernel(const float* __restrict__ pair_out, int ld, const float* 
   }
   float s2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     if (c < pieces) {
       if (scale != nullptr) {
-        const float4 f = row_piece(scale, c, pieces);
-        sum[i].x *= f.x;
-        sum[i].y *= f.y;
-        sum[i].z *= f.z;
-        sum[i].w *= f.w;
+        const float4 f = scales.piece(i);
+        sum[i] = make_float4(__fmul_rn(sum[i].x, f.x), __fmul_rn(sum[i].y, f.y),
+                             __fmul_rn(sum[i].z, f.z), __fmul_rn(sum[i].w, f.w));
       }
-      ds[i].x += sum[i].x;
-      ds[i].y += sum[i].y;
-      ds[i].z += sum[i].z;
-      ds[i].w += sum[i].w;
+      ds[i] = make_float4(__fadd_rn(ds[i].x, sum[i].x), __fadd_rn(ds[i].y, sum[i].y),
+                          __fadd_rn(ds[i].z, sum[i].z), __fadd_rn(ds[i].w, sum[i].w));
       put_piece(to, c, ds[i]);
       s2 += square_sum(ds[i]);
     }
   }
   if (next_out != nullptr) {
-    next_norm(ds, s2, scratch, width, next_weight, next_offset, next_eps,
+    next_norm(ds, s2, scratch, width, next, next_offset, next_eps,
               next_out + (size_t)row * ld_next);
   }
 }
@@ -822,20 +820,27 @@ AYK_API int ayk_moe_join(const float* pair_out, int ld, const float* share, cons
     return AYK_BAD_ARGUMENT;
   }
   const int by_piece = row_threads(width), size = type == 1 ? 2 : 4;
-  if (by_piece && row_takes(pair_out, ld, width, 4) && row_takes(hidden, ld_hidden, width, size) &&
+  // (without a next norm a row's entries do not hang together, and few rows are better spread over more
+  // CTAs; every sum and product is rounded by itself in both kernels, so a row's bits are the same: 8 rows of 2,048 1.8 microseconds against 2.5 in pieces, 512 rows 19 against 11)
+  if (by_piece && (next_out != nullptr || rows >= JOIN_PIECES_ROWS) &&
+      row_takes(pair_out, ld, width, 4) && row_takes(hidden, ld_hidden, width, size) &&
       row_takes(scale, 0, width, 4) && row_takes(dst, ld_dst, width, 4) &&
       row_takes(next_weight, 0, width, 4) && row_takes(next_out, ld_next, width, size)) {
+    const bool two = row_in_two(width, by_piece);
     if (type == 1) {
-      return launch_kernel(moe_join_pieces_kernel<__nv_bfloat16>, dim3(rows), dim3(by_piece), 0,
-                           (cudaStream_t)stream, 1, pair_out, ld, share, chosen,
-                           (const __nv_bfloat16*)hidden, ld_hidden, experts, top, scale, dst, ld_dst,
-                           width, accumulate, next_weight, next_offset, next_eps,
+      return launch_kernel(two ? moe_join_pieces_kernel<__nv_bfloat16, 2>
+                               : moe_join_pieces_kernel<__nv_bfloat16, ROW_PIECES>,
+                           dim3(rows), dim3(by_piece), 0, (cudaStream_t)stream, 1, pair_out, ld, share,
+                           chosen, (const __nv_bfloat16*)hidden, ld_hidden, experts, top, scale, dst,
+                           ld_dst, width, accumulate, next_weight, next_offset, next_eps,
                            (__nv_bfloat16*)next_out, ld_next);
     }
-    return launch_kernel(moe_join_pieces_kernel<float>, dim3(rows), dim3(by_piece), 0,
-                         (cudaStream_t)stream, 1, pair_out, ld, share, chosen, (const float*)hidden,
-                         ld_hidden, experts, top, scale, dst, ld_dst, width, accumulate, next_weight,
-                         next_offset, next_eps, (float*)next_out, ld_next);
+    return launch_kernel(two ? moe_join_pieces_kernel<float, 2>
+                               : moe_join_pieces_kernel<float, ROW_PIECES>,
+                         dim3(rows), dim3(by_piece), 0, (cudaStream_t)stream, 1, pair_out, ld, share,
+                         chosen, (const float*)hidden, ld_hidden, experts, top, scale, dst, ld_dst,
+                         width, accumulate, next_weight, next_offset, next_eps, (float*)next_out,
+                         ld_next);
   }
   if (type == 1) {
     return launch_kernel(moe_join_kernel<__nv_bfloat16>, dim3(rows, tiles), dim3(threads), 0,

@@ -108,8 +108,9 @@ __global__ void rms_norm_kernel(const float* __restrict__ x, int ld_x,
 }
 
 // The same for groups of whole pieces that a CTA's registers hold, without a weight's period.
-// Measured on a B200, 4,024 rows of 2,048 with a gate in front: 67 -> 18 microseconds.
-template <typename TOut>
+// Measured on a B200 with cold operands, 4,096 rows of 2,048 to bfloat16: 37 -> 18 microseconds (50 MB
+// are 8), 8 rows 2.2 -> 1.5.
+template <typename TOut, int P>
 __global__ void __launch_bounds__(512)
 rms_norm_pieces_kernel(const float* __restrict__ x, int ld_x, const int* __restrict__ rows,
                        const float* __restrict__ weight, float weight_offset, float eps,
@@ -120,16 +121,16 @@ rms_norm_pieces_kernel(const float* __restrict__ x, int ld_x, const int* __restr
   const int r = blockIdx.x, pieces = group_width / 4;
   const size_t first = (size_t)blockIdx.y * group_width;
   const int row = rows != nullptr ? rows[r] : r;
-  float4 ws[ROW_PIECES], xs[ROW_PIECES], zs[ROW_PIECES];
+  float4 ws[P], xs[P], zs[P];
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     ws[i] = weight != nullptr ? offset_piece(weight + first, weight_offset,
                                              threadIdx.x + i * blockDim.x, pieces)
                               : make_float4(1.f, 1.f, 1.f, 1.f);
   }
   pdl_wait_for(x, gate);
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     xs[i] = row_piece(x + (size_t)row * ld_x + first, c, pieces);
     if (gate_mode != GATE_NONE) {
@@ -139,7 +140,7 @@ rms_norm_pieces_kernel(const float* __restrict__ x, int ld_x, const int* __restr
   if (gate_mode != GATE_NONE) {  // the gate's factor
     const bool silu = gate_mode != GATE_SIGMOID_AFTER;
 #pragma unroll
-    for (int i = 0; i < ROW_PIECES; ++i) {
+    for (int i = 0; i < P; ++i) {
       zs[i].x = (silu ? zs[i].x : 1.f) * sigmoid_f(zs[i].x);
       zs[i].y = (silu ? zs[i].y : 1.f) * sigmoid_f(zs[i].y);
       zs[i].z = (silu ? zs[i].z : 1.f) * sigmoid_f(zs[i].z);
@@ -154,14 +155,14 @@ rms_norm_pieces_kernel(const float* __restrict__ x, int ld_x, const int* __restr
   };
   float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     if (gate_mode == GATE_SILU_BEFORE) times_gate(i);
     s += square_sum(xs[i]);
   }
   const float inv = 1.f / sqrtf(block_sum(s, scratch) / (float)group_width + eps);
   TOut* dst = out + (size_t)r * ld_out + first;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     xs[i].x = xs[i].x * inv * ws[i].x;
     xs[i].y = xs[i].y * inv * ws[i].y;
@@ -265,7 +266,9 @@ int rms_norm(const float* x, int ld_x, const int* rows, const float* weight, flo
   if (by_piece && weight_period == 0 && row_takes(x, ld_x, group_width, 4) &&
       row_takes(weight, 0, group_width, 4) && row_takes(gate, ld_gate, group_width, 4) &&
       row_takes(out, ld_out, group_width, sizeof(TOut))) {
-    return launch_kernel(rms_norm_pieces_kernel<TOut>, dim3(n, groups), dim3(by_piece), 0, stream, 1,
+    return launch_kernel(row_in_two(group_width, by_piece) ? rms_norm_pieces_kernel<TOut, 2>
+                                                           : rms_norm_pieces_kernel<TOut, ROW_PIECES>,
+                         dim3(n, groups), dim3(by_piece), 0, stream, 1,
                          x, ld_x, rows, weight, weight_offset, eps, group_width, gate, ld_gate,
                          gate_mode, (TOut*)out, ld_out);
   }
@@ -400,9 +403,9 @@ __global__ void norm_sum_kernel(Branches in, int count, float eps, float factor,
   }
 }
 
-// norm_sum_kernel for two sides and rows of whole pieces. Measured on a B200, 4,096 rows of 2,048 with
-// the next norm: 113 -> 27 microseconds (168 MB are 26).
-template <typename TOut>
+// norm_sum_kernel for two sides and rows of whole pieces. Measured on a B200 with cold operands, 4,096
+// rows of 2,048 with the next norm in bfloat16: 117 -> 39 microseconds (151 MB are 23), 8 rows 3.4 -> 2.4.
+template <typename TOut, int P>
 __global__ void __launch_bounds__(512)
 norm_sum_pieces_kernel(Branches in, float eps, float factor, const float* __restrict__ scale,
                        float* __restrict__ dst, int ld_dst, int width, int accumulate,
@@ -411,11 +414,13 @@ norm_sum_pieces_kernel(Branches in, float eps, float factor, const float* __rest
   __shared__ float scratch[33], other[33];
   pdl_launch_dependents();
   const int r = blockIdx.x, pieces = width / 4;
+  const RowWeights<P> first(in.weight[0], pieces, 1.f), second(in.weight[1], pieces, 1.f);
+  const RowWeights<P> scales(scale, pieces, 1.f), next(next_weight, pieces, 0.f);
   pdl_wait_for(dst, in.x[0], in.x[1]);
-  float4 xs[2][ROW_PIECES], ds[ROW_PIECES];
+  float4 xs[2][P], ds[P];
   float* to = dst + (size_t)r * ld_dst;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     xs[0][i] = row_piece(in.x[0] + (size_t)r * in.ld[0], c, pieces);
     xs[1][i] = row_piece(in.x[1] + (size_t)r * in.ld[1], c, pieces);
@@ -423,19 +428,17 @@ norm_sum_pieces_kernel(Branches in, float eps, float factor, const float* __rest
   }
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     s0 += square_sum(xs[0][i]);
     s1 += square_sum(xs[1][i]);
   }
   const float inv0 = factor / sqrtf(block_sum(s0, scratch) / (float)width + eps);
   const float inv1 = factor / sqrtf(block_sum(s1, other) / (float)width + eps);
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     if (c < pieces) {
-      const float4 a = row_piece(in.weight[0], c, pieces), b = row_piece(in.weight[1], c, pieces);
-      const float4 f = scale != nullptr ? row_piece(scale, c, pieces)
-                                        : make_float4(1.f, 1.f, 1.f, 1.f);
+      const float4 a = first.piece(i), b = second.piece(i), f = scales.piece(i);
       ds[i].x += f.x * (xs[0][i].x * inv0 * a.x + xs[1][i].x * inv1 * b.x);
       ds[i].y += f.y * (xs[0][i].y * inv0 * a.y + xs[1][i].y * inv1 * b.y);
       ds[i].z += f.z * (xs[0][i].z * inv0 * a.z + xs[1][i].z * inv1 * b.z);
@@ -445,7 +448,7 @@ norm_sum_pieces_kernel(Branches in, float eps, float factor, const float* __rest
     }
   }
   if (next_out != nullptr) {
-    next_norm(ds, s2, scratch, width, next_weight, next_offset, next_eps,
+    next_norm(ds, s2, scratch, width, next, next_offset, next_eps,
               next_out + (size_t)r * ld_next);
   }
 }
@@ -551,9 +554,9 @@ __global__ void norm_add_kernel(const float* __restrict__ x, int ld_x, float x_f
   }
 }
 
-// norm_add_kernel for rows of whole pieces. Measured on a B200, 4,096 rows of 2,048 with a bfloat16
-// copy: 38 -> 16 microseconds (117 MB are 18).
-template <typename TOut>
+// norm_add_kernel for rows of whole pieces. Measured on a B200 with cold operands, 4,096 rows of 2,048
+// with a bfloat16 copy and the next norm: 59 -> 29 microseconds (134 MB are 21), 8 rows 3.3 -> 2.3.
+template <typename TOut, int P>
 __global__ void __launch_bounds__(512)
 norm_add_pieces_kernel(const float* __restrict__ x, int ld_x, float x_factor,
                        const float* __restrict__ other, int ld_other, float other_factor,
@@ -564,22 +567,23 @@ norm_add_pieces_kernel(const float* __restrict__ x, int ld_x, float x_factor,
   __shared__ float scratch[33];
   pdl_launch_dependents();
   const int r = blockIdx.x, pieces = width / 4;
-  float4 ws[ROW_PIECES], xs[ROW_PIECES], ds[ROW_PIECES];
+  float4 ws[P], xs[P], ds[P];
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     ws[i] = offset_piece(weight, offset, threadIdx.x + i * blockDim.x, pieces);
   }
+  const RowWeights<P> next(next_weight, pieces, 0.f);
   pdl_wait_for(x, dst, other);
   float* to = dst + (size_t)r * ld_dst;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     xs[i] = row_piece(x + (size_t)r * ld_x, c, pieces);
     ds[i] = row_piece(to, c, pieces);
   }
   if (other != nullptr) {
 #pragma unroll
-    for (int i = 0; i < ROW_PIECES; ++i) {
+    for (int i = 0; i < P; ++i) {
       const float4 o = row_piece(other + (size_t)r * ld_other, threadIdx.x + i * blockDim.x, pieces);
       xs[i].x = xs[i].x * x_factor + o.x * other_factor;
       xs[i].y = xs[i].y * x_factor + o.y * other_factor;
@@ -589,10 +593,10 @@ norm_add_pieces_kernel(const float* __restrict__ x, int ld_x, float x_factor,
   }
   float s = 0.f, s2 = 0.f;
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) s += square_sum(xs[i]);
+  for (int i = 0; i < P; ++i) s += square_sum(xs[i]);
   const float inv = factor / sqrtf(block_sum(s, scratch) / (float)width + eps);
 #pragma unroll
-  for (int i = 0; i < ROW_PIECES; ++i) {
+  for (int i = 0; i < P; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
     if (c < pieces) {
       ds[i].x += xs[i].x * inv * ws[i].x;
@@ -605,7 +609,7 @@ norm_add_pieces_kernel(const float* __restrict__ x, int ld_x, float x_factor,
     }
   }
   if (next_out != nullptr) {
-    next_norm(ds, s2, scratch, width, next_weight, next_offset, next_eps,
+    next_norm(ds, s2, scratch, width, next, next_offset, next_eps,
               next_out + (size_t)r * ld_next);
   }
 }
@@ -662,13 +666,16 @@ AYK_API int ayk_norm_sum(const float* const* x, const int* ld, const float* cons
       row_takes(scale, 0, width, 4) && row_takes(dst, ld_dst, width, 4) &&
       row_takes(next_weight, 0, width, 4) &&
       row_takes(next_out, ld_next, width, next_type == 1 ? 2 : 4)) {
+    const bool two = row_in_two(width, by_piece);
     if (next_out != nullptr && next_type == 1) {
-      return launch_kernel(norm_sum_pieces_kernel<__nv_bfloat16>, dim3(n), dim3(by_piece), 0,
+      return launch_kernel(two ? norm_sum_pieces_kernel<__nv_bfloat16, 2>
+                               : norm_sum_pieces_kernel<__nv_bfloat16, ROW_PIECES>, dim3(n), dim3(by_piece), 0,
                            (cudaStream_t)stream, 1, in, eps, factor, scale, dst, ld_dst, width,
                            accumulate, next_weight, next_offset, next_eps,
                            (__nv_bfloat16*)next_out, ld_next);
     }
-    return launch_kernel(norm_sum_pieces_kernel<float>, dim3(n), dim3(by_piece), 0,
+    return launch_kernel(two ? norm_sum_pieces_kernel<float, 2>
+                               : norm_sum_pieces_kernel<float, ROW_PIECES>, dim3(n), dim3(by_piece), 0,
                          (cudaStream_t)stream, 1, in, eps, factor, scale, dst, ld_dst, width,
                          accumulate, next_weight, next_offset, next_eps, (float*)next_out, ld_next);
   }
@@ -720,14 +727,17 @@ AYK_API int ayk_norm_add_next(const float* x, int ld_x, float x_factor, const fl
       row_takes(other, ld_other, width, 4) && row_takes(weight, 0, width, 4) &&
       row_takes(dst, ld_dst, width, 4) && row_takes(copy, ld_copy, width, size) &&
       row_takes(next_weight, 0, width, 4) && row_takes(next_out, ld_next, width, size)) {
+    const bool two = row_in_two(width, by_piece);
     if (size == 2) {
-      return launch_kernel(norm_add_pieces_kernel<__nv_bfloat16>, dim3(n), dim3(by_piece), 0,
+      return launch_kernel(two ? norm_add_pieces_kernel<__nv_bfloat16, 2>
+                               : norm_add_pieces_kernel<__nv_bfloat16, ROW_PIECES>, dim3(n), dim3(by_piece), 0,
                            (cudaStream_t)stream, 1, x, ld_x, x_factor, other, ld_other,
                            other_factor, weight, offset, eps, factor, dst, ld_dst,
                            (__nv_bfloat16*)copy, ld_copy, width, next_weight, next_offset, next_eps,
                            (__nv_bfloat16*)next_out, ld_next);
     }
-    return launch_kernel(norm_add_pieces_kernel<float>, dim3(n), dim3(by_piece), 0,
+    return launch_kernel(two ? norm_add_pieces_kernel<float, 2>
+                               : norm_add_pieces_kernel<float, ROW_PIECES>, dim3(n), dim3(by_piece), 0,
                          (cudaStream_t)stream, 1, x, ld_x, x_factor, other, ld_other, other_factor,
                          weight, offset, eps, factor, dst, ld_dst, (float*)copy, ld_copy, width,
                          next_weight, next_offset, next_eps, (float*)next_out, ld_next);

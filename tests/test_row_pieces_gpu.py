@@ -1,6 +1,6 @@
 """Norms and joins over rows in pieces of four entries against float64, at the widths where the pieces
-end: one piece, a piece more or less than a block holds, the most that fits, and widths and offsets
-that take the kernels for any row."""
+end: one piece, a piece more or less than a block holds, the most that two pieces a thread and four
+hold, and widths and offsets that take the kernels for any row."""
 
 from __future__ import annotations
 
@@ -9,7 +9,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-WIDTHS = (4, 252, 1028, 2048, 8192, 8196, 1030)
+WIDTHS = (4, 252, 1028, 2048, 4096, 4100, 8192, 8196, 1030)
 ROWS = 3
 
 
@@ -105,3 +105,27 @@ def test_moe_join(width, dtype):
         want = mixed + start.double() if accumulate else mixed
         _close(dst, want)
         _close(out, _rms(want, c.double()))
+
+
+@pytest.mark.parametrize("width", [4, 1028, 2048, 4100, 1030])
+@pytest.mark.parametrize("rows", [127, 128, 300])
+def test_joins_of_few_and_of_many_rows(rows, width):
+    """Without a next norm the rows of a large step are taken in pieces, those of a small one entry by
+    entry: the same bits."""
+    ops = _ops()
+    top, experts = 3, 4
+    pair_out, share = _randn(rows * top, width), torch.rand(rows * top, device="cuda")
+    hidden, scale = _randn(rows, width, seed=1).bfloat16(), _randn(width, seed=2)
+    chosen = torch.arange(rows * top, device="cuda").int() % (experts + 1)
+    start = _randn(rows, width, seed=3)
+    for factor in (scale, None):
+        whole, parts = start.clone(), start.clone()
+        ops.moe_join(pair_out, share, whole, top=top, scale=factor, rows=rows, chosen=chosen,
+                     hidden=hidden, experts=experts)
+        for first in range(0, rows, 50):
+            few = slice(first, min(rows, first + 50))
+            pairs = slice(few.start * top, few.stop * top)
+            ops.moe_join(pair_out[pairs], share[pairs], parts[few], top=top, scale=factor,
+                         rows=few.stop - few.start, chosen=chosen[pairs], hidden=hidden[few],
+                         experts=experts)
+        assert torch.equal(whole, parts)
