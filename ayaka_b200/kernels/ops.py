@@ -1206,48 +1206,74 @@ def memory_chunks(host_rows: list[int]) -> int:
     return sum(-(-rows // MEMORY_CHUNK) for rows in host_rows)
 
 
-def _chunk_buffers(chunks: int, floats: int) -> tuple[int, int] | None:
-    """The scratch of a step of so many chunks, by the step alone (what the engine allows in one
-    says nothing of this one): a power of two of them, so that growing steps settle soon."""
-    if chunks * floats > MEMORY_MAX_FLOATS:
+def _chunk_buffers(row_by_row: float, in_chunks: float, chunks: int,
+                   floats: int) -> tuple[int, int] | None:
+    """The scratch of a step of so many chunks if it is done sooner in chunks (both times in
+    microseconds), by the step alone (what the engine allows in one says nothing of this one): a power
+    of two of them, so that growing steps settle soon."""
+    if in_chunks >= 0.95 * row_by_row or chunks * floats > MEMORY_MAX_FLOATS:
         return None
     return min(1 << (chunks - 1).bit_length(), MEMORY_MAX_FLOATS // floats), floats
 
 
-def memory_buffers(host_rows: list[int], heads: int, inner: int,
-                   columns: int) -> tuple[int, int] | None:
-    """``(chunks, floats per chunk)`` of the scratch if a step of these row
-    counts is taken in chunks by :func:`mamba2_scan` / :func:`mlstm_scan`, else ``None``: a request
-    brings at least a chunk of rows, and the step is not mostly single rows. (The scan row by row
-    takes about 0.9 microseconds a row of the longest request, whatever else runs beside it; in
-    chunks a step takes about 20 and then 2 a chunk of 2^18 state entries, a single row's chunk
-    as much as a whole one.)"""
-    longest, chunks = max(host_rows, default=0), memory_chunks(host_rows)
-    if longest < MEMORY_CHUNK or 2 * chunks > longest:
-        return None
-    return _chunk_buffers(chunks, heads * inner * (columns + 1))
+# Which way a step goes is a matter of its requests: row by row a step takes a row of its longest request
+# after the other, and all requests' rows share the device; in chunks a request of a single row costs as
+# much as a whole chunk (its state goes through scratch). The times below (S: entries of a request's
+# state in units of 2^18) are fitted to both ways measured on a B200 at two or three sizes and twenty
+# steps: one request of 64 to 2,000 rows, two to thirty of 70 to 300, and one of 64 to 1,000 beside 20
+# to 200 single rows. Where they choose the slower way it is by a fifth at most.
 
 
-def delta_buffers(host_rows: list[int], heads: int, dim: int) -> tuple[int, int] | None:
-    """The same for :func:`delta_scan`. (Row by row 0.48 microseconds a row of the longest request;
-    in chunks about 20 and then 0.13 a row.)"""
-    longest, chunks = max(host_rows, default=0), linear_chunks(host_rows)
-    if longest < MEMORY_CHUNK or chunks > longest or dim > 256:
+def memory_buffers(host_rows: list[int], heads: int, inner: int, columns: int,
+                   normed: bool = False) -> tuple[int, int] | None:
+    """``(chunks, floats per chunk)`` of the scratch if a step of these row counts is taken in chunks
+    by :func:`mamba2_scan` (``normed``: by :func:`mlstm_scan`), else ``None``. (Mamba-2 of S = 1, row
+    by row and in chunks: 200 rows 75 and 52 microseconds, 2,000 rows 667 and 283, but 128 rows
+    beside 60 single ones 119 and 263.)"""
+    rows, longest, requests = sum(host_rows), max(host_rows, default=0), len(host_rows)
+    if longest < MEMORY_CHUNK:
         return None
-    return _chunk_buffers(chunks, heads * _delta_floats(dim))
+    chunks, turns = memory_chunks(host_rows), -(-longest // MEMORY_CHUNK)
+    state = heads * inner * columns / (1 << 18)
+    if normed:
+        row_by_row = 8 + max(0.65 * longest, 0.2 * state * rows) + 2.1 * state * requests
+        in_chunks = 45 + 3 * turns + chunks * (0.3 + 3.7 * state)
+    else:
+        row_by_row = 8 + 0.22 * longest + state * (0.16 * rows + 1.2 * requests)
+        in_chunks = 31 + 4.5 * turns + chunks * (0.3 + 3.7 * state)
+    return _chunk_buffers(row_by_row, in_chunks, chunks, heads * inner * (columns + 1))
+
+
+def delta_buffers(host_rows: list[int], heads: int, dim: int,
+                  columns: int) -> tuple[int, int] | None:
+    """The same for :func:`delta_scan`, whose chunks have ``LINEAR_CHUNK`` rows. (S = 0.5: 200 rows 84
+    and 54 microseconds, 2,000 rows 761 and 404, 64 rows beside 31 single ones 69 and 151.)"""
+    rows, longest, requests = sum(host_rows), max(host_rows, default=0), len(host_rows)
+    if longest < MEMORY_CHUNK or dim > 256:
+        return None
+    chunks, turns = linear_chunks(host_rows), -(-longest // LINEAR_CHUNK)
+    state = heads * dim * columns / (1 << 18)
+    row_by_row = 8 + 0.33 * longest + state * (0.27 * rows + 2.2 * requests)
+    in_chunks = 25 + 1.7 * turns + state * (3 * requests + 4.5 * chunks)
+    return _chunk_buffers(row_by_row, in_chunks, chunks, heads * _delta_floats(dim))
 
 
 def _delta_floats(dim: int) -> int:
     return 4 * LINEAR_CHUNK * dim + -(-dim // 4) * 4 + LINEAR_CHUNK * LINEAR_CHUNK
 
 
-def gla_buffers(host_rows: list[int], heads: int, dim: int) -> tuple[int, int] | None:
-    """The same for :func:`gla_scan`, whose chunks have ``LINEAR_CHUNK`` rows. (Row by row 0.72
-    microseconds a row of the longest request; in chunks about 20 and then 0.1 a row.)"""
-    longest, chunks = max(host_rows, default=0), linear_chunks(host_rows)
-    if longest < MEMORY_CHUNK or chunks > longest:
+def gla_buffers(host_rows: list[int], heads: int, dim: int,
+                columns: int) -> tuple[int, int] | None:
+    """The same for :func:`gla_scan`, whose chunks have ``LINEAR_CHUNK`` rows. (S = 1: 200 rows 87 and
+    46 microseconds, 2,000 rows 804 and 239, 64 rows beside 31 single ones 79 and 142.)"""
+    rows, longest, requests = sum(host_rows), max(host_rows, default=0), len(host_rows)
+    if longest < MEMORY_CHUNK:
         return None
-    return _chunk_buffers(chunks, heads * _gla_floats(dim))
+    chunks, turns = linear_chunks(host_rows), -(-longest // LINEAR_CHUNK)
+    state = heads * dim * columns / (1 << 18)
+    row_by_row = 8 + max(0.4 * longest, 0.25 * state * rows) + 1.7 * state * requests
+    in_chunks = 25 + 1.6 * turns + state * (3.2 * requests + 0.7 * chunks)
+    return _chunk_buffers(row_by_row, in_chunks, chunks, heads * _gla_floats(dim))
 
 
 def _gla_floats(dim: int) -> int:

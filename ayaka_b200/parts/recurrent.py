@@ -29,7 +29,8 @@ def _chunks(step: StepContext, heads: int, inner: int, columns: int,
             planes: int) -> dict[str, object]:
     """The scan's further arguments for a step that is taken in chunks of rows."""
     states = _scratch(step, "memory.states",
-                      ops.memory_buffers(step.host_rows, heads, inner, columns))
+                      ops.memory_buffers(step.host_rows, heads, inner, columns,
+                                         normed=planes == 3))
     if states is None:
         return {}
     gates = step.workspace.buffer("memory.gates", planes * heads, torch.float32)
@@ -246,7 +247,8 @@ class GatedLinearAttention(Mixer):
         ops.linear(hidden, self.proj_weight, None, proj, rows=n)
         ops.linear(hidden, self.decay_down, None, low, rows=n)
         ops.linear(low, self.decay_up, self.decay_bias, decay, rows=n)
-        scratch = _scratch(step, "gla.chunks", ops.gla_buffers(step.host_rows, heads, self.dim))
+        scratch = _scratch(step, "gla.chunks", ops.gla_buffers(step.host_rows, heads, self.dim,
+                                                               self.columns))
         ops.gla_scan(proj, decay, state, answer, row_start=step.row_start,
                      state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                      dim=self.dim, columns=self.columns, k_offset=self.qk, v_offset=2 * self.qk,
@@ -332,7 +334,7 @@ class DeltaRule(Mixer):
         ops.unary_rows(proj[:, self.low_at:], low, activation="tanh", rows=n)
         ops.linear(low, self.decay_up, self.decay_bias, decay, rows=n)
         scratch = _scratch(step, "delta.chunks",
-                           ops.delta_buffers(step.host_rows, heads, self.dim))
+                           ops.delta_buffers(step.host_rows, heads, self.dim, self.columns))
         ops.delta_scan(proj, decay, self.rate_bias, state, answer, row_start=step.row_start,
                        state_slot=step.state_slot, requests=step.num_requests, heads=heads,
                        dim=self.dim, columns=self.columns, k_offset=self.k_at,

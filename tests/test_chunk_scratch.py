@@ -11,23 +11,35 @@ from ayaka_b200.parts.context import Workspace
 WIDE = (64, 128, 64)  # heads, inner, columns of a Mamba-2 layer 2,048 wide
 
 
-def test_the_step_alone_says_whether_it_is_taken_in_chunks():
-    for rows in ([1300, 700], [64], [100, 1, 1], [28000]):
-        for sizes in (ops.memory_buffers(rows, *WIDE), ops.gla_buffers(rows, 16, 128),
-                      ops.delta_buffers(rows, 32, 64)):
-            assert sizes is not None
-            assert sizes[0] * sizes[1] <= ops.MEMORY_MAX_FLOATS
-    for rows in ([1] * 64, [63], [64] + [1] * 40, [128 * 64 * 64]):
-        assert ops.memory_buffers(rows, *WIDE) is None
-    assert ops.delta_buffers([1000], 4, 257) is None
+SCANS = {  # a layer's scan at a size (S = 1 and 2, 1, 0.5)
+    "mamba2": lambda rows: ops.memory_buffers(rows, 32, 128, 64),
+    "wide mamba2": lambda rows: ops.memory_buffers(rows, *WIDE),
+    "mlstm": lambda rows: ops.memory_buffers(rows, 4, 256, 256, normed=True),
+    "gated": lambda rows: ops.gla_buffers(rows, 8, 128, 256),
+    "delta": lambda rows: ops.delta_buffers(rows, 32, 64, 64),
+}
+PORTIONS = ([1300, 700], [200], [300, 300], [2000, 1, 1], [27000])
+# a decode step, short portions, and portions beside so many single rows that these decide
+ROW_BY_ROW = ([1] * 64, [63], [10] * 12, [1] * 31 + [64], [1] * 60 + [128], [1] * 200 + [300])
 
 
-@pytest.mark.parametrize("rows", [[64], [65], [200, 70], [4096], [1300] * 3, [27000]])
-def test_the_scratch_holds_the_step_and_little_more(rows):
-    for sizes, chunks in ((ops.memory_buffers(rows, *WIDE), ops.memory_chunks(rows)),
-                          (ops.gla_buffers(rows, 16, 128), ops.linear_chunks(rows)),
-                          (ops.delta_buffers(rows, 32, 64), ops.linear_chunks(rows))):
-        assert chunks <= sizes[0] < 2 * chunks
+@pytest.mark.parametrize("scan", SCANS)
+def test_the_step_alone_says_whether_it_is_taken_in_chunks(scan):
+    for rows in PORTIONS:
+        assert SCANS[scan](rows) is not None, rows
+        assert SCANS[scan](rows)[0] * SCANS[scan](rows)[1] <= ops.MEMORY_MAX_FLOATS
+    for rows in ROW_BY_ROW:
+        assert SCANS[scan](rows) is None, rows
+    assert SCANS[scan]([1 << 20]) is None  # more scratch than there may be
+    assert SCANS[scan]([]) is None
+    assert ops.delta_buffers([1000], 4, 257, 64) is None
+
+
+@pytest.mark.parametrize("scan", SCANS)
+def test_the_scratch_holds_the_step_and_little_more(scan):
+    of = ops.memory_chunks if scan in ("mamba2", "wide mamba2", "mlstm") else ops.linear_chunks
+    for rows in PORTIONS:
+        assert of(rows) <= SCANS[scan](rows)[0] < 2 * of(rows)
 
 
 def test_a_spare_buffer_grows_gives_its_memory_back_and_may_be_refused(monkeypatch):
