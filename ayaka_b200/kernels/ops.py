@@ -476,6 +476,29 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
 PREFILL_ATTENTION = "tcgen05"
 
 
+def prefill_kernel(host_rows: list[int], head_dim: int, scale: float, plain: bool,
+                   same: bool) -> str:
+    """Which kernel :func:`attention_prefill` tries first (``plain``: without options, ``same``: the
+    values are the keys). The tcgen05 kernels work on tiles of 256 and 128 rows: a step of short
+    portions only is better served by the warp-level kernel's tiles of 64. mma against wide, 16 heads,
+    microseconds: head size 128, 128 rows 16.4 against 14.3, 64 rows 14.3 against 12.3; latent rows, 128
+    22.5 against 16.4, and twelve requests of 60 20.5 against 25.4; head size 64 with a gate, 128 rows
+    16.4 against 18.4, 300 rows 23.3 against 20.5, and there only where the tiles are fewer by a
+    quarter: 256 rows beside forty portions of 20 40 against 52, of 65 behind 1,500 keys 157 against
+    95."""
+    longest = max(host_rows, default=0)
+    if PREFILL_ATTENTION != "tcgen05" or scale <= 0:
+        return "mma"
+    if head_dim == 64 and plain:
+        return "tcgen05" if longest >= 256 else "mma"
+    if head_dim != 256 if same else head_dim not in (64, 128):
+        return "mma"
+    if head_dim == 64:
+        wide, narrow = (sum(-(-n // rows) for n in host_rows) for rows in (128, 64))
+        return "wide" if longest >= 256 and 4 * wide <= 3 * narrow else "mma"
+    return "wide" if longest >= 128 else "mma"
+
+
 def attention_prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                       block_table: torch.Tensor, row_start: torch.Tensor, kv_len: torch.Tensor,
                       out: torch.Tensor, *, num_heads: int, scale: float, host_rows: list[int],
@@ -547,20 +570,8 @@ def attention_prefill(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
         raise BackendError(f"{op}: slopes do not go with pooled rows, a sigmoid not with a sink")
     plain = value_dim == head_dim and gate is None and not (keep_first and window) and \
         not pooled and sink is None and not mode
-    # the tcgen05 kernels work on tiles of 256 and 128 rows: a step of short portions only is better
-    # served by the warp-level kernel's tiles of 64 (mma against wide, 16 heads: 128 rows of head
-    # size 128 16.4 against 14.3 us, 64 rows 14.3 against 12.3; latent rows 22.5 against 16.4, and
-    # twelve requests of 60 20.5 against 25.4; head size 64 with a gate, 128 rows 16.4 against
-    # 18.4, 300 rows 23.3 against 20.5)
-    longest = max(host_rows, default=0)
-    if kernel is not None:
-        which = kernel
-    elif PREFILL_ATTENTION != "tcgen05" or scale <= 0:
-        which = "mma"
-    elif head_dim == 64 and plain:
-        which = "tcgen05" if longest >= 256 else "mma"
-    else:
-        which = "wide" if longest >= (256 if head_dim == 64 else 128) else "mma"
+    which = kernel or prefill_kernel(host_rows, head_dim, scale, plain,
+                                     v_pages.data_ptr() == k_pages.data_ptr())
     if which == "wide" and not pooled and not mode and value_dim == head_dim:
         lib = library("attention_prefill_wide")
         tile_rows = lib.ayk_attention_prefill_wide_rows()
