@@ -1364,7 +1364,8 @@ AYK_API int ayk_linear_chunks(const ayk::LinearArgs* args, void* stream) {
 
 // The gated linear attention of csrc/recurrent.cu (a decay sigmoid(z)^(1/tau) per key channel, S as
 // [head][P][N]) in chunks; its rows, `z` and the state as there, the scratch as above (no delta
-// rule). AYK_NOT_TAKEN: the scratch does not start on 16 bytes; nothing ran.
+// rule). AYK_NOT_TAKEN: the scratch does not start on 16 bytes, or more heads than a grid counts; nothing
+// ran.
 AYK_API int ayk_gla_chunks(const float* proj, int ld_proj, int k_offset, int v_offset, const float* z,
                            int ld_z, float tau, float q_scale, float* state,
                            long long state_stride, const int* row_start, const int* state_slot,
@@ -1379,7 +1380,7 @@ AYK_API int ayk_gla_chunks(const float* proj, int ld_proj, int k_offset, int v_o
       state_stride < (long long)heads * N * P) {
     return AYK_BAD_ARGUMENT;
   }
-  if (((uintptr_t)scratch % 16) != 0) return AYK_NOT_TAKEN;
+  if (((uintptr_t)scratch % 16) != 0 || heads > 65535) return AYK_NOT_TAKEN;
   LinearArgs a = {};
   a.in = proj;
   a.decay_raw = z;
@@ -1409,7 +1410,8 @@ AYK_API int ayk_gla_chunks(const float* proj, int ld_proj, int k_offset, int v_o
 
 // The generalised delta rule of csrc/recurrent.cu in chunks; its operands as there, S as [head][P][N];
 // the scratch holds chunks * heads * ayk_delta_chunk_floats(N) floats. AYK_NOT_TAKEN: more than
-// LA_GENERAL_N key channels or a scratch that does not start on 16 bytes; nothing ran.
+// LA_GENERAL_N key channels, more heads than a grid counts or a scratch that does not start on 16 bytes;
+// nothing ran.
 constexpr int LA_GENERAL_N = 256;
 AYK_API int ayk_delta_chunk_floats(int n) { return ayk::la_chunk_floats(n, ayk::MODE_GENERAL); }
 AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v_offset,
@@ -1428,15 +1430,24 @@ AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v
       state_stride < (long long)heads * N * P) {
     return AYK_BAD_ARGUMENT;
   }
-  if (heads > 65535 || requests > 65535 || (P + LA_COLS - 1) / LA_COLS > 65535) return AYK_TOO_LARGE;
-  if (N > LA_GENERAL_N || ((uintptr_t)scratch % 16) != 0) return AYK_NOT_TAKEN;
+  if (requests > 65535 || (P + LA_COLS - 1) / LA_COLS > 65535) return AYK_TOO_LARGE;
+  if (N > LA_GENERAL_N || heads > 65535 || ((uintptr_t)scratch % 16) != 0) return AYK_NOT_TAKEN;
   const GeneralArgs g = {proj,    z,    a_bias,   row_start, scratch, ld_proj,
                          ld_z,    k_offset, a_offset, requests,  heads,   N,
                          decay_rate};
   const size_t smem = (size_t)5 * LA_C * la_pad4(N) * sizeof(float);
   cudaStream_t s = (cudaStream_t)stream;
   int status;
-#define AYK_GENERAL(M)                                                                             {                                                                                                  static const cudaError_t allowed =                                                                   cudaFuncSetAttribute(general_prepare_kernel<M>,                                                                       cudaFuncAttributeMaxDynamicSharedMemorySize,                                                     5 * LA_C * 64 * M * (int)sizeof(float));                                if (allowed != cudaSuccess) return (int)allowed;                                                 status = launch_kernel(general_prepare_kernel<M>, dim3(chunks, heads), dim3(LA_THREADS),                                smem, s, 1, g);                                                         }
+#define AYK_GENERAL(M)                                                                             \
+  {                                                                                                \
+    static const cudaError_t allowed =                                                             \
+        cudaFuncSetAttribute(general_prepare_kernel<M>,                                            \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,                          \
+                             5 * LA_C * 64 * M * (int)sizeof(float));                              \
+    if (allowed != cudaSuccess) return (int)allowed;                                               \
+    status = launch_kernel(general_prepare_kernel<M>, dim3(chunks, heads), dim3(LA_THREADS), smem, s,\
+                           1, g);                                                                  \
+  }
   if (N <= 64) AYK_GENERAL(1)
   else if (N <= 128) AYK_GENERAL(2)
   else AYK_GENERAL(4)

@@ -510,6 +510,12 @@ inline bool memory_takes(const MemoryArgs& a) {
          aligned(a.states);
 }
 
+// Whether the grids of the chunked kernels count the rows, heads and pieces of a state.
+inline bool memory_counts(int rows, int heads, int N, int P) {
+  return heads <= 65535 && (long long)rows * heads <= 0x7fffff00LL &&
+         (long long)((N + MC_TILE - 1) / MC_TILE) * ((P + MC_TILE - 1) / MC_TILE) <= 65535;
+}
+
 template <bool NORM>
 int launch_memory(const MemoryArgs& a, int chunks, cudaStream_t stream) {
   constexpr int STATES_BYTES = MC_STAGES * (2 * MC_STAGE * MC_TILE + 2 * MC_STAGE) * 4;

@@ -834,7 +834,7 @@ AYK_API int ayk_mlstm_scan(const float* proj, int ld_proj, int k_offset, int v_o
 // The same two recurrences over prompt portions (memory_chunks.cuh). `chunks`: every request's rows
 // in chunks of 64 rows, added up; `states`: chunks x heads x (N P, and dim more for mLSTM) floats;
 // `gates`: rows x heads x 2 (mLSTM: 3) floats. AYK_NOT_TAKEN: the operands are not whole 16-byte
-// pieces; nothing ran.
+// pieces, or there are more heads, rows or columns than a grid counts; nothing ran.
 AYK_API int ayk_mamba2_chunks(const float* xbc, int ld_xbc, const float* dt_raw, int ld_dt,
                               const float* dt_bias, const float* a_log, const float* skip,
                               float* state, long long state_stride, const int* row_start,
@@ -847,13 +847,11 @@ AYK_API int ayk_mamba2_chunks(const float* xbc, int ld_xbc, const float* dt_raw,
       P < 1 || xbc == nullptr || dt_raw == nullptr || dt_bias == nullptr || a_log == nullptr ||
       state == nullptr || row_start == nullptr || state_slot == nullptr || y == nullptr ||
       states == nullptr || gates == nullptr || ld_xbc < heads * P + 2 * groups * N ||
-      ld_dt < heads || ld_y < heads * P || requests > 65535 || heads > 65535) {
+      ld_dt < heads || ld_y < heads * P || requests > 65535) {
     return AYK_BAD_ARGUMENT;
   }
-  if (N > SCAN_MAX_N || (long long)rows * heads > 0x7fffffffLL ||
-      (long long)((N + MC_TILE - 1) / MC_TILE) * ((P + MC_TILE - 1) / MC_TILE) > 65535) {
-    return AYK_TOO_LARGE;
-  }
+  if (N > SCAN_MAX_N) return AYK_TOO_LARGE;
+  if (!memory_counts(rows, heads, N, P)) return AYK_NOT_TAKEN;
   MemoryArgs a = {};
   a.q = xbc + (size_t)heads * P + (size_t)groups * N;
   a.k = xbc + (size_t)heads * P;
@@ -894,14 +892,12 @@ AYK_API int ayk_mlstm_chunks(const float* proj, int ld_proj, int k_offset, int v
   if (requests < 0 || rows < 0 || chunks < 1 || heads < 1 || dim < 1 || P < 1 || proj == nullptr ||
       state == nullptr || row_start == nullptr || state_slot == nullptr || out == nullptr ||
       states == nullptr || gates == nullptr || !(cap > 0.f) || ld_out < heads * P ||
-      requests > 65535 || heads > 65535 ||
+      requests > 65535 ||
       state_stride < (long long)heads * dim * P + (long long)heads * tiles * (dim + 1)) {
     return AYK_BAD_ARGUMENT;
   }
-  if (dim > SCAN_MAX_N || (long long)rows * heads > 0x7fffffffLL ||
-      (long long)((dim + MC_TILE - 1) / MC_TILE) * ((P + MC_TILE - 1) / MC_TILE) > 65535) {
-    return AYK_TOO_LARGE;
-  }
+  if (dim > SCAN_MAX_N) return AYK_TOO_LARGE;
+  if (!memory_counts(rows, heads, dim, P)) return AYK_NOT_TAKEN;
   MemoryArgs a = {};
   a.q = proj;
   a.k = proj + k_offset;

@@ -62,3 +62,32 @@ def test_a_spare_buffer_grows_gives_its_memory_back_and_may_be_refused(monkeypat
     assert work.spare("chunks", 8, torch.float32, 256) is None
     assert asked == [128]  # not asked for again
     assert work.spare("chunks", 8, torch.float32, 64).shape == (64, 8)
+
+
+def test_what_a_grid_does_not_count_is_left_to_the_scans_row_by_row():
+    """The entry points of the chunked scans decline (and launch nothing) where the others serve."""
+    from ctypes import c_float, c_int, c_longlong, c_void_p
+
+    from ayaka_b200.kernels.lib import library
+
+    p, z, i, f = c_void_p(4096), c_void_p(0), c_int, c_float
+    heads, rows = 70000, 64
+
+    def wide(heads):
+        return i(heads * 24)
+
+    recurrent, linear = library("recurrent"), library("linear_attention")
+    for heads, rows in ((70000, 64), (60000, 40000)):
+        assert recurrent.ayk_mamba2_chunks(
+            p, wide(heads), p, i(heads), p, p, z, p, c_longlong(heads * 64), p, p, p, wide(heads),
+            i(1), i(rows), i(1), i(heads), i(1), i(8), i(8), p, p, z) == -6
+        assert recurrent.ayk_mlstm_chunks(
+            p, wide(heads), i(0), i(0), i(0), i(0), z, f(15.0), p, c_longlong(heads * 128), p, p, p,
+            wide(heads), i(1), i(rows), i(1), i(heads), i(8), i(8), p, p, z) == -6
+    heads = 70000
+    assert linear.ayk_gla_chunks(
+        p, wide(heads), i(0), i(0), p, wide(heads), f(4.0), f(1.0), p, c_longlong(heads * 64), p, p, p,
+        wide(heads), i(1), i(1), i(heads), i(8), i(8), p, z) == -6
+    assert linear.ayk_delta_chunks(
+        p, wide(heads), i(0), i(0), i(0), p, p, wide(heads), f(0.6), p, c_longlong(heads * 64), p, p,
+        p, wide(heads), i(1), i(1), i(heads), i(8), i(8), p, z) == -6
