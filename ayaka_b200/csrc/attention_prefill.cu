@@ -33,9 +33,10 @@
 // per key, normalised over nothing: no maximum, no sum, the tile's weights go straight to the
 // second product.
 //
-// This kernel uses the legacy warp-level tensor path (not tcgen05): attention is ~5% of a
-// prefill step's FLOPs and this dataflow is proven; the matrix products that dominate run on
-// tcgen05 (gemm_tc.cu).
+// This kernel uses the legacy warp-level tensor path. Most portions of head size 64 and 128 and of
+// latent rows run on tcgen05 (attention_prefill_tc.cu, attention_prefill_wide.cu); this one serves
+// short portions, the other head sizes, value rows of a size of their own, pooled rows, slopes and
+// sigmoid weights.
 #include "common.cuh"
 
 #ifndef AYK_HEAD_DIM

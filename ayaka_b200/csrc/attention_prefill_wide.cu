@@ -18,8 +18,9 @@
 //   warp 5     fetches Q (one TMA box per 64 entries of the head), then the K and V blocks by TMA, a
 //              box per page and 64 entries, into a ring in the order in which they are used: K0, K1,
 //              V0, K2, V1, ... (SAME: one block serves both products).
-// Bound by the tensor cores' shared-memory reads (64-wide products) and, at head size 128, by the
-// softmax, which is why two CTAs share an SM there (97 KB and 256 tensor-memory columns each).
+// Bound by the softmax of 64 keys a turn, which is why two CTAs share an SM where they fit (head sizes
+// 64 and 128: 97 KB and 256 tensor-memory columns each): the tensor pipe is active for 27 % of the time
+// at head size 128 and 21 % over latent rows, issue slots are used for 37 % and 19 %.
 // Rows of a value block that no row of the tile may see are zeroed after they land (their pages may be
 // gone, and 0 * NaN would poison the sum); keys out of sight are masked in the scores. Blocks are
 // aligned to absolute positions, so a row's result does not depend on how the prompt was cut.

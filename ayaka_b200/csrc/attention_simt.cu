@@ -10,9 +10,9 @@
 // and add p_j * V[j]. The tiling depends only on the position, so a row's output is the same
 // whether it arrives alone, in a prompt portion or beside other requests. It serves prefill,
 // decode and mixed batches of the float32 path; in bfloat16 it is the plain reference of the
-// tensor-core and split-KV kernels. Steps of more than ATT_ROWS_FROM rows take a kernel whose CTAs
-// share the tiles' keys and values between 32 rows, with the same arithmetic per row. head_dim: a
-// multiple of 8, at most 256. Any number of heads and of KV heads that divides it.
+// tensor-core and split-KV kernels. Steps of more than ATT_ROWS_FROM rows that bring portions take a
+// kernel whose CTAs share the tiles' keys and values between 32 rows, with the same arithmetic per
+// row, whatever the rows' positions are. head_dim: a multiple of 8, at most 256. Any number of heads and of KV heads that divides it.
 #include "common.cuh"
 
 namespace ayk {

@@ -12,8 +12,8 @@
 // packed pairs (fma.rn.f32x2, two exact fp32 FMAs an instruction): a pair is two neighbouring k of
 // one element, which lie side by side in shared memory as the operands do in global memory; pairs
 // along m or n would need moves. Tiles travel through a ring of four stages of 16 k (by cp.async, 16-bit
-// operands through registers: RowStage); rows of 20 floats let the eight rows that a quarter of a warp reads 16 bytes of fall into
-// different banks. The stretches of K run in the CTAs of a cluster, each of which adds up its share
+// operands through registers: RowStage); rows of 20 floats let the eight rows that a quarter of a warp
+// reads 16 bytes of fall into different banks. The stretches of K run in the CTAs of a cluster, each of which adds up its share
 // of the tile's rows through distributed shared memory: a few hundred rows of a model's products
 // are too few tiles for the device.
 // Measured on a B200 at 513 rows (2304 x 768, 768 x 768, 3072 x 768, 768 x 3072), against

@@ -821,7 +821,8 @@ AYK_API int ayk_moe_join(const float* pair_out, int ld, const float* share, cons
   }
   const int by_piece = row_threads(width), size = type == 1 ? 2 : 4;
   // (without a next norm a row's entries do not hang together, and few rows are better spread over more
-  // CTAs; every sum and product is rounded by itself in both kernels, so a row's bits are the same: 8 rows of 2,048 1.8 microseconds against 2.5 in pieces, 512 rows 19 against 11)
+  // CTAs: 8 rows of 2,048 1.8 microseconds against 2.5 in pieces, 512 rows 19 against 11; every sum and
+  // product is rounded by itself in both kernels, so a row's bits are the same)
   if (by_piece && (next_out != nullptr || rows >= JOIN_PIECES_ROWS) &&
       row_takes(pair_out, ld, width, 4) && row_takes(hidden, ld_hidden, width, size) &&
       row_takes(scale, 0, width, 4) && row_takes(dst, ld_dst, width, 4) &&

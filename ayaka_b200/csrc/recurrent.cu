@@ -1,8 +1,14 @@
 // Layers with a running per-request state instead of cached keys: the short causal
 // convolution and the selective state-space recurrence of a Mamba-2 layer, the matrix
-// memory of an mLSTM layer, and a gated linear attention with a decay per key channel. A step brings each request's next rows (a prompt portion or one
+// memory of an mLSTM layer, a gated linear attention with a decay per key channel and a
+// generalised delta rule. A step brings each request's next rows (a prompt portion or one
 // token); the state a request left behind is read from its slot, carried over the rows in
 // order, and written back. Everything here is fp32.
+//
+// Steps whose portions decide their time are taken in chunks of rows as small matrix products
+// (memory_chunks.cuh, entered from here, and linear_attention.cu); what follows is the scan row
+// by row, for steps of single rows, of short portions and of portions beside many single rows
+// (the caller compares both times), and for operands that the chunked kernels do not read.
 //
 // Both recurrences have the shape S_t = a_t S_(t-1) + b_t k_t v_t^T, y_t = S_t^T q_t with S
 // [n x p] per head, so the p columns of S never mix: a CTA owns one (head, request, tile of
