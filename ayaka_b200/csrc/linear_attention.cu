@@ -48,6 +48,7 @@ constexpr int LA_MAX_N = 512;      // key channels of a head
 constexpr int LA_MAX_TAPS = 16;
 constexpr int LA_CONV_ROWS = 8;    // rows per CTA of the portions' convolution
 constexpr int LA_THREADS = 256;
+constexpr int LA_PREPARE_THREADS = 128;
 
 // (DECAY_SIGMOID: per key channel, sigmoid(raw)^(1/tau); portions only)
 enum DecayMode : int { DECAY_FIXED = 0, DECAY_HEAD = 1, DECAY_CHANNEL = 2, DECAY_SIGMOID = 3 };
@@ -202,6 +203,19 @@ __host__ __device__ __forceinline__ int la_chunk_floats(int N, int mode) {
   return (2 + mode) * LA_C * N + la_pad4(N) + LA_C * LA_C;
 }
 
+// Heads whose scan runs in matrix instructions (linear_scan_mma.cuh), with the chunk's matrices as the
+// pieces described there instead: whole groups of 16 channels (a matrix instruction's k), at most 128
+// (beyond, a warp's state and its matrices leave too few registers and stages).
+__host__ __device__ __forceinline__ bool la_in_fragments(int N) { return N % 16 == 0 && N <= 128; }
+// Entry (k, column) of a piece.
+__host__ __device__ __forceinline__ int la_fragment(int k, int column) {
+  return (column * 4 + ((k & 7) >> 1)) * 4 + (k & 1) + 2 * (k >> 3);
+}
+// Floats between two rows of the chunk in shared memory: fragments read eight rows at once.
+__host__ __device__ __forceinline__ int la_row_floats(int N) {
+  return la_in_fragments(N) ? N + 8 : la_pad4(N);
+}
+
 // The request that owns chunk `index` of the step and the chunk's first row in it.
 __device__ __forceinline__ bool la_find_chunk(const int* row_start, int requests, int index, int& b,
                                               int& t0, int& count) {
@@ -218,18 +232,46 @@ __device__ __forceinline__ bool la_find_chunk(const int* row_start, int requests
   return false;
 }
 
-// grid (chunks, heads). Shared memory: k, q, g and D_(C-1) k as [C][NS], NS = N padded to a
-// multiple of 4 (the padding holds k = q = 0, g = 1). This kernel lets the scan start only when it
-// has ended: CTAs of the scan that took their places beside it would crowd on the SMs that empty
+// Sixteen values a lane, summed over the sixteen lanes of a half warp: lane l gets the sum of value l.
+// Fifteen exchanges in place of sixty-four: a lane keeps half of its values and hands the others over.
+__device__ __forceinline__ float la_transposed_sum(float (&v)[16]) {
+  const int lane = threadIdx.x;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    const bool upper = lane & o;
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const float send = upper ? v[k] : v[k + o];
+      v[k] = (upper ? v[k + o] : v[k]) + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+__device__ __forceinline__ float la_dot4(const float4& a, const float4& b, float s) {
+  return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, s))));
+}
+__device__ __forceinline__ float4 la_mul4(const float4& a, const float4& b) {
+  return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+}
+
+// grid (chunks, heads). Shared memory: k, q, g and D_(C-1) k as [C][NS], NS = N padded (to a
+// multiple of 4: the padding holds k = q = 0, g = 1). A half warp per row and then per pair of columns of
+// A and B, a lane with four neighbouring channels at a time. Bound by issue and shared memory: 128
+// threads whose half warps take two columns each fetch half of what 256 threads with one column did and
+// exchange a quarter of it. Measured on a B200, microseconds: 32 heads of 64 channels, 4,096 rows, a decay
+// per channel 177 -> 103, per head 138 -> 87; 8 heads of 128, 2,048 rows 38 -> 28. This kernel lets the scan start only when
+// it has ended: CTAs of the scan that took their places beside it would crowd on the SMs that empty
 // first, two or three on one (measured: 190 instead of 90 microseconds for 128 CTAs).
-template <int NREG, bool CHANNEL>  // ceil(N / 32); a decay per channel, or one per row
-__global__ void __launch_bounds__(LA_THREADS)
-la_prepare_kernel(const LinearArgs a) {
+template <int M, bool CHANNEL>  // ceil(N / 64); a decay per channel, or one per row
+__global__ void __launch_bounds__(LA_PREPARE_THREADS)
+la_prepare_kernel(const LinearArgs a, int vec) {
   extern __shared__ __align__(16) float la_smem[];
   __shared__ __align__(16) float A[LA_C][LA_C], B[LA_C][LA_C], T[LA_C][LA_C];
   __shared__ float beta_s[LA_C];
-  const int N = a.N, NS = la_pad4(N), h = blockIdx.y, kv = h / (a.heads / a.kv_heads);
+  const int N = a.N, NS = la_row_floats(N), h = blockIdx.y, kv = h / (a.heads / a.kv_heads);
+  const bool fragments = la_in_fragments(N);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int l = lane & 15, part = tid >> 4;  // the half warp of eight
   float* k_s = la_smem;
   float* q_s = k_s + LA_C * NS;
   float* g_s = q_s + LA_C * NS;
@@ -245,15 +287,25 @@ la_prepare_kernel(const LinearArgs a) {
   const int r0 = a.row_start[b] + t0;
   const float rate =
       a.decay_mode == DECAY_HEAD || a.decay_mode == DECAY_CHANNEL ? -expf(a.a_log[h]) : 0.f;
-  if (tid < LA_C * LA_C) {
-    A[tid / LA_C][tid % LA_C] = 0.f;
-    B[tid / LA_C][tid % LA_C] = 0.f;
+#pragma unroll
+  for (int idx = tid; idx < LA_C * LA_C; idx += LA_PREPARE_THREADS) {
+    A[idx / LA_C][idx % LA_C] = 0.f;
+    B[idx / LA_C][idx % LA_C] = 0.f;
   }
-  // a warp per row: q and k (rotated, of unit length, scaled), the decays, beta
-  for (int i = warp; i < LA_C; i += LA_THREADS / 32) {
+  // four channels from n on of a row, `rest` beyond the head
+  auto piece = [&](const float* row, int n, float rest) {
+    if (vec && n + 3 < N) return *reinterpret_cast<const float4*>(row + n);
+    return make_float4(n < N ? row[n] : rest, n + 1 < N ? row[n + 1] : rest,
+                       n + 2 < N ? row[n + 2] : rest, n + 3 < N ? row[n + 3] : rest);
+  };
+  // q and k (rotated, of unit length, scaled), the decays, beta
+#pragma unroll 1
+  for (int i = part; i < LA_C; i += LA_PREPARE_THREADS / 16) {
     const bool row = i < count;
     const float* src = in + (size_t)(r0 + i) * a.ld_in;
-    float k[NREG], q[NREG], g[NREG];
+    float* kr = k_s + i * NS;
+    float* qr = q_s + i * NS;
+    float4 k[M], q[M];
     float shared_g = 1.f;
     if (!CHANNEL && row) {
       shared_g = a.decay_mode == DECAY_FIXED
@@ -262,39 +314,45 @@ la_prepare_kernel(const LinearArgs a) {
                                           a.dt_bias[h]);
     }
 #pragma unroll
-    for (int m = 0; m < NREG; ++m) {
-      const int n = lane + 32 * m;
-      const bool live = row && n < N;
-      k[m] = live ? src[a.k_at + kv * N + n] : 0.f;
-      q[m] = live ? src[a.q_at + kv * N + n] : 0.f;
-      g[m] = shared_g;
-      if (CHANNEL) {
-        g[m] = 1.f;
-        if (live) {
-          const float z = decay_raw[(size_t)(r0 + i) * a.ld_decay + h * N + n];
-          g[m] = a.decay_mode == DECAY_SIGMOID ? la_sigmoid_decay(z, a.inv_tau)
-                                               : la_decay(rate, z + a.dt_bias[h * N + n]);
+    for (int m = 0; m < M; ++m) {
+      const int n = 4 * (l + 16 * m);
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      k[m] = row && n < N ? piece(src + a.k_at + kv * N, n, 0.f) : zero;
+      q[m] = row && n < N ? piece(src + a.q_at + kv * N, n, 0.f) : zero;
+      float4 g = make_float4(shared_g, shared_g, shared_g, shared_g);
+      if (CHANNEL && row && n < N) {
+        float4 z = piece(decay_raw + (size_t)(r0 + i) * a.ld_decay + h * N, n, 0.f);
+        if (a.decay_mode == DECAY_SIGMOID) {
+          g.x = la_sigmoid_decay(z.x, a.inv_tau);
+          g.y = la_sigmoid_decay(z.y, a.inv_tau);
+          g.z = la_sigmoid_decay(z.z, a.inv_tau);
+          g.w = la_sigmoid_decay(z.w, a.inv_tau);
+        } else {
+          const float4 bias = piece(a.dt_bias + h * N, n, 0.f);
+          g.x = la_decay(rate, z.x + bias.x);
+          g.y = la_decay(rate, z.y + bias.y);
+          g.z = la_decay(rate, z.z + bias.z);
+          g.w = la_decay(rate, z.w + bias.w);
         }
       }
+      if (n < NS) *reinterpret_cast<float4*>(g_s + i * NS + n) = g;
     }
-    if (lane == 0) {
+    if (l == 0) {
       beta_s[i] = (a.delta && row)
                       ? la_sigmoid(raw[(size_t)(r0 + i) * a.ld_raw + a.beta_at + h]) : 0.f;
     }
-    float* kr = k_s + i * NS;
-    float* qr = q_s + i * NS;
     if (a.rot_dims > 0) {
 #pragma unroll
-      for (int m = 0; m < NREG; ++m) {
-        const int n = lane + 32 * m;
-        if (n < N) {
-          kr[n] = k[m];
-          qr[n] = q[m];
+      for (int m = 0; m < M; ++m) {
+        const int n = 4 * (l + 16 * m);
+        if (n < NS) {
+          *reinterpret_cast<float4*>(kr + n) = k[m];
+          *reinterpret_cast<float4*>(qr + n) = q[m];
         }
       }
       __syncwarp();
       if (row) {
-        for (int pair = lane; pair < a.rot_dims / 2; pair += 32) {
+        for (int pair = l; pair < a.rot_dims / 2; pair += 16) {
           int x, y;
           rope_members(pair, a.rot_dims, a.rot_layout, x, y);
           float s, c;
@@ -308,30 +366,36 @@ la_prepare_kernel(const LinearArgs a) {
       }
       __syncwarp();
 #pragma unroll
-      for (int m = 0; m < NREG; ++m) {
-        const int n = lane + 32 * m;
-        k[m] = n < N ? kr[n] : 0.f;
-        q[m] = n < N ? qr[n] : 0.f;
+      for (int m = 0; m < M; ++m) {
+        const int n = 4 * (l + 16 * m);
+        if (n < NS) {
+          k[m] = *reinterpret_cast<const float4*>(kr + n);
+          q[m] = *reinterpret_cast<const float4*>(qr + n);
+        }
       }
     }
     float kf = a.k_scale, qf = a.q_scale;
     if (a.unit) {
       float kk = 0.f, qq = 0.f;
 #pragma unroll
-      for (int m = 0; m < NREG; ++m) {
-        kk = fmaf(k[m], k[m], kk);
-        qq = fmaf(q[m], q[m], qq);
+      for (int m = 0; m < M; ++m) {
+        kk = la_dot4(k[m], k[m], kk);
+        qq = la_dot4(q[m], q[m], qq);
       }
-      kf /= sqrtf(warp_sum(kk) + a.unit_eps);
-      qf /= sqrtf(warp_sum(qq) + a.unit_eps);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        kk += __shfl_xor_sync(0xffffffffu, kk, o);
+        qq += __shfl_xor_sync(0xffffffffu, qq, o);
+      }
+      kf /= sqrtf(kk + a.unit_eps);
+      qf /= sqrtf(qq + a.unit_eps);
     }
 #pragma unroll
-    for (int m = 0; m < NREG; ++m) {
-      const int n = lane + 32 * m;
+    for (int m = 0; m < M; ++m) {
+      const int n = 4 * (l + 16 * m);
       if (n < NS) {
-        kr[n] = k[m] * kf;
-        qr[n] = q[m] * qf;
-        g_s[i * NS + n] = g[m];
+        *reinterpret_cast<float4*>(kr + n) = la_mul4(k[m], make_float4(kf, kf, kf, kf));
+        *reinterpret_cast<float4*>(qr + n) = la_mul4(q[m], make_float4(qf, qf, qf, qf));
       }
     }
   }
@@ -342,58 +406,73 @@ la_prepare_kernel(const LinearArgs a) {
   float* g_out = kh_out + LA_C * N;
   float* r_out = g_out + la_pad4(N);
   {
-    // A, B and D_(C-1) k: warp w takes columns w and C - 1 - w, half a warp each, four
-    // neighbouring channels a lane at a time
-    constexpr int M = (NREG + 1) / 2;  // pieces of 16 lanes x 4 channels
-    const int half = lane >> 4, l = lane & 15, j = half ? LA_C - 1 - warp : warp;
-    float4 d[M];  // D_ij k_j (CHANNEL), else k_j, whose decays are one factor `dd`
-    float dd = 1.f;
+    // A, B and D_(C-1) k: a half warp takes columns `part` and C - 1 - part, four rows at a time
+    const int j[2] = {part, LA_C - 1 - part};
+    const int least[2] = {warp * 2, LA_C - 2 - 2 * warp};  // the smaller of the warp's two, each
+    float4 d[2][M];  // D_ij k_j (CHANNEL), else k_j, whose decays are one factor `dd`
+    float dd[2] = {1.f, 1.f};
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int n = 4 * (l + 16 * m);
-      d[m] = n < NS ? *reinterpret_cast<const float4*>(k_s + j * NS + n)
-                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int n = 4 * (l + 16 * m);
+        d[e][m] = n < NS ? *reinterpret_cast<const float4*>(k_s + j[e] * NS + n)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll 1
+    for (int i0 = least[0] & ~3; i0 < LA_C; i0 += 4) {
+      const bool both = i0 + 3 >= least[1];
+      float v[16];  // of row i0 + k: A and B in the first column, in the second
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = i0 + k;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          const int n = 4 * (l + 16 * m);
+          if (n < NS) {
+            const float4 ki = *reinterpret_cast<const float4*>(k_s + i * NS + n);
+            const float4 qi = *reinterpret_cast<const float4*>(q_s + i * NS + n);
+            float4 g = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (CHANNEL) g = *reinterpret_cast<const float4*>(g_s + i * NS + n);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              if (e == 0 || both) {
+                if (CHANNEL && i > j[e]) d[e][m] = la_mul4(d[e][m], g);
+                v[4 * k + 2 * e] = la_dot4(ki, d[e][m], v[4 * k + 2 * e]);
+                v[4 * k + 2 * e + 1] = la_dot4(qi, d[e][m], v[4 * k + 2 * e + 1]);
+              }
+            }
+          }
+        }
+        if (!CHANNEL) {
+          const float g = g_s[i * NS];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (i > j[e]) dd[e] *= g;
+            v[4 * k + 2 * e] *= dd[e];
+            v[4 * k + 2 * e + 1] *= dd[e];
+          }
+        }
+      }
+      const float sum = la_transposed_sum(v);
+      const int i = i0 + (l >> 2), column = l & 2 ? j[1] : j[0];
+      if (i >= column) (l & 1 ? B : A)[i][column] = sum;
     }
-    for (int i = warp; i < LA_C; ++i) {  // (warp: the smaller of the two columns)
-      float sa = 0.f, sb = 0.f;
-      if (!CHANNEL && i > j) dd *= g_s[i * NS];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
 #pragma unroll
       for (int m = 0; m < M; ++m) {
         const int n = 4 * (l + 16 * m);
         if (n < NS) {
-          const float4 k = *reinterpret_cast<const float4*>(k_s + i * NS + n);
-          const float4 q = *reinterpret_cast<const float4*>(q_s + i * NS + n);
-          if (CHANNEL && i > j) {
-            const float4 g = *reinterpret_cast<const float4*>(g_s + i * NS + n);
-            d[m].x *= g.x;
-            d[m].y *= g.y;
-            d[m].z *= g.z;
-            d[m].w *= g.w;
-          }
-          sa = fmaf(k.x, d[m].x, fmaf(k.y, d[m].y, fmaf(k.z, d[m].z, fmaf(k.w, d[m].w, sa))));
-          sb = fmaf(q.x, d[m].x, fmaf(q.y, d[m].y, fmaf(q.z, d[m].z, fmaf(q.w, d[m].w, sb))));
+          *reinterpret_cast<float4*>(w_s + j[e] * NS + n) =
+              la_mul4(d[e][m], make_float4(dd[e], dd[e], dd[e], dd[e]));
         }
       }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        sa += __shfl_xor_sync(0xffffffffu, sa, o);
-        sb += __shfl_xor_sync(0xffffffffu, sb, o);
-      }
-      if (l == 0 && i >= j) {
-        A[i][j] = sa * dd;
-        B[i][j] = sb * dd;
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int n = 4 * (l + 16 * m);
-      if (n < NS) {
-        *reinterpret_cast<float4*>(w_s + j * NS + n) =
-            make_float4(d[m].x * dd, d[m].y * dd, d[m].z * dd, d[m].w * dd);
-      }
-    }
   }
   __syncthreads();
+  constexpr int OTHERS = LA_PREPARE_THREADS - 32;
   if (warp == 0) {
     if (lane < LA_C) {  // column `lane` of T, from the top (x[m] is 0 above the diagonal)
       float x[LA_C];
@@ -409,11 +488,33 @@ la_prepare_kernel(const LinearArgs a) {
         T[i][lane] = s;
       }
     }
+  } else if (fragments) {  // meanwhile the cumulative decays, then Kt and Qt in pieces
+    for (int n = tid - 32; n < N; n += OTHERS) {
+      float g = 1.f;
+#pragma unroll
+      for (int i = 0; i < LA_C; ++i) {
+        g *= g_s[i * NS + n];
+        g_s[i * NS + n] = g;
+      }
+      g_out[n] = g;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(OTHERS) : "memory");
+    const int tiles = a.delta ? 4 : 2;
+    for (int idx = tid - 32; idx < N / 16 * tiles * 32; idx += OTHERS) {
+      const int at_lane = idx & 31, j = (idx >> 5) & (tiles - 1), group = (idx >> 5) / tiles;
+      const int at = ((j & 1) * 8 + (at_lane >> 2)) * NS + group * 16 + (at_lane & 3) * 2;
+      const float* x = (tiles == 4 && j < 2 ? k_s : q_s) + at;
+      const float2 x0 = *reinterpret_cast<const float2*>(x), x1 = *reinterpret_cast<const float2*>(x + 8);
+      const float2 g0 = *reinterpret_cast<const float2*>(g_s + at);
+      const float2 g1 = *reinterpret_cast<const float2*>(g_s + at + 8);
+      *reinterpret_cast<float4*>(m_out + (size_t)idx * 4) =
+          make_float4(g0.x * x0.x, g0.y * x0.y, g1.x * x1.x, g1.y * x1.y);
+    }
   } else {  // meanwhile Kt and Qt (four rows of a channel a thread) and G
     const int parts = a.delta ? 8 : 4;
-    for (int idx = tid - 32; idx < N * parts; idx += LA_THREADS - 32) {
-      const int n = idx / parts, part = idx % parts, first = (part & 3) * 4;
-      const float* x = part < parts - 4 ? k_s : q_s;
+    for (int idx = tid - 32; idx < N * parts; idx += OTHERS) {
+      const int n = idx / parts, at = idx % parts, first = (at & 3) * 4;
+      const float* x = at < parts - 4 ? k_s : q_s;
       float g = 1.f;
       for (int i = 0; i < first; ++i) g *= g_s[i * NS + n];
       float v[4];
@@ -422,32 +523,37 @@ la_prepare_kernel(const LinearArgs a) {
         g *= g_s[(first + i) * NS + n];
         v[i] = g * x[(first + i) * NS + n];
       }
-      *reinterpret_cast<float4*>(m_out + (size_t)n * parts * 4 + part * 4) =
+      *reinterpret_cast<float4*>(m_out + (size_t)n * parts * 4 + at * 4) =
           make_float4(v[0], v[1], v[2], v[3]);
-      if (part == 3) g_out[n] = g;
+      if (at == 3) g_out[n] = g;
     }
   }
   __syncthreads();
-  if (tid < LA_C * LA_C) {  // (B and T are zero above the diagonal)
-    const int i = tid / LA_C, j = tid % LA_C;
+#pragma unroll
+  for (int idx = tid; idx < LA_C * LA_C; idx += LA_PREPARE_THREADS) {
+    // (B and T are zero above the diagonal)
+    const int i = idx / LA_C, j = idx % LA_C;
     float s = 0.f;
 #pragma unroll
     for (int m = 0; m < LA_C; ++m) s = fmaf(B[i][m], T[m][j], s);
-    r_out[tid] = s;
+    r_out[fragments ? (i >> 3) * 128 + la_fragment(j, i & 7) : idx] = s;
   }
-  for (int idx = tid; idx < N * (LA_C / 4); idx += LA_THREADS) {
-    const int n = idx / (LA_C / 4), j = idx % (LA_C / 4) * 4;
+  // four rows of a channel of Kh: neighbouring ones, or (fragments) 2 t, 2 t + 1, 2 t + 8, 2 t + 9
+  for (int idx = tid; idx < N * (LA_C / 4); idx += LA_PREPARE_THREADS) {
+    const int n = idx >> 2, first = fragments ? 2 * (idx & 3) : 4 * (idx & 3);
+    const int second = first + (fragments ? 8 : 2);
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < LA_C; ++i) {
       const float d = w_s[i * NS + n];
-      const float4 t = *reinterpret_cast<const float4*>(&T[i][j]);
-      s.x = fmaf(t.x, d, s.x);
-      s.y = fmaf(t.y, d, s.y);
-      s.z = fmaf(t.z, d, s.z);
-      s.w = fmaf(t.w, d, s.w);
+      const float2 x = *reinterpret_cast<const float2*>(&T[i][first]);
+      const float2 y = *reinterpret_cast<const float2*>(&T[i][second]);
+      s.x = fmaf(x.x, d, s.x);
+      s.y = fmaf(x.y, d, s.y);
+      s.z = fmaf(y.x, d, s.z);
+      s.w = fmaf(y.y, d, s.w);
     }
-    *reinterpret_cast<float4*>(kh_out + (size_t)n * LA_C + j) = s;
+    *reinterpret_cast<float4*>(kh_out + (size_t)idx * 4) = s;
   }
 }
 
@@ -470,7 +576,8 @@ general_prepare_kernel(const GeneralArgs a) {
   extern __shared__ __align__(16) float la_smem[];
   __shared__ __align__(16) float Lk[LA_C][LA_C], La[LA_C][LA_C], Mk[LA_C][LA_C], Ma[LA_C][LA_C];
   __shared__ __align__(16) float T[LA_C][LA_C], Tk[LA_C][LA_C];
-  const int N = a.N, NS = la_pad4(N), h = blockIdx.y;
+  const int N = a.N, NS = la_row_floats(N), h = blockIdx.y;
+  const bool fragments = la_in_fragments(N);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* u_s = la_smem;
   float* r_s = u_s + LA_C * NS;
@@ -637,7 +744,7 @@ general_prepare_kernel(const GeneralArgs a) {
     for (int m = 0; m < LA_C; ++m) {
       if (m <= i) s = fmaf(-Ma[i][m], Tk[m][j], s);
     }
-    r_out[tid] = s;
+    r_out[fragments ? (i >> 3) * 128 + la_fragment(j, i & 7) : tid] = s;
   }
   for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
     const int n = idx % N, first = idx / N * 8;
@@ -672,6 +779,14 @@ general_prepare_kernel(const GeneralArgs a) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) kh[e] = fmaf(-Tk[m][first + e], d, kh[e]);
     }
+    if (fragments) {  // (nobody else reads these entries)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        r_s[(first + e) * NS + n] = q[e];
+        k_s[(first + e) * NS + n] = kh[e];
+      }
+      continue;
+    }
     float* m_row = m_out + (size_t)n * 2 * LA_C + first;
 #pragma unroll
     for (int e = 0; e < 8; e += 4) {  // (32 bytes at a time: whole sectors)
@@ -685,6 +800,20 @@ general_prepare_kernel(const GeneralArgs a) {
           make_float4(au_s[(first + e) * NS + n], au_s[(first + e + 1) * NS + n],
                       au_s[(first + e + 2) * NS + n], au_s[(first + e + 3) * NS + n]);
     }
+  }
+  if (!fragments) return;
+  __syncthreads();
+  for (int idx = tid; idx < N * 8; idx += LA_THREADS) {  // U' and Rt in pieces
+    const int l = idx & 31, j = (idx >> 5) & 3, group = idx >> 7;
+    const float* x = (j < 2 ? g_s : r_s) + ((j & 1) * 8 + (l >> 2)) * NS + group * 16 + (l & 3) * 2;
+    const float2 x0 = *reinterpret_cast<const float2*>(x), x1 = *reinterpret_cast<const float2*>(x + 8);
+    *reinterpret_cast<float4*>(m_out + (size_t)idx * 4) = make_float4(x0.x, x0.y, x1.x, x1.y);
+  }
+  for (int idx = tid; idx < N * 8; idx += LA_THREADS) {  // Kh, then Ah
+    const int which = idx / (N * 4), at = idx - which * N * 4, n = at >> 2, t = at & 3;
+    const float* x = (which ? au_s : k_s) + 2 * t * NS + n;
+    *reinterpret_cast<float4*>(kh_out + (size_t)idx * 4) =
+        make_float4(x[0], x[NS], x[8 * NS], x[9 * NS]);
   }
 }
 
@@ -951,6 +1080,12 @@ la_scan_kernel(const LinearArgs a, int vec) {
     }
   }
 }
+
+}  // namespace ayk
+
+#include "linear_scan_mma.cuh"
+
+namespace ayk {
 
 // ---------------------------------------------------------------------------------------------
 // Single rows. grid (heads, rows). A tile of PT columns of S at a time: thread (group, column)
@@ -1247,36 +1382,55 @@ static int la_chunks(const LinearArgs& a, cudaStream_t s) {
   if (a.N > LA_MAX_N || a.heads > 65535 || a.requests > 65535 || tiles > 65535) {
     return AYK_TOO_LARGE;
   }
-  const size_t smem = (size_t)4 * LA_C * la_pad4(a.N) * sizeof(float);
+  const size_t smem = (size_t)4 * LA_C * la_row_floats(a.N) * sizeof(float);
   int status;
-#define AYK_LA_PREPARE_AS(NREG, CHANNEL)                                                         \
+  const int vec = a.N % 4 == 0 && a.ld_in % 4 == 0 && a.k_at % 4 == 0 && a.q_at % 4 == 0 &&
+                  a.ld_decay % 4 == 0 &&
+                  ((uintptr_t)a.in | (uintptr_t)a.decay_raw | (uintptr_t)a.dt_bias) % 16 == 0;
+#define AYK_LA_PREPARE_AS(M, CHANNEL)                                                            \
   {                                                                                              \
     static const bool allowed =                                                                  \
-        (cudaFuncSetAttribute(la_prepare_kernel<NREG, CHANNEL>,                                  \
+        (cudaFuncSetAttribute(la_prepare_kernel<M, CHANNEL>,                                     \
                               cudaFuncAttributeMaxDynamicSharedMemorySize,                       \
-                              4 * LA_C * 32 * NREG * (int)sizeof(float)), true);                 \
+                              4 * LA_C * (64 * M + 8) * (int)sizeof(float)), true);              \
     (void)allowed;                                                                               \
-    status = launch_kernel(la_prepare_kernel<NREG, CHANNEL>, dim3(a.chunks, a.heads),            \
-                           dim3(LA_THREADS), smem, s, 1, a);                                     \
+    status = launch_kernel(la_prepare_kernel<M, CHANNEL>, dim3(a.chunks, a.heads),               \
+                           dim3(LA_PREPARE_THREADS), smem, s, 1, a, vec);                        \
   }
-#define AYK_LA_PREPARE(NREG)                                                                     \
+#define AYK_LA_PREPARE(M)                                                                        \
   {                                                                                              \
-    if (a.decay_mode >= DECAY_CHANNEL) AYK_LA_PREPARE_AS(NREG, true)                             \
-    else AYK_LA_PREPARE_AS(NREG, false)                                                          \
+    if (a.decay_mode >= DECAY_CHANNEL) AYK_LA_PREPARE_AS(M, true)                                \
+    else AYK_LA_PREPARE_AS(M, false)                                                             \
   }
-  if (a.N <= 32) AYK_LA_PREPARE(1)
-  else if (a.N <= 64) AYK_LA_PREPARE(2)
-  else if (a.N <= 128) AYK_LA_PREPARE(4)
-  else if (a.N <= 256) AYK_LA_PREPARE(8)
-  else AYK_LA_PREPARE(16)
+  if (a.N <= 64) AYK_LA_PREPARE(1)
+  else if (a.N <= 128) AYK_LA_PREPARE(2)
+  else if (a.N <= 256) AYK_LA_PREPARE(4)
+  else AYK_LA_PREPARE(8)
 #undef AYK_LA_PREPARE
 #undef AYK_LA_PREPARE_AS
   if (status != AYK_OK) return status;
   return la_scan(a, a.delta ? MODE_DELTA : MODE_PLAIN, s);
 }
 
+template <int MODE, int KS> static int la_scan_mma_as(const LinearArgs& a, cudaStream_t s) {
+  static const cudaError_t allowed = cudaFuncSetAttribute(
+      la_scan_mma_kernel<MODE, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      (int)LaShare<MODE, KS>::BYTES);
+  if (allowed != cudaSuccess) return (int)allowed;
+  return launch_kernel(la_scan_mma_kernel<MODE, KS>,
+                       dim3(a.heads, a.requests, (a.P + LA_COLS - 1) / LA_COLS), dim3(128),
+                       LaShare<MODE, KS>::BYTES, s, 1, a);
+}
+
 // The scan over the chunks' matrices.
 static int la_scan(const LinearArgs& a, int mode, cudaStream_t s) {
+  if (la_in_fragments(a.N)) {
+#define AYK_LA_MMA(MODE) return a.N <= 64 ? la_scan_mma_as<MODE, 1>(a, s) : la_scan_mma_as<MODE, 2>(a, s)
+    if (mode == MODE_GENERAL) AYK_LA_MMA(MODE_GENERAL);
+    if (mode == MODE_DELTA) AYK_LA_MMA(MODE_DELTA);
+    AYK_LA_MMA(MODE_PLAIN);
+#undef AYK_LA_MMA
+  }
   const int tiles = (a.P + LA_COLS - 1) / LA_COLS;
   const int vec = ((uintptr_t)a.in % 16) == 0 && a.ld_in % 4 == 0 && a.v_at % 4 == 0 &&
                   a.P % 4 == 0;
@@ -1435,7 +1589,7 @@ AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v
   const GeneralArgs g = {proj,    z,    a_bias,   row_start, scratch, ld_proj,
                          ld_z,    k_offset, a_offset, requests,  heads,   N,
                          decay_rate};
-  const size_t smem = (size_t)5 * LA_C * la_pad4(N) * sizeof(float);
+  const size_t smem = (size_t)5 * LA_C * la_row_floats(N) * sizeof(float);
   cudaStream_t s = (cudaStream_t)stream;
   int status;
 #define AYK_GENERAL(M)                                                                             \
@@ -1443,7 +1597,7 @@ AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v
     static const cudaError_t allowed =                                                             \
         cudaFuncSetAttribute(general_prepare_kernel<M>,                                            \
                              cudaFuncAttributeMaxDynamicSharedMemorySize,                          \
-                             5 * LA_C * 64 * M * (int)sizeof(float));                              \
+                             5 * LA_C * (64 * M + 8) * (int)sizeof(float));                        \
     if (allowed != cudaSuccess) return (int)allowed;                                               \
     status = launch_kernel(general_prepare_kernel<M>, dim3(chunks, heads), dim3(LA_THREADS), smem, s,\
                            1, g);                                                                  \

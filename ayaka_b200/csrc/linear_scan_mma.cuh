@@ -1,0 +1,414 @@
+// The scan over a request's chunk matrices (linear_attention.cu) in matrix instructions: heads of whole
+// 16-channel groups, at most 128 channels. Included by linear_attention.cu.
+//
+// A CTA of four warps holds 16 columns of a head's state, S^T as the accumulator fragments of
+// mma.sync.m16n8k16 (a warp: KS groups of 16 channels), which are at the same time the layout the next
+// product takes its left operand in: the state never leaves the registers. Per chunk a warp multiplies
+// its channels of S^T with its channels of the chunk's first matrix, the four shares meet in shared
+// memory (the one barrier of a chunk; two buffers in turn), every warp forms W^T from them, in registers
+// again, and from W^T its channels of the new state; two warps do the rows of O.
+//
+// mma.sync has no 32-bit mode. Operands are taken apart into three bfloat16 numbers each (24 bits) and the
+// six products that 32 bits can hold are added up, the first apart from the five smaller ones, 16 terms
+// in an instruction at a time; what is kept across instructions is added in fp32, rounded to nearest.
+// Errors against float64 beside those of fp32 FMAs (2-norm of the rows, of the states, 1e-7; 2,048 to 4,096
+// rows): decay per channel 2.58 -> 2.34, 2.18 -> 2.00; per head 2.44 -> 2.16, 1.98 -> 1.72; retention 23.1
+// -> 22.1, 29.9 -> 28.8; gated linear attention 1.75 -> 1.55, 1.57 -> 1.38. An operand that is no number or infinite
+// makes every sum it enters no number, also where its factor is zero: such sums are formed again with
+// FMAs (la_plain_tile), so a later row never reaches an earlier one.
+//
+// Bound by the chain of a chunk (split, 24 and 12 MMAs, the exchange) where a request is long, else by
+// MMA issue. With 4 x 4 register tiles on the FMA pipes (la_scan_kernel, which serves other sizes)
+// shared memory bounds a chunk: every lane fetches its own copy of what an MMA shares. Measured on a B200,
+// the scan alone, before and after, microseconds: delta rule, 32 heads of 64 x 64, 4,096 rows of one
+// request 347 -> 312, 2,748 rows of twelve 211 -> 134; retention, 16 heads of 64 x 128, 4,096 rows 318 ->
+// 286; gated linear attention, 8 heads of 128 x 256, 2,048 rows of three 190 -> 139; general delta rule,
+// 16 heads of 64 x 64, 4 x 1,024 rows 174 -> 108.
+//
+// The chunk's matrices lie in the scratch as the fragments of the right operand, piece by piece of 16 k x
+// 8 columns: 32 lanes x 4 floats, lane 4 g + t holding k = 2 t, 2 t + 1, 2 t + 8, 2 t + 9 of column g.
+//   M  [N / 16][J][32][4]  column tiles: rows of Kt (2, with the delta rule), rows of Qt (2)
+//   Kh [N / 16][2][32][4]  k: rows of the chunk, columns: channels;  Ah likewise (MODE_GENERAL)
+//   G  [N],  R [2][32][4]  k: rows of W, columns: rows of O
+#pragma once
+
+namespace ayk {
+
+constexpr int LM_STAGES = 4;
+
+__device__ __forceinline__ void la_split2(float x, float y, uint32_t (&u)[3]) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const __nv_bfloat162 pair = __floats2bfloat162_rn(x, y);
+    u[p] = *reinterpret_cast<const uint32_t*>(&pair);
+    if (p < 2) {  // what is left (exact)
+      x -= __uint_as_float(u[p] << 16);
+      y -= __uint_as_float(u[p] & 0xffff0000u);
+    }
+  }
+}
+
+struct LaLeft {  // 16 columns x 16 k, three parts
+  uint32_t r[3][4];
+  // from two neighbouring accumulator tiles
+  __device__ __forceinline__ void set(const float (&a)[4], const float (&b)[4]) {
+    uint32_t u[3];
+    la_split2(a[0], a[1], u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) r[p][0] = u[p];
+    la_split2(a[2], a[3], u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) r[p][1] = u[p];
+    la_split2(b[0], b[1], u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) r[p][2] = u[p];
+    la_split2(b[2], b[3], u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) r[p][3] = u[p];
+  }
+};
+struct LaRight {  // 16 k x 8 columns, three parts
+  uint32_t r[3][2];
+  LaRight() = default;
+  __device__ __forceinline__ explicit LaRight(const float4& f) {
+    uint32_t u[3];
+    la_split2(f.x, f.y, u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) r[p][0] = u[p];
+    la_split2(f.z, f.w, u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) r[p][1] = u[p];
+  }
+};
+
+__device__ __forceinline__ void la_mma(float (&d)[4], const uint32_t (&a)[4],
+                                       const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// d = a b. (Three short chains of instructions, by the products' sizes.)
+__device__ __forceinline__ void la_mma6(float (&d)[4], const LaLeft& a, const LaRight& b) {
+  float first[4], rest[4], least[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) first[e] = rest[e] = least[e] = 0.f;
+  la_mma(least, a.r[0], b.r[2]);
+  la_mma(rest, a.r[0], b.r[1]);
+  la_mma(first, a.r[0], b.r[0]);
+  la_mma(least, a.r[2], b.r[0]);
+  la_mma(rest, a.r[1], b.r[0]);
+  la_mma(least, a.r[1], b.r[1]);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) d[e] = first[e] + (rest[e] + least[e]);
+}
+__device__ __forceinline__ bool la_odd(const float (&x)[4]) {
+  return x[0] != x[0] || x[1] != x[1] || x[2] != x[2] || x[3] != x[3];
+}
+// The product of one piece with FMAs: entries of d that are no number are replaced (added up over the
+// calls for several pieces in `sum`, which starts at zero). `causal` >= 0: k counts the rows of W and
+// the piece's column g is row causal + g of O; later rows are left out. All lanes of the warp.
+__device__ __forceinline__ void la_plain_tile(float (&sum)[4], const float (&a)[4],
+                                              const float (&b)[4], const float* piece, int causal) {
+  const int lane = threadIdx.x & 31, t = lane & 3;
+#pragma unroll 1
+  for (int n = 0; n < 8; ++n) {
+    const float4 f = *reinterpret_cast<const float4*>(piece + (n * 4 + t) * 4);
+    const int last = causal < 0 ? LA_C : causal + n;  // the last k that counts
+    float x = 0.f, y = 0.f;
+    if (2 * t <= last) x = a[0] * f.x, y = a[2] * f.x;
+    if (2 * t + 1 <= last) x = fmaf(a[1], f.y, x), y = fmaf(a[3], f.y, y);
+    if (2 * t + 8 <= last) x = fmaf(b[0], f.z, x), y = fmaf(b[2], f.z, y);
+    if (2 * t + 9 <= last) x = fmaf(b[1], f.w, x), y = fmaf(b[3], f.w, y);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    y += __shfl_xor_sync(0xffffffffu, y, 2);
+    if ((n >> 1) == t) {
+      sum[0] += n & 1 ? 0.f : x;
+      sum[1] += n & 1 ? x : 0.f;
+      sum[2] += n & 1 ? 0.f : y;
+      sum[3] += n & 1 ? y : 0.f;
+    }
+  }
+}
+__device__ __forceinline__ void la_mend(float (&d)[4], const float (&sum)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) d[e] = d[e] != d[e] ? sum[e] : d[e];
+}
+
+// floats of a warp's share of a chunk
+template <int MODE, int KS> struct LaShare {
+  static constexpr int J = MODE == MODE_PLAIN ? 2 : 4;
+  static constexpr int M = 0, KH = KS * J * 128, AH = KH + KS * 256;
+  static constexpr int R = AH + (MODE == MODE_GENERAL ? KS * 256 : 0), G = R + 128;
+  static constexpr int FLOATS = G + KS * 16;
+  static constexpr int EXCHANGE = 2 * 4 * J * 128;  // [buffer][warp][tile][lane][4]
+  static constexpr size_t BYTES = (size_t)(LM_STAGES * 4 * FLOATS + EXCHANGE) * sizeof(float);
+};
+
+// grid (heads, requests, tiles of 16 columns)
+template <int MODE, int KS>  // KS >= N / 64
+__global__ void __launch_bounds__(128, 3)
+la_scan_mma_kernel(const LinearArgs a) {
+  using L = LaShare<MODE, KS>;
+  constexpr int J = L::J;
+  constexpr bool DELTA = MODE != MODE_PLAIN;
+  extern __shared__ __align__(16) float la_smem[];
+  pdl_launch_dependents();
+  const int N = a.N, P = a.P, h = blockIdx.x, b = blockIdx.y, p0 = blockIdx.z * LA_COLS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  float* ring = la_smem + warp * LM_STAGES * L::FLOATS;  // this warp's
+  float* exchange = la_smem + 4 * LM_STAGES * L::FLOATS;
+  const int r0 = a.row_start[b], rows = a.row_start[b + 1] - r0;
+  if (a.state_slot[b] < 0 || rows <= 0) return;
+  int before = 0;  // chunks of the requests ahead
+  for (int i = 0; i < b; ++i) {
+    before += (a.row_start[i + 1] - a.row_start[i] + LA_C - 1) / LA_C;
+  }
+  float* mine = a.state + (size_t)a.state_slot[b] * a.state_stride + (size_t)h * N * P;
+  const float* in = a.in;
+  const float* scratch = a.scratch;
+  pdl_wait_for(in, scratch, mine);
+  const int chunks = (rows + LA_C - 1) / LA_C, chunk_floats = la_chunk_floats(N, MODE);
+  const int group = warp * KS, groups = N / 16;  // this warp's first group of 16 channels
+  const float* next = scratch + ((size_t)before * a.heads + h) * chunk_floats + lane * 4;
+  auto stage = [&](int c) {  // (called for one chunk after the other)
+    float* at = ring + c % LM_STAGES * L::FLOATS + lane * 4;
+    const float* from = next;
+    next += (size_t)a.heads * chunk_floats;
+    const float* kh = from + 8 * J * N;
+    const float* ah = kh + LA_C * N;
+    const float* rest = ah + (MODE == MODE_GENERAL ? LA_C * N : 0);  // G, R
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      if (group + k < groups) {
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          la_copy16(at + L::M + (k * J + j) * 128, from + ((group + k) * J + j) * 128);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          la_copy16(at + L::KH + (k * 2 + j) * 128, kh + ((group + k) * 2 + j) * 128);
+          if (MODE == MODE_GENERAL) {
+            la_copy16(at + L::AH + (k * 2 + j) * 128, ah + ((group + k) * 2 + j) * 128);
+          }
+        }
+        if (lane < 4) la_copy16(at + L::G + k * 16, rest + (group + k) * 16);
+      }
+    }
+    if (warp < 2) la_copy16(at + L::R, rest + N + warp * 128);
+  };
+  const bool in0 = p0 + g < P, in1 = p0 + g + 8 < P;  // this lane's two columns
+  float v[2][4];  // V^T of the chunk: tiles of 8 rows
+  const float* v_row = in + (size_t)(r0 + 2 * t) * a.ld_in + a.v_at + h * P + p0 + g;
+  auto values = [&](int c) {
+    const int count = rows - c * LA_C - 2 * t;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float* from = v_row + (size_t)(8 * j + e) * a.ld_in;
+        const bool row = 8 * j + e < count;
+        v[j][e] = row && in0 ? from[0] : 0.f;
+        v[j][2 + e] = row && in1 ? from[8] : 0.f;
+      }
+    v_row += (size_t)LA_C * a.ld_in;
+  };
+#pragma unroll
+  for (int c = 0; c < LM_STAGES - 1; ++c) {
+    if (c < chunks) stage(c);
+    la_commit();
+  }
+  values(0);
+  float s[KS][2][4];  // columns g and g + 8, channels 2 t and 2 t + 1 of every 8
+  auto state_at = [&](int k, int j, int e) {
+    const int n = (group + k) * 16 + j * 8 + 2 * t + (e & 1), p = p0 + g + (e >> 1) * 8;
+    return a.transposed ? (size_t)p * N + n : (size_t)n * P + p;
+  };
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[k][j][e] = group + k < groups && (e < 2 ? in0 : in1) ? mine[state_at(k, j, e)] : 0.f;
+      }
+  for (int c = 0; c < chunks; ++c) {
+    la_wait<LM_STAGES - 2>();
+    __syncwarp();  // chunk c has landed, and every lane is done with chunk c - 1
+    if (c + LM_STAGES - 1 < chunks) stage(c + LM_STAGES - 1);
+    la_commit();
+    const float* at = ring + c % LM_STAGES * L::FLOATS;
+    // what does not depend on the state is taken apart beside the first products
+    auto piece = [&](int at_floats) {
+      return LaRight(*reinterpret_cast<const float4*>(at + at_floats + lane * 4));
+    };
+    LaRight kh[KS][2], ah[KS][2], r;
+    // this warp's share of S_0^T [Kt; Qt]^T
+    float part[J][4];
+    {
+      bool odd = false;
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) part[j][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        if (group + k < groups) {
+          LaLeft left;
+          left.set(s[k][0], s[k][1]);
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            float x[4];
+            la_mma6(x, left, piece(L::M + (k * J + j) * 128));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[j][e] = k == 0 ? x[e] : part[j][e] + x[e];
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            kh[k][j] = piece(L::KH + (k * 2 + j) * 128);
+            if (MODE == MODE_GENERAL) ah[k][j] = piece(L::AH + (k * 2 + j) * 128);
+          }
+        }
+      }
+      if (warp < 2) r = piece(L::R);
+#pragma unroll
+      for (int j = 0; j < J; ++j) odd |= la_odd(part[j]);
+      if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int k = 0; k < KS; ++k) {
+            if (group + k < groups) {
+              la_plain_tile(sum, s[k][0], s[k][1], at + L::M + (k * J + j) * 128, -1);
+            }
+          }
+          la_mend(part[j], sum);
+        }
+      }
+    }
+    float* shares = exchange + (c & 1) * 4 * J * 128;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      *reinterpret_cast<float4*>(shares + (warp * J + j) * 128 + lane * 4) =
+          make_float4(part[j][0], part[j][1], part[j][2], part[j][3]);
+    }
+    __syncthreads();
+    auto total = [&](int j, float (&x)[4]) {  // the four warps' shares, in order
+      float4 y = *reinterpret_cast<const float4*>(shares + j * 128 + lane * 4);
+#pragma unroll
+      for (int w = 1; w < 4; ++w) {
+        const float4 z =
+            *reinterpret_cast<const float4*>(shares + (w * J + j) * 128 + lane * 4);
+        y.x += z.x;
+        y.y += z.y;
+        y.z += z.z;
+        y.w += z.w;
+      }
+      x[0] = y.x;
+      x[1] = y.y;
+      x[2] = y.z;
+      x[3] = y.w;
+    };
+    float w[2][4];  // W^T (V^T without the delta rule)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if (DELTA) {
+        total(j, w[j]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          w[j][e] = MODE == MODE_DELTA ? v[j][e] - w[j][e] : -w[j][e];
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[j][e] = v[j][e];
+      }
+    }
+    float u[2][4];  // what R and Kh take
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) u[j][e] = MODE == MODE_GENERAL ? v[j][e] : w[j][e];
+    if (c + 1 < chunks) values(c + 1);
+    LaLeft left, removed;
+    left.set(u[0], u[1]);
+    if (MODE == MODE_GENERAL) removed.set(w[0], w[1]);
+    // the new state
+#pragma unroll
+    for (int k = 0; k < KS; ++k) {
+      if (group + k < groups) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float x[4];
+          la_mma6(x, left, kh[k][j]);
+          if (MODE == MODE_GENERAL) {
+            float away[4];
+            la_mma6(away, removed, ah[k][j]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] += away[e];
+          }
+          if (__any_sync(0xffffffffu, la_odd(x))) {
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            la_plain_tile(sum, u[0], u[1], at + L::KH + (k * 2 + j) * 128, -1);
+            if (MODE == MODE_GENERAL) {
+              la_plain_tile(sum, w[0], w[1], at + L::AH + (k * 2 + j) * 128, -1);
+            }
+            la_mend(x, sum);
+          }
+          const float2 fade =
+              *reinterpret_cast<const float2*>(at + L::G + k * 16 + j * 8 + 2 * t);
+          s[k][j][0] = fmaf(fade.x, s[k][j][0], x[0]);
+          s[k][j][1] = fmaf(fade.y, s[k][j][1], x[1]);
+          s[k][j][2] = fmaf(fade.x, s[k][j][2], x[2]);
+          s[k][j][3] = fmaf(fade.y, s[k][j][3], x[3]);
+        }
+      }
+    }
+    // O: warp 0 the chunk's first eight rows, warp 1 the others
+    if (warp < 2) {
+      float o[4];
+      total(J - 2 + warp, o);
+      float x[4];
+      la_mma6(x, left, r);
+      if (__any_sync(0xffffffffu, la_odd(x))) {
+        // R is zero above the diagonal, but a later row's W may be no number: rows ahead of it get what
+        // they get beside a W of finite entries, its own and later ones what FMAs give
+        float finite[2][4], sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            finite[j][e] = fabsf(u[j][e]) < INFINITY ? u[j][e] : 0.f;
+          }
+        LaLeft again;
+        again.set(finite[0], finite[1]);
+        la_mma6(x, again, r);
+        la_plain_tile(sum, u[0], u[1], at + L::R, 8 * warp);
+        la_mend(x, sum);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = fabsf(sum[e]) < INFINITY ? x[e] : sum[e];
+      }
+      const int row = c * LA_C + warp * 8 + 2 * t;
+      float* to = a.out + (size_t)(r0 + row) * a.ld_out + h * P + p0 + g;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (row + e < rows) {
+          if (in0) to[(size_t)e * a.ld_out] = o[e] + x[e];
+          if (in1) to[(size_t)e * a.ld_out + 8] = o[2 + e] + x[2 + e];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (group + k < groups && (e < 2 ? in0 : in1)) mine[state_at(k, j, e)] = s[k][j][e];
+      }
+}
+
+}  // namespace ayk
