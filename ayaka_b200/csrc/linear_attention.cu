@@ -254,12 +254,19 @@ __device__ __forceinline__ float4 la_mul4(const float4& a, const float4& b) {
   return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
 }
 
+// Four channels of a row from n on, zeros beyond the head.
+__device__ __forceinline__ float4 la_piece(const float* row, int n, int N, int vec) {
+  if (vec && n + 3 < N) return *reinterpret_cast<const float4*>(row + n);
+  return make_float4(n < N ? row[n] : 0.f, n + 1 < N ? row[n + 1] : 0.f,
+                     n + 2 < N ? row[n + 2] : 0.f, n + 3 < N ? row[n + 3] : 0.f);
+}
+
 // grid (chunks, heads). Shared memory: k, q, g and D_(C-1) k as [C][NS], NS = N padded (to a
 // multiple of 4: the padding holds k = q = 0, g = 1). A half warp per row and then per pair of columns of
 // A and B, a lane with four neighbouring channels at a time. Bound by issue and shared memory: 128
 // threads whose half warps take two columns each fetch half of what 256 threads with one column did and
 // exchange a quarter of it. Measured on a B200, microseconds: 32 heads of 64 channels, 4,096 rows, a decay
-// per channel 177 -> 103, per head 138 -> 87; 8 heads of 128, 2,048 rows 38 -> 28. This kernel lets the scan start only when
+// per channel 177 -> 103; 8 heads of 128, 2,048 rows 38 -> 28. This kernel lets the scan start only when
 // it has ended: CTAs of the scan that took their places beside it would crowd on the SMs that empty
 // first, two or three on one (measured: 190 instead of 90 microseconds for 128 CTAs).
 template <int M, bool CHANNEL>  // ceil(N / 64); a decay per channel, or one per row
@@ -292,12 +299,6 @@ la_prepare_kernel(const LinearArgs a, int vec) {
     A[idx / LA_C][idx % LA_C] = 0.f;
     B[idx / LA_C][idx % LA_C] = 0.f;
   }
-  // four channels from n on of a row, `rest` beyond the head
-  auto piece = [&](const float* row, int n, float rest) {
-    if (vec && n + 3 < N) return *reinterpret_cast<const float4*>(row + n);
-    return make_float4(n < N ? row[n] : rest, n + 1 < N ? row[n + 1] : rest,
-                       n + 2 < N ? row[n + 2] : rest, n + 3 < N ? row[n + 3] : rest);
-  };
   // q and k (rotated, of unit length, scaled), the decays, beta
 #pragma unroll 1
   for (int i = part; i < LA_C; i += LA_PREPARE_THREADS / 16) {
@@ -317,18 +318,18 @@ la_prepare_kernel(const LinearArgs a, int vec) {
     for (int m = 0; m < M; ++m) {
       const int n = 4 * (l + 16 * m);
       const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      k[m] = row && n < N ? piece(src + a.k_at + kv * N, n, 0.f) : zero;
-      q[m] = row && n < N ? piece(src + a.q_at + kv * N, n, 0.f) : zero;
+      k[m] = row ? la_piece(src + a.k_at + kv * N, n, N, vec) : zero;
+      q[m] = row ? la_piece(src + a.q_at + kv * N, n, N, vec) : zero;
       float4 g = make_float4(shared_g, shared_g, shared_g, shared_g);
       if (CHANNEL && row && n < N) {
-        float4 z = piece(decay_raw + (size_t)(r0 + i) * a.ld_decay + h * N, n, 0.f);
+        const float4 z = la_piece(decay_raw + (size_t)(r0 + i) * a.ld_decay + h * N, n, N, vec);
         if (a.decay_mode == DECAY_SIGMOID) {
           g.x = la_sigmoid_decay(z.x, a.inv_tau);
           g.y = la_sigmoid_decay(z.y, a.inv_tau);
           g.z = la_sigmoid_decay(z.z, a.inv_tau);
           g.w = la_sigmoid_decay(z.w, a.inv_tau);
         } else {
-          const float4 bias = piece(a.dt_bias + h * N, n, 0.f);
+          const float4 bias = la_piece(a.dt_bias + h * N, n, N, vec);
           g.x = la_decay(rate, z.x + bias.x);
           g.y = la_decay(rate, z.y + bias.y);
           g.z = la_decay(rate, z.z + bias.z);
@@ -560,6 +561,8 @@ la_prepare_kernel(const LinearArgs a, int vec) {
 // The chunk matrices of the generalised delta rule (see the head of this file), laid out for the scan.
 // grid (chunks, heads). Shared memory: u (then Ut), r (then Rt), k (then Kh), a u (then Ah) and w
 // (then U') as [C][NS].
+// Half warps as in la_prepare_kernel: 16 heads of 64 channels, 4 x 1,024 rows 188 -> 88 microseconds against
+// 256 threads with a column each.
 struct GeneralArgs {
   const float* proj;    // r at 0, k at k_at, raw rates at a_at (heads x N each)
   const float* z;       // raw decays, heads x N a row
@@ -571,14 +574,15 @@ struct GeneralArgs {
 };
 
 template <int M>  // ceil(N / 64)
-__global__ void __launch_bounds__(LA_THREADS)
-general_prepare_kernel(const GeneralArgs a) {
+__global__ void __launch_bounds__(LA_PREPARE_THREADS)
+general_prepare_kernel(const GeneralArgs a, int vec) {
   extern __shared__ __align__(16) float la_smem[];
   __shared__ __align__(16) float Lk[LA_C][LA_C], La[LA_C][LA_C], Mk[LA_C][LA_C], Ma[LA_C][LA_C];
   __shared__ __align__(16) float T[LA_C][LA_C], Tk[LA_C][LA_C];
   const int N = a.N, NS = la_row_floats(N), h = blockIdx.y;
   const bool fragments = la_in_fragments(N);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int l = lane & 15, part = tid >> 4;  // the half warp of eight
   float* u_s = la_smem;
   float* r_s = u_s + LA_C * NS;
   float* k_s = r_s + LA_C * NS;
@@ -592,86 +596,115 @@ general_prepare_kernel(const GeneralArgs a) {
   pdl_wait_for(proj, z, scratch);
   if (!found) return;
   const int r0 = a.row_start[b] + t0;
-  if (tid < LA_C * LA_C) {
-    Lk[tid / LA_C][tid % LA_C] = La[tid / LA_C][tid % LA_C] = 0.f;
-    Mk[tid / LA_C][tid % LA_C] = Ma[tid / LA_C][tid % LA_C] = 0.f;
+#pragma unroll
+  for (int idx = tid; idx < LA_C * LA_C; idx += LA_PREPARE_THREADS) {
+    Lk[idx / LA_C][idx % LA_C] = La[idx / LA_C][idx % LA_C] = 0.f;
+    Mk[idx / LA_C][idx % LA_C] = Ma[idx / LA_C][idx % LA_C] = 0.f;
   }
-  for (int i = warp; i < LA_C; i += LA_THREADS / 32) {  // a warp per row
+#pragma unroll 1
+  for (int i = part; i < LA_C; i += LA_PREPARE_THREADS / 16) {  // a half warp per row
     const bool row = i < count;
     const float* src = proj + (size_t)(r0 + i) * a.ld_proj + (size_t)h * N;
+    const float* raw = z + (size_t)(r0 + i) * a.ld_z + (size_t)h * N;
+    const float* bias = a.a_bias + (size_t)h * N;
+    float4 k[M];
     float kk = 0.f;
-    for (int n = lane; n < NS; n += 32) {
-      const float k = row && n < N ? src[a.k_at + n] : 0.f;
-      k_s[i * NS + n] = k;
-      kk = fmaf(k, k, kk);
-    }
-    const float inv = 1.f / sqrtf(warp_sum(kk) + 1e-6f);
-    for (int n = lane; n < NS; n += 32) {
-      const bool live = row && n < N;
-      const float u = k_s[i * NS + n] * inv;
-      u_s[i * NS + n] = u;
-      r_s[i * NS + n] = live ? src[n] : 0.f;
-      au_s[i * NS + n] = live ? u * la_sigmoid(src[a.a_at + n] + a.a_bias[h * N + n]) : 0.f;
-      g_s[i * NS + n] =
-          live ? expf(-a.decay_rate * la_sigmoid(z[(size_t)(r0 + i) * a.ld_z + h * N + n])) : 1.f;
-    }
-  }
-  __syncthreads();
-  {  // the four matrices: warp w takes columns w and C - 1 - w, half a warp each, four neighbouring
-     // channels a lane at a time; what a column's row carries (k_j and a_j u_j, faded) ends as Kh, Ah
-    const int half = lane >> 4, l = lane & 15, j = half ? LA_C - 1 - warp : warp;
-    float4 dk[M], da[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       const int n = 4 * (l + 16 * m);
-      dk[m] = n < NS ? *reinterpret_cast<const float4*>(k_s + j * NS + n)
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
-      da[m] = n < NS ? *reinterpret_cast<const float4*>(au_s + j * NS + n)
-                     : make_float4(0.f, 0.f, 0.f, 0.f);
+      k[m] = row ? la_piece(src + a.k_at, n, N, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+      kk = la_dot4(k[m], k[m], kk);
     }
-    for (int i = warp; i < LA_C; ++i) {  // (warp: the smaller of the two columns)
-      float lk = 0.f, la = 0.f, mk = 0.f, ma = 0.f;
-      if (i >= j) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
+    const float inv = 1.f / sqrtf(kk + 1e-6f);
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int n = 4 * (l + 16 * m);
+      if (n >= NS) continue;
+      const float4 u = la_mul4(k[m], make_float4(inv, inv, inv, inv));
+      float4 r = make_float4(0.f, 0.f, 0.f, 0.f), au = r, g = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (row) {  // (channels beyond the head have u = 0, and no weight in any sum)
+        const float4 y = la_piece(src + a.a_at, n, N, vec), c = la_piece(bias, n, N, vec);
+        const float4 w = la_piece(raw, n, N, vec);
+        r = la_piece(src, n, N, vec);
+        au = make_float4(u.x * la_sigmoid(y.x + c.x), u.y * la_sigmoid(y.y + c.y),
+                         u.z * la_sigmoid(y.z + c.z), u.w * la_sigmoid(y.w + c.w));
+        g = make_float4(expf(-a.decay_rate * la_sigmoid(w.x)), expf(-a.decay_rate * la_sigmoid(w.y)),
+                        expf(-a.decay_rate * la_sigmoid(w.z)), expf(-a.decay_rate * la_sigmoid(w.w)));
+      }
+      *reinterpret_cast<float4*>(u_s + i * NS + n) = u;
+      *reinterpret_cast<float4*>(r_s + i * NS + n) = r;
+      *reinterpret_cast<float4*>(k_s + i * NS + n) = k[m];
+      *reinterpret_cast<float4*>(au_s + i * NS + n) = au;
+      *reinterpret_cast<float4*>(g_s + i * NS + n) = g;
+    }
+  }
+  __syncthreads();
+  {  // the four matrices: a half warp takes columns `part` and C - 1 - part, two rows at a time, four
+     // neighbouring channels a lane; what a column's row carries (k_j and a_j u_j, faded) ends as Kh, Ah
+    const int j[2] = {part, LA_C - 1 - part};
+    const int least[2] = {warp * 2, LA_C - 2 - 2 * warp};  // the smaller of the warp's two, each
+    float4 dk[2][M], da[2][M];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int n = 4 * (l + 16 * m);
+        dk[e][m] = n < NS ? *reinterpret_cast<const float4*>(k_s + j[e] * NS + n)
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+        da[e][m] = n < NS ? *reinterpret_cast<const float4*>(au_s + j[e] * NS + n)
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll 1
+    for (int i0 = least[0]; i0 < LA_C; i0 += 2) {
+      const bool both = i0 + 1 >= least[1];
+      float v[16];  // of row i0 + k, column e: Lk, La, Mk, Ma
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int i = i0 + k;
 #pragma unroll
         for (int m = 0; m < M; ++m) {
           const int n = 4 * (l + 16 * m);
           if (n < NS) {
-            if (i > j) {
-              const float4 u = *reinterpret_cast<const float4*>(u_s + i * NS + n);
-              const float4 g = *reinterpret_cast<const float4*>(g_s + i * NS + n);
-              lk = fmaf(u.x, dk[m].x, fmaf(u.y, dk[m].y, fmaf(u.z, dk[m].z, fmaf(u.w, dk[m].w, lk))));
-              la = fmaf(u.x, da[m].x, fmaf(u.y, da[m].y, fmaf(u.z, da[m].z, fmaf(u.w, da[m].w, la))));
-              dk[m] = make_float4(dk[m].x * g.x, dk[m].y * g.y, dk[m].z * g.z, dk[m].w * g.w);
-              da[m] = make_float4(da[m].x * g.x, da[m].y * g.y, da[m].z * g.z, da[m].w * g.w);
-            }
+            const float4 u = *reinterpret_cast<const float4*>(u_s + i * NS + n);
+            const float4 g = *reinterpret_cast<const float4*>(g_s + i * NS + n);
             const float4 r = *reinterpret_cast<const float4*>(r_s + i * NS + n);
-            mk = fmaf(r.x, dk[m].x, fmaf(r.y, dk[m].y, fmaf(r.z, dk[m].z, fmaf(r.w, dk[m].w, mk))));
-            ma = fmaf(r.x, da[m].x, fmaf(r.y, da[m].y, fmaf(r.z, da[m].z, fmaf(r.w, da[m].w, ma))));
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              if (e == 0 || both) {
+                float* x = v + 8 * k + 4 * e;
+                x[0] = la_dot4(u, dk[e][m], x[0]);
+                x[1] = la_dot4(u, da[e][m], x[1]);
+                if (i > j[e]) {
+                  dk[e][m] = la_mul4(dk[e][m], g);
+                  da[e][m] = la_mul4(da[e][m], g);
+                }
+                x[2] = la_dot4(r, dk[e][m], x[2]);
+                x[3] = la_dot4(r, da[e][m], x[3]);
+              }
+            }
           }
         }
       }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        lk += __shfl_xor_sync(0xffffffffu, lk, o);
-        la += __shfl_xor_sync(0xffffffffu, la, o);
-        mk += __shfl_xor_sync(0xffffffffu, mk, o);
-        ma += __shfl_xor_sync(0xffffffffu, ma, o);
-      }
-      if (l == 0 && i >= j) {
-        Lk[i][j] = lk;
-        La[i][j] = la;
-        Mk[i][j] = mk;
-        Ma[i][j] = ma;
+      const float sum = la_transposed_sum(v);
+      const int i = i0 + (l >> 3), column = l & 4 ? j[1] : j[0];
+      if (i > column || (i == column && (l & 2))) {
+        (l & 2 ? (l & 1 ? Ma : Mk) : (l & 1 ? La : Lk))[i][column] = sum;
       }
     }
 #pragma unroll
-    for (int m = 0; m < M; ++m) {  // (nobody else reads these rows)
-      const int n = 4 * (l + 16 * m);
-      if (n < NS) {
-        *reinterpret_cast<float4*>(k_s + j * NS + n) = dk[m];
-        *reinterpret_cast<float4*>(au_s + j * NS + n) = da[m];
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {  // (nobody else reads these rows)
+        const int n = 4 * (l + 16 * m);
+        if (n < NS) {
+          *reinterpret_cast<float4*>(k_s + j[e] * NS + n) = dk[e][m];
+          *reinterpret_cast<float4*>(au_s + j[e] * NS + n) = da[e][m];
+        }
       }
-    }
   }
   __syncthreads();
   float* m_out = scratch + ((size_t)blockIdx.x * a.heads + h) * la_chunk_floats(N, MODE_GENERAL);
@@ -692,7 +725,7 @@ general_prepare_kernel(const GeneralArgs a) {
       }
     }
   } else {  // meanwhile Ut, Rt and G, a channel a thread
-    for (int n = tid - 32; n < N; n += LA_THREADS - 32) {
+    for (int n = tid - 32; n < N; n += LA_PREPARE_THREADS - 32) {
       float g = 1.f;
       for (int i = 0; i < LA_C; ++i) {
         u_s[i * NS + n] *= g;
@@ -703,8 +736,9 @@ general_prepare_kernel(const GeneralArgs a) {
     }
   }
   __syncthreads();
-  if (tid < LA_C * LA_C) {
-    const int i = tid / LA_C, j = tid % LA_C;
+#pragma unroll
+  for (int idx = tid; idx < LA_C * LA_C; idx += LA_PREPARE_THREADS) {
+    const int i = idx / LA_C, j = idx % LA_C;
     float s = 0.f;
 #pragma unroll
     for (int m = 0; m < LA_C; ++m) {
@@ -716,7 +750,7 @@ general_prepare_kernel(const GeneralArgs a) {
   // a warp 32 channels of the same rows: no bank conflicts, and the small matrices are broadcast.
   // What lies above a matrix's diagonal is never multiplied: an entry of a later row may be infinite,
   // and zero times that is not zero.
-  for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
+  for (int idx = tid; idx < 2 * N; idx += LA_PREPARE_THREADS) {
     const int n = idx % N, first = idx / N * 8;
     float s[8];
 #pragma unroll
@@ -737,16 +771,17 @@ general_prepare_kernel(const GeneralArgs a) {
     for (int e = 0; e < 8; ++e) g_s[(first + e) * NS + n] = s[e];
   }
   __syncthreads();
-  if (tid < LA_C * LA_C) {
-    const int i = tid / LA_C, j = tid % LA_C;
+#pragma unroll
+  for (int idx = tid; idx < LA_C * LA_C; idx += LA_PREPARE_THREADS) {
+    const int i = idx / LA_C, j = idx % LA_C;
     float s = Mk[i][j];
 #pragma unroll
     for (int m = 0; m < LA_C; ++m) {
       if (m <= i) s = fmaf(-Ma[i][m], Tk[m][j], s);
     }
-    r_out[fragments ? (i >> 3) * 128 + la_fragment(j, i & 7) : tid] = s;
+    r_out[fragments ? (i >> 3) * 128 + la_fragment(j, i & 7) : idx] = s;
   }
-  for (int idx = tid; idx < 2 * N; idx += LA_THREADS) {
+  for (int idx = tid; idx < 2 * N; idx += LA_PREPARE_THREADS) {
     const int n = idx % N, first = idx / N * 8;
     float q[8], kh[8];
 #pragma unroll
@@ -803,13 +838,13 @@ general_prepare_kernel(const GeneralArgs a) {
   }
   if (!fragments) return;
   __syncthreads();
-  for (int idx = tid; idx < N * 8; idx += LA_THREADS) {  // U' and Rt in pieces
+  for (int idx = tid; idx < N * 8; idx += LA_PREPARE_THREADS) {  // U' and Rt in pieces
     const int l = idx & 31, j = (idx >> 5) & 3, group = idx >> 7;
     const float* x = (j < 2 ? g_s : r_s) + ((j & 1) * 8 + (l >> 2)) * NS + group * 16 + (l & 3) * 2;
     const float2 x0 = *reinterpret_cast<const float2*>(x), x1 = *reinterpret_cast<const float2*>(x + 8);
     *reinterpret_cast<float4*>(m_out + (size_t)idx * 4) = make_float4(x0.x, x0.y, x1.x, x1.y);
   }
-  for (int idx = tid; idx < N * 8; idx += LA_THREADS) {  // Kh, then Ah
+  for (int idx = tid; idx < N * 8; idx += LA_PREPARE_THREADS) {  // Kh, then Ah
     const int which = idx / (N * 4), at = idx - which * N * 4, n = at >> 2, t = at & 3;
     const float* x = (which ? au_s : k_s) + 2 * t * NS + n;
     *reinterpret_cast<float4*>(kh_out + (size_t)idx * 4) =
@@ -1590,6 +1625,9 @@ AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v
                          ld_z,    k_offset, a_offset, requests,  heads,   N,
                          decay_rate};
   const size_t smem = (size_t)5 * LA_C * la_row_floats(N) * sizeof(float);
+  const int vec = N % 4 == 0 && ld_proj % 4 == 0 && ld_z % 4 == 0 && k_offset % 4 == 0 &&
+                  a_offset % 4 == 0 &&
+                  ((uintptr_t)proj | (uintptr_t)z | (uintptr_t)a_bias) % 16 == 0;
   cudaStream_t s = (cudaStream_t)stream;
   int status;
 #define AYK_GENERAL(M)                                                                             \
@@ -1599,8 +1637,8 @@ AYK_API int ayk_delta_chunks(const float* proj, int ld_proj, int k_offset, int v
                              cudaFuncAttributeMaxDynamicSharedMemorySize,                          \
                              5 * LA_C * (64 * M + 8) * (int)sizeof(float));                        \
     if (allowed != cudaSuccess) return (int)allowed;                                               \
-    status = launch_kernel(general_prepare_kernel<M>, dim3(chunks, heads), dim3(LA_THREADS), smem, s,\
-                           1, g);                                                                  \
+    status = launch_kernel(general_prepare_kernel<M>, dim3(chunks, heads),                         \
+                           dim3(LA_PREPARE_THREADS), smem, s, 1, g, vec);                          \
   }
   if (N <= 64) AYK_GENERAL(1)
   else if (N <= 128) AYK_GENERAL(2)

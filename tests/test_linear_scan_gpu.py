@@ -1,0 +1,70 @@
+"""The chunked scans of heads of whole groups of 16 channels (matrix instructions) against the recurrences
+in float64: one to eight groups, ragged columns and rows; and rows that are no numbers."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+import test_memory_chunks_gpu as chunks
+import test_senurax_kernels_gpu as senurax
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(3, 16, 17), (2, 48, 7), (2, 64, 40), (1, 80, 64), (2, 112, 16), (1, 128, 33)]
+
+
+@pytest.mark.parametrize("rows", [*chunks.ROWS, [16, 15, 17]])
+@pytest.mark.parametrize("heads,inner,columns", SIZES)
+def test_gated_and_general_delta_scans(heads, inner, columns, rows):
+    chunks.test_gated_linear_attention_in_chunks(heads, inner, columns, rows)
+    chunks.test_generalised_delta_rule_in_chunks(heads, inner, columns, rows)
+
+
+@pytest.mark.parametrize("decay,heads,kv,dim,columns,rot", [
+    ("head", 4, 2, 48, 20, None), ("channel", 2, 2, 128, 40, None), ("fixed", 2, 2, 16, 16, 16),
+    ("fixed", 1, 1, 112, 9, None), ("head", 2, 1, 16, 17, None), ("channel", 2, 1, 80, 16, None)])
+def test_delta_rule_and_retention(decay, heads, kv, dim, columns, rot):
+    senurax.test_the_recurrences_in_chunks(decay, heads, kv, dim, columns, rot)
+
+
+@pytest.mark.parametrize("row", [1, 10, 15, 37, 63, 90])
+@pytest.mark.parametrize("inner", [48, 96])
+def test_no_later_row_reaches_an_earlier_one(inner, row):
+    from ayaka_b200.kernels import ops
+
+    rows, heads, columns = [70, 130, 66], 2, 36
+    g = torch.Generator("cuda").manual_seed(row)
+    randn = lambda *shape: torch.randn(*shape, generator=g, device="cuda")  # noqa: E731
+    total, qk, width = sum(rows), heads * inner, heads * columns
+    bias = randn(qk)
+
+    def scratch(floats):
+        return torch.full((ops.linear_chunks(rows), heads * (floats * inner + inner + 256)),
+                          float("nan"), device="cuda")
+
+    def gated(q, k, v, z):
+        out = torch.zeros(total, width, device="cuda")
+        ops.gla_scan(torch.cat([q, k, v], 1), z, torch.zeros(4, qk * columns, device="cuda"), out,
+                     heads=heads, dim=inner, columns=columns, k_offset=qk, v_offset=2 * qk, tau=4.0,
+                     q_scale=0.2, scratch=scratch(32), **chunks._step(rows))
+        return out
+
+    def delta(r, k, y, v, z):
+        out = torch.zeros(total, width, device="cuda")
+        ops.delta_scan(torch.cat([r, k, y, v], 1), z, bias,
+                       torch.zeros(4, qk * columns, device="cuda"), out, heads=heads, dim=inner,
+                       columns=columns, k_offset=qk, a_offset=2 * qk, v_offset=3 * qk,
+                       decay_rate=0.6065, scratch=scratch(64), **chunks._step(rows))
+        return out
+
+    operands = dict(k=randn(total, qk), v=randn(total, width), z=randn(total, qk))
+    chunks._rows_before(gated, dict(q=randn(total, qk), **operands), row, rows)
+    chunks._rows_before(delta, dict(r=randn(total, qk), y=randn(total, qk), **operands), row, rows)
+    # what a value that is infinite leaves behind is infinite or no number, in its own column alone
+    first, v = rows[0] + row, operands["v"].clone()
+    v[first, 5] = float("inf")
+    hit = ~torch.isfinite(gated(randn(total, qk), operands["k"], v, operands["z"]))
+    assert hit[first, 5] and not hit[:first].any() and not hit[sum(rows[:2]):].any()
+    hit[:, 5] = False
+    assert not hit.any()
