@@ -1,0 +1,100 @@
+"""The float32 product in bfloat16 parts against float64: remainders of every tile, stretches of K, rows
+that are no numbers, infinite, huge or tiny; and that a row's bits do not depend on its batch."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# rows, columns, K (one stretch, 2, 3, 8; blocks of 64 k with and without a remainder)
+SHAPES = [(1, 1, 4), (16, 128, 64), (17, 129, 68), (129, 2500, 60), (513, 640, 516), (300, 200, 1540),
+          (7, 16, 2048), (81, 256, 3076), (1300, 70, 200)]
+# an element: 64-term sums of exact products, each rounded to 32 bits a few times, then up to 48 added
+TOLERANCE = 5e-7
+
+
+def _operands(m, n, k):
+    g = torch.Generator("cuda").manual_seed(m + n + k)
+    a = torch.randn(m, k + 4, generator=g, device="cuda")[:, :k]
+    w = torch.randn(n, k, generator=g, device="cuda") * k ** -0.5
+    return a, w, torch.randn(n, generator=g, device="cuda"), torch.randn(m, n, generator=g,
+                                                                        device="cuda")
+
+
+def _product(a, w, bias, out, *, residual=False, activation="none", tile=0):
+    from ctypes import c_int, c_void_p
+
+    from ayaka_b200.kernels import flags, lib, ops
+
+    status = lib.entry("gemm_f32", "ayk_gemm_f32")(
+        c_void_p(a.data_ptr()), c_int(a.stride(0)), c_void_p(w.data_ptr()), c_int(w.stride(0)),
+        c_void_p(0 if bias is None else bias.data_ptr()), c_void_p(out.data_ptr()),
+        c_int(out.stride(0)), c_int(a.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]),
+        c_int(ops.ACTIVATIONS[activation]), c_int(int(residual)), c_int(tile),
+        c_void_p(flags.status_word(a.device).data_ptr()), c_void_p(lib.raw_stream()))
+    lib.check(status, "gemm_f32")
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_against_float64(m, n, k):
+    from ayaka_b200.kernels import flags
+
+    a, w, bias, base = _operands(m, n, k)
+    want = a.double() @ w.double().T + bias.double()
+    out, acc = torch.full((m, n), float("nan"), device="cuda"), base.clone()
+    _product(a, w, bias, out)
+    _product(a, w, bias, acc, residual=True)
+    assert (out.double() - want).norm() <= TOLERANCE * want.norm()
+    assert (acc.double() - want - base.double()).norm() <= TOLERANCE * (want + base.double()).norm()
+    _product(a, w, bias, out, activation="gelu_tanh")
+    torch.testing.assert_close(out.double(), torch.nn.functional.gelu(want, approximate="tanh"),
+                               rtol=1e-5, atol=1e-5)
+    assert int(flags.status_word(a.device).item()) == 0
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+def test_a_rows_bits_do_not_depend_on_its_tile(m, n, k):
+    a, w, bias, _ = _operands(m, n, k)
+    whole = torch.empty(m, n, device="cuda")
+    _product(a, w, bias, whole)
+    for tile in range(16, 129, 16):
+        out = torch.empty(m, n, device="cuda")
+        _product(a, w, bias, out, tile=tile)
+        assert torch.equal(out, whole), tile
+    part = torch.empty(1, n, device="cuda")
+    _product(a[m // 2:m // 2 + 1], w, bias, part)
+    assert torch.equal(part[0], whole[m // 2])
+
+
+@pytest.mark.parametrize("m,n,k", [(40, 130, 200), (9, 16, 2048)])
+def test_what_is_no_number_infinite_huge_or_tiny(m, n, k):
+    from ayaka_b200.kernels import ops
+
+    a, w, bias, _ = _operands(m, n, k)
+    a, bias = a.contiguous(), None
+    clean = torch.empty(m, n, device="cuda")
+    _product(a, w, bias, clean)
+    a[1, 3], a[2, k - 1], a[3, 5] = float("inf"), float("nan"), -float("inf")
+    # rounds to an infinite bfloat16; alone, so that no order of its row's sums overflows (|w| < 0.6)
+    a[4, 2] = 3.4e38
+    a[5] *= 1e-36  # parts below what bfloat16 holds
+    a[6] = 0.0
+    w[7, 3] = 0.0  # infinity times zero
+    w[8] *= 1e30
+    want, out = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+    ops.linear(a, w, bias, want, kernel="simt")
+    _product(a, w, bias, out)
+    rows = [i for i in range(m) if not 1 <= i <= 6]
+    same = [i for i in range(n) if i not in (7, 8)]
+    assert torch.equal(out[rows][:, same], clean[rows][:, same])
+    assert torch.equal(out[1:5].isnan(), want[1:5].isnan())
+    assert torch.equal(out[1:5].isinf(), want[1:5].isinf())
+    torch.testing.assert_close(out[4, same], want[4, same], rtol=1e-6, atol=0.0)
+    assert torch.equal(out[6], torch.zeros(n, device="cuda"))
+    # (column 8: entries below 2^-107 lack up to 2^-134 each, against weights of up to 3e29 here)
+    exact, row = a[5].double() @ w.double().T, out[5].double()
+    assert (row[same] - exact[same]).norm() <= 2e-6 * exact[same].norm()
+    assert (row[8:9] - exact[8:9]).norm() <= 2.0 ** -134 * float(w[8:9].double().abs().sum()) + \
+        2e-6 * exact[8:9].norm()
