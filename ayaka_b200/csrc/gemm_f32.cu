@@ -4,20 +4,22 @@
 // which between them hold its 24 bits and its range (to within 2^-27 |x|), and of the nine products of
 // the parts the six that 32 bits can hold are added up:
 //   a w = a1 w1 + (a1 w2 + a2 w1 + a1 w3 + a3 w1 + a2 w2)   to within 2^-26 |a w|.
-// A product of two bfloat16 numbers is exact in fp32. The tensor core's own sums are kept short: 64 k are
-// summed in tensor memory, the first products and the five smaller ones apart, and those sums are added
-// in fp32 registers, rounded to nearest. So the result is a true 32-bit product; against float64 its
+// A product of two bfloat16 numbers is exact in fp32. The tensor core's own sums are kept short: 128 k are
+// summed in tensor memory, products of different size apart, and those sums are added in fp32 registers,
+// rounded to nearest. So the result is a true 32-bit product; against float64 its
 // 2-norm is off by 1.0e-7 (K 768 to 1,024) and 1.1e-7 (3,072), that of FMAs in gemm_simt.cu by 1.8e-7 to
 // 3.5e-7.
 //
 // The weights are the 128-row operand and a tile of NT rows of A the other one, so D[n, m] has a lane
-// per output column whatever M is. Blocks of 32 k travel by TMA into a ring of raw fp32 tiles; warps 0-7
-// turn a block into bf16 tiles of 128-byte rows (x1 | x2, and x3 | nothing) in the layout of TMA's
-// 128-byte swizzle, two in turn; warp 8 issues the MMAs, six per 16 k; warps 8-15 add the accumulators
-// (two in turn) to their registers, lane n of 32 and half of the rows each. K may be cut into stretches by
-// N and K alone (f3_splits); their CTAs are a cluster and add up their sums in order through distributed
-// shared memory. An element's sum has one order whatever M or the tile it falls in: a row's bits do not
-// depend on its batch.
+// per output column whatever M is. Blocks of 32 k travel by TMA into a ring of raw fp32 tiles; all sixteen
+// warps turn a block into bf16 tiles in the layout of TMA's 128-byte swizzle, two in turn: rows of W as
+// w1 | w2 and w3 | nothing, the parts of A's rows below one another, so that three MMAs per 16 k form the
+// six products, w1 [a1 a2 a3], w2 [a1 a2] and w3 a1, in accumulators of their own. One thread issues them;
+// an MMA is short (N up to 240) and what a single thread does for each, descriptors above all, is what
+// bounds a block, so both are kept few. Behind every fourth block the warps add the accumulators to their
+// registers, lane n of 32 and a quarter of the rows each. One block barrier a block. K may be cut into stretches by N and K alone (f3_splits); their CTAs are a cluster and add up their sums in order
+// through distributed shared memory. An element's sum has one order whatever M or the tile it falls in: a
+// row's bits do not depend on its batch.
 //
 // An entry that is no number, infinite, or rounds to infinity makes x2 and so every sum it enters no
 // number; entries below 2^-107 have parts that bfloat16 cannot hold, which may show in a sum that is
@@ -31,26 +33,25 @@
 namespace ayk {
 
 constexpr int F3_BM = 128, F3_BK = 32, F3_STAGES = 2;
-constexpr int F3_SUM_K = 64;  // k of an accumulator
-constexpr int F3_CONVERT_WARPS = 8, F3_SUM_WARPS = 8;
-constexpr int F3_MMA_WARP = F3_CONVERT_WARPS;  // the first sum warp issues the MMAs, a sum ahead
-constexpr int F3_THREADS = 32 * (F3_CONVERT_WARPS + F3_SUM_WARPS);
-constexpr int F3_MAX_NT = 128;
+constexpr int F3_SUM_K = 128;  // k of an accumulator
+constexpr int F3_THREADS = 512;
+constexpr int F3_SUM_BLOCKS = F3_SUM_K / F3_BK;
+constexpr int F3_MAX_NT = 80;  // six accumulators in tensor memory
 
 template <int NT>
 struct F3Smem {
   static constexpr int ROWS = F3_BM + NT;
-  // a stage: rows of W, then of A, 128 bytes x1 | x2 each; then the same rows' x3 | nothing
-  static constexpr int STAGE_BYTES = 2 * ROWS * 128;
+  // a stage, rows of 128 bytes: W's w1 | w2, W's w3 | nothing, A's a1 | nothing, a2 and a3
+  static constexpr int A_OFFSET = 2 * F3_BM * 128;
+  static constexpr int STAGE_BYTES = A_OFFSET + 3 * NT * 128;
   static constexpr int RAW_BYTES = ROWS * F3_BK * 4;
   static constexpr int RAW_OFFSET = F3_STAGES * STAGE_BYTES;
   static constexpr int LIMIT = 226 * 1024;
   static constexpr int FITS = (LIMIT - 1024 - 256 - RAW_OFFSET) / RAW_BYTES;
   static constexpr int RAW = FITS > 6 ? 6 : FITS;  // raw tiles in the ring
   static constexpr int BAR_OFFSET = RAW_OFFSET + RAW * RAW_BYTES;
-  // raw_full[RAW], raw_empty[RAW], full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], then the tmem
-  // slot and the failure flag
-  static constexpr int TOTAL = BAR_OFFSET + (2 * RAW + 2 * F3_STAGES + 4) * 8 + 16;
+  // raw_full[RAW], empty[STAGES], acc_full, then the tmem slot and the failure flag
+  static constexpr int TOTAL = BAR_OFFSET + (RAW + F3_STAGES + 1) * 8 + 16;
   static constexpr int DYNAMIC = TOTAL + 1024;
   static_assert(RAW >= 3, "two blocks on their way while one is converted");
   static_assert(NT * F3_BM * 4 <= RAW_OFFSET, "the stages hold the partial sums at the end");
@@ -89,13 +90,11 @@ __device__ __noinline__ float f3_plain(const float* a, const float* w, int k_fir
   return s;
 }
 
-__device__ __forceinline__ void f3_ld_32x8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7])
-      : "r"(taddr)
-      : "memory");
+__device__ __forceinline__ void f3_ld_32x4(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(taddr)
+               : "memory");
 }
 
 // grid (weight tiles * splits, row tiles), clusters of `splits` along x.
@@ -110,44 +109,32 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
-  uint64_t* raw_empty = raw_full + L::RAW;
-  uint64_t* full = raw_empty + L::RAW;
-  uint64_t* empty = full + F3_STAGES;
+  uint64_t* empty = raw_full + L::RAW;
   uint64_t* acc_full = empty + F3_STAGES;
-  uint64_t* acc_empty = acc_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // two accumulators in turn, each NT columns of first products and NT of the smaller ones
-  constexpr int PITCH = (NT + 31) / 32 * 32;
-  constexpr uint32_t TMEM_COLS = PITCH <= 32 ? 128 : (PITCH <= 64 ? 256 : 512);
-  constexpr int NH = NT / 2;  // rows of a sum warp
+  // the accumulators of w1, w2 and w3
+  constexpr int D2 = (3 * NT + 31) / 32 * 32, D3 = D2 + 2 * NT, D_END = D3 + (NT + 31) / 32 * 32;
+  constexpr uint32_t TMEM_COLS = D_END <= 128 ? 128 : (D_END <= 256 ? 256 : 512);
+  static_assert(D_END <= 512 && D2 % 32 == 0 && D3 % 32 == 0, "tensor memory");
+  constexpr int NQ = NT / 4;  // rows of a warp's sums
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = splits > 1 ? (int)(blockIdx.x % splits) : 0;
   const int n0 = (int)(blockIdx.x / splits) * F3_BM, m0 = blockIdx.y * NT;
   const int k_first = rank * k_split, k_last = min(K, k_first + k_split);
   const int num_kb = (k_last - k_first + F3_BK - 1) / F3_BK;  // blocks
-  const int num_sums = (num_kb + 1) / 2;                      // accumulators, of two blocks each
 
   if (tid == 0) {
-    for (int s = 0; s < L::RAW; ++s) {
-      mbar_init(&raw_full[s], 1);
-      mbar_init(&raw_empty[s], F3_CONVERT_WARPS);
-    }
-    for (int s = 0; s < F3_STAGES; ++s) {
-      mbar_init(&full[s], F3_CONVERT_WARPS);
-      mbar_init(&empty[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], F3_SUM_WARPS);
-    }
+    for (int s = 0; s < L::RAW; ++s) mbar_init(&raw_full[s], 1);
+    for (int s = 0; s < F3_STAGES; ++s) mbar_init(&empty[s], 1);
+    mbar_init(acc_full, 1);
     *failed = 0;
     mbar_fence_init();
     tma_prefetch_map(&map_w);
     tma_prefetch_map(&map_a);
   }
-  if (warp == F3_MMA_WARP) {
+  if (warp == 0) {
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
@@ -157,169 +144,143 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
 
-  float acc[NH];
-  const int quarter = warp & 3, half = (warp - F3_CONVERT_WARPS) >> 2;
-  const int n = n0 + quarter * 32 + lane;  // (sum warps) this lane's output column
-  int issued = 0;                          // blocks whose copies this thread has started
-  if (warp < F3_CONVERT_WARPS) {
-    auto raw_tile = [&](int kb) { return smem + L::RAW_OFFSET + kb % L::RAW * L::RAW_BYTES; };
-    auto bring_w = [&](int kb) {
-      mbar_expect_tx(&raw_full[kb % L::RAW], L::RAW_BYTES);
-      tma_load_2d(raw_tile(kb), &map_w, &raw_full[kb % L::RAW], k_first + kb * F3_BK, n0);
-    };
-    auto bring_a = [&](int kb) {
-      tma_load_2d(raw_tile(kb) + F3_BM * F3_BK * 4, &map_a, &raw_full[kb % L::RAW],
-                  k_first + kb * F3_BK, m0);
-      issued = kb + 1;
-    };
-    constexpr int AHEAD = L::RAW - 1;  // blocks on their way ahead of the one that is converted
-    if (tid == 0) {
-      const int ahead = num_kb < AHEAD ? num_kb : AHEAD;
-      for (int kb = 0; kb < ahead; ++kb) bring_w(kb);  // weights: ahead of the dependency wait
-      pdl_wait();
-      for (int kb = 0; kb < ahead; ++kb) bring_a(kb);
-    }
-    __syncwarp();
-    // ---- a thread: 8 neighbouring k (piece p of 4) of rows r, r + 64, ... of both tiles
-    const int r = tid >> 2, p = tid & 3, x = r & 7;
-    for (int kb = 0; kb < num_kb; ++kb) {
-      const int s = kb % F3_STAGES, at = kb % L::RAW;
-      bool ok = true;
-      if (tid == 0 && kb + AHEAD < num_kb) {
-        // the place of the block converted last, which every warp has read
-        ok = kb == 0 || mbar_wait(&raw_empty[(kb - 1) % L::RAW], ((kb - 1) / L::RAW) & 1);
-        if (ok) {
-          bring_w(kb + AHEAD);
-          bring_a(kb + AHEAD);
-        }
-      }
-      if (lane == 0 && ok) {
-        ok = mbar_wait(&raw_full[at], (kb / L::RAW) & 1) &&
-             (kb < F3_STAGES || mbar_wait(&empty[s], ((kb / F3_STAGES) & 1) ^ 1));
-      }
-      if (!__shfl_sync(0xffffffffu, ok, 0)) {
-        *failed = 1;
-        break;
-      }
-      const uint8_t* raw = raw_tile(kb);
-      uint8_t* tile = smem + s * L::STAGE_BYTES;
-#pragma unroll
-      for (int i = 0; i < (L::ROWS + 63) / 64; ++i) {
-        const int row = r + 64 * i;
-        if (L::ROWS % 64 == 0 || row < L::ROWS) {
-          uint4 plane[3];
-          const uint8_t* from = raw + row * 128;
-          f3_split(*reinterpret_cast<const float4*>(from + (((2 * p) ^ x) << 4)),
-                   *reinterpret_cast<const float4*>(from + (((2 * p + 1) ^ x) << 4)), plane);
-          uint8_t* to = tile + row * 128;
-          // (odd rows store x2 first: two rows side by side in different halves of the banks)
-          const bool odd = x & 1;
-          *reinterpret_cast<uint4*>(to + ((((odd ? 4 : 0) + p) ^ x) << 4)) = odd ? plane[1] : plane[0];
-          *reinterpret_cast<uint4*>(to + ((((odd ? 0 : 4) + p) ^ x) << 4)) = odd ? plane[0] : plane[1];
-          *reinterpret_cast<uint4*>(to + L::ROWS * 128 + ((p ^ x) << 4)) = plane[2];
-        }
-      }
-      fence_proxy_async_shared();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&full[s]);
-        if (kb + L::RAW < num_kb) mbar_arrive(&raw_empty[at]);  // (waited for only then)
-      }
-    }
-  } else {
-    constexpr uint32_t idesc = umma_idesc_bf16(F3_BM, NT);
-    auto issue = [&](int c) {  // the MMAs of an accumulator (one lane)
-      const int buf = c & 1;
-      if (c >= 2 && !mbar_wait(&acc_empty[buf], ((c >> 1) & 1) ^ 1)) return false;
-      const uint32_t first = tmem_base + (uint32_t)(buf * 2 * PITCH), rest = first + PITCH;
-      for (int kb = 2 * c; kb < min(2 * c + 2, num_kb); ++kb) {
-        const int s = kb % F3_STAGES;
-        if (!mbar_wait(&full[s], (kb / F3_STAGES) & 1)) return false;
-        tc_fence_after();
-        const uint8_t* w12 = smem + s * L::STAGE_BYTES;
-        const uint8_t* a12 = w12 + F3_BM * 128;
-        const uint8_t* w3 = w12 + L::ROWS * 128;
-        const uint8_t* a3 = w3 + F3_BM * 128;
-        const uint32_t more = kb != 2 * c;
-        // (one accumulator after the other, not in turn)
-#pragma unroll
-        for (int k = 0; k < F3_BK / 16; ++k) {
-          umma_f16(first, umma_desc_k128(w12, k * 32), umma_desc_k128(a12, k * 32), idesc,
-                   more | (k != 0));
-        }
-#pragma unroll
-        for (int k = 0; k < F3_BK / 16; ++k) {
-          const uint64_t wd[3] = {umma_desc_k128(w12, k * 32), umma_desc_k128(w12, 64 + k * 32),
-                                  umma_desc_k128(w3, k * 32)};
-          const uint64_t ad[3] = {umma_desc_k128(a12, k * 32), umma_desc_k128(a12, 64 + k * 32),
-                                  umma_desc_k128(a3, k * 32)};
-          umma_f16(rest, wd[0], ad[2], idesc, more | (k != 0));
-          umma_f16(rest, wd[2], ad[0], idesc, 1);
-          umma_f16(rest, wd[1], ad[1], idesc, 1);
-          umma_f16(rest, wd[0], ad[1], idesc, 1);
-          umma_f16(rest, wd[1], ad[0], idesc, 1);
-        }
-        umma_commit(&empty[s]);
-      }
-      umma_commit(&acc_full[buf]);
-      return true;
-    };
-    // ---- the sums: lane n, rows half * NH ..
-#pragma unroll
-    for (int j = 0; j < NH; ++j) acc[j] = 0.f;
-    for (int c = 0; c < num_sums; ++c) {
-      const int buf = c & 1;
-      bool have = true;
-      if (lane == 0) {
-        if (warp == F3_MMA_WARP) {
-          if (c == 0) have = issue(0);
-          if (have && c + 1 < num_sums) have = issue(c + 1);
-        }
-        have = have && mbar_wait(&acc_full[buf], (c >> 1) & 1);
-      }
-      if (!__shfl_sync(0xffffffffu, have, 0)) {
-        *failed = 1;
-        break;
-      }
-      tc_fence_after();
-      const uint32_t from = tmem_base + (uint32_t)(buf * 2 * PITCH + half * NH) +
-                            ((uint32_t)(quarter * 32) << 16);
-#pragma unroll
-      for (int j = 0; j < NH; j += 8) {
-        uint32_t y[8], z[8];
-        f3_ld_32x8(from + j, y);
-        f3_ld_32x8(from + PITCH + j, z);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(y[e]) + __uint_as_float(z[e]);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
-    }
+  int issued = 0;  // (thread 32) blocks whose copies it has started
+  auto raw_tile = [&](int slot) { return smem + L::RAW_OFFSET + slot * L::RAW_BYTES; };
+  auto bring_w = [&](int kb, int slot) {
+    mbar_expect_tx(&raw_full[slot], L::RAW_BYTES);
+    tma_load_2d(raw_tile(slot), &map_w, &raw_full[slot], k_first + kb * F3_BK, n0);
+  };
+  auto bring_a = [&](int kb, int slot) {
+    tma_load_2d(raw_tile(slot) + F3_BM * F3_BK * 4, &map_a, &raw_full[slot], k_first + kb * F3_BK, m0);
+    issued = kb + 1;
+  };
+  if (tid == 32) {
+    const int ahead = num_kb < L::RAW ? num_kb : L::RAW;
+    for (int kb = 0; kb < ahead; ++kb) bring_w(kb, kb);  // weights: ahead of the dependency wait
+    pdl_wait();
+    for (int kb = 0; kb < ahead; ++kb) bring_a(kb, kb);
   }
   __syncwarp();
+
+  const int quarter = warp & 3, part = warp >> 2;
+  const int n = n0 + quarter * 32 + lane;  // this lane's output column
+  float acc[NQ];
+#pragma unroll
+  for (int j = 0; j < NQ; ++j) acc[j] = 0.f;
+  uint32_t sums = 0;  // accumulators added so far
+  auto add = [&]() {  // the accumulators to the sums: lane n, rows part * NQ ..
+    if (*failed == 0 && !mbar_wait(acc_full, sums & 1)) *failed = 1;
+    ++sums;
+    __syncwarp();
+    tc_fence_after();
+    const uint32_t from = tmem_base + (uint32_t)(part * NQ) + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+    for (int j = 0; j < NQ; j += 4) {
+      uint32_t x[6][4];
+      f3_ld_32x4(from + j, x[0]);
+      f3_ld_32x4(from + NT + j, x[1]);
+      f3_ld_32x4(from + D2 + j, x[2]);
+      f3_ld_32x4(from + 2 * NT + j, x[3]);
+      f3_ld_32x4(from + D2 + NT + j, x[4]);
+      f3_ld_32x4(from + D3 + j, x[5]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float least = __uint_as_float(x[3][e]) + __uint_as_float(x[4][e]) + __uint_as_float(x[5][e]);
+        const float rest = __uint_as_float(x[1][e]) + __uint_as_float(x[2][e]) + least;
+        acc[j + e] += __uint_as_float(x[0][e]) + rest;
+      }
+    }
+    tc_fence_before();
+  };
+  // descriptors: the low words differ by where a tile starts (in 16 bytes), the high ones not
+  const uint64_t desc0 = umma_desc_k128(smem, 0);
+  auto desc = [&](uint32_t bytes) {
+    return (desc0 & 0xffffffff00000000ull) | ((uint32_t)desc0 + (bytes >> 4));
+  };
+  constexpr uint32_t idesc1 = umma_idesc_bf16(F3_BM, 3 * NT), idesc2 = umma_idesc_bf16(F3_BM, 2 * NT),
+                     idesc3 = umma_idesc_bf16(F3_BM, NT);
+  // a thread: 8 neighbouring k (piece p of 4) of row r of W and, for the first NT, of A
+  const int r = tid >> 2, p = tid & 3, x = r & 7;
+  const bool odd_row = x & 1;
+  const uint32_t raw0 = (uint32_t)(((2 * p) ^ x) << 4), raw1 = (uint32_t)(((2 * p + 1) ^ x) << 4);
+  // (of W, odd rows store x2 first: two rows side by side in different halves of the banks)
+  const uint32_t to0 = (uint32_t)((((odd_row ? 4 : 0) + p) ^ x) << 4);
+  const uint32_t to1 = (uint32_t)((((odd_row ? 0 : 4) + p) ^ x) << 4);
+  const uint32_t to2 = (uint32_t)((p ^ x) << 4);
+  int slot = 0;          // of the raw ring
+  uint32_t round = 0;    // parity of the ring's turn
+  for (int kb = 0; kb < num_kb; ++kb) {
+    const int s = kb & 1;
+    if (*failed == 0 && (!mbar_wait(&raw_full[slot], round) ||
+                         (kb >= F3_STAGES && !mbar_wait(&empty[s], ((kb >> 1) & 1) ^ 1)))) {
+      *failed = 1;
+    }
+    const uint8_t* raw = raw_tile(slot) + r * 128;
+    uint8_t* tile = smem + s * L::STAGE_BYTES + r * 128;
+    uint4 plane[3];
+    f3_split(*reinterpret_cast<const float4*>(raw + raw0), *reinterpret_cast<const float4*>(raw + raw1),
+             plane);
+    *reinterpret_cast<uint4*>(tile + to0) = odd_row ? plane[1] : plane[0];
+    *reinterpret_cast<uint4*>(tile + to1) = odd_row ? plane[0] : plane[1];
+    *reinterpret_cast<uint4*>(tile + F3_BM * 128 + to2) = plane[2];
+    if (r < NT) {
+      f3_split(*reinterpret_cast<const float4*>(raw + F3_BM * 128 + raw0),
+               *reinterpret_cast<const float4*>(raw + F3_BM * 128 + raw1), plane);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        *reinterpret_cast<uint4*>(tile + L::A_OFFSET + q * NT * 128 + to2) = plane[q];
+      }
+    }
+    fence_proxy_async_shared();
+    // (before the accumulators begin anew; their last MMAs ran under this block's conversion)
+    const bool begins = kb % F3_SUM_BLOCKS == 0;
+    if (begins && kb > 0) add();
+    __syncthreads();  // the block is converted
+    if (tid == 0) {
+      tc_fence_after();
+      const uint32_t w12 = s * L::STAGE_BYTES, w3 = w12 + F3_BM * 128, a1 = w12 + L::A_OFFSET;
+#pragma unroll
+      for (int k = 0; k < F3_BK / 16; ++k) {
+        const uint32_t more = !begins || k != 0;
+        umma_f16(tmem_base, desc(w12 + k * 32), desc(a1 + k * 32), idesc1, more);
+        umma_f16(tmem_base + D2, desc(w12 + 64 + k * 32), desc(a1 + k * 32), idesc2, more);
+        umma_f16(tmem_base + D3, desc(w3 + k * 32), desc(a1 + k * 32), idesc3, more);
+      }
+      umma_commit(&empty[s]);
+      if (kb % F3_SUM_BLOCKS == F3_SUM_BLOCKS - 1 || kb + 1 == num_kb) umma_commit(acc_full);
+    }
+    if (tid == 32 && kb + L::RAW < num_kb && *failed == 0) {  // (every warp has read the raw tile)
+      bring_w(kb + L::RAW, slot);
+      bring_a(kb + L::RAW, slot);
+    }
+    __syncwarp();
+    if (++slot == L::RAW) {
+      slot = 0;
+      round ^= 1;
+    }
+  }
+  add();
   pdl_wait_for(a, out);
 
   // ---- this stretch's sums; what is odd once more
-  const bool sums = warp >= F3_CONVERT_WARPS;
-  if (sums) {
+  {
     bool odd = false;
 #pragma unroll
-    for (int j = 0; j < NH; ++j) odd |= f3_odd(acc[j]);
+    for (int j = 0; j < NQ; ++j) odd |= f3_odd(acc[j]);
     if (odd && n < N && *failed == 0) {
-      float again[NH];
+      float again[NQ];
 #pragma unroll
-      for (int j = 0; j < NH; ++j) again[j] = acc[j];
+      for (int j = 0; j < NQ; ++j) again[j] = acc[j];
 #pragma unroll 1
-      for (int j = 0; j < NH; ++j) {
-        const int m = m0 + half * NH + j;
+      for (int j = 0; j < NQ; ++j) {
+        const int m = m0 + part * NQ + j;
         if (m < M && f3_odd(again[j])) {
           again[j] = f3_plain(a + (size_t)m * lda, w + (size_t)n * ldw, k_first, k_last);
         }
       }
 #pragma unroll
-      for (int j = 0; j < NH; ++j) acc[j] = again[j];
+      for (int j = 0; j < NQ; ++j) acc[j] = again[j];
     }
     __syncwarp();
   }
@@ -327,10 +288,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   // free), and from there, added up over the stretches, a row of 128 columns a time. (One small loop: with
   // the activation unrolled over a lane's own sums the kernel waited for its code.)
   float* partial = reinterpret_cast<float*>(smem);  // [NT][128]
-  if (sums) {
 #pragma unroll
-    for (int j = 0; j < NH; ++j) partial[(half * NH + j) * F3_BM + quarter * 32 + lane] = acc[j];
-  }
+  for (int j = 0; j < NQ; ++j) partial[(part * NQ + j) * F3_BM + quarter * 32 + lane] = acc[j];
   if (splits > 1) {
     cluster_sync_all();
   } else {
@@ -372,7 +331,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
-  if (*failed != 0 && tid == 0) {
+  if (*failed != 0 && tid == 32) {
     // copies this thread started may still be landing: wait for each, bounded
     for (int kb = issued > L::RAW ? issued - L::RAW : 0; kb < issued; ++kb) {
       mbar_wait(&raw_full[kb % L::RAW], (kb / L::RAW) & 1);
@@ -380,7 +339,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     atomicExch(status, AYK_WAIT_TIMEOUT);
   }
   __syncthreads();
-  if (warp == F3_MMA_WARP) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 // Stretches of K, by N and K alone: about 20 CTAs a tile of rows (what seven tiles of rows can fill the
@@ -388,13 +347,12 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 inline int f3_splits(int N, int K) {
   const int tiles = (N + F3_BM - 1) / F3_BM, blocks = (K + F3_SUM_K - 1) / F3_SUM_K;
   int splits = 1;
-  while (splits < 8 && tiles * (splits + 1) <= 20 && blocks >= 4 * (splits + 1)) ++splits;
+  while (splits < 8 && tiles * (splits + 1) <= 20 && blocks >= 2 * (splits + 1)) ++splits;
   const int each = (blocks + splits - 1) / splits;
   return (blocks + each - 1) / each;  // (no stretch without a block)
 }
 
-// Rows of a tile: the width with the least (rounds over the SMs) x (time of a CTA). 64 k take the MMAs
-// 24 x max(47, NT / 2) clocks, a CTA about 5,000 more.
+// Rows of a tile: the width with the least (rounds over the SMs) x (time of a CTA).
 inline int f3_rows(int M, int ctas, int blocks) {
   const int sms = sm_count();
   long long best = -1;
@@ -402,7 +360,7 @@ inline int f3_rows(int M, int ctas, int blocks) {
   for (int tiles = (M + F3_MAX_NT - 1) / F3_MAX_NT, tried = 0; tried < 8; ++tiles, ++tried) {
     const int nt = ((M + tiles - 1) / tiles + 15) / 16 * 16;
     const long long rounds = ((long long)ctas * ((M + nt - 1) / nt) + sms - 1) / sms;
-    const long long cost = rounds * (5000 + (long long)blocks * 12 * (nt < 94 ? 94 : nt));
+    const long long cost = rounds * (5000 + (long long)blocks * (1000 + 10 * nt));
     if (best < 0 || cost < best) {
       best = cost;
       best_nt = nt;
@@ -435,7 +393,7 @@ int launch_gemm_f32(const float* a, int lda, const float* w, int ldw, const floa
 
 AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
 
-// `residual` != 0: out is added to. `tile_rows`: 0 chooses, else 16, 32, ... 128 rows of A a tile (for
+// `residual` != 0: out is added to. `tile_rows`: 0 chooses, else 16, 32, ... 80 rows of A a tile (for
 // tests). AYK_NOT_TAKEN, and nothing ran: operands whose rows do not start on 16 bytes, or more row tiles
 // than a grid counts; the FMA kernel of gemm_simt.cu takes any.
 AYK_API int ayk_gemm_f32(const float* a, int lda, const float* w, int ldw, const float* bias,
@@ -465,9 +423,6 @@ AYK_API int ayk_gemm_f32(const float* a, int lda, const float* w, int ldw, const
     AYK_F3(48);
     AYK_F3(64);
     AYK_F3(80);
-    AYK_F3(96);
-    AYK_F3(112);
-    AYK_F3(128);
   }
 #undef AYK_F3
   return AYK_BAD_ARGUMENT;
