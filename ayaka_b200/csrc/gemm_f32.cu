@@ -7,19 +7,33 @@
 // A product of two bfloat16 numbers is exact in fp32. The tensor core's own sums are kept short: 128 k are
 // summed in tensor memory, products of different size apart, and those sums are added in fp32 registers,
 // rounded to nearest. So the result is a true 32-bit product; against float64 its
-// 2-norm is off by 1.0e-7 (K 768 to 1,024) and 1.1e-7 (3,072), that of FMAs in gemm_simt.cu by 1.8e-7 to
-// 3.5e-7.
+// 2-norm is off by 7e-8 (K 64), 1.2e-7 (256), 1.3e-7 (768 to 3,072) and 1.4e-7 (6,400), that of FMAs in
+// gemm_simt.cu by 1.1e-7, 2.1e-7, 1.8e-7 to 3.5e-7 and 5.1e-7.
 //
 // The weights are the 128-row operand and a tile of NT rows of A the other one, so D[n, m] has a lane
-// per output column whatever M is. Blocks of 32 k travel by TMA into a ring of raw fp32 tiles; all sixteen
-// warps turn a block into bf16 tiles in the layout of TMA's 128-byte swizzle, two in turn: rows of W as
-// w1 | w2 and w3 | nothing, the parts of A's rows below one another, so that three MMAs per 16 k form the
-// six products, w1 [a1 a2 a3], w2 [a1 a2] and w3 a1, in accumulators of their own. One thread issues them;
-// an MMA is short (N up to 240) and what a single thread does for each, descriptors above all, is what
-// bounds a block, so both are kept few. Behind every fourth block the warps add the accumulators to their
-// registers, lane n of 32 and a quarter of the rows each. One block barrier a block. K may be cut into stretches by N and K alone (f3_splits); their CTAs are a cluster and add up their sums in order
-// through distributed shared memory. An element's sum has one order whatever M or the tile it falls in: a
-// row's bits do not depend on its batch.
+// per output column whatever M is. Blocks of 32 k travel by TMA into a ring of raw fp32 tiles (a warp of
+// its own); sixteen warps turn a block into bf16 tiles in the layout of TMA's 128-byte swizzle, two in
+// turn: rows of W as w1 | w2 and w3 | nothing, the parts of A's rows below one another, so that three MMAs
+// per 16 k form the six products, w1 [a1 a2 a3], w2 [a1 a2] and w3 a1, in accumulators of their own (an
+// MMA is short, N up to 240, and what one thread does for each would bound a block of six). A warp of its
+// own issues them beside the next block's conversion. Behind every fourth block the sixteen warps add the
+// accumulators to their registers, lane n of 32 and a quarter of the rows each.
+//
+// An element's sum has one order whatever M or the tile it falls in, so a row's bits do not depend on its
+// batch: N and K alone cut K into stretches of up to eight parts in all (F3Cut), the blocks of 128 k of a
+// part are added in order, the parts of a stretch, the stretches. With many rows a CTA has a stretch, with
+// few (f3_plan) a part; the CTAs of a tile are a cluster and add up their sums through distributed shared
+// memory.
+//
+// Bound by the conversion: some 190 instructions a thread and block, 1,700 clocks a block with 80 rows
+// a tile (the MMAs take a fifth of them) and 900 with 16; a launch and a cold pipeline are 14 microseconds
+// of a short product. Measured on a B200, cold caches, microseconds, FMAs -> this kernel, at 1, 64 and 513
+// rows:  2304 x 768 30 -> 24, 31 -> 25, 99 -> 42;  768 x 768 21 -> 18, 22 -> 20, 46 -> 27;  3072 x 768
+// 27 -> 22, 32 -> 26, 102 -> 57;  768 x 3072 27 -> 27, 30 -> 29, 118 -> 46;  50257 x 768 160 -> 71,
+// 164 -> 85, 1,103 -> 491;  1024 x 4096 29 -> 26, 37 -> 30, 175 -> 67;  1024 x 64 17 -> 14, 16 -> 14,
+// 17 -> 16. (With a stretch a CTA also for few rows, 64 x 1024 x 4096 took 57 and 8 x 768 x 3072 37; with
+// one warp converting and issuing MMAs, six an MMA step, 513 x 2304 x 768 took 61.) There is nothing left
+// for FMAs but operands that TMA cannot read.
 //
 // An entry that is no number, infinite, or rounds to infinity makes x2 and so every sum it enters no
 // number; entries below 2^-107 have parts that bfloat16 cannot hold, which may show in a sum that is
@@ -34,9 +48,14 @@ namespace ayk {
 
 constexpr int F3_BM = 128, F3_BK = 32, F3_STAGES = 2;
 constexpr int F3_SUM_K = 128;  // k of an accumulator
-constexpr int F3_THREADS = 512;
+constexpr int F3_WARPS = 16, F3_WORKERS = F3_WARPS * 32;  // that convert and add
+constexpr int F3_THREADS = F3_WORKERS + 64;  // and a warp for the MMAs, one for the copies
+constexpr int F3_PARTS = 8;  // at most, the CTAs of a portable cluster
+constexpr int F3_FULL = 112;  // CTAs that run at once in such clusters (fewer than SMs)
 constexpr int F3_SUM_BLOCKS = F3_SUM_K / F3_BK;
 constexpr int F3_MAX_NT = 80;  // six accumulators in tensor memory
+// clocks of a CTA, of a block of 32 k and of a row of it (fitted to the measurements above)
+constexpr int F3_FIXED = 20000, F3_BLOCK = 800, F3_ROW = 8;
 
 template <int NT>
 struct F3Smem {
@@ -50,8 +69,8 @@ struct F3Smem {
   static constexpr int FITS = (LIMIT - 1024 - 256 - RAW_OFFSET) / RAW_BYTES;
   static constexpr int RAW = FITS > 6 ? 6 : FITS;  // raw tiles in the ring
   static constexpr int BAR_OFFSET = RAW_OFFSET + RAW * RAW_BYTES;
-  // raw_full[RAW], empty[STAGES], acc_full, then the tmem slot and the failure flag
-  static constexpr int TOTAL = BAR_OFFSET + (RAW + F3_STAGES + 1) * 8 + 16;
+  // raw_full[RAW], raw_empty[RAW], full[STAGES], empty[STAGES], acc_full, the tmem slot, the failure flag
+  static constexpr int TOTAL = BAR_OFFSET + (2 * RAW + 2 * F3_STAGES + 1) * 8 + 16;
   static constexpr int DYNAMIC = TOTAL + 1024;
   static_assert(RAW >= 3, "two blocks on their way while one is converted");
   static_assert(NT * F3_BM * 4 <= RAW_OFFSET, "the stages hold the partial sums at the end");
@@ -97,19 +116,47 @@ __device__ __forceinline__ void f3_ld_32x4(uint32_t taddr, uint32_t* v) {
                : "memory");
 }
 
-// grid (weight tiles * splits, row tiles), clusters of `splits` along x.
+// An element's sum over the CTAs of a cluster that have a part each, `group` of them a stretch of `span`
+// k; `mine` is where this CTA has its own.
+__device__ __noinline__ float f3_sum_parts(const float* mine, int ctas, int group, const float* a,
+                                           const float* w, int K, int span) {
+  float x[F3_PARTS];
+#pragma unroll
+  for (int r = 0; r < F3_PARTS; ++r) x[r] = r < ctas ? ld_peer_f32(mine, r) : 0.f;
+  float sum = 0.f, stretch = 0.f;
+  int parts = 0, k = 0;
+#pragma unroll
+  for (int r = 0; r < F3_PARTS; ++r) {
+    if (r < ctas) {
+      stretch += x[r];
+      if (++parts == group || r == ctas - 1) {
+        if (f3_odd(stretch)) stretch = f3_plain(a, w, k, min(K, k + span));
+        sum = k == 0 ? stretch : sum + stretch;
+        stretch = 0.f;
+        parts = 0;
+        k += span;
+      }
+    }
+  }
+  return sum;
+}
+
+// grid (weight tiles * splits, row tiles), clusters of `splits` along x; a CTA has `k_split` k: a stretch
+// of parts of `part_k` (group 1), or a part, `group` of them a stretch.
 template <int NT>
 __global__ void __launch_bounds__(F3_THREADS, 1)
 gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                 const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw,
                 const float* __restrict__ bias, float* __restrict__ out, int ldo, int M, int N,
-                int K, int act, int residual, int splits, int k_split,
+                int K, int act, int residual, int splits, int k_split, int part_k, int group,
                 int* __restrict__ status) {
   using L = F3Smem<NT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
-  uint64_t* empty = raw_full + L::RAW;
+  uint64_t* raw_empty = raw_full + L::RAW;
+  uint64_t* full = raw_empty + L::RAW;
+  uint64_t* empty = full + F3_STAGES;
   uint64_t* acc_full = empty + F3_STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -126,8 +173,14 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const int num_kb = (k_last - k_first + F3_BK - 1) / F3_BK;  // blocks
 
   if (tid == 0) {
-    for (int s = 0; s < L::RAW; ++s) mbar_init(&raw_full[s], 1);
-    for (int s = 0; s < F3_STAGES; ++s) mbar_init(&empty[s], 1);
+    for (int s = 0; s < L::RAW; ++s) {
+      mbar_init(&raw_full[s], 1);
+      mbar_init(&raw_empty[s], F3_WARPS);
+    }
+    for (int s = 0; s < F3_STAGES; ++s) {
+      mbar_init(&full[s], F3_WARPS);
+      mbar_init(&empty[s], 1);
+    }
     mbar_init(acc_full, 1);
     *failed = 0;
     mbar_fence_init();
@@ -144,29 +197,18 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
 
-  int issued = 0;  // (thread 32) blocks whose copies it has started
-  auto raw_tile = [&](int slot) { return smem + L::RAW_OFFSET + slot * L::RAW_BYTES; };
-  auto bring_w = [&](int kb, int slot) {
-    mbar_expect_tx(&raw_full[slot], L::RAW_BYTES);
-    tma_load_2d(raw_tile(slot), &map_w, &raw_full[slot], k_first + kb * F3_BK, n0);
-  };
-  auto bring_a = [&](int kb, int slot) {
-    tma_load_2d(raw_tile(slot) + F3_BM * F3_BK * 4, &map_a, &raw_full[slot], k_first + kb * F3_BK, m0);
-    issued = kb + 1;
-  };
-  if (tid == 32) {
-    const int ahead = num_kb < L::RAW ? num_kb : L::RAW;
-    for (int kb = 0; kb < ahead; ++kb) bring_w(kb, kb);  // weights: ahead of the dependency wait
-    pdl_wait();
-    for (int kb = 0; kb < ahead; ++kb) bring_a(kb, kb);
-  }
-  __syncwarp();
-
-  const int quarter = warp & 3, part = warp >> 2;
+  const int quarter = warp & 3, part = (warp >> 2) & 3;
   const int n = n0 + quarter * 32 + lane;  // this lane's output column
-  float acc[NQ];
+  float acc[NQ], total[NQ];  // the part's, the stretch's sums
 #pragma unroll
-  for (int j = 0; j < NQ; ++j) acc[j] = 0.f;
+  for (int j = 0; j < NQ; ++j) acc[j] = total[j] = 0.f;
+  auto fold = [&]() {
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) {
+      total[j] += acc[j];
+      acc[j] = 0.f;
+    }
+  };
   uint32_t sums = 0;  // accumulators added so far
   auto add = [&]() {  // the accumulators to the sums: lane n, rows part * NQ ..
     if (*failed == 0 && !mbar_wait(acc_full, sums & 1)) *failed = 1;
@@ -193,85 +235,132 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
     tc_fence_before();
   };
-  // descriptors: the low words differ by where a tile starts (in 16 bytes), the high ones not
-  const uint64_t desc0 = umma_desc_k128(smem, 0);
-  auto desc = [&](uint32_t bytes) {
-    return (desc0 & 0xffffffff00000000ull) | ((uint32_t)desc0 + (bytes >> 4));
-  };
-  constexpr uint32_t idesc1 = umma_idesc_bf16(F3_BM, 3 * NT), idesc2 = umma_idesc_bf16(F3_BM, 2 * NT),
-                     idesc3 = umma_idesc_bf16(F3_BM, NT);
-  // a thread: 8 neighbouring k (piece p of 4) of row r of W and, for the first NT, of A
-  const int r = tid >> 2, p = tid & 3, x = r & 7;
-  const bool odd_row = x & 1;
-  const uint32_t raw0 = (uint32_t)(((2 * p) ^ x) << 4), raw1 = (uint32_t)(((2 * p + 1) ^ x) << 4);
-  // (of W, odd rows store x2 first: two rows side by side in different halves of the banks)
-  const uint32_t to0 = (uint32_t)((((odd_row ? 4 : 0) + p) ^ x) << 4);
-  const uint32_t to1 = (uint32_t)((((odd_row ? 0 : 4) + p) ^ x) << 4);
-  const uint32_t to2 = (uint32_t)((p ^ x) << 4);
-  int slot = 0;          // of the raw ring
-  uint32_t round = 0;    // parity of the ring's turn
-  for (int kb = 0; kb < num_kb; ++kb) {
-    const int s = kb & 1;
-    if (*failed == 0 && (!mbar_wait(&raw_full[slot], round) ||
-                         (kb >= F3_STAGES && !mbar_wait(&empty[s], ((kb >> 1) & 1) ^ 1)))) {
-      *failed = 1;
-    }
-    const uint8_t* raw = raw_tile(slot) + r * 128;
-    uint8_t* tile = smem + s * L::STAGE_BYTES + r * 128;
-    uint4 plane[3];
-    f3_split(*reinterpret_cast<const float4*>(raw + raw0), *reinterpret_cast<const float4*>(raw + raw1),
-             plane);
-    *reinterpret_cast<uint4*>(tile + to0) = odd_row ? plane[1] : plane[0];
-    *reinterpret_cast<uint4*>(tile + to1) = odd_row ? plane[0] : plane[1];
-    *reinterpret_cast<uint4*>(tile + F3_BM * 128 + to2) = plane[2];
-    if (r < NT) {
-      f3_split(*reinterpret_cast<const float4*>(raw + F3_BM * 128 + raw0),
-               *reinterpret_cast<const float4*>(raw + F3_BM * 128 + raw1), plane);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        *reinterpret_cast<uint4*>(tile + L::A_OFFSET + q * NT * 128 + to2) = plane[q];
+  if (warp == F3_WARPS + 1) {
+    if (lane == 0) {
+      auto raw_w = [&](int slot) { return smem + L::RAW_OFFSET + slot * L::RAW_BYTES; };
+      auto bring_w = [&](int kb, int slot) {
+        mbar_expect_tx(&raw_full[slot], L::RAW_BYTES);
+        tma_load_2d(raw_w(slot), &map_w, &raw_full[slot], k_first + kb * F3_BK, n0);
+      };
+      auto bring_a = [&](int kb, int slot) {
+        tma_load_2d(raw_w(slot) + F3_BM * F3_BK * 4, &map_a, &raw_full[slot], k_first + kb * F3_BK, m0);
+      };
+      const int ahead = num_kb < L::RAW ? num_kb : L::RAW;
+      for (int kb = 0; kb < ahead; ++kb) bring_w(kb, kb);  // weights: ahead of the dependency wait
+      pdl_wait();
+      for (int kb = 0; kb < ahead; ++kb) bring_a(kb, kb);
+      int issued = ahead, slot = 0;
+      uint32_t round = 0;
+      while (issued < num_kb && *failed == 0) {
+        if (!mbar_wait(&raw_empty[slot], round)) {
+          *failed = 1;
+          break;
+        }
+        bring_w(issued, slot);
+        bring_a(issued, slot);
+        ++issued;
+        if (++slot == L::RAW) {
+          slot = 0;
+          round ^= 1;
+        }
       }
-    }
-    fence_proxy_async_shared();
-    // (before the accumulators begin anew; their last MMAs ran under this block's conversion)
-    const bool begins = kb % F3_SUM_BLOCKS == 0;
-    if (begins && kb > 0) add();
-    __syncthreads();  // the block is converted
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t w12 = s * L::STAGE_BYTES, w3 = w12 + F3_BM * 128, a1 = w12 + L::A_OFFSET;
-#pragma unroll
-      for (int k = 0; k < F3_BK / 16; ++k) {
-        const uint32_t more = !begins || k != 0;
-        umma_f16(tmem_base, desc(w12 + k * 32), desc(a1 + k * 32), idesc1, more);
-        umma_f16(tmem_base + D2, desc(w12 + 64 + k * 32), desc(a1 + k * 32), idesc2, more);
-        umma_f16(tmem_base + D3, desc(w3 + k * 32), desc(a1 + k * 32), idesc3, more);
+      // every copy has landed before the CTA ends, whatever the others gave up on
+      for (int kb = issued > L::RAW ? issued - L::RAW : 0; kb < issued; ++kb) {
+        mbar_wait(&raw_full[kb % L::RAW], (kb / L::RAW) & 1);
       }
-      umma_commit(&empty[s]);
-      if (kb % F3_SUM_BLOCKS == F3_SUM_BLOCKS - 1 || kb + 1 == num_kb) umma_commit(acc_full);
-    }
-    if (tid == 32 && kb + L::RAW < num_kb && *failed == 0) {  // (every warp has read the raw tile)
-      bring_w(kb + L::RAW, slot);
-      bring_a(kb + L::RAW, slot);
     }
     __syncwarp();
-    if (++slot == L::RAW) {
-      slot = 0;
-      round ^= 1;
+  } else if (warp == F3_WARPS) {
+    if (lane == 0) {
+      // descriptors: the low words differ by where a tile starts (in 16 bytes), the high ones not
+      const uint64_t desc0 = umma_desc_k128(smem, 0);
+      auto desc = [&](uint32_t bytes) {
+        return (desc0 & 0xffffffff00000000ull) | ((uint32_t)desc0 + (bytes >> 4));
+      };
+      constexpr uint32_t idesc1 = umma_idesc_bf16(F3_BM, 3 * NT), idesc2 = umma_idesc_bf16(F3_BM, 2 * NT),
+                         idesc3 = umma_idesc_bf16(F3_BM, NT);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        const int s = kb & 1;
+        if (*failed == 0 && !mbar_wait(&full[s], (kb >> 1) & 1)) *failed = 1;
+        tc_fence_after();
+        const bool begins = kb % F3_SUM_BLOCKS == 0;
+        const uint32_t w12 = s * L::STAGE_BYTES, w3 = w12 + F3_BM * 128, a1 = w12 + L::A_OFFSET;
+#pragma unroll
+        for (int k = 0; k < F3_BK / 16; ++k) {
+          const uint32_t more = !begins || k != 0;
+          umma_f16(tmem_base, desc(w12 + k * 32), desc(a1 + k * 32), idesc1, more);
+          umma_f16(tmem_base + D2, desc(w12 + 64 + k * 32), desc(a1 + k * 32), idesc2, more);
+          umma_f16(tmem_base + D3, desc(w3 + k * 32), desc(a1 + k * 32), idesc3, more);
+        }
+        umma_commit(&empty[s]);
+        if (kb % F3_SUM_BLOCKS == F3_SUM_BLOCKS - 1 || kb + 1 == num_kb) umma_commit(acc_full);
+      }
     }
+    __syncwarp();
+  } else {
+    // a thread: 8 neighbouring k (piece p of 4) of row r of W and, for the first NT, of A
+    const int r = tid >> 2, p = tid & 3, x = r & 7;
+    const bool odd_row = x & 1;
+    const uint32_t raw0 = (uint32_t)(((2 * p) ^ x) << 4), raw1 = (uint32_t)(((2 * p + 1) ^ x) << 4);
+    // (of W, odd rows store x2 first: two rows side by side in different halves of the banks)
+    const uint32_t to0 = (uint32_t)((((odd_row ? 4 : 0) + p) ^ x) << 4);
+    const uint32_t to1 = (uint32_t)((((odd_row ? 0 : 4) + p) ^ x) << 4);
+    const uint32_t to2 = (uint32_t)((p ^ x) << 4);
+    const int part_blocks = part_k / F3_BK;
+    int slot = 0;          // of the raw ring
+    uint32_t round = 0;    // parity of the ring's turn
+    for (int kb = 0; kb < num_kb; ++kb) {
+      const int s = kb & 1;
+      if (*failed == 0 && (!mbar_wait(&raw_full[slot], round) ||
+                           (kb >= F3_STAGES && !mbar_wait(&empty[s], ((kb >> 1) & 1) ^ 1)))) {
+        *failed = 1;
+      }
+      const uint8_t* raw = smem + L::RAW_OFFSET + slot * L::RAW_BYTES + r * 128;
+      uint8_t* tile = smem + s * L::STAGE_BYTES + r * 128;
+      uint4 plane[3];
+      f3_split(*reinterpret_cast<const float4*>(raw + raw0), *reinterpret_cast<const float4*>(raw + raw1),
+               plane);
+      *reinterpret_cast<uint4*>(tile + to0) = odd_row ? plane[1] : plane[0];
+      *reinterpret_cast<uint4*>(tile + to1) = odd_row ? plane[0] : plane[1];
+      *reinterpret_cast<uint4*>(tile + F3_BM * 128 + to2) = plane[2];
+      if (r < NT) {
+        f3_split(*reinterpret_cast<const float4*>(raw + F3_BM * 128 + raw0),
+                 *reinterpret_cast<const float4*>(raw + F3_BM * 128 + raw1), plane);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          *reinterpret_cast<uint4*>(tile + L::A_OFFSET + q * NT * 128 + to2) = plane[q];
+        }
+      }
+      fence_proxy_async_shared();
+      // (before the accumulators begin anew; their last MMAs ran under this block's conversion)
+      if (kb % F3_SUM_BLOCKS == 0 && kb > 0) {
+        add();
+        if (kb % part_blocks == 0) fold();
+      }
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&full[s]);
+        mbar_arrive(&raw_empty[slot]);
+      }
+      if (++slot == L::RAW) {
+        slot = 0;
+        round ^= 1;
+      }
+    }
+    add();
+    fold();
   }
-  add();
   pdl_wait_for(a, out);
 
   // ---- this stretch's sums; what is odd once more
-  {
+  if (warp < F3_WARPS && group == 1) {
     bool odd = false;
 #pragma unroll
-    for (int j = 0; j < NQ; ++j) odd |= f3_odd(acc[j]);
+    for (int j = 0; j < NQ; ++j) odd |= f3_odd(total[j]);
     if (odd && n < N && *failed == 0) {
       float again[NQ];
 #pragma unroll
-      for (int j = 0; j < NQ; ++j) again[j] = acc[j];
+      for (int j = 0; j < NQ; ++j) again[j] = total[j];
 #pragma unroll 1
       for (int j = 0; j < NQ; ++j) {
         const int m = m0 + part * NQ + j;
@@ -280,7 +369,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
       }
 #pragma unroll
-      for (int j = 0; j < NQ; ++j) acc[j] = again[j];
+      for (int j = 0; j < NQ; ++j) total[j] = again[j];
     }
     __syncwarp();
   }
@@ -288,17 +377,19 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   // free), and from there, added up over the stretches, a row of 128 columns a time. (One small loop: with
   // the activation unrolled over a lane's own sums the kernel waited for its code.)
   float* partial = reinterpret_cast<float*>(smem);  // [NT][128]
+  if (warp < F3_WARPS) {
 #pragma unroll
-  for (int j = 0; j < NQ; ++j) partial[(part * NQ + j) * F3_BM + quarter * 32 + lane] = acc[j];
+    for (int j = 0; j < NQ; ++j) partial[(part * NQ + j) * F3_BM + quarter * 32 + lane] = total[j];
+  }
   if (splits > 1) {
     cluster_sync_all();
   } else {
     __syncthreads();
   }
   const int column = n0 + (tid & 127);
-  if (*failed == 0 && column < N) {
+  if (*failed == 0 && column < N && warp < F3_WARPS) {
     const float b = bias != nullptr ? __ldg(bias + column) : 0.f;
-    const int step = splits * (F3_THREADS / 128), rows = min(NT, M - m0);
+    const int step = splits * (F3_WORKERS / 128), rows = min(NT, M - m0);
 #pragma unroll 1
     for (int row = rank + splits * (tid >> 7); row < rows; row += 4 * step) {
       float v[4], old[4];
@@ -309,7 +400,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         old[i] = residual && row + i * step < rows
                      ? out[(size_t)(m0 + at) * ldo + column] : 0.f;
       }
-      if (splits > 1) {
+      if (group > 1) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int at = row + i * step;
+          if (at < rows) {
+            v[i] = f3_sum_parts(partial + at * F3_BM + (tid & 127), splits, group,
+                                a + (size_t)(m0 + at) * lda, w + (size_t)column * ldw, K, group * k_split);
+          }
+        }
+      } else if (splits > 1) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float* mine = partial + min(row + i * step, NT - 1) * F3_BM + (tid & 127);
@@ -331,48 +431,98 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 
   tc_fence_before();
   __syncthreads();
-  if (*failed != 0 && tid == 32) {
-    // copies this thread started may still be landing: wait for each, bounded
-    for (int kb = issued > L::RAW ? issued - L::RAW : 0; kb < issued; ++kb) {
-      mbar_wait(&raw_full[kb % L::RAW], (kb / L::RAW) & 1);
-    }
-    atomicExch(status, AYK_WAIT_TIMEOUT);
-  }
-  __syncthreads();
+  if (*failed != 0 && tid == 0) atomicExch(status, AYK_WAIT_TIMEOUT);
   if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// Stretches of K, by N and K alone: about 20 CTAs a tile of rows (what seven tiles of rows can fill the
-// device with) as long as a stretch has at least 256 k.
-inline int f3_splits(int N, int K) {
+// How K is cut, by N and K alone. Stretches: about 20 CTAs a tile of rows (what seven tiles of rows can
+// fill the device with) as long as a stretch has at least 256 k. Parts: as many as fit in a cluster and,
+// of one tile of rows, on the device at once.
+struct F3Cut {
+  int stretches, parts, group, part_k;  // group: parts of a stretch
+};
+inline F3Cut f3_cut(int N, int K) {
   const int tiles = (N + F3_BM - 1) / F3_BM, blocks = (K + F3_SUM_K - 1) / F3_SUM_K;
   int splits = 1;
-  while (splits < 8 && tiles * (splits + 1) <= 20 && blocks >= 2 * (splits + 1)) ++splits;
-  const int each = (blocks + splits - 1) / splits;
-  return (blocks + each - 1) / each;  // (no stretch without a block)
+  while (splits < F3_PARTS && tiles * (splits + 1) <= 20 && blocks >= 2 * (splits + 1)) ++splits;
+  F3Cut cut;
+  const int each = (blocks + splits - 1) / splits, room = F3_FULL / (tiles * splits);
+  cut.group = F3_PARTS / splits;
+  if (cut.group > room) cut.group = room > 1 ? room : 1;
+  if (cut.group > each) cut.group = each;
+  const int part = (each + cut.group - 1) / cut.group;
+  cut.part_k = part * F3_SUM_K;
+  cut.parts = (blocks + part - 1) / part;  // (none is empty)
+  if (cut.group > cut.parts) cut.group = cut.parts;
+  cut.stretches = (cut.parts + cut.group - 1) / cut.group;
+  return cut;
 }
 
-// Rows of a tile: the width with the least (rounds over the SMs) x (time of a CTA).
-inline int f3_rows(int M, int ctas, int blocks) {
-  const int sms = sm_count();
-  long long best = -1;
-  int best_nt = F3_MAX_NT;
-  for (int tiles = (M + F3_MAX_NT - 1) / F3_MAX_NT, tried = 0; tried < 8; ++tiles, ++tried) {
-    const int nt = ((M + tiles - 1) / tiles + 15) / 16 * 16;
-    const long long rounds = ((long long)ctas * ((M + nt - 1) / nt) + sms - 1) / sms;
-    const long long cost = rounds * (5000 + (long long)blocks * (1000 + 10 * nt));
-    if (best < 0 || cost < best) {
-      best = cost;
-      best_nt = nt;
+// CTAs that run at once in clusters of `ctas` (which lie within a part of the device; one CTA an SM).
+inline int f3_at_once(int ctas) {
+  struct Table {
+    int at_once[F3_PARTS + 1];
+    Table() {
+      using L = F3Smem<F3_MAX_NT>;
+      const bool allowed =
+          cudaFuncSetAttribute(gemm_f32_kernel<F3_MAX_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               L::DYNAMIC) == cudaSuccess;
+      for (int n = 1; n <= F3_PARTS; ++n) {
+        at_once[n] = sm_count() / n * n;
+        if (n == 1 || !allowed) continue;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(n);
+        config.blockDim = dim3(F3_THREADS);
+        config.dynamicSmemBytes = L::DYNAMIC;
+        cudaLaunchAttribute cluster[1];
+        cluster[0].id = cudaLaunchAttributeClusterDimension;
+        cluster[0].val.clusterDim.x = n;
+        cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+        config.attrs = cluster;
+        config.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_f32_kernel<F3_MAX_NT>, &config) ==
+                cudaSuccess && clusters > 0) {
+          at_once[n] = clusters * n;
+        }
+      }
     }
-    if (nt == 16) break;
+  };
+  static const Table table;
+  return table.at_once[ctas];
+}
+
+// Rows of a tile, and whether a CTA has a part or a stretch: the least (rounds over the SMs) x (time of a
+// CTA), in clocks.
+struct F3Plan {
+  int rows;
+  bool by_part;
+};
+inline F3Plan f3_plan(int M, int N, int K, const F3Cut& cut, int rows, int by_part) {
+  const int tiles_n = (N + F3_BM - 1) / F3_BM;
+  F3Plan plan = {F3_MAX_NT, false};
+  long long best = -1;
+  for (int nt = F3_MAX_NT; nt >= 16; nt -= 16) {
+    for (int fine = 0; fine < 2; ++fine) {
+      if ((rows != 0 && nt != rows) || (by_part >= 0 && fine != by_part)) continue;
+      if (fine && cut.group == 1) continue;
+      const int ctas = fine ? cut.parts : cut.stretches;
+      const int at_once = f3_at_once(ctas);
+      const long long rounds = ((long long)tiles_n * ctas * ((M + nt - 1) / nt) + at_once - 1) / at_once;
+      const long long blocks = min(K, fine ? cut.part_k : cut.part_k * cut.group) / F3_BK;
+      const long long cost = rounds * (F3_FIXED + blocks * (F3_BLOCK + F3_ROW * nt));
+      if (best < 0 || cost < best) {
+        best = cost;
+        plan = {nt, fine != 0};
+      }
+    }
   }
-  return best_nt;
+  return plan;
 }
 
 template <int NT>
 int launch_gemm_f32(const float* a, int lda, const float* w, int ldw, const float* bias, float* out,
-                    int ldo, int M, int N, int K, int act, int residual, int splits, int k_split,
+                    int ldo, int M, int N, int K, int act, int residual, const F3Cut& cut, bool by_part,
                     int* status, cudaStream_t stream) {
   using L = F3Smem<NT>;
   CUtensorMap map_w, map_a;
@@ -383,41 +533,44 @@ int launch_gemm_f32(const float* a, int lda, const float* w, int ldw, const floa
   static const cudaError_t allowed = cudaFuncSetAttribute(
       gemm_f32_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::DYNAMIC);
   if (allowed != cudaSuccess) return (int)allowed;
+  const int splits = by_part ? cut.parts : cut.stretches;
+  const int k_split = by_part ? cut.part_k : cut.part_k * cut.group;
   const dim3 grid((N + F3_BM - 1) / F3_BM * splits, (M + NT - 1) / NT);
   return launch_kernel_x(gemm_f32_kernel<NT>, grid, dim3(F3_THREADS), L::DYNAMIC, stream, splits,
                          map_w, map_a, a, lda, w, ldw, bias, out, ldo, M, N, K, act, residual, splits,
-                         k_split, status);
+                         k_split, cut.part_k, by_part ? cut.group : 1, status);
 }
 
 }  // namespace ayk
 
 AYK_API void ayk_set_pdl(int on) { ayk::pdl_enabled() = on; }
 
-// `residual` != 0: out is added to. `tile_rows`: 0 chooses, else 16, 32, ... 80 rows of A a tile (for
-// tests). AYK_NOT_TAKEN, and nothing ran: operands whose rows do not start on 16 bytes, or more row tiles
-// than a grid counts; the FMA kernel of gemm_simt.cu takes any.
+// `residual` != 0: out is added to. `tile_rows`: 0 chooses, else (for tests) 16, 32, ... 80 rows of A a
+// tile, and 1 more: a part of K a CTA. AYK_NOT_TAKEN, and nothing ran: operands whose rows do not start on
+// 16 bytes or lie in one another, no K, or more row tiles than a grid counts; the FMA kernel of
+// gemm_simt.cu takes any.
 AYK_API int ayk_gemm_f32(const float* a, int lda, const float* w, int ldw, const float* bias,
                          float* out, int ldo, int M, int N, int K, int act, int residual,
                          int tile_rows, int* status, void* stream) {
   using namespace ayk;
   if (M == 0 || N == 0) return AYK_OK;
-  if (M < 0 || N < 0 || K < 1 || lda < K || ldw < K || ldo < N || status == nullptr ||
-      act < ACT_NONE || act > ACT_RELU_SQUARED || (residual && act != ACT_NONE) || tile_rows < 0 ||
-      tile_rows > F3_MAX_NT || tile_rows % 16) {
+  if (M < 0 || N < 0 || K < 0 || status == nullptr || act < ACT_NONE || act > ACT_RELU_SQUARED ||
+      (residual && act != ACT_NONE) || tile_rows < 0 || tile_rows > F3_MAX_NT + 1 ||
+      tile_rows % 16 > 1 || tile_rows == 1) {
     return AYK_BAD_ARGUMENT;
   }
-  if (lda % 4 || ldw % 4 || (uintptr_t)a % 16 || (uintptr_t)w % 16) return AYK_NOT_TAKEN;
-  const int blocks = (K + F3_SUM_K - 1) / F3_SUM_K, splits = f3_splits(N, K);
-  const int each = (blocks + splits - 1) / splits;
-  const long long ctas = (long long)((N + F3_BM - 1) / F3_BM) * splits;
-  if (ctas > 0x7fffffffLL) return AYK_NOT_TAKEN;
-  const int nt = tile_rows ? tile_rows : f3_rows(M, (int)ctas, each);
-  if ((M + nt - 1) / nt > 65535) return AYK_NOT_TAKEN;
+  if (K == 0 || lda < K || ldw < K || lda % 4 || ldw % 4 || (uintptr_t)a % 16 || (uintptr_t)w % 16) {
+    return AYK_NOT_TAKEN;
+  }
+  const F3Cut cut = f3_cut(N, K);
+  if ((long long)((N + F3_BM - 1) / F3_BM) * cut.parts > 0x7fffffffLL) return AYK_NOT_TAKEN;
+  const F3Plan plan = f3_plan(M, N, K, cut, tile_rows / 16 * 16, tile_rows ? tile_rows % 16 : -1);
+  if ((M + plan.rows - 1) / plan.rows > 65535) return AYK_NOT_TAKEN;
 #define AYK_F3(NT)                                                                               \
   case NT:                                                                                       \
-    return launch_gemm_f32<NT>(a, lda, w, ldw, bias, out, ldo, M, N, K, act, residual, splits,   \
-                               each * F3_SUM_K, status, (cudaStream_t)stream)
-  switch (nt) {
+    return launch_gemm_f32<NT>(a, lda, w, ldw, bias, out, ldo, M, N, K, act, residual, cut,      \
+                               plan.by_part, status, (cudaStream_t)stream)
+  switch (plan.rows) {
     AYK_F3(16);
     AYK_F3(32);
     AYK_F3(48);

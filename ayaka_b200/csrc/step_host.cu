@@ -29,6 +29,8 @@ typedef int (*GemmTcKvFn)(const void*, int, const void*, int, const float*, void
                           int, const int*, void*, void*, int, int, int, int, int, int*, void*);
 typedef int (*GemmSimtFn)(const void*, int, const void*, int, const float*, void*, int, int, int,
                           int, int, int, int, int, void*);
+typedef int (*GemmF32Fn)(const void*, int, const void*, int, const float*, void*, int, int, int,
+                         int, int, int, int, int*, void*);
 typedef int (*KvStoreFn)(const void*, const void*, int, const int*, void*, void*, int, int, int,
                          int, int, void*);
 typedef int (*AttnDecodeFn)(const void*, int, const void*, const void*, const int*, int,
@@ -88,6 +90,7 @@ struct AykKernels {
   void* gemm_tc;
   void* gemm_tc_kv;
   void* gemm_simt;
+  void* gemm_f32;
   void* kv_store;
   void* attention_decode;
   void* attention_simt;
@@ -151,8 +154,8 @@ inline bool tma_readable(const void* a, int lda, const void* w, int ldw) {
   return ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0 && lda % 8 == 0 && ldw % 8 == 0;
 }
 
-// ops.linear: bfloat16 on the tensor cores when TMA can read the operands, else (and for
-// float32) the CUDA-core kernel. `residual`: out is fp32 and is added to.
+// ops.linear: on the tensor cores when TMA can read the operands (float32 in three bfloat16
+// parts), else the CUDA-core kernel. `residual`: out is fp32 and is added to.
 int linear(const AykKernels& k, AykStep* step, int type, const void* a, int lda, const void* w,
            int ldw, const float* bias, void* out, int ldo, int out_type, int M, int N, int K,
            int act, int residual) {
@@ -163,8 +166,13 @@ int linear(const AykKernels& k, AykStep* step, int type, const void* a, int lda,
     return ((GemmTcFn)k.gemm_tc)(a, lda, w, ldw, bias, out, ldo, M, N, K, act, mode,
                                  step->tile_n, step->status, step->stream);
   }
-  if (k.gemm_simt == nullptr) return AYK_DRIVER;
   ++step->launches;
+  if (type == 0 && k.gemm_f32 != nullptr) {
+    const int status = ((GemmF32Fn)k.gemm_f32)(a, lda, w, ldw, bias, out, ldo, M, N, K, act,
+                                               residual, 0, step->status, step->stream);
+    if (status != AYK_NOT_TAKEN) return status;
+  }
+  if (k.gemm_simt == nullptr) return AYK_DRIVER;
   return ((GemmSimtFn)k.gemm_simt)(a, lda, w, ldw, bias, out, ldo, M, N, K, act, residual, type,
                                    out_type, step->stream);
 }

@@ -43,7 +43,8 @@ class Step(Structure):
 
 class Kernels(Structure):
     _fields_ = [(name, c_void_p) for name in (
-        "layer_norm_f32", "layer_norm_bf16", "gemm_tc", "gemm_tc_kv", "gemm_simt", "kv_store",
+        "layer_norm_f32", "layer_norm_bf16", "gemm_tc", "gemm_tc_kv", "gemm_simt",
+        "gemm_f32", "kv_store",
         "attention_decode", "attention_simt", "attention_prefill", "attention_prefill_tc",
         "attention_prefill_tc_rows")]
 
@@ -103,7 +104,7 @@ def _address(library_name: str, symbol: str, **defines: int) -> int:
 
 def _kernels(dtype: torch.dtype, head_dim: int | None = None) -> Kernels:
     """The entry points a part of this dtype may reach. A float32 model never loads (or
-    compiles) the tensor-core libraries."""
+    compiles) the bfloat16 tensor-core libraries."""
     table = Kernels()
     table.gemm_simt = _address("gemm_simt", "ayk_gemm_simt")
     if dtype == torch.bfloat16:
@@ -112,6 +113,7 @@ def _kernels(dtype: torch.dtype, head_dim: int | None = None) -> Kernels:
         table.gemm_tc_kv = _address("gemm_tc", "ayk_gemm_bf16_tc_kv")
     else:
         table.layer_norm_f32 = _address("norm", "ayk_layer_norm_f32")
+        table.gemm_f32 = _address("gemm_f32", "ayk_gemm_f32")
     if head_dim is not None:
         table.kv_store = _address("attention_simt", "ayk_kv_store")
         table.attention_decode = _address("attention_decode", "ayk_attention_decode")

@@ -17,7 +17,8 @@ from ctypes import Structure, byref, c_float, c_int, c_longlong, c_void_p, sizeo
 import torch
 
 from ayaka_b200.errors import BackendError
-from ayaka_b200.kernels.lib import check, library, raw_stream
+from ayaka_b200.kernels import flags
+from ayaka_b200.kernels.lib import check, entry, library, raw_stream
 
 __all__ = [
     "ACTIVATIONS",
@@ -304,9 +305,10 @@ def linear(a: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, out
 
     ``a`` is ``[M, K]``, ``weight`` ``[N, K]`` (both float32, or both bfloat16), ``bias``
     float32 ``[N]``. ``out`` is ``[M, N]``: float32 always allowed (and required with
-    ``residual``), bfloat16 for bfloat16 inputs. ``rows`` limits M. float32 inputs run on
-    the CUDA cores with fp32 FMA (no reduced-precision matrix mode); bfloat16 inputs on the
-    tensor cores unless ``kernel="simt"``.
+    ``residual``), bfloat16 for bfloat16 inputs. ``rows`` limits M. Both run on the tensor cores
+    unless ``kernel="simt"`` or their rows are not TMA's: bfloat16 as it is, a float32 operand in
+    three bfloat16 parts that hold all its bits (the sums are at least as precise as the CUDA
+    cores' fp32 FMAs).
     """
     op = "linear"
     if _left_out and f"linear:{weight.shape[0]}x{weight.shape[1]}" in _left_out:
@@ -340,6 +342,16 @@ def linear(a: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, out
         if kernel == "tcgen05" or gemm_tc.usable(a, weight):
             gemm_tc.linear_bf16(a, weight, bias, out, m, ACTIVATIONS[activation], residual)
             return
+    if a.dtype == torch.float32 and kernel is None:
+        status = entry("gemm_f32", "ayk_gemm_f32")(
+            _ptr(a), c_int(a.stride(0)), _ptr(weight), c_int(weight.stride(0)), _ptr(bias),
+            _ptr(out), c_int(out.stride(0)), c_int(m), c_int(n), c_int(k),
+            c_int(ACTIVATIONS[activation]), c_int(1 if residual else 0), c_int(0),
+            c_void_p(flags.status_word(a.device).data_ptr()), _stream())
+        if status != -6:
+            check(status, op)
+            return
+        _nothing_ran()
     fn = library("gemm_simt").ayk_gemm_simt
     status = fn(_ptr(a), c_int(a.stride(0)), _ptr(weight), c_int(weight.stride(0)), _ptr(bias),
                 _ptr(out), c_int(out.stride(0)), c_int(m), c_int(n), c_int(k),

@@ -59,7 +59,7 @@ def test_a_rows_bits_do_not_depend_on_its_tile(m, n, k):
     a, w, bias, _ = _operands(m, n, k)
     whole = torch.empty(m, n, device="cuda")
     _product(a, w, bias, whole)
-    for tile in range(16, 81, 16):
+    for tile in [*range(16, 81, 16), *range(17, 82, 16)]:  # a stretch, a part of K a CTA
         out = torch.empty(m, n, device="cuda")
         _product(a, w, bias, out, tile=tile)
         assert torch.equal(out, whole), tile
@@ -98,3 +98,30 @@ def test_what_is_no_number_infinite_huge_or_tiny(m, n, k):
     assert (row[same] - exact[same]).norm() <= 2e-6 * exact[same].norm()
     assert (row[8:9] - exact[8:9]).norm() <= 2.0 ** -134 * float(w[8:9].double().abs().sum()) + \
         2e-6 * exact[8:9].norm()
+
+
+@pytest.mark.parametrize("form", ["whole", "strided", "odd stride", "odd start", "one row for all",
+                                  "rows over one another", "one narrow row", "weights strided"])
+def test_linear_takes_any_form(form):
+    """``ops.linear`` in every layout its rows may have, against the FMA kernel: those of TMA go
+    to the parts, the others stay where they were."""
+    from ayaka_b200.kernels import flags, ops
+
+    g = torch.Generator("cuda").manual_seed(5)
+    m, n, k = (1, 70, 96) if form == "one narrow row" else (21, 70, 96)
+    flat = torch.randn(m * (k + 8) + 8, generator=g, device="cuda")
+    a = {"strided": flat.as_strided((m, k), (k + 4, 1)), "odd stride": flat.as_strided((m, k), (k + 3, 1)),
+         "odd start": flat[1:].as_strided((m, k), (k, 1)), "one row for all": flat[:k].expand(m, k),
+         "rows over one another": flat.as_strided((m, k), (4, 1)),
+         "one narrow row": flat.as_strided((1, k), (4, 1))}.get(form, flat.as_strided((m, k), (k, 1)))
+    w = torch.randn(n, 2 * k, generator=g, device="cuda")
+    w = w[:, k:] if form == "weights strided" else w[:, :k].contiguous()
+    bias = torch.randn(n, generator=g, device="cuda")
+    out, want = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+    before = ops.launch_count()
+    ops.linear(a, w, bias, out)
+    assert ops.launch_count() == before + 1
+    ops.linear(a, w, bias, want, kernel="simt")
+    # (each within 5e-7 of the exact product)
+    assert (out - want).norm() <= 1e-6 * want.norm()
+    assert int(flags.status_word(a.device).item()) == 0
