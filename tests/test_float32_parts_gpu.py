@@ -105,6 +105,7 @@ def test_what_is_no_number_infinite_huge_or_tiny(m, n, k):
 def test_linear_takes_any_form(form):
     """``ops.linear`` in every layout its rows may have, against the FMA kernel: those of TMA go
     to the parts, the others stay where they were."""
+    from ayaka_b200.errors import BackendError
     from ayaka_b200.kernels import flags, ops
 
     g = torch.Generator("cuda").manual_seed(5)
