@@ -49,6 +49,23 @@ template <> struct Vec8<__nv_bfloat16> {
   }
 };
 
+// Eight entries on their way to shared memory, as fp32 (zeros where `in` is not set).
+__device__ __forceinline__ void bring8(float* dst, const float* src, bool in) {
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {  // (with a source size of 0 nothing is read)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + 16 * e), "l"(src + 4 * e),
+                 "r"(in ? 16 : 0)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void bring8(float* dst, const __nv_bfloat16* src, bool in) {
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (in) Vec8<__nv_bfloat16>::load(src, v);
+  reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+  reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
 // One row of one head, by one warp: q_s, p_s and off_s are the warp's shared memory.
 template <typename T>
 __device__ __forceinline__ void attend_row(const T* __restrict__ q, int ld_q,
@@ -157,15 +174,22 @@ attention_simt_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k
 // bytes a lane at a time, which bounds it). Per row the arithmetic and its order are those of
 // attend_row: the results are the same bits. Rows that are not a few stretches of neighbouring
 // positions (of several requests, or asked for in any other order) are taken one by one.
-// Measured on a B200, GPT-2 small's 12 heads of 64, prompts of 333 and 180: 111 -> 61 microseconds.
+// Bound by the latencies of a tile (keys on their way, the sums over the warp) and by shared memory, a
+// broadcast of four floats costing as much as four. Measured on a B200, 12 heads of 64, keys and values by
+// cp.async, the four rows' sums side by side and whole tiles without their tests, before -> after:
+// prompts of 333 and 180 84 -> 78 microseconds, 200 rows 59 -> 54, 1,024 rows 248 -> 204, 500 rows behind
+// 1,500 keys 447 -> 377, forty requests of 6 93 -> 83; 16 heads of 128, 2,000 and 1,500 rows 1,726 -> 1,396.
+// (16 rows a CTA: 78, 53, 174, 340, 109 and 1,489.)
 // ATT_TILE_PARTS CTAs a block: where its rows are taken one by one each has a warp for every row of its
 // part (one CTA for all 32 walked four rows a warp: 32 single rows and a portion of 200, 12 heads of 64,
 // 240 microseconds where this takes 84), else the first one works for all.
 constexpr int ATT_TILE_WARPS = 8, ATT_TILE_ROWS = 32;
 constexpr int ATT_TILE_PARTS = ATT_TILE_ROWS / ATT_TILE_WARPS;
 constexpr int ATT_TILE_STRETCHES = 4;  // of more stretches the 32 rows are taken one by one
+// (Three CTAs an SM up to heads of 64: with 128 registers it is two, the cases above take 69, 48, 183 and
+// 284, but forty requests of 6 rows 101 and 200 rows beside 32 single ones 112 where three take 83 and 100.)
 template <typename T, int NI>  // ceil(head_dim / 32)
-__global__ void __launch_bounds__(ATT_TILE_WARPS * 32)
+__global__ void __launch_bounds__(ATT_TILE_WARPS * 32, NI <= 2 ? 3 : 2)
 attention_simt_tile_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__ k_pages,
                            const T* __restrict__ v_pages, const int* __restrict__ block_table,
                            int table_stride, const int* __restrict__ request_of_row,
@@ -243,24 +267,14 @@ attention_simt_tile_kernel(const T* __restrict__ q, int ld_q, const T* __restric
       __syncthreads();  // the tile before has been used (and q is there)
       for (int idx = threadIdx.x; idx < 32 * pieces; idx += ATT_TILE_WARPS * 32) {
         const int j = idx / pieces, d = (idx - j * pieces) * 8, key = t0 + j;
-        float kv[8], vv[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) kv[e] = vv[e] = 0.f;
-        if (key >= lo_cta && key <= last_pos) {
-          const int page = table[key / page_size];
-          const size_t base = (((size_t)page * num_kv_heads + kv_head) * page_size +
-                               key % page_size) * head_dim + d;
-          Vec8<T>::load(k_pages + base, kv);
-          Vec8<T>::load(v_pages + base, vv);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; e += 4) {
-          *reinterpret_cast<float4*>(k_s + j * ld_s + d + e) =
-              make_float4(kv[e], kv[e + 1], kv[e + 2], kv[e + 3]);
-          *reinterpret_cast<float4*>(v_s + j * ld_s + d + e) =
-              make_float4(vv[e], vv[e + 1], vv[e + 2], vv[e + 3]);
-        }
+        const bool in = key >= lo_cta && key <= last_pos;
+        const int page = in ? table[key / page_size] : 0;
+        const size_t base = (((size_t)page * num_kv_heads + kv_head) * page_size +
+                             (in ? key % page_size : 0)) * head_dim + d;
+        bring8(k_s + j * ld_s + d, k_pages + base, in);
+        bring8(v_s + j * ld_s + d, v_pages + base, in);
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
       if (t0 > max(max(pos[0], pos[1]), max(pos[2], pos[3]))) continue;
       float dot[4] = {0.f, 0.f, 0.f, 0.f};
@@ -277,31 +291,57 @@ attention_simt_tile_kernel(const T* __restrict__ q, int ld_q, const T* __restric
         }
       }
       const int key = t0 + lane;
-      float p[4];
+      // (the four rows' reductions side by side: one behind the other they were a third of the time. A row
+      // that sees none of the tile keeps what it has, times 1 and plus 0.)
+      float p[4], top[4], corr[4];
       int j_lo[4], j_hi[4];  // the tile's keys that a row sees
       int from = 32, to = 0;
+      bool all_see = true;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         j_lo[r] = lo[r] > t0 ? lo[r] - t0 : 0;
         j_hi[r] = pos[r] - t0 + 1 < 32 ? pos[r] - t0 + 1 : 32;
-        p[r] = 0.f;
-        if (j_lo[r] >= j_hi[r]) continue;  // none of it (uniform over the warp)
-        from = min(from, j_lo[r]);
-        to = max(to, j_hi[r]);
-        const bool valid = key >= lo[r] && key <= pos[r];
-        const float s = valid ? dot[r] * scale : -INFINITY;
-        const float new_max = fmaxf(run_max[r], warp_max(s));
-        const float corr = expf(run_max[r] - new_max);  // exp(-inf) = 0 on the first tile
-        p[r] = valid ? expf(s - new_max) : 0.f;
-        run_sum[r] = run_sum[r] * corr + warp_sum(p[r]);
-        run_max[r] = new_max;
+        if (j_lo[r] < j_hi[r]) {
+          from = min(from, j_lo[r]);
+          to = max(to, j_hi[r]);
+        }
+        all_see = all_see && j_lo[r] == 0 && j_hi[r] == 32;
+        top[r] = key >= lo[r] && key <= pos[r] ? dot[r] * scale : -INFINITY;
+        p[r] = top[r];
+      }
 #pragma unroll
-        for (int i = 0; i < NI; ++i) acc[r][i] *= corr;
+      for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], o));
+        }
+      }
+      float sum[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const bool sees = j_lo[r] < j_hi[r];
+        const float new_max = fmaxf(run_max[r], top[r]);
+        const float shrink = expf(run_max[r] - new_max);  // exp(-inf) = 0 on the first tile
+        corr[r] = sees ? shrink : 1.f;
+        run_max[r] = sees ? new_max : run_max[r];
+        const float weight = expf(p[r] - new_max);
+        p[r] = key >= lo[r] && key <= pos[r] ? weight : 0.f;
+        sum[r] = p[r];
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        run_sum[r] = run_sum[r] * corr[r] + sum[r];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) acc[r][i] *= corr[r];
       }
       *reinterpret_cast<float4*>(p_s[warp][lane]) = make_float4(p[0], p[1], p[2], p[3]);
       __syncwarp();
-#pragma unroll 4
-      for (int j = from; j < to; ++j) {
+      auto weigh = [&](int j, bool whole) {
         const float4 w4 = *reinterpret_cast<const float4*>(p_s[warp][j]);
         const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
@@ -310,9 +350,16 @@ attention_simt_tile_kernel(const T* __restrict__ q, int ld_q, const T* __restric
           const float v = v_s[j * ld_s + lane + 32 * i];
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
-            if (j >= j_lo[r] && j < j_hi[r]) acc[r][i] = fmaf(w[r], v, acc[r][i]);
+            if (whole || (j >= j_lo[r] && j < j_hi[r])) acc[r][i] = fmaf(w[r], v, acc[r][i]);
           }
         }
+      };
+      if (all_see) {
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) weigh(j, true);
+      } else {
+#pragma unroll 4
+        for (int j = from; j < to; ++j) weigh(j, false);
       }
       __syncwarp();
     }
